@@ -143,6 +143,8 @@ struct RunArgs {
   int src_on;                // 1: src holds the accretion and spot constants
   int regen;                 // k_wave regeneration threshold: waiting lanes of a warp before they take new packets
   int qchunk;                // k_wave: peel-off queue slots a lane reserves at a time
+  int lanes;                 // k_wave: lanes of a warp that take packets (fewer than 32 in small batches)
+  int dump;                  // k_wave: busy lanes of a warp below which it leaves them to k_tail
   int imcube;                // 1: tally the per-frequency image cube
   int iter1;                 // 1: the first Lucy iteration (small grains emit from spectrum row 2)
   hc3d_sources src;
@@ -175,8 +177,16 @@ struct WaveBufs {
   void* pool;
   void* queue[2];
   unsigned long long* qcount[2];
-  unsigned int* alive;
+  unsigned int* alive[2];           // packets in flight after the wave that filled queue q,
+  unsigned int* live[2];            // and their pool slots, the input of k_tail
+  unsigned int* next_live;          // k_tail's counter over them
   unsigned long long* next_ray[2];  // ray counters of k_peel
+};
+
+// Buffers of an unpeeled run: the packets that k_wave leaves to k_tail.
+struct TailBufs {
+  void* pool;
+  unsigned int* count;  // [0] packets left, [1] k_tail's counter over them
 };
 
 // k_wave: advance every live packet by up to E events, appending peel-off
@@ -189,6 +199,24 @@ cudaError_t launch_wave_transport_fp64(const DevModel& m, const DevTallies& t, c
                                        const WaveBufs& w, int q, int E, const LaunchCfg& cfg);
 cudaError_t launch_wave_peel_fp64(const DevModel& m, const DevTallies& t, const TallyDims& d, const RunArgs& a,
                                   const WaveBufs& w, int q, const LaunchCfg& cfg);
+// k_tail: advance the packets in flight after the wave of queue 1 - q by up to
+// E events, a warp each, appending to queue q.
+cudaError_t launch_wave_tail_mixed(const DevModel& m, const DevTallies& t, const TallyDims& d, const RunArgs& a,
+                                   const WaveBufs& w, int q, int E, const LaunchCfg& cfg);
+cudaError_t launch_wave_tail_fp64(const DevModel& m, const DevTallies& t, const TallyDims& d, const RunArgs& a,
+                                  const WaveBufs& w, int q, int E, const LaunchCfg& cfg);
+// An unpeeled batch: k_wave without a queue, then k_tail for the packets it
+// leaves.  b.count is zero before it.
+cudaError_t launch_packets_mixed(const DevModel& m, const DevTallies& t, const TallyDims& d, const RunArgs& a,
+                                 const TailBufs& b, const LaunchCfg& cfg, int tail_blocks);
+cudaError_t launch_packets_fp64(const DevModel& m, const DevTallies& t, const TallyDims& d, const RunArgs& a,
+                                const TailBufs& b, const LaunchCfg& cfg, int tail_blocks);
+const void* packets_fn_mixed();
+const void* packets_fn_fp64();
+const void* tail_fn_mixed(bool peel);
+const void* tail_fn_fp64(bool peel);
+int tail_smem_mixed(const DevModel& m);  // dynamic shared memory of k_tail
+int tail_smem_fp64(const DevModel& m);
 size_t slot_bytes_mixed();
 size_t slot_bytes_fp64();
 size_t rec_bytes_mixed();

@@ -122,6 +122,96 @@ template <> __device__ __forceinline__ float ran<float>(Rng& r) {
   return ((float)(next_u32(r) >> 8) + 0.5f) * (1.0f / 16777216.0f);
 }
 
+// The functions of a draw that a packet's history needs, from one draw each:
+// the optical depth -ln u, and an isotropic direction (cos theta = 1 - 2u, sin
+// theta; cos phi and sin phi of phi = 2 pi u).
+template <class R> __device__ __forceinline__ R neg_log(Rng& r) { return -xlog(ran<R>(r)); }
+template <class R> __device__ __forceinline__ void draw_mu(Rng& r, R& mu, R& smu) {
+  mu = R(1) - R(2) * ran<R>(r);
+  smu = xsqrt(R(1) - mu * mu);
+}
+template <class R> __device__ __forceinline__ void draw_phi(Rng& r, R& phi, R& cphi, R& sphi) {
+  phi = (R)kR2p * ran<R>(r);
+  cphi = xcos(phi);
+  sphi = xsin(phi);
+}
+
+// Draws of a packet that a whole warp runs (k_tail): the next 128 draws of its
+// stream and the functions above of each, formed 32 lanes at a time in shared
+// memory, so that the packet's chain of events reads them instead of running
+// Philox, a logarithm, a sine and a cosine one after another.  Every lane
+// holds the same position; ensure() is called by the whole warp.
+template <class R>
+struct DrawTable {
+  static constexpr int kDraws = 128;
+  R u[kDraws], nl[kDraws], mu[kDraws], smu[kDraws], cphi[kDraws], sphi[kDraws];
+};
+template <class R>
+struct WarpRng {
+  DrawTable<R>* t;
+  uint32_t k0, k1, c2, c3;
+  uint32_t block;  // Philox block of the table's first four draws
+  int at;          // next draw of the table
+};
+
+template <class G> struct IsWarp { static constexpr bool value = false; };
+template <class R> struct IsWarp<WarpRng<R>> { static constexpr bool value = true; };
+
+template <class R> __device__ __forceinline__ void fill_draws(WarpRng<R>& r) {
+  r.block += (uint32_t)(r.at >> 2);
+  r.at &= 3;
+  const int lane = threadIdx.x & 31;
+  uint32_t b[4];
+  philox(r.block + (uint32_t)lane, 0u, r.c2, r.c3, r.k0, r.k1, b);
+  __syncwarp();  // the lanes have read what they need of the old table
+#pragma unroll 1
+  for (int j = 0; j < 4; ++j) {
+    R u;
+    const uint32_t w = pick4(b, j);
+    if constexpr (sizeof(R) == 4) u = ((float)(w >> 8) + 0.5f) * (1.0f / 16777216.0f);
+    else u = ((double)w + 0.5) * (1.0 / 4294967296.0);
+    const int k = 4 * lane + j;
+    r.t->u[k] = u;
+    r.t->nl[k] = -xlog(u);
+    const R mu = R(1) - R(2) * u;
+    r.t->mu[k] = mu;
+    r.t->smu[k] = xsqrt(R(1) - mu * mu);
+    const R phi = (R)kR2p * u;
+    r.t->cphi[k] = xcos(phi);
+    r.t->sphi[k] = xsin(phi);
+  }
+  __syncwarp();
+}
+template <class R> __device__ __forceinline__ void ensure(WarpRng<R>& r, int n) {
+  if (r.at + n > DrawTable<R>::kDraws) fill_draws(r);
+}
+// start or resume a stream: c0 blocks drawn so far, `left` draws of the last unused
+template <class R>
+__device__ __forceinline__ void rng_init(WarpRng<R>& r, DrawTable<R>* t, uint32_t key0, uint32_t key1, uint64_t pid,
+                                         uint32_t c0, int left) {
+  r.t = t;
+  r.k0 = key0; r.k1 = key1;
+  r.c2 = (uint32_t)pid; r.c3 = (uint32_t)(pid >> 32);
+  r.block = left > 0 ? c0 - 1u : c0;
+  r.at = left > 0 ? 4 - left : 0;
+  fill_draws(r);
+}
+template <class R> __device__ __forceinline__ void rng_save(const WarpRng<R>& r, uint32_t& c0, int& left) {
+  c0 = r.block + (uint32_t)((r.at + 3) >> 2);
+  left = (4 - (r.at & 3)) & 3;
+}
+template <class R> __device__ __forceinline__ R ran(WarpRng<R>& r) { return r.t->u[r.at++]; }
+template <class R> __device__ __forceinline__ R neg_log(WarpRng<R>& r) { return r.t->nl[r.at++]; }
+template <class R> __device__ __forceinline__ void draw_mu(WarpRng<R>& r, R& mu, R& smu) {
+  mu = r.t->mu[r.at];
+  smu = r.t->smu[r.at++];
+}
+template <class R> __device__ __forceinline__ void draw_phi(WarpRng<R>& r, R& phi, R& cphi, R& sphi) {
+  phi = (R)kR2p * r.t->u[r.at];
+  cphi = r.t->cphi[r.at];
+  sphi = r.t->sphi[r.at++];
+}
+
 // ---- packet state: the tts_mod/stokesvar_mod globals of one packet ------------
 // Positions: FP64 in the FP64 form.  The mixed form carries each coordinate
 // as an unevaluated FP32 pair hi + lo (about 44 significant bits), advanced
@@ -163,16 +253,30 @@ struct Pkt {
   LucyRow lrow;  // mixed form: cached Lucy CDF rows of the current cell
 };
 
-// Event counters (HC3D_CNT_*) of a thread and its last fault code.  The
-// counters live in the block's shared memory, so they take no registers on
-// the packet's chain of events; local_init() clears them, flush() adds them
-// to the device counters once per block.  The peel-off walks count in
-// registers instead (PeelCount): their crossings would make every lane hit
-// the same shared counter.
+// Event counters (HC3D_CNT_*) of a thread and its last fault code.  The rare
+// ones live in the block's shared memory, so they take no registers on the
+// packet's chain of events; local_init() clears them, flush() adds them to the
+// device counters once per block.  The counts of every crossing and every
+// interaction are kept in registers (cross, events, pcross) and settled into
+// the shared counters when a packet ends: a 64-bit shared add is a
+// compare-and-swap loop, which the lanes of a warp that cross a wall together
+// run one after another.  32 bits hold one packet's counts: at most
+// max_interactions walks of at most 4 (nrg + ntg + npg) crossings, or one
+// event's peel-off rays.
 struct Local {
   unsigned long long* sc;  // the block's 16 counters
   int fault;
-  __device__ __forceinline__ void add(int k, unsigned long long v = 1ull) const { atomicAdd(sc + k, v); }
+  unsigned cross, events, pcross;
+  bool on;  // this lane tallies: false for the lanes of k_tail that repeat lane 0's packet
+  __device__ __forceinline__ void add(int k, unsigned long long v = 1ull) const {
+    if (on) atomicAdd(sc + k, v);
+  }
+  __device__ __forceinline__ void settle() {
+    if (cross) add(HC3D_CNT_CROSS_PROP, cross);
+    if (events) add(HC3D_CNT_EVENTS, events);
+    if (pcross) add(HC3D_CNT_CROSS_PEEL, pcross);
+    cross = events = pcross = 0u;
+  }
 };
 
 __device__ __forceinline__ void local_init(Local& L, unsigned long long* sc) {
@@ -180,6 +284,8 @@ __device__ __forceinline__ void local_init(Local& L, unsigned long long* sc) {
   __syncthreads();
   L.sc = sc;
   L.fault = 0;
+  L.cross = L.events = L.pcross = 0u;
+  L.on = true;
 }
 
 struct PeelCount {
@@ -338,12 +444,16 @@ struct Ray {
   bool dbl;
 };
 
+// The mixed-form walk names every rounding (fmaf, or the _rn intrinsics, which
+// the compiler does not contract) wherever a product meets a sum, so that the
+// kernels that walk packets -- several of them, and free to be rearranged --
+// form the same bits.  A packet's history depends on every bit of them.
 __device__ __forceinline__ void ray_init(Ray& r, const Pos2& x, const Pos2& y, const Pos2& z, float ux, float uy,
                                          float uz) {
   r.x0 = x.hi; r.y0 = y.hi; r.z0 = z.hi;
   r.ux = ux; r.uy = uy; r.uz = uz;
-  r.urho2 = ux * ux + uy * uy;
-  r.uz2 = uz * uz;
+  r.urho2 = fmaf(ux, ux, __fmul_rn(uy, uy));
+  r.uz2 = __fmul_rn(uz, uz);
   r.xs = x; r.ys = y; r.zs = z;
   r.dbl = false;
 }
@@ -352,9 +462,9 @@ __device__ __forceinline__ void ray_f64(Ray& r) {
   if (r.dbl) return;
   const double uxd = r.ux, uyd = r.uy, uzd = r.uz;
   const double x = dval(r.xs), y = dval(r.ys), z = dval(r.zs);
-  r.rr0 = x * x + y * y + z * z;
-  r.hb0 = x * uxd + y * uyd + z * uzd;
-  r.u2 = uxd * uxd + uyd * uyd + uzd * uzd;
+  r.rr0 = fma(z, z, fma(x, x, __dmul_rn(y, y)));
+  r.hb0 = fma(z, uzd, fma(x, uxd, __dmul_rn(y, uyd)));
+  r.u2 = fma(uzd, uzd, fma(uxd, uxd, __dmul_rn(uyd, uyd)));
   r.dbl = true;
 }
 
@@ -368,13 +478,13 @@ __device__ __forceinline__ void ray_at(const Ray& r, const PathLen& S, double& x
 
 // x + S u as a pair: x a pair, S a pair, u FP32 (error-free product and sum)
 __device__ __forceinline__ Pos2 pos_step(const Pos2& x, const PathLen& S, float u) {
-  const float pr = S.hi * u;
-  const float pe = fmaf(S.hi, u, -pr) + S.lo * u;
-  const float sm = x.hi + pr;
-  const float bp = sm - x.hi;
-  const float e = ((x.hi - (sm - bp)) + (pr - bp)) + (x.lo + pe);
-  const float hi = sm + e;
-  return Pos2{hi, e - (hi - sm)};
+  const float pr = __fmul_rn(S.hi, u);
+  const float pe = fmaf(S.lo, u, fmaf(S.hi, u, -pr));
+  const float sm = __fadd_rn(x.hi, pr);
+  const float bp = __fsub_rn(sm, x.hi);
+  const float e = __fadd_rn(__fadd_rn(__fsub_rn(x.hi, __fsub_rn(sm, bp)), __fsub_rn(pr, bp)), __fadd_rn(x.lo, pe));
+  const float hi = __fadd_rn(sm, e);
+  return Pos2{hi, __fsub_rn(e, __fsub_rn(hi, sm))};
 }
 
 // the point of the ray at path length S, as pairs
@@ -402,10 +512,11 @@ __device__ __forceinline__ float fsqrt_pos(float x) { return x * rsqrtf(x); }
 // only their far root, and the next wall is the smallest non-negative root
 // of the rest, a minimum over at most six candidates.  FP32, except the
 // near-sphere and grazing sphere roots (FP64).
-// kCache: keep the FP64 terms of the start point in the Ray once formed (the
-// transport walk, where one event's steps repeat the refinement); the
-// peel-off walk forms them afresh each time and keeps its registers.
-template <bool kCache>
+// kFused: how |x|^2 and x.u take their z term: by an FMA (the peeled runs) or
+// by a separate product and sum (the unpeeled ones).  The two round
+// differently in the last bit; each kind of run keeps the one that its
+// results have always had.
+template <bool kFused>
 __device__ __forceinline__ bool next_wall_ray(const DevModel& m, Ray& r, const PathLen& S, int ir, int it, int ip,
                                               int own, float& dt, int& iface) {
   float best = 3.402823466e38f;
@@ -421,48 +532,38 @@ __device__ __forceinline__ bool next_wall_ray(const DevModel& m, Ray& r, const P
   const float yr = fmaf(S.hi, uy, fmaf(S.lo, uy, r.y0));
   const float zr = fmaf(S.hi, uz, fmaf(S.lo, uz, r.z0));
   // terms shared by the spheres and the cones
-  const float pxy = xr * ux + yr * uy, pz = zr * uz;
-  const float rho2 = xr * xr + yr * yr, z2 = zr * zr;
+  const float pxy = fmaf(xr, ux, __fmul_rn(yr, uy)), pz = __fmul_rn(zr, uz);
+  const float rho2 = fmaf(xr, xr, __fmul_rn(yr, yr)), z2 = __fmul_rn(zr, zr);
   // spheres: t^2 + 2 hb t + c = 0 with hb = x.u, c = |x|^2 - R^2, disc = hb^2 - c
   const bool in_own = (own & 2) != 0, out_own = (own & 4) != 0;
-  float hb = pxy + pz;
-  const float rr = rho2 + z2;
+  float hb = kFused ? fmaf(zr, uz, pxy) : __fadd_rn(pxy, pz);
+  const float rr = kFused ? fmaf(zr, zr, rho2) : __fadd_rn(rho2, z2);
   const float2 r2io = __ldg(m.r2pair + ir - 1);
   const float r2i = r2io.x, r2o = r2io.y;
-  float ci = rr - r2i, co = rr - r2o;
-  float di = hb * hb - ci, dq = hb * hb - co;
+  float ci = __fsub_rn(rr, r2i), co = __fsub_rn(rr, r2o);
+  float di = fmaf(hb, hb, -ci), dq = fmaf(hb, hb, -co);
   const bool fix = (!in_own && hb < 0.f && (fabsf(ci) < kNearSphere * r2i || fabsf(di) < kGrazeSphere * r2i)) ||
                    (!out_own && (fabsf(co) < kNearSphere * r2o || fabsf(dq) < kGrazeSphere * r2o));
   if (fix) {
-    double rr0, hb0, u2;
-    if constexpr (kCache) {
-      ray_f64(r);
-      rr0 = r.rr0; hb0 = r.hb0; u2 = r.u2;
-    } else {
-      const double uxd = ux, uyd = uy, uzd = uz;
-      const double x = dval(r.xs), y = dval(r.ys), z = dval(r.zs);
-      rr0 = x * x + y * y + z * z;
-      hb0 = x * uxd + y * uyd + z * uzd;
-      u2 = uxd * uxd + uyd * uyd + uzd * uzd;
-    }
+    ray_f64(r);
     const double s = path_f64(S);
-    const double hbd = fma(s, u2, hb0);
-    const double rrd = fma(s, fma(s, u2, hb0 + hb0), rr0);
+    const double hbd = fma(s, r.u2, r.hb0);
+    const double rrd = fma(s, fma(s, r.u2, r.hb0 + r.hb0), r.rr0);
     const double cid = rrd - __ldg(m.r2arr + ir - 1), cod = rrd - __ldg(m.r2arr + ir);
     hb = (float)hbd;
     ci = (float)cid; co = (float)cod;
-    di = (float)(hbd * hbd - cid); dq = (float)(hbd * hbd - cod);
+    di = (float)fma(hbd, hbd, -cid); dq = (float)fma(hbd, hbd, -cod);
   }
   if (in_own) {
     if (hb < 0.f) cand(-2.f * hb, 1);
   } else if (hb < 0.f && di > 0.f) {  // inner sphere: reached only moving inwards
-    cand(__fdividef(fmaxf(ci, 0.f), fsqrt_pos(di) - hb), 1);
+    cand(__fdividef(fmaxf(ci, 0.f), fmaf(di, rsqrtf(di), -hb)), 1);
   }
   if (out_own) {
     if (hb < 0.f) cand(-2.f * hb, 2);
   } else if (dq > 0.f) {  // outer sphere: the exit root
-    const float sq = fsqrt_pos(dq);
-    cand(hb > 0.f ? __fdividef(fmaxf(-co, 0.f), hb + sq) : sq - hb, 2);
+    const float sq = __fmul_rn(dq, rsqrtf(dq));
+    cand(hb > 0.f ? __fdividef(fmaxf(-co, 0.f), __fadd_rn(hb, sq)) : __fsub_rn(sq, hb), 2);
   }
   if (m.ntg > 2) {
     // cones x^2 + y^2 = tan2 z^2: a t^2 + b t + cq = 0
@@ -482,7 +583,7 @@ __device__ __forceinline__ bool next_wall_ray(const DevModel& m, Ray& r, const P
       if (mine) {
         if (a != 0.f) {
           const float t = __fdividef(-b, a);
-          if ((zr + t * uz) * hemi > 0.f) cand(t, id);
+          if (fmaf(t, uz, zr) * hemi > 0.f) cand(t, id);
         }
         continue;
       }
@@ -490,29 +591,29 @@ __device__ __forceinline__ bool next_wall_ray(const DevModel& m, Ray& r, const P
       if (a == 0.f) {
         if (b != 0.f) {
           const float t = __fdividef(-cq, b);
-          if ((zr + t * uz) * hemi > 0.f) cand(t, id);
+          if (fmaf(t, uz, zr) * hemi > 0.f) cand(t, id);
         }
         continue;
       }
-      const float disc = b * b - 4.f * a * cq;
+      const float disc = fmaf(b, b, -__fmul_rn(4.f * a, cq));
       if (disc > 0.f) {
-        const float sq = fsqrt_pos(disc), inv = __fdividef(0.5f, a);
-        const float t1 = (-b + sq) * inv, t2 = (-b - sq) * inv;
-        if ((zr + t1 * uz) * hemi > 0.f) cand(t1, id);
-        if ((zr + t2 * uz) * hemi > 0.f) cand(t2, id);
+        const float rs = rsqrtf(disc), inv = __fdividef(0.5f, a);
+        const float t1 = __fmul_rn(fmaf(disc, rs, -b), inv), t2 = __fmul_rn(fmaf(-disc, rs, -b), inv);
+        if (fmaf(t1, uz, zr) * hemi > 0.f) cand(t1, id);
+        if (fmaf(t2, uz, zr) * hemi > 0.f) cand(t2, id);
       }
     }
     if (m.npg > 2) {
       // The azimuth of a straight line changes monotonically (by less than
       // pi), so only the plane on the side it turns towards can be met:
       // phi(ip) (id 6) when (x cross u)_z > 0, phi(ip-1) (id 5) otherwise.
-      const int k = xr * uy - yr * ux > 0.f ? 1 : 0;
+      const int k = fmaf(xr, uy, -__fmul_rn(yr, ux)) > 0.f ? 1 : 0;
       const int id = 5 + k;
       if (!((own >> id) & 1)) {
         const float2 ab = __ldg(m.planef + ip - 1 + k);
         const float A = ab.x, B = ab.y;
-        const float d = A * ux + B * uy;
-        if (d != 0.f) cand(__fdividef(-(A * xr + B * yr), d), id);
+        const float d = fmaf(A, ux, __fmul_rn(B, uy));
+        if (d != 0.f) cand(__fdividef(-fmaf(A, xr, __fmul_rn(B, yr)), d), id);
       }
     }
   }
@@ -746,21 +847,70 @@ __device__ __forceinline__ unsigned long long fxf(float v, float scale) {
   return (unsigned long long)f2ll(v * scale);
 }
 
-// The small grains' absorption path of a step ds in cell c (models with
-// small-grain slots): ds kappa(nu)/kappa_V (1 - albedo(nu)) of slot sg_slot,
-// over the cell's outer radius like jmean.  int_mean turns it into the mean
-// intensity in units of the ISRF absorbed by the same grains (the tally of
-// the reference's tauint is restated; its source is absent).
+// The Lucy tallies of a step ds in cell c: the absorbed path of every species
+// with density, kappa (1 - albedo) rho ds; the path over the cell's outer
+// radius (jmean); and in models with small-grain slots their absorption path,
+// ds kappa(nu)/kappa_V (1 - albedo(nu)) of slot sg_slot over the outer radius,
+// which int_mean turns into the mean intensity in units of the ISRF absorbed
+// by the same grains (the tally of the reference's tauint is restated; its
+// source is absent).
 template <class R>
-__device__ __forceinline__ void tally_jsg(const DevModel& m, const DevTallies& t, const Pkt<R>& p, int64_t c, R ds,
-                                          R rout) {
-  if (!m.sg_on) return;
+__device__ __forceinline__ void tally_path(const DevModel& m, const DevTallies& t, const Pkt<R>& p, const Rho<R>& rho,
+                                           int64_t c, R ds, R rout) {
   if constexpr (sizeof(R) == 4) {
-    const float w = pick4(p.kapd, m.sg_slot) * (1.f - pick4(p.albedo, m.sg_slot)) * m.sg_jfac;
-    atomicAdd(t.jsg + c, fxf(ds * w / rout, (float)t.path_scale));
+    const float ps = (float)t.path_scale;
+#pragma unroll
+    for (int s = 0; s < kSlots; ++s)
+      if (rho.v[s] > 0.f)
+        atomicAdd(t.dtauabs + (int64_t)s * m.ncell + c, fxf(p.kapd[s] * (1.f - p.albedo[s]) * rho.v[s] * ds, ps));
+    atomicAdd(t.jmean + c, fxf(ds / rout, ps));
+    if (m.sg_on) {
+      const float w = pick4(p.kapd, m.sg_slot) * (1.f - pick4(p.albedo, m.sg_slot)) * m.sg_jfac;
+      atomicAdd(t.jsg + c, fxf(ds * w / rout, ps));
+    }
   } else {
-    const double w = pick4(p.kapd, m.sg_slot) * (1.0 - pick4(p.albedo, m.sg_slot)) * m.sg_jfacd;
-    atomicAdd(t.jsg + c, fx((double)ds * w / (double)rout, t.path_scale));
+#pragma unroll
+    for (int s = 0; s < kSlots; ++s)
+      if (rho.v[s] > R(0)) {
+        const R v = p.kapd[s] * (R(1) - p.albedo[s]) * rho.v[s] * ds;
+        atomicAdd(t.dtauabs + (int64_t)s * m.ncell + c, fx((double)v, t.path_scale));
+      }
+    atomicAdd(t.jmean + c, fx((double)ds / (double)rout, t.path_scale));
+    if (m.sg_on) {
+      const double w = pick4(p.kapd, m.sg_slot) * (1.0 - pick4(p.albedo, m.sg_slot)) * m.sg_jfacd;
+      atomicAdd(t.jsg + c, fx((double)ds * w / (double)rout, t.path_scale));
+    }
+  }
+}
+
+// The same by the lanes of a warp that runs one packet: lane s < 4 tallies
+// species s, lane 4 the path, lane 5 the small grains' path -- one fixed-point
+// conversion and one atomic instruction instead of up to six.
+template <class R>
+__device__ __forceinline__ void tally_path_warp(const DevModel& m, const DevTallies& t, const Pkt<R>& p,
+                                                const Rho<R>& rho, int64_t c, R ds, R rout) {
+  const int lane = threadIdx.x & 31;
+  unsigned long long* q = nullptr;
+  R v = R(0);
+  if (lane < kSlots) {
+    const R r = pick4(rho.v, lane);
+    if (r > R(0)) {
+      q = t.dtauabs + (int64_t)lane * m.ncell + c;
+      v = pick4(p.kapd, lane) * (R(1) - pick4(p.albedo, lane)) * r * ds;
+    }
+  } else if (lane == 4) {
+    q = t.jmean + c;
+    v = ds / rout;
+  } else if (lane == 5 && m.sg_on) {
+    q = t.jsg + c;
+    if constexpr (sizeof(R) == 4)
+      v = ds * (pick4(p.kapd, m.sg_slot) * (1.f - pick4(p.albedo, m.sg_slot)) * m.sg_jfac) / rout;
+    else
+      v = ds * (pick4(p.kapd, m.sg_slot) * (1.0 - pick4(p.albedo, m.sg_slot)) * m.sg_jfacd) / rout;
+  }
+  if (q) {
+    if constexpr (sizeof(R) == 4) atomicAdd(q, fxf(v, (float)t.path_scale));
+    else atomicAdd(q, fx(v, t.path_scale));
   }
 }
 
@@ -770,28 +920,30 @@ __device__ __forceinline__ void tally_jsg(const DevModel& m, const DevTallies& t
 // midplane gives |z|, a pole is no wall) and the planes |A x + B y|, less a
 // margin for FP32 rounding of the point and of the walls.
 __device__ __forceinline__ float safe_dist(const DevModel& m, float x, float y, float z, int ir, int it, int ip) {
-  const float rc2 = x * x + y * y;
-  const float r = sqrtf(rc2 + z * z), rc = sqrtf(rc2);
+  const float rc2 = fmaf(x, x, __fmul_rn(y, y));
+  const float r = sqrtf(fmaf(z, z, rc2)), rc = sqrtf(rc2);
   float d = fminf(r - __ldg(m.rarrf + ir - 1), __ldg(m.rarrf + ir) - r);
   if (m.ntg > 2) {
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
       if (__ldg(m.tan2f + it - 1 + k) == 0.f) continue;
       const float2 cs = __ldg(m.thcs + it - 1 + k);
-      d = fminf(d, fabsf(rc * cs.x - z * cs.y));
+      d = fminf(d, fabsf(fmaf(rc, cs.x, -__fmul_rn(z, cs.y))));
     }
     if (m.npg > 2) {
 #pragma unroll
       for (int k = 0; k < 2; ++k)
-        d = fminf(d, fabsf(__ldg(m.aarrf + ip - 1 + k) * x + __ldg(m.barrf + ip - 1 + k) * y));
+        d = fminf(d, fabsf(fmaf(__ldg(m.aarrf + ip - 1 + k), x, __fmul_rn(__ldg(m.barrf + ip - 1 + k), y))));
     }
   }
-  return d - 1.0e-6f * r;
+  return fmaf(-1.0e-6f, r, d);
 }
 
 // Mixed form of tauint: the step of one event is a Ray from the event point;
 // the walk, the tau integral and the Lucy tallies are FP32, the FP64 point
-// where the walk stops is formed once, at the end.
+// where the walk stops is formed once, at the end.  kWarp: a whole warp runs
+// the packet (k_tail), every lane holding the same state.
+template <bool kFused, bool kWarp>
 static __device__ __forceinline__ int tauint_mixed(const DevModel& m, const DevTallies& t, Pkt<float>& p, float tau, Local& L,
                                    Tracer& tr) {
   float tsum = 0.f;
@@ -800,7 +952,16 @@ static __device__ __forceinline__ int tauint_mixed(const DevModel& m, const DevT
   Ray ray;
   ray_init(ray, p.x, p.y, p.z, p.ux, p.uy, p.uz);
   PathLen S{0.f, 0.f};
-  const float ps = (float)t.path_scale;
+  auto tally = [&](const Rho<float>& rho, int64_t c, float ds, float rout) {
+    if constexpr (kWarp) tally_path_warp<float>(m, t, p, rho, c, ds, rout);
+    else tally_path<float>(m, t, p, rho, c, ds, rout);
+  };
+  auto opacity = [&](const Rho<float>& rho) {
+    float opac = __fmul_rn(p.kapd[0], rho.v[0]);
+#pragma unroll
+    for (int s = 1; s < kSlots; ++s) opac = fmaf(p.kapd[s], rho.v[s], opac);
+    return opac;
+  };
   if (p.on_wall == 0 && p.ir >= 1 && p.ir <= m.nrg - 1 && p.it >= 1 && p.it <= m.ntg - 1) {
     // From a point inside the cell, a step shorter than the safe distance
     // ends in the cell: the interaction the walk would find, without the
@@ -808,20 +969,13 @@ static __device__ __forceinline__ int tauint_mixed(const DevModel& m, const DevT
     // where it was formed; each such step uses up its length.
     const int64_t c = cidx(m, p.ir, p.it, p.ip);
     const Rho<float> rho = load_rho<float>(m, c);
-    float opac = 0.f;
-#pragma unroll
-    for (int s = 0; s < kSlots; ++s) opac += p.kapd[s] * rho.v[s];
+    const float opac = opacity(rho);
     const float ds = tau / opac;
     if (opac > 0.f && !(ds < p.safe)) p.safe = safe_dist(m, p.x.hi, p.y.hi, p.z.hi, p.ir, p.it, p.ip);
     if (opac > 0.f && ds < p.safe) {
-      p.safe -= ds;
-      L.add(HC3D_CNT_CROSS_PROP);
-#pragma unroll
-      for (int s = 0; s < kSlots; ++s)
-        if (rho.v[s] > 0.f)
-          atomicAdd(t.dtauabs + (int64_t)s * m.ncell + c, fxf(p.kapd[s] * (1.f - p.albedo[s]) * rho.v[s] * ds, ps));
-      atomicAdd(t.jmean + c, fxf(ds / __ldg(m.rarrf + p.ir), ps));
-      tally_jsg<float>(m, t, p, c, ds, __ldg(m.rarrf + p.ir));
+      p.safe = __fsub_rn(p.safe, ds);
+      L.cross++;
+      tally(rho, c, ds, __ldg(m.rarrf + p.ir));
       path_add(S, ds);
       ray_pos(ray, S, p.x, p.y, p.z);
       tr.add(2, p.ir, p.it, p.ip, 0, (double)tau, dval(p.x), dval(p.y), dval(p.z));
@@ -849,7 +1003,7 @@ static __device__ __forceinline__ int tauint_mixed(const DevModel& m, const DevT
     const Rho<float> rho = load_rho<float>(m, c);
     float dt;
     int iface;
-    if (!next_wall_ray<true>(m, ray, S, p.ir, p.it, p.ip, p.on_wall, dt, iface)) {
+    if (!next_wall_ray<kFused>(m, ray, S, p.ir, p.it, p.ip, p.on_wall, dt, iface)) {
       at();
       if (nreloc < 4) {
         ++nreloc;
@@ -862,20 +1016,13 @@ static __device__ __forceinline__ int tauint_mixed(const DevModel& m, const DevT
       L.fault = F_NOWALL;
       return TI_FAULT;
     }
-    float opac = 0.f;
-#pragma unroll
-    for (int s = 0; s < kSlots; ++s) opac += p.kapd[s] * rho.v[s];
-    const float dtau = opac * dt;
+    const float opac = opacity(rho);
+    const float tnext = fmaf(opac, dt, tsum);  // the optical depth at the wall
     const float rout = __ldg(m.rarrf + p.ir);
-    L.add(HC3D_CNT_CROSS_PROP);
-    const bool stop = tsum + dtau > tau;
+    L.cross++;
+    const bool stop = tnext > tau;
     const float ds = stop ? (tau - tsum) / opac : dt;
-#pragma unroll
-    for (int s = 0; s < kSlots; ++s)
-      if (rho.v[s] > 0.f)
-        atomicAdd(t.dtauabs + (int64_t)s * m.ncell + c, fxf(p.kapd[s] * (1.f - p.albedo[s]) * rho.v[s] * ds, ps));
-    atomicAdd(t.jmean + c, fxf(ds / rout, ps));
-    tally_jsg<float>(m, t, p, c, ds, rout);
+    tally(rho, c, ds, rout);
     if (stop) {
       path_add(S, ds);
       at();
@@ -883,7 +1030,7 @@ static __device__ __forceinline__ int tauint_mixed(const DevModel& m, const DevT
       tr.add(2, p.ir, p.it, p.ip, 0, (double)tau, dval(p.x), dval(p.y), dval(p.z));
       return TI_INTERACT;
     }
-    tsum += dtau;
+    tsum = tnext;
     step_index(m.npg, iface, p.ir, p.it, p.ip);
     path_add(S, dt);
     p.on_wall = 1 << own_after(iface);
@@ -909,14 +1056,18 @@ static __device__ __forceinline__ int tauint_mixed(const DevModel& m, const DevT
 
 // tauint in either form: the FP64 form walks with the reference's wall
 // machinery (closest_wall rule), the mixed form with tauint_mixed.
-template <class R>
+template <class R, bool kFused, bool kWarp>
 __device__ __forceinline__ int tauint(const DevModel& m, const DevTallies& t, Pkt<R>& p, R tau, Local& L, Tracer& tr) {
   if constexpr (sizeof(R) == 4) {
-    return tauint_mixed(m, t, p, tau, L, tr);
+    return tauint_mixed<kFused, kWarp>(m, t, p, tau, L, tr);
   } else {
     R tsum = R(0);
     const int cap = 4 * (m.nrg + m.ntg + m.npg) + 64;
     const double uxd = (double)p.ux, uyd = (double)p.uy, uzd = (double)p.uz;
+    auto tally = [&](const Rho<R>& rho, int64_t c, R ds, R rout) {
+      if constexpr (kWarp) tally_path_warp<R>(m, t, p, rho, c, ds, rout);
+      else tally_path<R>(m, t, p, rho, c, ds, rout);
+    };
     for (int n = 0;; ++n) {
       if (n > cap || p.it < 1 || p.it > m.ntg - 1 || p.ir < 1 || p.ir > m.nrg - 1) {
         L.fault = n > cap ? F_CAP : F_RANGE;
@@ -935,32 +1086,18 @@ __device__ __forceinline__ int tauint(const DevModel& m, const DevTallies& t, Pk
       for (int s = 0; s < kSlots; ++s) opac += p.kapd[s] * rho.v[s];
       const R dtau = opac * dt;
       const double rout = __ldg(m.rarr + p.ir);
-      L.add(HC3D_CNT_CROSS_PROP);
+      L.cross++;
       if (tsum + dtau > tau) {
         const R ds = (tau - tsum) / opac;
         p.x += (double)ds * uxd;
         p.y += (double)ds * uyd;
         p.z += (double)ds * uzd;
         p.on_wall = 0;
-#pragma unroll
-        for (int s = 0; s < kSlots; ++s)
-          if (rho.v[s] > R(0)) {
-            const R v = p.kapd[s] * (R(1) - p.albedo[s]) * rho.v[s] * ds;
-            atomicAdd(t.dtauabs + (int64_t)s * m.ncell + c, fx((double)v, t.path_scale));
-          }
-        atomicAdd(t.jmean + c, fx((double)ds / rout, t.path_scale));
-        tally_jsg<R>(m, t, p, c, ds, (R)rout);
+        tally(rho, c, ds, (R)rout);
         tr.add(2, p.ir, p.it, p.ip, 0, (double)tau, p.x, p.y, p.z);
         return TI_INTERACT;
       }
-#pragma unroll
-      for (int s = 0; s < kSlots; ++s)
-        if (rho.v[s] > R(0)) {
-          const R v = p.kapd[s] * (R(1) - p.albedo[s]) * rho.v[s] * dt;
-          atomicAdd(t.dtauabs + (int64_t)s * m.ncell + c, fx((double)v, t.path_scale));
-        }
-      atomicAdd(t.jmean + c, fx((double)dt / rout, t.path_scale));
-      tally_jsg<R>(m, t, p, c, dt, (R)rout);
+      tally(rho, c, dt, (R)rout);
       tsum += dtau;
       step_index(m.npg, iface, p.ir, p.it, p.ip);
       p.x += (double)dt * uxd;
@@ -975,8 +1112,8 @@ __device__ __forceinline__ int tauint(const DevModel& m, const DevTallies& t, Pk
 }
 
 // ---- select_dust.f90:16-42 ---------------------------------------------------
-template <class R>
-__device__ __forceinline__ int select_dust(const DevModel& m, const Pkt<R>& p, Rng& rng) {
+template <class R, class G>
+__device__ __forceinline__ int select_dust(const DevModel& m, const Pkt<R>& p, G& rng) {
   const R xran = ran<R>(rng);
   const Rho<R> rho = load_rho<R>(m, cidx(m, p.ir, p.it, p.ip));
   R opac = R(0), frac = R(0);
@@ -1046,31 +1183,95 @@ __device__ __forceinline__ void mueller(bool upper, R p1, R p2, R p3, R s2x, R c
 }
 
 // ---- stokes.f90:46-388 --------------------------------------------------------------
+// One try of the rejection loop: a scattering angle and azimuth from two
+// draws, their phase-matrix elements and the probability of the direction for
+// the packet's polarisation.
 template <class R>
-__device__ __forceinline__ void stokes(Pkt<R>& p, int id, Rng& rng) {
+struct ScatTry {
+  R bmu, sinbt, p1, p2, p3, ci, si, rprob;
+  bool upper;
+};
+template <class R>
+__device__ __forceinline__ void scat_try(const Pkt<R>& p, R g, R pl, R u0, R u1, ScatTry<R>& q) {
+  q.bmu = R(1) - R(2) * u0;
+  R cosb2 = q.bmu * q.bmu;
+  dustmat<R>(g, pl, q.bmu, cosb2, q.p1, q.p2, q.p3);
+  if (xabs(q.bmu) > R(1)) { q.bmu = q.bmu > R(1) ? R(1) : R(-1); cosb2 = R(1); }
+  q.sinbt = xsqrt(R(1) - cosb2);
+  const R ri1 = (R)kR2p * u1;
+  q.upper = ri1 > (R)kPi;
+  const R ang = q.upper ? (R)kR2p - ri1 : ri1;
+  q.ci = xcos(ang);
+  q.si = xsin(ang);
+  const R s2 = R(2) * q.si * q.ci, c2 = R(2) * q.ci * q.ci - R(1);
+  const R a12 = q.p2 * c2, a13 = q.upper ? q.p2 * s2 : -q.p2 * s2;
+  q.rprob = (q.p1 * p.sip + a12 * p.sqp + a13 * p.sup) / p.sip;
+}
+
+// the rejection loop, its tries one after another
+template <class R>
+__device__ __forceinline__ void scat_draw(const Pkt<R>& p, R g, R pl, Rng& rng, ScatTry<R>& q) {
+  R peak = peak_of<R>(g);
+  for (;;) {
+    const R u0 = ran<R>(rng), u1 = ran<R>(rng);
+    scat_try<R>(p, g, pl, u0, u1, q);
+    if (q.rprob > peak) peak = q.rprob;
+    const R xran = ran<R>(rng);
+    if (!(peak * xran > q.rprob)) break;
+  }
+}
+
+// The rejection loop of a packet that a whole warp runs: ten tries at once,
+// one per lane, on the draws each would have had (a try takes three); the
+// first accepted one is the loop's.  A probability above the peak raises the
+// peak for the tries after it (stokes.f90 updates it in the loop): a running
+// maximum over the lanes.
+template <class R>
+__device__ __forceinline__ void scat_draw(const Pkt<R>& p, R g, R pl, WarpRng<R>& rng, ScatTry<R>& q) {
+  constexpr int kTries = 10;
+  const int lane = threadIdx.x & 31;
+  R peak = peak_of<R>(g);
+  for (;;) {
+    ensure(rng, 3 * kTries);
+    const int k = rng.at + 3 * min(lane, kTries - 1);
+    scat_try<R>(p, g, pl, rng.t->u[k], rng.t->u[k + 1], q);
+    R top = peak;
+    if (__any_sync(0xffffffffu, q.rprob > peak)) {
+      top = fmax(q.rprob, peak);
+#pragma unroll
+      for (int o = 1; o < 16; o <<= 1) {
+        const R v = __shfl_up_sync(0xffffffffu, top, o);
+        if (lane >= o) top = fmax(top, v);
+      }
+    }
+    const unsigned ok = __ballot_sync(0xffffffffu, lane < kTries && !(top * rng.t->u[k + 2] > q.rprob));
+    const int win = ok ? __ffs(ok) - 1 : kTries - 1;
+    rng.at += 3 * (win + 1);
+    if (ok) {
+      q.bmu = __shfl_sync(0xffffffffu, q.bmu, win);
+      q.sinbt = __shfl_sync(0xffffffffu, q.sinbt, win);
+      q.p1 = __shfl_sync(0xffffffffu, q.p1, win);
+      q.p2 = __shfl_sync(0xffffffffu, q.p2, win);
+      q.p3 = __shfl_sync(0xffffffffu, q.p3, win);
+      q.ci = __shfl_sync(0xffffffffu, q.ci, win);
+      q.si = __shfl_sync(0xffffffffu, q.si, win);
+      q.rprob = __shfl_sync(0xffffffffu, q.rprob, win);
+      q.upper = __shfl_sync(0xffffffffu, (int)q.upper, win) != 0;
+      return;
+    }
+    peak = __shfl_sync(0xffffffffu, top, kTries - 1);
+  }
+}
+
+template <class R, class G>
+__device__ __forceinline__ void stokes(Pkt<R>& p, int id, G& rng) {
   const R costp = p.cost, sintp = p.sint, phip = p.phi;
   const R g = pick4(p.g, id), pl = pick4(p.pl, id);
-  R peak = peak_of<R>(g);
-  R bmu, cosb2, sinbt, p1, p2, p3, rprob, ci, si_;
-  bool upper;
-  for (;;) {
-    bmu = R(1) - R(2) * ran<R>(rng);
-    cosb2 = bmu * bmu;
-    dustmat<R>(g, pl, bmu, cosb2, p1, p2, p3);
-    if (xabs(bmu) > R(1)) { bmu = bmu > R(1) ? R(1) : R(-1); cosb2 = R(1); }
-    sinbt = xsqrt(R(1) - cosb2);
-    const R ri1 = (R)kR2p * ran<R>(rng);
-    upper = ri1 > (R)kPi;
-    const R ang = upper ? (R)kR2p - ri1 : ri1;
-    ci = xcos(ang);
-    si_ = xsin(ang);
-    const R s2 = R(2) * si_ * ci, c2 = R(2) * ci * ci - R(1);
-    const R a12 = p2 * c2, a13 = upper ? p2 * s2 : -p2 * s2;
-    rprob = (p1 * p.sip + a12 * p.sqp + a13 * p.sup) / p.sip;
-    if (rprob > peak) peak = rprob;
-    const R xran = ran<R>(rng);
-    if (!(peak * xran > rprob)) break;
-  }
+  ScatTry<R> q;
+  scat_draw<R>(p, g, pl, rng, q);
+  const R bmu = q.bmu, sinbt = q.sinbt, p1 = q.p1, p2 = q.p2, p3 = q.p3, rprob = q.rprob;
+  R ci = q.ci, si_ = q.si;
+  const bool upper = q.upper;
   const R a = rprob;
   if (bmu == R(1)) return;
   const R s2x = R(2) * si_ * ci, c2x = R(2) * ci * ci - R(1);
@@ -1273,7 +1474,7 @@ __device__ void peel_ray(const DevModel& m, const DevTallies& t, const TallyDims
     for (int s = 0; s < kSlots; ++s)
       if (mask & (1u << s)) opac += e.kapd[s] * rho.v[s];
     tsum += (double)(opac * dt);
-    L.add(HC3D_CNT_CROSS_PEEL);
+    L.pcross++;
     if (tsum > kTauMax) return;
     step_index(m.npg, iface, ir, it, ip);
     xp1 += (double)dt * uxd;
@@ -1729,6 +1930,7 @@ __device__ __forceinline__ void peel_all(const DevModel& m, const DevTallies& t,
     if constexpr (sizeof(R) == 4) peel_ray_mixed(m, t, d, a, rec, k, L);
     else peel_ray<R>(m, t, d, a, rec, k, L);
   }
+  L.settle();
 }
 
 // ---- lucydustfreq.f90:19-157 -------------------------------------------------------------
@@ -1738,7 +1940,8 @@ __device__ __forceinline__ void peel_all(const DevModel& m, const DevTallies& t,
 // index is the same bracket of the interpolated CDF as the reference's
 // bisection (the CDF is non-decreasing, so the bracket is unique), found
 // from the guide table and a short bisection over the interleaved rows.
-__device__ __forceinline__ float lucy_freq_mixed(const DevModel& m, LucyRow& lr, int64_t c, int id, Rng& rng) {
+template <class G>
+__device__ __forceinline__ float lucy_freq_mixed(const DevModel& m, LucyRow& lr, int64_t c, int id, G& rng) {
   const int nT = m.nT, nnu = m.nnu;
   const float* nuint = m.nuintf;
   const int key = (int)(4 * c + id);
@@ -1772,6 +1975,23 @@ __device__ __forceinline__ float lucy_freq_mixed(const DevModel& m, LucyRow& lr,
   auto P = [&](int i) { return fminf((1.f - f) * __ldg(KP + i - 1).x + f * __ldg(KP + i - 1).y, 1.f); };
   const short2 g = __ldg(m.kguide + (size_t)lr.pr * kGuide + min((int)(xi * (float)kGuide), kGuide - 1));
   int i0 = g.x, i1 = g.y;
+  bool found = false;
+  if constexpr (IsWarp<G>::value) {
+    // the guide's bracket in one step: lane j has P(i0 + j); the CDF does not
+    // decrease, so the last value <= xi and the first > xi are neighbours
+    const int j = threadIdx.x & 31;
+    const float v = P(min(i0 + j, i1));
+    const unsigned above = __ballot_sync(0xffffffffu, v > xi);
+    if (above != 0u && (above & 1u) == 0u) {
+      const int w1 = __ffs(above) - 1;
+      i1 = min(i0 + w1, i1);
+      i0 += w1 - 1;
+      P0 = __shfl_sync(0xffffffffu, v, w1 - 1);
+      P1 = __shfl_sync(0xffffffffu, v, w1);
+      found = true;
+    }
+  }
+  if (!found) {
   const float Pa = P(i0), Pb = P(i1);
   if (Pa <= xi) P0 = Pa; else i0 = 1;
   if (Pb > xi) P1 = Pb; else i1 = nnu;
@@ -1781,6 +2001,7 @@ __device__ __forceinline__ float lucy_freq_mixed(const DevModel& m, LucyRow& lr,
     const float v = P(i);
     if (v > xi) { i1 = i; P1 = v; }
     else { i0 = i; P0 = v; }
+  }
   }
   float w;
   if (xi < P0) w = 0.f;
@@ -1799,8 +2020,8 @@ template <> __device__ __forceinline__ double xpow<double>(double a, double b) {
 __device__ __forceinline__ float xlog10(float x) { return log10f(x); }
 __device__ __forceinline__ double xlog10(double x) { return log10(x); }
 
-template <class R>
-__device__ __forceinline__ R lucydustfreq(const DevModel& m, R T0, int id, Rng& rng) {
+template <class R, class G>
+__device__ __forceinline__ R lucydustfreq(const DevModel& m, R T0, int id, G& rng) {
   const int nT = m.nT, nnu = m.nnu;
   const R* lTint = tab<R>(m.lTint, m.lTintf);
   const R* nuint = tab<R>(m.nuint, m.nuintf);
@@ -1905,8 +2126,8 @@ __device__ __forceinline__ double draine_logfreq(const DevModel& m, int j, doubl
   return (lx - l0) / (l1 - l0) * (f1 - f0) + f0;
 }
 
-template <class R>
-__device__ __forceinline__ double rep_draine(const DevModel& m, int im, double jmf, Rng& rng) {
+template <class R, class G>
+__device__ __forceinline__ double rep_draine(const DevModel& m, int im, double jmf, G& rng) {
   const double xran = (double)ran<R>(rng);
   const double lx = log10(xran);
   const double lf1 = draine_logfreq(m, im, xran, lx);
@@ -2030,7 +2251,8 @@ __device__ __forceinline__ void set_status(const RunArgs& a, int code) {
 }
 
 // Record a faulted packet (global id and fault code) in the fault log.
-__device__ __forceinline__ void log_fault(const DevTallies& t, const Rng& rng, int code) {
+template <class G>
+__device__ __forceinline__ void log_fault(const DevTallies& t, const G& rng, int code) {
   if (!t.fault_log) return;
   const unsigned long long k = atomicAdd(t.fault_count, 1ull);
   if (k < (unsigned long long)kFaultLog)
@@ -2357,19 +2579,20 @@ __device__ __forceinline__ bool emit(const DevModel& m, const DustView<R>& dv, c
 
 
 // tau sample + tauint + outcome, propagate.f90:46-62 (first) and 169-202.
-template <class R>
-__device__ __forceinline__ int walk(const DevModel& m, const DevTallies& t, const TallyDims& d, const RunArgs& a, Pkt<R>& p, Rng& rng,
+// G: the packet's draws, one lane's (Rng) or a warp's (WarpRng, k_tail).
+template <class R, bool kFused, class G>
+__device__ __forceinline__ int walk(const DevModel& m, const DevTallies& t, const TallyDims& d, const RunArgs& a, Pkt<R>& p, G& rng,
                     Flow<R>& f, Local& L, Tracer& tr, bool first) {
-  const R tau = -xlog(ran<R>(rng));
+  const R tau = neg_log<R>(rng);
   if (!first) {
     f.xpold = p.x; f.ypold = p.y; f.zpold = p.z;
     p.ux = p.sint * p.cosp; p.uy = p.sint * p.sinp; p.uz = p.cost;
   }
   const int pir = p.ir, pit = p.it, pip = p.ip;
-  const int st = tauint<R>(m, t, p, tau, L, tr);
+  const int st = tauint<R, kFused, IsWarp<G>::value>(m, t, p, tau, L, tr);
   if (st == TI_ESCAPE) {
     tr.add(3, p.ir, p.it, p.ip, 0, 0.0, dval(p.x), dval(p.y), dval(p.z));
-    bin_escape<R>(t, d, a, p, dval(f.xpold), dval(f.ypold), dval(f.zpold), f.iflag, f.iscat, L);
+    if (L.on) bin_escape<R>(t, d, a, p, dval(f.xpold), dval(f.ypold), dval(f.zpold), f.iflag, f.iscat, L);
     return ST_DONE;
   }
   if (st == TI_STAR) {
@@ -2379,14 +2602,16 @@ __device__ __forceinline__ int walk(const DevModel& m, const DevTallies& t, cons
   }
   if (st == TI_FAULT) {
     L.add(HC3D_CNT_STUCK);
-    set_status(a, 1);
-    log_fault(t, rng, L.fault);
+    if (L.on) {
+      set_status(a, 1);
+      log_fault(t, rng, L.fault);
+    }
     return ST_DONE;
   }
   if (!first) {
     if (p.ir != pir || p.it != pit || p.ip != pip) f.iint = 0;
     if (f.iint > a.iintmax || (a.max_interactions > 0 && f.ntot >= a.max_interactions)) {
-      atomicAdd(t.killed + cidx(m, p.ir, p.it, p.ip), 1u);
+      if (L.on) atomicAdd(t.killed + cidx(m, p.ir, p.it, p.ip), 1u);
       L.add(HC3D_CNT_ABFLUX);
       tr.add(7, p.ir, p.it, p.ip, 0, 0.0, dval(p.x), dval(p.y), dval(p.z));
       return ST_DONE;
@@ -2395,8 +2620,10 @@ __device__ __forceinline__ int walk(const DevModel& m, const DevTallies& t, cons
   f.idust2 = select_dust<R>(m, p, rng);
   if (f.idust2 < 0) {
     L.add(HC3D_CNT_STUCK);
-    set_status(a, 2);
-    log_fault(t, rng, F_SELECT);
+    if (L.on) {
+      set_status(a, 2);
+      log_fault(t, rng, F_SELECT);
+    }
     return ST_DONE;
   }
   if (first) L.add(HC3D_CNT_TOT);
@@ -2430,12 +2657,12 @@ __device__ __forceinline__ bool deep_peel(const DevModel& m, const Pkt<R>& p, in
 // stokes) or absorption and thermal re-emission (rec = the re-emitted packet).
 // Returns whether rec was written: only in peeled runs, and not for an event
 // whose peel-off rays all end in its cell (deep_peel).
-template <class R>
-__device__ __forceinline__ bool interact(const DevModel& m, const DustView<R>& dv, const DevTallies& t, const RunArgs& a, Pkt<R>& p, Rng& rng, Flow<R>& f,
+template <class R, class G>
+__device__ __forceinline__ bool interact(const DevModel& m, const DustView<R>& dv, const DevTallies& t, const RunArgs& a, Pkt<R>& p, G& rng, Flow<R>& f,
                          Local& L, Tracer& tr, PeelRec<R>& rec) {
   const int64_t c = cidx(m, p.ir, p.it, p.ip);
   const int idust2 = f.idust2;
-  L.add(HC3D_CNT_EVENTS);
+  L.events++;
   f.ntot++;
   // issued before the albedo test so that its latency overlaps the draw
   R tave = R(0);
@@ -2444,14 +2671,14 @@ __device__ __forceinline__ bool interact(const DevModel& m, const DustView<R>& d
   if (ran<R>(rng) <= pick4(p.albedo, idust2)) {  // scattered
     f.iflag = 1; f.iscat++; f.iint++;
     keep = a.ipeel == 1 && !deep_peel<R>(m, p, c);
-    if (keep) make_rec<R>(rec, p, a, 1, idust2);
+    if (keep && L.on) make_rec<R>(rec, p, a, 1, idust2);
     stokes<R>(p, idust2, rng);
     tr.add(5, p.ir, p.it, p.ip, 0, 0.0, dval(p.x), dval(p.y), dval(p.z));
   } else {  // absorbed + re-emitted (emit_common thermal branch, reemit; small grains: rep_draine, emit_sg)
     const bool sg = (m.sg_mask >> idust2) & 1u;
-    atomicAdd((sg ? t.dsg : t.dbig) + c, 1u);
+    if (L.on) atomicAdd((sg ? t.dsg : t.dbig) + c, 1u);
     p.i_orig = ((m.disk_mask >> idust2) & 1u) ? 2 : 3;
-    atomicAdd(t.nabs + (int64_t)idust2 * m.ncell + c, 1ull);
+    if (L.on) atomicAdd(t.nabs + (int64_t)idust2 * m.ncell + c, 1ull);
     p.sip = R(1); p.sqp = R(0); p.sup = R(0); p.svp = R(0);
     if (sg) {
       // emit_common.f90:31-53: the spectrum row of the cell's mean intensity
@@ -2461,11 +2688,8 @@ __device__ __forceinline__ bool interact(const DevModel& m, const DustView<R>& d
       const double imf = a.iter1 ? 0.0 : __ldg(m.imfract + c);
       p.nub = (R)rep_draine<R>(m, im, imf, rng);
     }
-    p.cost = R(1) - R(2) * ran<R>(rng);
-    p.sint = xsqrt(R(1) - p.cost * p.cost);
-    p.phi = (R)kR2p * ran<R>(rng);
-    p.cosp = xcos(p.phi);
-    p.sinp = xsin(p.phi);
+    draw_mu<R>(rng, p.cost, p.sint);
+    draw_phi<R>(rng, p.phi, p.cosp, p.sinp);
     if (!sg) {
       if constexpr (sizeof(R) == 4) p.nub = lucy_freq_mixed(m, p.lrow, c, idust2, rng);
       else p.nub = lucydustfreq<R>(m, tave, idust2, rng);
@@ -2473,7 +2697,7 @@ __device__ __forceinline__ bool interact(const DevModel& m, const DustView<R>& d
     f.iflag = 0;
     opacset<R>(m, dv, p, p.nub, a);
     keep = a.ipeel == 1 && !deep_peel<R>(m, p, c);
-    if (keep) make_rec<R>(rec, p, a, 0, idust2);
+    if (keep && L.on) make_rec<R>(rec, p, a, 0, idust2);
     f.iint++;
     tr.add(6, p.ir, p.it, p.ip, 0, 0.0, dval(p.x), dval(p.y), dval(p.z));
   }
@@ -2482,6 +2706,7 @@ __device__ __forceinline__ bool interact(const DevModel& m, const DustView<R>& d
 
 // every thread of the block calls it, after its last event
 __device__ __forceinline__ void flush(const DevTallies& t, Local& L) {
+  L.settle();
   __syncthreads();
   if (threadIdx.x < 16 && L.sc[threadIdx.x]) atomicAdd(t.counters + threadIdx.x, L.sc[threadIdx.x]);
 }
@@ -2489,7 +2714,7 @@ __device__ __forceinline__ void flush(const DevTallies& t, Local& L) {
 // ---- per-thread form: one packet at a time, its peel-off rays inline --------------
 // Used for the trace harness and for runs without peel-off (the Lucy
 // iterations), where a packet's history is its only work.
-template <class R>
+template <class R, bool kFused>
 __device__ void run_packet(const DevModel& m, const DustView<R>& dv, const DevTallies& t, const TallyDims& d, const RunArgs& a, Rng& rng,
                            Local& L, Tracer& tr) {
   Pkt<R> p;
@@ -2499,10 +2724,10 @@ __device__ void run_packet(const DevModel& m, const DustView<R>& dv, const DevTa
   Flow<R> f;
   f.xpold = p.x; f.ypold = p.y; f.zpold = p.z;
   f.iflag = 0; f.iscat = 0; f.iint = 0; f.idust2 = 0; f.ntot = 0;
-  int st = walk<R>(m, t, d, a, p, rng, f, L, tr, true);
+  int st = walk<R, kFused>(m, t, d, a, p, rng, f, L, tr, true);
   while (st == ST_INTERACT) {
     if (interact<R>(m, dv, t, a, p, rng, f, L, tr, rec)) peel_all<R>(m, t, d, a, rec, L);
-    st = walk<R>(m, t, d, a, p, rng, f, L, tr, false);
+    st = walk<R, kFused>(m, t, d, a, p, rng, f, L, tr, false);
   }
 }
 
@@ -2523,7 +2748,7 @@ __global__ void __launch_bounds__(128) k_transport(DevModel m, DevTallies t, Tal
       rng.inj = a.inj + (size_t)k * a.ninj;
       rng.ninj = a.ninj;
       Tracer tr{reinterpret_cast<TraceRec*>(a.trace) + (size_t)k * a.max_rec, a.max_rec, 0};
-      run_packet<R>(m, dv, t, d, a, rng, L, tr);
+      run_packet<R, false>(m, dv, t, d, a, rng, L, tr);
       a.nrec[k] = tr.n;
     }
   } else {
@@ -2533,7 +2758,8 @@ __global__ void __launch_bounds__(128) k_transport(DevModel m, DevTallies t, Tal
       if (pid >= (unsigned long long)a.np) break;
       Rng rng;
       rng_init(rng, a.key0, a.key1, (uint64_t)(a.packet_offset + (int64_t)pid));
-      run_packet<R>(m, dv, t, d, a, rng, L, tr);
+      run_packet<R, false>(m, dv, t, d, a, rng, L, tr);
+      L.settle();
     }
   }
   flush(t, L);
@@ -2568,9 +2794,12 @@ __global__ void __launch_bounds__(128) k_transport_batch(const BatchItem* items,
     Local L;
     L.sc = b.t.counters;
     L.fault = 0;
+    L.cross = L.events = L.pcross = 0u;
+    L.on = true;
     Rng rng;
     rng_init(rng, b.a.key0, b.a.key1, (uint64_t)(b.a.packet_offset + ((int64_t)g - sfirst[lo])));
-    run_packet<R>(b.m, dv, b.t, b.d, b.a, rng, L, tr);
+    run_packet<R, true>(b.m, dv, b.t, b.d, b.a, rng, L, tr);
+    L.settle();
   }
 }
 
@@ -2591,10 +2820,22 @@ struct Slot {
   int stage;  // 0 = empty, 1 = an interaction is pending
 };
 
-template <class R>
+// The packets of a batch, one per lane, regenerated from the batch counter as
+// they end.  kPeel: one wave of a peeled run, at most E events a lane, its
+// records in the queue and its packets in flight in the pool (slot = thread),
+// listed in live[0 .. *alive).  Otherwise (the Lucy iterations, which make no
+// records) the whole batch in one launch.
+//
+// A history of an optically thick cell runs to 10^4 .. 10^6 events while most
+// packets end after tens, so at the end of a batch a few lanes of a few warps
+// would run on alone, each event a chain of about 1800 dependent
+// instructions, 5 us.  Once the batch has no packet left, a warp with fewer
+// than a.dump busy lanes therefore stops and leaves its packets to k_tail:
+// in their pool slots (kPeel), or as the first *alive slots of the pool.
+template <class R, bool kPeel>
 __global__ void __launch_bounds__(128, 3) k_wave(DevModel m, DevTallies t, TallyDims d, RunArgs a, Slot<R>* pool,
                                                PeelRec<R>* queue, unsigned long long* qcount, int E,
-                                               unsigned int* alive) {
+                                               unsigned int* alive, unsigned int* live) {
   extern __shared__ double dust_smem[];
   DustView<R> dv;
   dust_view<R>(m, reinterpret_cast<R*>(dust_smem), dv);
@@ -2602,10 +2843,12 @@ __global__ void __launch_bounds__(128, 3) k_wave(DevModel m, DevTallies t, Tally
   Local L;
   local_init(L, block_counters);
   const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  Slot<R> s = pool[gid];
+  Slot<R> s;
+  if constexpr (kPeel) s = pool[gid];
+  else { s.stage = 0; s.pid = 0; }
   Rng rng;
   rng_init(rng, a.key0, a.key1, s.pid);
-  if (s.stage) {
+  if (kPeel && s.stage) {
     rng.c0 = s.c0;
     rng.left = s.left;
     if (rng.left > 0) philox(rng.c0 - 1, 0u, rng.c2, rng.c3, rng.k0, rng.k1, rng.b);
@@ -2616,52 +2859,136 @@ __global__ void __launch_bounds__(128, 3) k_wave(DevModel m, DevTallies t, Tally
   // only when at least a.regen lanes of its warp are waiting, or no lane is
   // busy, so that emissions run together instead of beside the other lanes'
   // interactions.  The tallies do not depend on it (each packet's stream is
-  // keyed by its id).
-  bool done = false;  // the batch has no packet left for this lane
+  // keyed by its id).  A batch of fewer packets than threads is spread over
+  // the warps: only the first a.lanes lanes of each take packets.
+  bool done = (int)(threadIdx.x & 31) >= a.lanes;  // the batch has no packet left for this lane
   // Queue slots are reserved a.qchunk at a time, so that the atomic whose
   // result addresses the record is paid once per qchunk events (in the tail
   // of a batch, where a few long histories run alone, it is otherwise a
   // round trip on every event); slots left over are marked empty at the end.
   unsigned long long slot = 0ull, slot_end = 0ull;
-  for (int nrec = 0; nrec < E; ++nrec) {
+  bool exhausted = false;  // every packet of the batch has been taken
+  for (int nrec = 0; !kPeel || nrec < E; ++nrec) {
     const unsigned waiting = __ballot_sync(0xffffffffu, s.stage == 0 && !done);
     const unsigned busy = __ballot_sync(0xffffffffu, s.stage != 0);
-    if (waiting == 0u && busy == 0u) break;  // warp-uniform
-    if (s.stage == 0) {
-      if (done || (busy != 0u && __popc(waiting) < a.regen)) continue;
+    if ((waiting == 0u || exhausted) && busy == 0u) break;  // warp-uniform
+    if (exhausted && __popc(busy) < a.dump) break;
+    // read here and used in the next round, so that its latency is hidden
+    const unsigned long long taken = *reinterpret_cast<volatile unsigned long long*>(a.work);
+    bool run = s.stage != 0;
+    if (!run && !done && (busy == 0u || __popc(waiting) >= a.regen)) {
       const unsigned long long pid = atomicAdd(a.work, 1ull);
       if (pid >= (unsigned long long)a.np) {
         done = true;
-        continue;
+      } else {
+        s.pid = (uint64_t)(a.packet_offset + (int64_t)pid);
+        rng_init(rng, a.key0, a.key1, s.pid);
+        run = true;
       }
-      s.pid = (uint64_t)(a.packet_offset + (int64_t)pid);
-      rng_init(rng, a.key0, a.key1, s.pid);
     }
-    // The event's record is written field by field into its queue slot as
-    // emission or the interaction produces it: the record occupies no
-    // registers across the walk.
-    if (slot == slot_end) {
-      slot = atomicAdd(qcount, (unsigned long long)a.qchunk);
-      slot_end = slot + (unsigned long long)a.qchunk;
+    if (run) {
+      // The event's record is written field by field into its queue slot as
+      // emission or the interaction produces it: the record occupies no
+      // registers across the walk.
+      PeelRec<R> none;
+      if (kPeel && slot == slot_end) {
+        slot = atomicAdd(qcount, (unsigned long long)a.qchunk);
+        slot_end = slot + (unsigned long long)a.qchunk;
+      }
+      PeelRec<R>& rec = kPeel ? queue[slot] : none;
+      bool emitted = true;
+      if (s.stage == 0) {
+        ++slot;
+        emitted = emit<R>(m, dv, t, a, s.p, rng, rec, tr, L);  // else dropped: the lane takes the next packet
+        if (emitted) {
+          s.f.xpold = s.p.x; s.f.ypold = s.p.y; s.f.zpold = s.p.z;
+          s.f.iflag = 0; s.f.iscat = 0; s.f.iint = 0; s.f.idust2 = 0; s.f.ntot = 0;
+          s.stage = 2;  // emitted: walk to the first interaction after the record
+        }
+      } else if (interact<R>(m, dv, t, a, s.p, rng, s.f, L, tr, rec)) {
+        ++slot;  // the slot is kept only when the event made a record
+      }
+      if (emitted) {
+        const int st = walk<R, kPeel>(m, t, d, a, s.p, rng, s.f, L, tr, s.stage == 2);
+        s.stage = st == ST_INTERACT ? 1 : 0;
+        if (!kPeel && s.stage == 0) L.settle();
+      }
     }
-    PeelRec<R>& rec = queue[slot];
-    if (s.stage == 0) {
-      ++slot;
-      if (!emit<R>(m, dv, t, a, s.p, rng, rec, tr, L)) continue;  // dropped: the lane takes the next packet
-      s.f.xpold = s.p.x; s.f.ypold = s.p.y; s.f.zpold = s.p.z;
-      s.f.iflag = 0; s.f.iscat = 0; s.f.iint = 0; s.f.idust2 = 0; s.f.ntot = 0;
-      s.stage = 2;  // emitted: walk to the first interaction after the record
-    } else if (interact<R>(m, dv, t, a, s.p, rng, s.f, L, tr, rec)) {
-      ++slot;  // the slot is kept only when the event made a record
-    }
-    const int st = walk<R>(m, t, d, a, s.p, rng, s.f, L, tr, s.stage == 2);
-    s.stage = st == ST_INTERACT ? 1 : 0;
+    exhausted = __any_sync(0xffffffffu, taken >= (unsigned long long)a.np);
   }
-  for (; slot < slot_end; ++slot) queue[slot].flags = kRecNoPeel;
   s.c0 = rng.c0;
   s.left = rng.left;
-  pool[gid] = s;
-  if (s.stage) atomicAdd(alive, 1u);
+  if constexpr (kPeel) {
+    for (; slot < slot_end; ++slot) queue[slot].flags = kRecNoPeel;
+    pool[gid] = s;
+    if (s.stage) live[atomicAdd(alive, 1u)] = (unsigned)gid;
+  } else {
+    if (s.stage) pool[atomicAdd(alive, 1u)] = s;
+  }
+  flush(t, L);
+}
+
+// The packets that k_wave left, one per warp: every lane holds the packet and
+// runs its events, and the parts of an event that a lane alone would do one
+// after another are shared between the lanes -- the draws and their
+// logarithms, sines and cosines (DrawTable), the tries of the scattering
+// angle (scat_draw), the search of the Lucy CDF (lucy_freq_mixed) and the
+// tallies of a step (tally_path_warp).  What bounds it is the latency of one
+// packet's chain of events: 3.4 us an event in the plain model's disk against
+// 5.0 us for a lane of k_wave, and no other lane of the warp runs beside it.
+// The arithmetic is that of k_wave, bit for bit.
+template <class R, bool kPeel>
+__global__ void __launch_bounds__(128, 4) k_tail(DevModel m, DevTallies t, TallyDims d, RunArgs a, Slot<R>* pool,
+                                                 const unsigned int* nlive, const unsigned int* live,
+                                                 unsigned int* next, PeelRec<R>* queue, unsigned long long* qcount,
+                                                 int E, unsigned int* alive_out, unsigned int* live_out) {
+  extern __shared__ double dust_smem[];
+  DustView<R> dv;
+  dust_view<R>(m, reinterpret_cast<R*>(dust_smem), dv);
+  __shared__ unsigned long long block_counters[16];
+  __shared__ DrawTable<R> draws[4];
+  Local L;
+  local_init(L, block_counters);
+  const int lane = threadIdx.x & 31;
+  L.on = lane == 0;
+  const unsigned n = *nlive;
+  Tracer tr{nullptr, 0, 0};
+  for (;;) {
+    unsigned k = 0;
+    if (lane == 0) k = atomicAdd(next, 1u);
+    k = __shfl_sync(0xffffffffu, k, 0);
+    if (k >= n) break;
+    const unsigned gid = kPeel ? live[k] : k;
+    Slot<R> s = pool[gid];
+    WarpRng<R> rng;
+    rng_init(rng, draws + (threadIdx.x >> 5), a.key0, a.key1, s.pid, s.c0, s.left);
+    unsigned long long slot = 0ull, slot_end = 0ull;
+    for (int nrec = 0; !kPeel || nrec < E; ++nrec) {
+      ensure(rng, 8);  // an event draws at most 7 beside the tries of a scattering
+      PeelRec<R> none;
+      if (kPeel && slot == slot_end) {
+        if (lane == 0) slot = atomicAdd(qcount, (unsigned long long)a.qchunk);
+        slot = __shfl_sync(0xffffffffu, slot, 0);
+        slot_end = slot + (unsigned long long)a.qchunk;
+      }
+      if (interact<R>(m, dv, t, a, s.p, rng, s.f, L, tr, kPeel ? queue[slot] : none)) ++slot;
+      ensure(rng, 8);
+      if (walk<R, kPeel>(m, t, d, a, s.p, rng, s.f, L, tr, false) != ST_INTERACT) {
+        s.stage = 0;
+        break;
+      }
+    }
+    L.settle();
+    if constexpr (kPeel) {
+      if (lane == 0) {
+        for (; slot < slot_end; ++slot) queue[slot].flags = kRecNoPeel;
+        rng_save(rng, s.c0, s.left);
+        pool[gid] = s;
+        if (s.stage) live_out[atomicAdd(alive_out, 1u)] = gid;
+      }
+    }
+    __syncwarp();
+  }
   flush(t, L);
 }
 
