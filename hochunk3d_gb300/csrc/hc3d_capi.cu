@@ -33,6 +33,7 @@ struct hc3d_ctx {
   double* d_tdust = nullptr;   // (ncell*4), also dm.tdust
   float* d_tdustf = nullptr;   // (ncell*4) FP32 copy, also dm.tdustf
   unsigned char* d_peelmask = nullptr;
+  int2* d_lucyrow = nullptr;  // (ncell*4) weight and CDF row pair of each temperature, also dm.lucyrow
   float4* d_rho4p = nullptr;  // (ncell) peel-masked FP32 densities, also dm.rho4p
   int ndg_in = 0;
   // species (1..8, reference numbering) of the four device slots (hc3d_set_species)
@@ -199,7 +200,25 @@ __device__ __forceinline__ float4 masked_rho(float4 r, unsigned mask) {
                      (mask & 8u) ? r.w : 0.f);
 }
 
-__global__ void k_lucy(LucyArgs a, const unsigned long long* dtauabs, const double* rho4d, const double* massarr,
+// The Lucy CDF row pair of a temperature and the weight of its second row
+// (lucydustfreq.f90:19-40), as the mixed form reads them (DevModel::lucyrow).
+struct LucyRows {
+  const float* lT;  // (nT) FP32
+  int nT;
+  int2* rows;       // NULL: no tables loaded yet
+};
+
+__device__ __forceinline__ int2 lucy_row(const LucyRows& q, float T0, int s) {
+  const float lT0 = logf(T0);
+  const float l1 = __ldg(q.lT), lN = __ldg(q.lT + q.nT - 1);
+  int j = (int)((float)(q.nT - 1) * (lT0 - l1) / (lN - l1)) + 1;
+  j = j < 1 ? 1 : (j > q.nT - 1 ? q.nT - 1 : j);
+  float f = (lT0 - __ldg(q.lT + j - 1)) / (__ldg(q.lT + j) - __ldg(q.lT + j - 1));
+  f = f < 0.f ? 0.f : (f > 1.f ? 1.f : f);
+  return make_int2(__float_as_int(f), s * (q.nT - 1) + (j - 1));
+}
+
+__global__ void k_lucy(LucyArgs a, LucyRows rows, const unsigned long long* dtauabs, const double* rho4d, const double* massarr,
                        double* tdust, float* tdustf, unsigned char* peelmask, unsigned long long* maxrel,
                        const float4* rho4f, float4* rho4p) {
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < a.ncell; c += (int64_t)gridDim.x * blockDim.x) {
@@ -216,6 +235,7 @@ __global__ void k_lucy(LucyArgs a, const unsigned long long* dtauabs, const doub
         T = Td;
         tdust[4 * c + s] = Td;
         tdustf[4 * c + s] = (float)Td;
+        rows.rows[4 * c + s] = lucy_row(rows, (float)Td, s);
       }
       if (T < a.tsub / 11605.0) mask |= 1u << s;
     }
@@ -224,12 +244,16 @@ __global__ void k_lucy(LucyArgs a, const unsigned long long* dtauabs, const doub
   }
 }
 
-__global__ void k_peelmask(int64_t ncell, const double* tdust, double tsub, unsigned char* peelmask,
-                           const float4* rho4f, float4* rho4p) {
+// What follows from the temperatures of a loaded grid: the peel mask, the
+// peel-masked densities and the rows of the Lucy CDF.
+__global__ void k_peelmask(int64_t ncell, LucyRows rows, const double* tdust, const float* tdustf, double tsub,
+                           unsigned char* peelmask, const float4* rho4f, float4* rho4p) {
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < ncell; c += (int64_t)gridDim.x * blockDim.x) {
     unsigned mask = 0;
-    for (int s = 0; s < kSlots; ++s)
+    for (int s = 0; s < kSlots; ++s) {
       if (tdust[4 * c + s] < tsub / 11605.0) mask |= 1u << s;
+      if (rows.rows) rows.rows[4 * c + s] = lucy_row(rows, tdustf[4 * c + s], s);
+    }
     peelmask[c] = (unsigned char)mask;
     rho4p[c] = masked_rho(rho4f[c], mask);
   }
@@ -290,6 +314,15 @@ int grid_blocks_for(hc3d_ctx* c, int64_t n) {
   int64_t b = (n + 255) / 256;
   int64_t cap = (int64_t)c->sm_count * 8;
   return (int)std::max<int64_t>(1, std::min(b, cap));
+}
+
+LucyRows lucy_rows(hc3d_ctx* c) {
+  return LucyRows{c->dm.lTintf, c->dm.nT, c->tables ? c->d_lucyrow : nullptr};
+}
+
+void launch_peelmask(hc3d_ctx* c) {
+  k_peelmask<<<grid_blocks_for(c, c->dm.ncell), 256, 0, c->stream>>>(
+      c->dm.ncell, lucy_rows(c), c->d_tdust, c->d_tdustf, c->tsub, c->d_peelmask, c->dm.rho4f, c->d_rho4p);
 }
 
 int alloc_run_tallies(hc3d_ctx* c, const TallyDims& d) {
@@ -905,6 +938,7 @@ extern "C" int hc3d_reset(hc3d_ctx* c) {
   c->dims = TallyDims{};
   c->d_kappap = c->d_massarr = c->d_tdust = nullptr;
   c->d_tdustf = nullptr;
+  c->d_lucyrow = nullptr;
   c->d_peelmask = nullptr;
   c->d_rho4p = nullptr;
   c->ndg_in = 0;
@@ -1140,14 +1174,21 @@ extern "C" int hc3d_load_tables(hc3d_ctx* c, const hc3d_dust_tables* t) {
     if ((r = dupload(c, own, &d_pair, pair.data(), pair.size())) ||
         (r = dupload(c, own, &d_guide, guide.data(), guide.size())))
       return r;
+    std::vector<float2> ratio(nnu);
+    for (int i = 0; i < nnu; ++i) {
+      const float n0 = (float)t->nuint[i], n1 = (float)t->nuint[std::min(i + 1, nnu - 1)];
+      ratio[i] = make_float2(n0, n1 / n0);
+    }
+    float2* d_ratio = nullptr;
+    if ((r = dupload(c, own, &d_ratio, ratio.data(), ratio.size()))) return r;
+    c->dm.nuratio = d_ratio;
     c->dm.kpairf = d_pair;
     c->dm.kguide = d_guide;
   }
   c->tsub = t->tsub > 0.0 ? t->tsub : 1600.0;
   c->tables = true;
   if (c->grid) {
-    k_peelmask<<<grid_blocks_for(c, c->dm.ncell), 256, 0, c->stream>>>(c->dm.ncell, c->d_tdust, c->tsub, c->d_peelmask,
-                                                                       c->dm.rho4f, c->d_rho4p);
+    launch_peelmask(c);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(c->stream));
   }
@@ -1235,6 +1276,7 @@ extern "C" int hc3d_load_grid(hc3d_ctx* c, const hc3d_grid* g) {
   {
     const std::vector<float> tdf(td.begin(), td.end());
     if ((r = dupload(c, own, &c->d_tdustf, tdf.data(), tdf.size()))) return r;
+    if ((r = dalloc(c, own, &c->d_lucyrow, (size_t)4 * ncell))) return r;
   }
   DevTallies& t = c->dt;
   if ((r = dalloc(c, own, &t.nabs, (size_t)kSlots * ncell)) || (r = dalloc(c, own, &t.dtauabs, (size_t)kSlots * ncell)) ||
@@ -1301,10 +1343,10 @@ extern "C" int hc3d_load_grid(hc3d_ctx* c, const hc3d_grid* g) {
   }
   m.aarrd = d_a; m.barrd = d_b; m.aarrf = d_af; m.barrf = d_bf; m.rho4f = d_rf; m.rho4d = d_rd;
   m.peelmask = c->d_peelmask; m.rho4p = c->d_rho4p; m.tdust = c->d_tdust; m.tdustf = c->d_tdustf;
+  m.lucyrow = c->d_lucyrow;
   m.imean = c->d_imean; m.imfract = c->d_imfract;
   c->ndg_in = g->ndg;
-  k_peelmask<<<grid_blocks_for(c, ncell), 256, 0, c->stream>>>(ncell, c->d_tdust, c->tsub, c->d_peelmask, d_rf,
-                                                                c->d_rho4p);
+  launch_peelmask(c);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(c->stream));
   c->grid = true;
@@ -1351,8 +1393,7 @@ extern "C" int hc3d_set_tdust(hc3d_ctx* c, const double* tdust) {
   const std::vector<float> tdf(td.begin(), td.end());
   CK(cudaMemcpyAsync(c->d_tdust, td.data(), td.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemcpyAsync(c->d_tdustf, tdf.data(), tdf.size() * sizeof(float), cudaMemcpyHostToDevice, c->stream));
-  k_peelmask<<<grid_blocks_for(c, ncell), 256, 0, c->stream>>>(ncell, c->d_tdust, c->tsub, c->d_peelmask, c->dm.rho4f,
-                                                                c->d_rho4p);
+  launch_peelmask(c);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(c->stream));
   return HC3D_OK;
@@ -1873,7 +1914,7 @@ extern "C" int hc3d_lucy_update(hc3d_ctx* c, double ltot, int64_t np, double* td
   CK(cudaSetDevice(c->device));
   const LucyArgs a = lucy_args(c, ltot, np);
   CK(cudaMemsetAsync(c->d_maxrel, 0, sizeof(unsigned long long), c->stream));
-  k_lucy<<<grid_blocks_for(c, a.ncell), 256, 0, c->stream>>>(a, c->dt.dtauabs, c->dm.rho4d, c->d_massarr, c->d_tdust, c->d_tdustf,
+  k_lucy<<<grid_blocks_for(c, a.ncell), 256, 0, c->stream>>>(a, lucy_rows(c), c->dt.dtauabs, c->dm.rho4d, c->d_massarr, c->d_tdust, c->d_tdustf,
                                                            c->d_peelmask, c->d_maxrel, c->dm.rho4f, c->d_rho4p);
   CK(cudaGetLastError());
   if (c->dm.sg_on) {
@@ -1950,7 +1991,7 @@ extern "C" int hc3d_lucy_iterations(hc3d_ctx* c, const hc3d_run_params* p, int n
     if (e == cudaSuccess) e = cudaMemsetAsync(c->d_work, 0, sizeof(unsigned long long), st);
     if (e == cudaSuccess) e = launch_packets(c, args[(size_t)k], cfg, tail_blocks);
     if (e == cudaSuccess) {
-      k_lucy<<<grid_blocks_for(c, la.ncell), 256, 0, st>>>(la, c->dt.dtauabs, c->dm.rho4d, c->d_massarr, c->d_tdust,
+      k_lucy<<<grid_blocks_for(c, la.ncell), 256, 0, st>>>(la, lucy_rows(c), c->dt.dtauabs, c->dm.rho4d, c->d_massarr, c->d_tdust,
                                                            c->d_tdustf, c->d_peelmask, d_rel + k, c->dm.rho4f,
                                                            c->d_rho4p);
       e = cudaGetLastError();

@@ -103,6 +103,8 @@ struct DevModel {
   // frequency index where the interpolated CDF of rows j, j+1 crosses a level in [b, b+1)/kGuide
   const float2* kpairf;
   const short2* kguide;
+  const float2* nuratio;  // (nnu) nuint(i) and nuint(i+1)/nuint(i), FP32 (ratio 1 in the last row)
+  const int2* lucyrow;    // (ncell*4) per cell and slot: the weight f (FP32 bits) and the row pair of tdustf (lucy_row)
   // dust-table guide of the mixed form: dguide[u*kDustGuide + b] = (lo, hi) brackets the row i0 of
   // table u (nud(i0) >= nu > nud(i0+1)) for ln(nu) in bucket b of [dlnlo[u], dlnlo[u] + kDustGuide/dginv[u])
   const short2* dguide;

@@ -92,7 +92,7 @@ int64_t footprint_bytes(const hc3d::Model& m, int npeel) {
   const int64_t sg = m.sg_slot >= 0 ? ncell * (4 /*dsg*/ + 8 /*jsg*/ + 4 /*imean*/ + 8 /*imfract*/ + 8 /*vcell*/) +
                                           (int64_t)2 * hc3d::kNemit * hc3d::kNdraine * 8
                                     : 0;
-  const int64_t grid = ncell * (4 * 4 /*rho f32*/ + 4 * 8 /*rho f64*/ + 2 * 4 * 8 /*tdust, massarr*/ + 4 * 4 /*tdust f32*/ +
+  const int64_t grid = ncell * (4 * 4 /*rho f32*/ + 4 * 8 /*rho f64*/ + 2 * 4 * 8 /*tdust, massarr*/ + 4 * 4 /*tdust f32*/ + 4 * 8 /*Lucy rows*/ +
                                 1 /*peel mask*/ + 2 * 4 * 8 /*nabs, dtauabs*/ + 8 /*jmean*/ + 2 * 4 /*killed, dbig*/) +
                        sg;
   const int64_t walls = (int64_t)(m.nrg + m.ntg + m.npg) * 64 + n4 * 8 /*vcell*/;

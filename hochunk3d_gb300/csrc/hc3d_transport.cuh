@@ -136,15 +136,20 @@ template <class R> __device__ __forceinline__ void draw_phi(Rng& r, R& phi, R& c
   sphi = xsin(phi);
 }
 
-// Draws of a packet that a whole warp runs (k_tail): the next 128 draws of its
-// stream and the functions above of each, formed 32 lanes at a time in shared
-// memory, so that the packet's chain of events reads them instead of running
-// Philox, a logarithm, a sine and a cosine one after another.  Every lane
-// holds the same position; ensure() is called by the whole warp.
-template <class R>
-struct DrawTable {
+// Draws of a packet that a whole warp runs (k_tail): the next draws of its
+// stream, formed 32 lanes at a time in shared memory.  The FP64 form keeps the
+// functions above of each beside them -- a lone FP64 logarithm is a chain of
+// 2100 cycles -- and reads them instead; the mixed form runs its events side by
+// side in the lanes (tail_batch), which form what they need.  Every lane holds
+// the same position; ensure() is called by the whole warp.
+template <class R> struct DrawTable;
+template <> struct DrawTable<float> {
+  static constexpr int kDraws = 256;
+  float u[kDraws];
+};
+template <> struct DrawTable<double> {
   static constexpr int kDraws = 128;
-  R u[kDraws], nl[kDraws], mu[kDraws], smu[kDraws], cphi[kDraws], sphi[kDraws];
+  double u[kDraws], nl[kDraws], mu[kDraws], smu[kDraws], cphi[kDraws], sphi[kDraws];
 };
 template <class R>
 struct WarpRng {
@@ -156,29 +161,41 @@ struct WarpRng {
 
 template <class G> struct IsWarp { static constexpr bool value = false; };
 template <class R> struct IsWarp<WarpRng<R>> { static constexpr bool value = true; };
+// whether the caller of select_dust has the density of the cell at hand
+struct OneDraw;
+template <class G> struct KnowsRho { static constexpr bool value = IsWarp<G>::value; };
+template <> struct KnowsRho<OneDraw> { static constexpr bool value = true; };
 
 template <class R> __device__ __forceinline__ void fill_draws(WarpRng<R>& r) {
   r.block += (uint32_t)(r.at >> 2);
   r.at &= 3;
   const int lane = threadIdx.x & 31;
-  uint32_t b[4];
-  philox(r.block + (uint32_t)lane, 0u, r.c2, r.c3, r.k0, r.k1, b);
   __syncwarp();  // the lanes have read what they need of the old table
+  if constexpr (sizeof(R) == 4) {
+#pragma unroll
+    for (int h = 0; h < DrawTable<R>::kDraws / 128; ++h) {
+      uint32_t b[4];
+      philox(r.block + (uint32_t)(32 * h + lane), 0u, r.c2, r.c3, r.k0, r.k1, b);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        r.t->u[128 * h + 4 * lane + j] = ((float)(b[j] >> 8) + 0.5f) * (1.0f / 16777216.0f);
+    }
+  } else {
+    uint32_t b[4];
+    philox(r.block + (uint32_t)lane, 0u, r.c2, r.c3, r.k0, r.k1, b);
 #pragma unroll 1
-  for (int j = 0; j < 4; ++j) {
-    R u;
-    const uint32_t w = pick4(b, j);
-    if constexpr (sizeof(R) == 4) u = ((float)(w >> 8) + 0.5f) * (1.0f / 16777216.0f);
-    else u = ((double)w + 0.5) * (1.0 / 4294967296.0);
-    const int k = 4 * lane + j;
-    r.t->u[k] = u;
-    r.t->nl[k] = -xlog(u);
-    const R mu = R(1) - R(2) * u;
-    r.t->mu[k] = mu;
-    r.t->smu[k] = xsqrt(R(1) - mu * mu);
-    const R phi = (R)kR2p * u;
-    r.t->cphi[k] = xcos(phi);
-    r.t->sphi[k] = xsin(phi);
+    for (int j = 0; j < 4; ++j) {
+      const R u = ((double)pick4(b, j) + 0.5) * (1.0 / 4294967296.0);
+      const int k = 4 * lane + j;
+      r.t->u[k] = u;
+      r.t->nl[k] = -xlog(u);
+      const R mu = R(1) - R(2) * u;
+      r.t->mu[k] = mu;
+      r.t->smu[k] = xsqrt(R(1) - mu * mu);
+      const R phi = (R)kR2p * u;
+      r.t->cphi[k] = xcos(phi);
+      r.t->sphi[k] = xsin(phi);
+    }
   }
   __syncwarp();
 }
@@ -201,16 +218,35 @@ template <class R> __device__ __forceinline__ void rng_save(const WarpRng<R>& r,
   left = (4 - (r.at & 3)) & 3;
 }
 template <class R> __device__ __forceinline__ R ran(WarpRng<R>& r) { return r.t->u[r.at++]; }
-template <class R> __device__ __forceinline__ R neg_log(WarpRng<R>& r) { return r.t->nl[r.at++]; }
+template <class R> __device__ __forceinline__ R neg_log(WarpRng<R>& r) {
+  if constexpr (sizeof(R) == 4) return -xlog(r.t->u[r.at++]);
+  else return r.t->nl[r.at++];
+}
 template <class R> __device__ __forceinline__ void draw_mu(WarpRng<R>& r, R& mu, R& smu) {
-  mu = r.t->mu[r.at];
-  smu = r.t->smu[r.at++];
+  if constexpr (sizeof(R) == 4) {
+    mu = R(1) - R(2) * r.t->u[r.at++];
+    smu = xsqrt(R(1) - mu * mu);
+  } else {
+    mu = r.t->mu[r.at];
+    smu = r.t->smu[r.at++];
+  }
 }
 template <class R> __device__ __forceinline__ void draw_phi(WarpRng<R>& r, R& phi, R& cphi, R& sphi) {
   phi = (R)kR2p * r.t->u[r.at];
-  cphi = r.t->cphi[r.at];
-  sphi = r.t->sphi[r.at++];
+  if constexpr (sizeof(R) == 4) {
+    cphi = xcos(phi);
+    sphi = xsin(phi);
+    r.at++;
+  } else {
+    cphi = r.t->cphi[r.at];
+    sphi = r.t->sphi[r.at++];
+  }
 }
+// one draw, of a lane that works ahead (tail_batch)
+struct OneDraw {
+  float u;
+};
+template <class R> __device__ __forceinline__ R ran(OneDraw& r) { return r.u; }
 
 // ---- packet state: the tts_mod/stokesvar_mod globals of one packet ------------
 // Positions: FP64 in the FP64 form.  The mixed form carries each coordinate
@@ -230,13 +266,6 @@ __device__ __forceinline__ void set_pos(Pos2& d, double v) {
   d.lo = (float)(v - (double)d.hi);
 }
 
-// Lucy CDF rows of one cell and species slot (mixed form, lucy_freq_mixed)
-struct LucyRow {
-  int key;  // 4 * cell + slot; -1 = empty
-  int pr;   // row pair: slot * (nT - 1) + j - 1
-  float T0, f, P0, P1;
-};
-
 template <class R>
 struct Pkt {
   typename PosOf<R>::T x, y, z;
@@ -250,7 +279,6 @@ struct Pkt {
   int i_orig;
   R kapd[kSlots], albedo[kSlots], g[kSlots], pl[kSlots];
   float safe;  // mixed form: a step shorter than this from here stays in the cell (0 = unknown)
-  LucyRow lrow;  // mixed form: cached Lucy CDF rows of the current cell
 };
 
 // Event counters (HC3D_CNT_*) of a thread and its last fault code.  The rare
@@ -622,6 +650,93 @@ __device__ __forceinline__ bool next_wall_ray(const DevModel& m, Ray& r, const P
   return bi != 0;
 }
 
+// The same search by the lanes of a warp that runs one packet (k_tail): lane 0
+// the inner sphere, 1 the outer, 2 and 3 the lower and upper cone, 4 the plane
+// on the side the ray turns towards.  Every lane forms all three kinds of root
+// from its own wall's parameters without a branch, so that their latencies
+// overlap, and keeps the one of its wall; the next wall is the minimum over
+// the lanes, the lowest lane of equal ones as in the search above.  About 300
+// cycles against 900 for the walls one after another.
+template <bool kFused>
+__device__ __forceinline__ bool next_wall_warp(const DevModel& m, Ray& r, const PathLen& S, int ir, int it, int ip,
+                                               int own, float& dt, int& iface) {
+  const int lane = threadIdx.x & 31;
+  const float ux = r.ux, uy = r.uy, uz = r.uz;
+  const float xr = fmaf(S.hi, ux, fmaf(S.lo, ux, r.x0));
+  const float yr = fmaf(S.hi, uy, fmaf(S.lo, uy, r.y0));
+  const float zr = fmaf(S.hi, uz, fmaf(S.lo, uz, r.z0));
+  const int side = fmaf(xr, uy, -__fmul_rn(yr, ux)) > 0.f ? 1 : 0;
+  const float2* wp = m.r2pair + ir - 1;
+  if (lane == 2) wp = m.conef + it - 1;
+  if (lane == 3) wp = m.conef + it;
+  if (lane == 4) wp = m.planef + ip - 1 + side;
+  const float2 w = __ldg(wp);
+  const int id = lane + 1 + (lane == 4 ? side : 0);
+  const bool mine = (own >> min(id, 7)) & 1;
+  const float pxy = fmaf(xr, ux, __fmul_rn(yr, uy)), pz = __fmul_rn(zr, uz);
+  const float rho2 = fmaf(xr, xr, __fmul_rn(yr, yr)), z2 = __fmul_rn(zr, zr);
+  constexpr float kNone = 3.402823466e38f;
+  // cones
+  const float tan2 = w.x, hemi = w.y;
+  const float a = fmaf(-tan2, r.uz2, r.urho2);
+  const float b = 2.f * fmaf(-tan2, pz, pxy);
+  const float cq = fmaf(-tan2, z2, rho2);
+  const float disc = fmaf(b, b, -__fmul_rn(4.f * a, cq));
+  const float rs = rsqrtf(disc), inv = __fdividef(0.5f, a);
+  const float t1 = __fmul_rn(fmaf(disc, rs, -b), inv), t2 = __fmul_rn(fmaf(-disc, rs, -b), inv);
+  // the midplane; the far root on one's own cone; a ray along the cone: one root
+  const bool mid = tan2 < 0.f;
+  const float ts = __fdividef(mid ? -zr : (mine ? -b : -cq), mid ? uz : (mine ? a : b));
+  auto ahead = [&](float t) { return t >= 0.f && fmaf(t, uz, zr) * hemi > 0.f; };
+  float tc = kNone;
+  if (mid) {
+    if (!mine && uz != 0.f && ts >= 0.f) tc = ts;
+  } else if (mine || a == 0.f) {
+    if ((mine ? a : b) != 0.f && ahead(ts)) tc = ts;
+  } else if (disc > 0.f) {
+    if (ahead(t1)) tc = t1;
+    if (ahead(t2)) tc = fminf(tc, t2);
+  }
+  if (tan2 == 0.f) tc = kNone;  // a pole
+  // planes
+  const float d = fmaf(w.x, ux, __fmul_rn(w.y, uy));
+  const float tq = __fdividef(-fmaf(w.x, xr, __fmul_rn(w.y, yr)), d);
+  const float tp = m.npg > 2 && !mine && d != 0.f && tq >= 0.f ? tq : kNone;
+  // spheres
+  const float r2 = lane == 0 ? w.x : w.y;
+  float hb = kFused ? fmaf(zr, uz, pxy) : __fadd_rn(pxy, pz);
+  const float rr = kFused ? fmaf(zr, zr, rho2) : __fadd_rn(rho2, z2);
+  float c = __fsub_rn(rr, r2), ds = fmaf(hb, hb, -c);
+  const bool near = lane < 2 && !mine && (lane == 1 || hb < 0.f) &&
+                    (fabsf(c) < kNearSphere * r2 || fabsf(ds) < kGrazeSphere * r2);
+  if (__any_sync(0xffffffffu, near)) {
+    ray_f64(r);
+    const double s = path_f64(S);
+    const double hbd = fma(s, r.u2, r.hb0);
+    const double rrd = fma(s, fma(s, r.u2, r.hb0 + r.hb0), r.rr0);
+    const double cd = rrd - __ldg(m.r2arr + ir - (lane == 0 ? 1 : 0));
+    hb = (float)hbd;
+    c = (float)cd;
+    ds = (float)fma(hbd, hbd, -cd);
+  }
+  const float rd = rsqrtf(ds), sq = __fmul_rn(ds, rd);
+  const float tn = __fdividef(fmaxf(lane == 0 ? c : -c, 0.f), lane == 0 ? fmaf(ds, rd, -hb) : __fadd_rn(hb, sq));
+  float tr = lane == 0 || hb > 0.f ? tn : __fsub_rn(sq, hb);
+  bool ok = ds > 0.f && (lane == 1 || hb < 0.f);
+  if (mine) {
+    tr = -2.f * hb;
+    ok = hb < 0.f;
+  }
+  if (!(ok && tr >= 0.f)) tr = kNone;
+  const float t = lane < 2 ? tr : (lane < 4 ? tc : (lane == 4 ? tp : kNone));
+  const unsigned bits = __float_as_uint(__fadd_rn(t, 0.f));  // t >= 0: ordered as unsigned (-0 becomes +0)
+  const unsigned best = __reduce_min_sync(0xffffffffu, bits);
+  const int win = __ffs(__ballot_sync(0xffffffffu, bits == best)) - 1;
+  dt = __uint_as_float(best);
+  iface = win + 1 + (win == 4 ? side : 0);
+  return best != __float_as_uint(kNone);
+}
+
 // wall -> index step, peeloff_3d.f90:120-139
 __device__ __forceinline__ void step_index(int npg, int iface, int& ir, int& it, int& ip) {
   ir += (int)(iface == 2) - (int)(iface == 1);
@@ -710,12 +825,13 @@ __device__ __forceinline__ void dust_view(const DevModel& m, R* smem, DustView<R
 // Computed once per unique table; species slots sharing a dust file share
 // the result (only kappa_V differs), which is what the per-slot loop of the
 // reference computes for them.
-template <class R>
+// kWarp: a whole warp forms the opacities of one packet, and searches the
+// table two levels of 32 rows deep by ballots.
+template <class R, bool kWarp>
 __device__ __forceinline__ void opacset(const DevModel& m, const DustView<R>& v, Pkt<R>& p, R nu, const RunArgs& a) {
   if constexpr (sizeof(R) == 4) {
     // mixed form: the same bracket from the ln(nu) guide of each table, then
     // a short bisection inside it; values kept in registers
-    const float lnu = logf(nu);
     float gt[kSlots], plt[kSlots], kt[kSlots], at[kSlots];
 #pragma unroll
     for (int u = 0; u < kSlots; ++u) {
@@ -728,8 +844,15 @@ __device__ __forceinline__ void opacset(const DevModel& m, const DustView<R>& v,
         i0 = i1 = 1;
       } else if (nu <= nud[nl - 1]) {
         i0 = i1 = nl;
+      } else if (kWarp && nl <= 1024) {
+        const int lane = threadIdx.x & 31, st = (nl + 31) >> 5;
+        const int k1 = lane * st;
+        const int base = (__popc(__ballot_sync(0xffffffffu, k1 < nl && nud[min(k1, nl - 1)] >= nu)) - 1) * st;
+        const int k2 = base + lane;
+        i0 = base + __popc(__ballot_sync(0xffffffffu, lane < st && k2 < nl && nud[min(k2, nl - 1)] >= nu));
+        i1 = i0 + 1;
       } else {
-        const int b = min(max((int)((lnu - m.dlnlo[u]) * m.dginv[u]), 0), kDustGuide - 1);
+        const int b = min(max((int)((logf(nu) - m.dlnlo[u]) * m.dginv[u]), 0), kDustGuide - 1);
         const short2 gb = __ldg(m.dguide + u * kDustGuide + b);
         if (nud[gb.x - 1] >= nu && nu > nud[gb.y]) { i0 = gb.x; i1 = gb.y + 1; }
         while (i1 - i0 > 1) {
@@ -742,11 +865,19 @@ __device__ __forceinline__ void opacset(const DevModel& m, const DustView<R>& v,
       } else {
         const float n1 = nud[i1 - 1], n0 = nud[i0 - 1];
         const float f = (nu - n1) / (n0 - n1), fm1 = 1.f - f;
-        gt[u] = fm1 * v.g[u][i1 - 1] + f * v.g[u][i0 - 1];
-        plt[u] = fm1 * v.pl[u][i1 - 1] + f * v.pl[u][i0 - 1];
-        kt[u] = fm1 * v.kap[u][i1 - 1] + f * v.kap[u][i0 - 1];
-        at[u] = fm1 * v.alb[u][i1 - 1] + f * v.alb[u][i0 - 1];
+        gt[u] = fmaf(fm1, v.g[u][i1 - 1], __fmul_rn(f, v.g[u][i0 - 1]));
+        plt[u] = fmaf(fm1, v.pl[u][i1 - 1], __fmul_rn(f, v.pl[u][i0 - 1]));
+        kt[u] = fmaf(fm1, v.kap[u][i1 - 1], __fmul_rn(f, v.kap[u][i0 - 1]));
+        at[u] = fmaf(fm1, v.alb[u][i1 - 1], __fmul_rn(f, v.alb[u][i0 - 1]));
       }
+    }
+    if (m.ntab == 1) {  // every slot reads one table
+#pragma unroll
+      for (int id = 0; id < kSlots; ++id) {
+        p.g[id] = gt[0]; p.pl[id] = plt[0]; p.albedo[id] = at[0];
+        p.kapd[id] = kt[0] * a.kapfac[id];
+      }
+      return;
     }
 #pragma unroll
     for (int id = 0; id < kSlots; ++id) {
@@ -883,9 +1014,10 @@ __device__ __forceinline__ void tally_path(const DevModel& m, const DevTallies& 
   }
 }
 
-// The same by the lanes of a warp that runs one packet: lane s < 4 tallies
-// species s, lane 4 the path, lane 5 the small grains' path -- one fixed-point
-// conversion and one atomic instruction instead of up to six.
+// The same by the lanes of a warp that runs one packet (FP64 form; the mixed
+// form's is in tauint_warp): lane s < 4 tallies species s, lane 4 the path,
+// lane 5 the small grains' path -- one fixed-point conversion and one atomic
+// instruction instead of up to six.
 template <class R>
 __device__ __forceinline__ void tally_path_warp(const DevModel& m, const DevTallies& t, const Pkt<R>& p,
                                                 const Rho<R>& rho, int64_t c, R ds, R rout) {
@@ -939,11 +1071,18 @@ __device__ __forceinline__ float safe_dist(const DevModel& m, float x, float y, 
   return fmaf(-1.0e-6f, r, d);
 }
 
+// the opacity of a cell to the packet's frequency, per unit length
+__device__ __forceinline__ float opacity(const Pkt<float>& p, const Rho<float>& rho) {
+  float opac = __fmul_rn(p.kapd[0], rho.v[0]);
+#pragma unroll
+  for (int s = 1; s < kSlots; ++s) opac = fmaf(p.kapd[s], rho.v[s], opac);
+  return opac;
+}
+
 // Mixed form of tauint: the step of one event is a Ray from the event point;
 // the walk, the tau integral and the Lucy tallies are FP32, the FP64 point
-// where the walk stops is formed once, at the end.  kWarp: a whole warp runs
-// the packet (k_tail), every lane holding the same state.
-template <bool kFused, bool kWarp>
+// where the walk stops is formed once, at the end.
+template <bool kFused>
 static __device__ __forceinline__ int tauint_mixed(const DevModel& m, const DevTallies& t, Pkt<float>& p, float tau, Local& L,
                                    Tracer& tr) {
   float tsum = 0.f;
@@ -952,16 +1091,6 @@ static __device__ __forceinline__ int tauint_mixed(const DevModel& m, const DevT
   Ray ray;
   ray_init(ray, p.x, p.y, p.z, p.ux, p.uy, p.uz);
   PathLen S{0.f, 0.f};
-  auto tally = [&](const Rho<float>& rho, int64_t c, float ds, float rout) {
-    if constexpr (kWarp) tally_path_warp<float>(m, t, p, rho, c, ds, rout);
-    else tally_path<float>(m, t, p, rho, c, ds, rout);
-  };
-  auto opacity = [&](const Rho<float>& rho) {
-    float opac = __fmul_rn(p.kapd[0], rho.v[0]);
-#pragma unroll
-    for (int s = 1; s < kSlots; ++s) opac = fmaf(p.kapd[s], rho.v[s], opac);
-    return opac;
-  };
   if (p.on_wall == 0 && p.ir >= 1 && p.ir <= m.nrg - 1 && p.it >= 1 && p.it <= m.ntg - 1) {
     // From a point inside the cell, a step shorter than the safe distance
     // ends in the cell: the interaction the walk would find, without the
@@ -969,13 +1098,13 @@ static __device__ __forceinline__ int tauint_mixed(const DevModel& m, const DevT
     // where it was formed; each such step uses up its length.
     const int64_t c = cidx(m, p.ir, p.it, p.ip);
     const Rho<float> rho = load_rho<float>(m, c);
-    const float opac = opacity(rho);
+    const float opac = opacity(p, rho);
     const float ds = tau / opac;
     if (opac > 0.f && !(ds < p.safe)) p.safe = safe_dist(m, p.x.hi, p.y.hi, p.z.hi, p.ir, p.it, p.ip);
     if (opac > 0.f && ds < p.safe) {
       p.safe = __fsub_rn(p.safe, ds);
       L.cross++;
-      tally(rho, c, ds, __ldg(m.rarrf + p.ir));
+      tally_path<float>(m, t, p, rho, c, ds, __ldg(m.rarrf + p.ir));
       path_add(S, ds);
       ray_pos(ray, S, p.x, p.y, p.z);
       tr.add(2, p.ir, p.it, p.ip, 0, (double)tau, dval(p.x), dval(p.y), dval(p.z));
@@ -1016,13 +1145,13 @@ static __device__ __forceinline__ int tauint_mixed(const DevModel& m, const DevT
       L.fault = F_NOWALL;
       return TI_FAULT;
     }
-    const float opac = opacity(rho);
+    const float opac = opacity(p, rho);
     const float tnext = fmaf(opac, dt, tsum);  // the optical depth at the wall
     const float rout = __ldg(m.rarrf + p.ir);
     L.cross++;
     const bool stop = tnext > tau;
     const float ds = stop ? (tau - tsum) / opac : dt;
-    tally(rho, c, ds, rout);
+    tally_path<float>(m, t, p, rho, c, ds, rout);
     if (stop) {
       path_add(S, ds);
       at();
@@ -1054,12 +1183,137 @@ static __device__ __forceinline__ int tauint_mixed(const DevModel& m, const DevT
   }
 }
 
+// tauint_mixed of a packet that a whole warp runs (k_tail), every lane holding
+// the same state.  rho: the density of the packet's cell, kept from one call
+// to the next, so that the next event's step starts without its load.  The
+// safe distance is formed only where it can be larger than the step: it is at
+// most half the cell's radial depth, less a margin above FP32 rounding.
+// tried: the caller has found the step to be longer than it.
+template <bool kFused>
+static __device__ __forceinline__ int tauint_warp(const DevModel& m, const DevTallies& t, Pkt<float>& p, float tau,
+                                                  Rho<float>& rho, bool tried, Local& L) {
+  const int lane = threadIdx.x & 31;
+  const int cap = 4 * (m.nrg + m.ntg + m.npg) + 64;
+  int nreloc = 0, ntiny = 0;
+  Ray ray;
+  ray_init(ray, p.x, p.y, p.z, p.ux, p.uy, p.uz);
+  PathLen S{0.f, 0.f};
+  // what this lane tallies of a step: lane s < 4 the absorbed path of species
+  // s, lane 4 the path, lane 5 the small grains' path
+  const float ps = (float)t.path_scale;
+  const float kabs = pick4(p.kapd, lane & 3) * (1.f - pick4(p.albedo, lane & 3));
+  const float ksg = m.sg_on ? pick4(p.kapd, m.sg_slot) * (1.f - pick4(p.albedo, m.sg_slot)) * m.sg_jfac : 0.f;
+  unsigned long long* const base = lane < 4 ? t.dtauabs + (int64_t)lane * m.ncell : (lane == 4 ? t.jmean : t.jsg);
+  auto tally = [&](int64_t c, float ds, float rout) {
+    const float r = pick4(rho.v, lane & 3);
+    float q = ds / rout;
+    if (m.sg_on && lane == 5) q = ds * ksg / rout;
+    const float v = lane < 4 ? kabs * r * ds : q;
+    if (lane < 4 ? r > 0.f : (lane == 4 || (lane == 5 && m.sg_on))) atomicAdd(base + c, fxf(v, ps));
+  };
+  int64_t c = cidx(m, p.ir, p.it, p.ip);
+  if (!tried && p.on_wall == 0 && p.ir >= 1 && p.ir <= m.nrg - 1 && p.it >= 1 && p.it <= m.ntg - 1) {
+    const float opac = opacity(p, rho);
+    const float ds = tau / opac;
+    const float rin = __ldg(m.rarrf + p.ir - 1), rout = __ldg(m.rarrf + p.ir);
+    if (opac > 0.f && ds < 0.5f * (rout - rin)) {
+      if (!(ds < p.safe)) p.safe = safe_dist(m, p.x.hi, p.y.hi, p.z.hi, p.ir, p.it, p.ip);
+      if (ds < p.safe) {
+        p.safe = __fsub_rn(p.safe, ds);
+        L.cross++;
+        tally(c, ds, rout);
+        path_add(S, ds);
+        ray_pos(ray, S, p.x, p.y, p.z);
+        return TI_INTERACT;
+      }
+    }
+  }
+  p.safe = 0.f;
+  float tsum = 0.f;
+  auto at = [&]() { ray_pos(ray, S, p.x, p.y, p.z); };
+  auto reloc = [&]() {
+    double x, y, z;
+    ray_at(ray, S, x, y, z);
+    int jr = p.ir, jt = p.it, jp = p.ip;
+    const int where = relocate(m, x, y, z, jr, jt, jp);
+    p.ir = jr; p.it = jt; p.ip = jp;
+    c = cidx(m, p.ir, p.it, p.ip);
+    if (where == 0) rho = load_rho<float>(m, c);
+    return where;
+  };
+  for (int n = 0;; ++n) {
+    if (n > cap || p.it < 1 || p.it > m.ntg - 1 || p.ir < 1 || p.ir > m.nrg - 1) {
+      L.fault = n > cap ? F_CAP : F_RANGE;
+      at();
+      return TI_FAULT;
+    }
+    float dt;
+    int iface;
+    if (!next_wall_warp<kFused>(m, ray, S, p.ir, p.it, p.ip, p.on_wall, dt, iface)) {
+      at();
+      if (nreloc < 4) {
+        ++nreloc;
+        const int where = reloc();
+        if (where == 1) { p.ir = m.nrg; return TI_ESCAPE; }
+        if (where == 2) { p.ir = 0; return TI_STAR; }
+        p.on_wall = 0;
+        continue;
+      }
+      L.fault = F_NOWALL;
+      return TI_FAULT;
+    }
+    const float opac = opacity(p, rho);
+    const float tnext = fmaf(opac, dt, tsum);  // the optical depth at the wall
+    const float rout = __ldg(m.rarrf + p.ir);
+    L.cross++;
+    const bool stop = tnext > tau;
+    float ds = dt;
+    if (stop) ds = (tau - tsum) / opac;
+    if (stop) {
+      tally(c, ds, rout);
+      path_add(S, ds);
+      at();
+      p.on_wall = 0;
+      return TI_INTERACT;
+    }
+    const int64_t c0 = c;
+    tsum = tnext;
+    step_index(m.npg, iface, p.ir, p.it, p.ip);
+    // the next cell's density, loaded before the tally of this one
+    Rho<float> next = rho;
+    if (p.ir >= 1 && p.ir <= m.nrg - 1 && p.it >= 1 && p.it <= m.ntg - 1) {
+      c = cidx(m, p.ir, p.it, p.ip);
+      next = load_rho<float>(m, c);
+    }
+    tally(c0, ds, rout);
+    rho = next;
+    path_add(S, dt);
+    p.on_wall = 1 << own_after(iface);
+    if (p.ir == m.nrg) { at(); return TI_ESCAPE; }
+    if (p.ir == 0) { at(); return TI_STAR; }
+    if (!tiny_step(m, dt, p.ir)) {
+      ntiny = 0;
+    } else if (++ntiny > 6 && nreloc < 4) {
+      ++nreloc;
+      ntiny = 0;
+      at();
+      const int where = reloc();
+      if (where == 1) { p.ir = m.nrg; return TI_ESCAPE; }
+      if (where == 2) { p.ir = 0; return TI_STAR; }
+      p.on_wall = 0;
+    }
+  }
+}
+
 // tauint in either form: the FP64 form walks with the reference's wall
 // machinery (closest_wall rule), the mixed form with tauint_mixed.
+// kWarp: a whole warp runs the packet; rho is then the density of its cell.
 template <class R, bool kFused, bool kWarp>
-__device__ __forceinline__ int tauint(const DevModel& m, const DevTallies& t, Pkt<R>& p, R tau, Local& L, Tracer& tr) {
+__device__ __forceinline__ int tauint(const DevModel& m, const DevTallies& t, Pkt<R>& p, R tau, Rho<R>& rho_, bool tried,
+                                      Local& L, Tracer& tr) {
   if constexpr (sizeof(R) == 4) {
-    return tauint_mixed<kFused, kWarp>(m, t, p, tau, L, tr);
+    if constexpr (kWarp) return tauint_warp<kFused>(m, t, p, tau, rho_, tried, L);
+    else return tauint_mixed<kFused>(m, t, p, tau, L, tr);
   } else {
     R tsum = R(0);
     const int cap = 4 * (m.nrg + m.ntg + m.npg) + 64;
@@ -1113,9 +1367,20 @@ __device__ __forceinline__ int tauint(const DevModel& m, const DevTallies& t, Pk
 
 // ---- select_dust.f90:16-42 ---------------------------------------------------
 template <class R, class G>
-__device__ __forceinline__ int select_dust(const DevModel& m, const Pkt<R>& p, G& rng) {
+__device__ __forceinline__ int select_dust(const DevModel& m, const Pkt<R>& p, const Rho<R>& rho_, G& rng) {
   const R xran = ran<R>(rng);
-  const Rho<R> rho = load_rho<R>(m, cidx(m, p.ir, p.it, p.ip));
+  Rho<R> rho;
+  if constexpr (KnowsRho<G>::value && sizeof(R) == 4) {
+    rho = rho_;
+    // one species with opacity takes every draw (the draw past the rounded
+    // sum of the fractions too, see below)
+    unsigned some = 0u;
+#pragma unroll
+    for (int s = 0; s < kSlots; ++s) some |= p.kapd[s] * rho.v[s] > 0.f ? 1u << s : 0u;
+    if (some != 0u && (some & (some - 1u)) == 0u) return __ffs(some) - 1;
+  } else {
+    rho = load_rho<R>(m, cidx(m, p.ir, p.it, p.ip));
+  }
   R opac = R(0), frac = R(0);
 #pragma unroll
   for (int s = 0; s < kSlots; ++s) opac += p.kapd[s] * rho.v[s];
@@ -1386,17 +1651,22 @@ __device__ __forceinline__ int nu_bin(const RunArgs& a, R nub) {
 }
 
 template <class R>
-__device__ __forceinline__ void make_rec(PeelRec<R>& e, const Pkt<R>& p, const RunArgs& a, int iflag, int idust2,
-                                         int extra = 0) {
+__device__ __forceinline__ void make_rec(PeelRec<R>& e, const Pkt<R>& p, int inub, int iflag, int idust2, int extra) {
   e.x = p.x; e.y = p.y; e.z = p.z;
   e.ir = p.ir; e.it = p.it; e.ip = p.ip;
   e.flags = (p.on_wall ? 1 : 0) | (iflag << 1) | (p.i_orig << 2) | (idust2 << 5) | (p.on_wall << 8) | extra;
-  e.inub = nu_bin<R>(a, p.nub);
+  e.inub = inub;
   e.sip = p.sip; e.sqp = p.sqp; e.sup = p.sup; e.svp = p.svp;
   e.d0 = p.cost; e.d1 = p.sint; e.d2 = p.phi; e.d3 = p.cosp; e.d4 = p.sinp;
   e.g = pick4(p.g, idust2); e.pl = pick4(p.pl, idust2);
 #pragma unroll
   for (int s = 0; s < kSlots; ++s) e.kapd[s] = p.kapd[s];
+}
+
+template <class R>
+__device__ __forceinline__ void make_rec(PeelRec<R>& e, const Pkt<R>& p, const RunArgs& a, int iflag, int idust2,
+                                         int extra = 0) {
+  make_rec<R>(e, p, nu_bin<R>(a, p.nub), iflag, idust2, extra);
 }
 
 __device__ __forceinline__ void add9(unsigned long long* base, int64_t stride, int64_t b, double i, double q, double u,
@@ -1935,82 +2205,78 @@ __device__ __forceinline__ void peel_all(const DevModel& m, const DevTallies& t,
 
 // ---- lucydustfreq.f90:19-157 -------------------------------------------------------------
 // Mixed form.  The row pair j, j+1 of the Lucy CDF and the weight f follow
-// from the cell temperature, which is fixed during a run: they are cached in
-// the packet while it stays in the cell and species slot.  The frequency
+// from the cell temperature, which is fixed during a run: they are formed
+// once per temperature update (lucy_row) and read here, 8 bytes.  The frequency
 // index is the same bracket of the interpolated CDF as the reference's
 // bisection (the CDF is non-decreasing, so the bracket is unique), found
-// from the guide table and a short bisection over the interleaved rows.
+// from the guide table and a short bisection over the interleaved rows; a
+// warp that runs one packet reads the guide's whole bracket at once.
 template <class G>
-__device__ __forceinline__ float lucy_freq_mixed(const DevModel& m, LucyRow& lr, int64_t c, int id, G& rng) {
-  const int nT = m.nT, nnu = m.nnu;
+__device__ __forceinline__ float lucy_freq_mixed(const DevModel& m, int64_t c, int id, G& rng) {
+  const int nnu = m.nnu;
   const float* nuint = m.nuintf;
-  const int key = (int)(4 * c + id);
-  if (key != lr.key) {
-    const float T0 = __ldg(m.tdustf + 4 * c + id);
-    const float* lTint = m.lTintf;
-    const float lT0 = logf(T0);
-    const float l1 = __ldg(lTint), lN = __ldg(lTint + nT - 1);
-    int j = (int)((float)(nT - 1) * (lT0 - l1) / (lN - l1)) + 1;
-    j = j < 1 ? 1 : (j > nT - 1 ? nT - 1 : j);
-    float f = (lT0 - __ldg(lTint + j - 1)) / (__ldg(lTint + j) - __ldg(lTint + j - 1));
-    f = f < 0.f ? 0.f : (f > 1.f ? 1.f : f);
-    const int pr = id * (nT - 1) + (j - 1);
-    const float2 k1 = __ldg(m.kpairf + (size_t)pr * nnu), kn = __ldg(m.kpairf + (size_t)pr * nnu + nnu - 1);
-    lr.key = key;
-    lr.pr = pr;
-    lr.T0 = T0;
-    lr.f = f;
-    lr.P0 = fminf((1.f - f) * k1.x + f * k1.y, 1.f);
-    lr.P1 = fminf((1.f - f) * kn.x + f * kn.y, 1.f);
-  }
-  const float T0 = lr.T0, f = lr.f;
+  const float T0 = __ldg(m.tdustf + 4 * c + id);
+  const int2 row = __ldg(m.lucyrow + 4 * c + id);
+  const float f = __int_as_float(row.x);
+  const int pr = row.y;
+  const float2* KP = m.kpairf + (size_t)pr * nnu;
+  auto P = [&](int i) {
+    const float2 k = __ldg(KP + i - 1);
+    return fminf(fmaf(1.f - f, k.x, __fmul_rn(f, k.y)), 1.f);
+  };
   const float xi = ran<float>(rng);
-  float P0 = lr.P0, P1 = lr.P1;
+  const short2 g = __ldg(m.kguide + (size_t)pr * kGuide + min((int)(xi * (float)kGuide), kGuide - 1));
+  const float Pf = P(1), Pl = P(nnu);
+  float P0 = Pf, P1 = Pl;
   if (xi < P0) return P0 > 0.f ? T0 * xi * __ldg(nuint) / P0 : T0 * __ldg(nuint);
   if (xi >= P1) {
     if (P1 < 1.f && xi < 1.f) return T0 * __ldg(nuint + nnu - 1) * (1.f - P1) / (1.f - xi);
     return T0 * __ldg(nuint + nnu - 1);
   }
-  const float2* KP = m.kpairf + (size_t)lr.pr * nnu;
-  auto P = [&](int i) { return fminf((1.f - f) * __ldg(KP + i - 1).x + f * __ldg(KP + i - 1).y, 1.f); };
-  const short2 g = __ldg(m.kguide + (size_t)lr.pr * kGuide + min((int)(xi * (float)kGuide), kGuide - 1));
   int i0 = g.x, i1 = g.y;
   bool found = false;
+  float2 nn;  // the frequency of row i0 and its ratio to the next
   if constexpr (IsWarp<G>::value) {
-    // the guide's bracket in one step: lane j has P(i0 + j); the CDF does not
-    // decrease, so the last value <= xi and the first > xi are neighbours
-    const int j = threadIdx.x & 31;
-    const float v = P(min(i0 + j, i1));
+    // lane j has P(i0 + j); the CDF does not decrease, so the last value <= xi
+    // and the first > xi are neighbours
+    const int i = min(i0 + (int)(threadIdx.x & 31), i1);
+    const float v = P(i);
+    const float2 nv = __ldg(m.nuratio + i - 1);
     const unsigned above = __ballot_sync(0xffffffffu, v > xi);
     if (above != 0u && (above & 1u) == 0u) {
       const int w1 = __ffs(above) - 1;
-      i1 = min(i0 + w1, i1);
-      i0 += w1 - 1;
       P0 = __shfl_sync(0xffffffffu, v, w1 - 1);
       P1 = __shfl_sync(0xffffffffu, v, w1);
+      nn.x = __shfl_sync(0xffffffffu, nv.x, w1 - 1);
+      nn.y = __shfl_sync(0xffffffffu, nv.y, w1 - 1);
       found = true;
     }
   }
   if (!found) {
-  const float Pa = P(i0), Pb = P(i1);
-  if (Pa <= xi) P0 = Pa; else i0 = 1;
-  if (Pb > xi) P1 = Pb; else i1 = nnu;
-  if (i1 <= i0) { i0 = 1; i1 = nnu; P0 = lr.P0; P1 = lr.P1; }
-  while (i1 - i0 > 1) {
-    const int i = (i0 + i1) / 2;
-    const float v = P(i);
-    if (v > xi) { i1 = i; P1 = v; }
-    else { i0 = i; P0 = v; }
-  }
+    const float Pa = P(i0), Pb = P(i1);
+    if (Pa <= xi) P0 = Pa; else i0 = 1;
+    if (Pb > xi) P1 = Pb; else i1 = nnu;
+    if (i1 <= i0) { i0 = 1; i1 = nnu; P0 = Pf; P1 = Pl; }
+    while (i1 - i0 > 1) {
+      const int i = (i0 + i1) / 2;
+      const float v = P(i);
+      if (v > xi) { i1 = i; P1 = v; }
+      else { i0 = i; P0 = v; }
+    }
+    nn = __ldg(m.nuratio + i0 - 1);
   }
   float w;
   if (xi < P0) w = 0.f;
   else if (xi > P1) w = 1.f;
   else if (P0 <= 0.f) w = 0.5f;
   else if (P1 <= 0.f || xi <= 0.f) w = f;
-  else w = logf(xi / P0) / logf(P1 / P0);
-  const float n0 = __ldg(nuint + i0 - 1), n1 = __ldg(nuint + i1 - 1);
-  return T0 * n0 * powf(n1 / n0, w);
+  else if constexpr (IsWarp<G>::value) {
+    const float l = logf(((threadIdx.x & 31) == 0 ? xi : P1) / P0);  // lane 0 the numerator, the others the denominator
+    w = __shfl_sync(0xffffffffu, l, 0) / __shfl_sync(0xffffffffu, l, 1);
+  } else {
+    w = logf(xi / P0) / logf(P1 / P0);
+  }
+  return T0 * nn.x * powf(nn.y, w);
 }
 
 // FP64 form: the reference's bisection.
@@ -2291,7 +2557,6 @@ __device__ bool emit_star(const DevModel& m, const DustView<R>& dv, const RunArg
                           PeelRec<R>& rec, Tracer& tr, int spotph) {
   p.on_wall = 0;
   p.safe = 0.f;
-  p.lrow.key = -1;
   p.sip = R(1); p.sqp = R(0); p.sup = R(0); p.svp = R(0);
   const bool spots = a.src_on && a.src.ispot;
   for (int tries = 0;; ++tries) {
@@ -2337,7 +2602,7 @@ __device__ bool emit_star(const DevModel& m, const DustView<R>& dv, const RunArg
     p.nub = atmosfreq<R>(m, rng);
   }
   p.i_orig = 1;
-  opacset<R>(m, dv, p, p.nub, a);
+  opacset<R, false>(m, dv, p, p.nub, a);
   const R coslp = xcos(p.lp), sinlp = xsin(p.lp);
   const double rp_ = (double)p.sinb;
   set_pos(p.z, (double)p.cosb);
@@ -2382,7 +2647,6 @@ __device__ void emit_external(const DevModel& m, const DustView<R>& dv, const Ru
                               PeelRec<R>& rec, Tracer& tr) {
   p.on_wall = 0;
   p.safe = 0.f;
-  p.lrow.key = -1;
   p.sip = R(1); p.sqp = R(0); p.sup = R(0); p.svp = R(0);
   p.cosb = R(1) - R(2) * ran<R>(rng);
   p.sinb = xsqrt(R(1) - p.cosb * p.cosb);
@@ -2395,7 +2659,7 @@ __device__ void emit_external(const DevModel& m, const DustView<R>& dv, const Ru
   initp_transform<R>(p);
   p.nub = rep_isrf<R>(m, rng);
   p.i_orig = 4;
-  opacset<R>(m, dv, p, p.nub, a);
+  opacset<R, false>(m, dv, p, p.nub, a);
   const R coslp = xcos(p.lp), sinlp = xsin(p.lp);
   const double zp = (double)p.cosb * a.rmax * 0.999999, rp_ = (double)p.sinb * a.rmax * 0.999999;
   set_pos(p.z, zp);
@@ -2460,7 +2724,6 @@ __device__ __forceinline__ bool emit_acc(const DevModel& m, const DustView<R>& d
   const hc3d_sources& S = a.src;
   p.on_wall = 0;
   p.safe = 0.f;
-  p.lrow.key = -1;
   Gauss g{0, 0.0};
   double rp, xp, yp, zp;
   int tries = 0;
@@ -2534,7 +2797,7 @@ __device__ __forceinline__ bool emit_acc(const DevModel& m, const DustView<R>& d
     p.phi = (R)kR2p * ran<R>(rng);
     p.cosp = xcos(p.phi);
     p.sinp = xsin(p.phi);
-    if constexpr (sizeof(R) == 4) p.nub = lucy_freq_mixed(m, p.lrow, c, idust2, rng);
+    if constexpr (sizeof(R) == 4) p.nub = lucy_freq_mixed(m, c, idust2, rng);
     else p.nub = lucydustfreq<R>(m, __ldg(m.tdust + 4 * c + idust2), idust2, rng);
   } else {
     // gas at the accretion disk temperature (Pringle 1981, eq. 3.23)
@@ -2549,7 +2812,7 @@ __device__ __forceinline__ bool emit_acc(const DevModel& m, const DustView<R>& d
   }
   p.ux = p.sint * p.cosp; p.uy = p.sint * p.sinp; p.uz = p.cost;
   p.i_orig = 2;
-  opacset<R>(m, dv, p, p.nub, a);
+  opacset<R, false>(m, dv, p, p.nub, a);
   tr.add(0, p.ir, p.it, p.ip, 0, 0.0, dval(p.x), dval(p.y), dval(p.z));
   make_rec<R>(rec, p, a, 0, idust2 < 0 ? 0 : idust2);
   return true;
@@ -2582,14 +2845,15 @@ __device__ __forceinline__ bool emit(const DevModel& m, const DustView<R>& dv, c
 // G: the packet's draws, one lane's (Rng) or a warp's (WarpRng, k_tail).
 template <class R, bool kFused, class G>
 __device__ __forceinline__ int walk(const DevModel& m, const DevTallies& t, const TallyDims& d, const RunArgs& a, Pkt<R>& p, G& rng,
-                    Flow<R>& f, Local& L, Tracer& tr, bool first) {
+                    Flow<R>& f, Rho<R>& rho, Local& L, Tracer& tr, bool first,
+                    bool tried = false) {
   const R tau = neg_log<R>(rng);
   if (!first) {
     f.xpold = p.x; f.ypold = p.y; f.zpold = p.z;
     p.ux = p.sint * p.cosp; p.uy = p.sint * p.sinp; p.uz = p.cost;
   }
   const int pir = p.ir, pit = p.it, pip = p.ip;
-  const int st = tauint<R, kFused, IsWarp<G>::value>(m, t, p, tau, L, tr);
+  const int st = tauint<R, kFused, IsWarp<G>::value>(m, t, p, tau, rho, tried, L, tr);
   if (st == TI_ESCAPE) {
     tr.add(3, p.ir, p.it, p.ip, 0, 0.0, dval(p.x), dval(p.y), dval(p.z));
     if (L.on) bin_escape<R>(t, d, a, p, dval(f.xpold), dval(f.ypold), dval(f.zpold), f.iflag, f.iscat, L);
@@ -2617,7 +2881,7 @@ __device__ __forceinline__ int walk(const DevModel& m, const DevTallies& t, cons
       return ST_DONE;
     }
   }
-  f.idust2 = select_dust<R>(m, p, rng);
+  f.idust2 = select_dust<R>(m, p, rho, rng);
   if (f.idust2 < 0) {
     L.add(HC3D_CNT_STUCK);
     if (L.on) {
@@ -2640,15 +2904,18 @@ __device__ __forceinline__ int walk(const DevModel& m, const DevTallies& t, cons
 // (about 2^-23 |x|), the walk would end every ray at its first wall: no
 // record is made and no ray is walked.  The tallies are unchanged; the
 // peel-off ray and crossing counters count only the rays walked.
+__device__ __forceinline__ float peel_opacity(const DevModel& m, const Pkt<float>& p, int64_t c) {
+  const float4 q = __ldg(m.rho4p + c);
+  return fmaf(p.kapd[0], q.x, fmaf(p.kapd[1], q.y, fmaf(p.kapd[2], q.z, __fmul_rn(p.kapd[3], q.w))));
+}
+__device__ __forceinline__ bool deep_peel_at(const Pkt<float>& p, float safe, float op) {
+  const float r = fabsf(p.x.hi) + fabsf(p.y.hi) + fabsf(p.z.hi);
+  return safe * op > 1.01f * (float)kTauMax && safe > r * 1.220703125e-4f;
+}
 template <class R>
 __device__ __forceinline__ bool deep_peel(const DevModel& m, const Pkt<R>& p, int64_t c) {
   if constexpr (sizeof(R) == 4) {
-    if (p.safe > 0.f) {
-      const float4 q = __ldg(m.rho4p + c);
-      const float op = fmaf(p.kapd[0], q.x, fmaf(p.kapd[1], q.y, fmaf(p.kapd[2], q.z, p.kapd[3] * q.w)));
-      const float r = fabsf(p.x.hi) + fabsf(p.y.hi) + fabsf(p.z.hi);
-      return p.safe * op > 1.01f * (float)kTauMax && p.safe > r * 1.220703125e-4f;
-    }
+    if (p.safe > 0.f) return deep_peel_at(p, p.safe, peel_opacity(m, p, c));
   }
   return false;
 }
@@ -2691,11 +2958,11 @@ __device__ __forceinline__ bool interact(const DevModel& m, const DustView<R>& d
     draw_mu<R>(rng, p.cost, p.sint);
     draw_phi<R>(rng, p.phi, p.cosp, p.sinp);
     if (!sg) {
-      if constexpr (sizeof(R) == 4) p.nub = lucy_freq_mixed(m, p.lrow, c, idust2, rng);
+      if constexpr (sizeof(R) == 4) p.nub = lucy_freq_mixed(m, c, idust2, rng);
       else p.nub = lucydustfreq<R>(m, tave, idust2, rng);
     }
     f.iflag = 0;
-    opacset<R>(m, dv, p, p.nub, a);
+    opacset<R, IsWarp<G>::value>(m, dv, p, p.nub, a);
     keep = a.ipeel == 1 && !deep_peel<R>(m, p, c);
     if (keep && L.on) make_rec<R>(rec, p, a, 0, idust2);
     f.iint++;
@@ -2724,10 +2991,11 @@ __device__ void run_packet(const DevModel& m, const DustView<R>& dv, const DevTa
   Flow<R> f;
   f.xpold = p.x; f.ypold = p.y; f.zpold = p.z;
   f.iflag = 0; f.iscat = 0; f.iint = 0; f.idust2 = 0; f.ntot = 0;
-  int st = walk<R, kFused>(m, t, d, a, p, rng, f, L, tr, true);
+  Rho<R> rho;
+  int st = walk<R, kFused>(m, t, d, a, p, rng, f, rho, L, tr, true);
   while (st == ST_INTERACT) {
     if (interact<R>(m, dv, t, a, p, rng, f, L, tr, rec)) peel_all<R>(m, t, d, a, rec, L);
-    st = walk<R, kFused>(m, t, d, a, p, rng, f, L, tr, false);
+    st = walk<R, kFused>(m, t, d, a, p, rng, f, rho, L, tr, false);
   }
 }
 
@@ -2909,7 +3177,8 @@ __global__ void __launch_bounds__(128, 3) k_wave(DevModel m, DevTallies t, Tally
         ++slot;  // the slot is kept only when the event made a record
       }
       if (emitted) {
-        const int st = walk<R, kPeel>(m, t, d, a, s.p, rng, s.f, L, tr, s.stage == 2);
+        Rho<R> rho;
+        const int st = walk<R, kPeel>(m, t, d, a, s.p, rng, s.f, rho, L, tr, s.stage == 2);
         s.stage = st == ST_INTERACT ? 1 : 0;
         if (!kPeel && s.stage == 0) L.settle();
       }
@@ -2928,15 +3197,177 @@ __global__ void __launch_bounds__(128, 3) k_wave(DevModel m, DevTallies t, Tally
   flush(t, L);
 }
 
-// The packets that k_wave left, one per warp: every lane holds the packet and
-// runs its events, and the parts of an event that a lane alone would do one
-// after another are shared between the lanes -- the draws and their
-// logarithms, sines and cosines (DrawTable), the tries of the scattering
-// angle (scat_draw), the search of the Lucy CDF (lucy_freq_mixed) and the
-// tallies of a step (tally_path_warp).  What bounds it is the latency of one
-// packet's chain of events: 3.4 us an event in the plain model's disk against
-// 5.0 us for a lane of k_wave, and no other lane of the warp runs beside it.
-// The arithmetic is that of k_wave, bit for bit.
+// Up to kAhead events of one packet side by side in the lanes of its warp.
+//
+// An absorption re-emits the packet with a frequency drawn from the cell's
+// temperature, in an isotropic direction: what it leaves depends on its draws
+// and on the cell, and not on the packet that was absorbed.  In an optically
+// thick cell most events are absorptions that end in the cell (safe steps), so
+// their frequencies, opacities, directions and step lengths are formed at once:
+// lane k takes the k-th event from here, on the draws it has if all before it
+// are absorptions (six each: albedo, mu, phi, frequency, tau, species).  The
+// chain holds as far as the albedo draw of each event absorbs it, by the
+// albedo its predecessor left, and the species it assumed is the one its
+// predecessor's last draw selects.  What depends on the packet's way -- the
+// position, and whether a step is safe -- is then followed event by event, in
+// the order and rounding of the walk, and the events up to the first one that
+// needs the wall search are tallied by their lanes.  That one (`wall`) is left
+// re-emitted, for the caller to walk; a scattering is left to interact().
+//
+// One event after another took 5700 cycles each, nearly all of them in the
+// part that the lanes share here.
+constexpr int kAhead = 16;
+
+struct Batch {
+  int n;      // events done, walked and tallied
+  bool wall;  // and one more absorbed and re-emitted, to be walked
+  bool far;   // whose step is longer than the safe distance
+};
+
+template <bool kPeel>
+__device__ __forceinline__ Batch tail_batch(const DevModel& m, const DustView<float>& dv, const DevTallies& t,
+                                            const RunArgs& a, Pkt<float>& p, WarpRng<float>& rng, Flow<float>& f,
+                                            const Rho<float>& rho, Local& L, PeelRec<float>* queue,
+                                            unsigned long long* qcount, unsigned long long& slot,
+                                            unsigned long long& slot_end, int most) {
+  Batch b{0, false, false};
+  const int lane = threadIdx.x & 31;
+  const int64_t c = cidx(m, p.ir, p.it, p.ip);
+  const int at = rng.at + 6 * min(lane, kAhead - 1);
+  const float* u = rng.t->u + at;
+  // the species each event is assumed to meet: the pending one's is known,
+  // the later ones' as the packet's present opacities select it
+  OneDraw d{u[lane == 0 ? 0 : -1]};
+  int s = select_dust<float>(m, p, rho, d);
+  if (lane == 0) s = f.idust2;
+  const bool thermal = s >= 0 && !((m.sg_mask >> s) & 1u);
+  // lane 0: is the pending event an absorption at all?
+  if (__shfl_sync(0xffffffffu, (int)(thermal && u[0] > pick4(p.albedo, f.idust2)), 0) == 0) return b;
+  if (!thermal) s = f.idust2;
+  Pkt<float> q;
+  q.cost = 1.f - 2.f * u[1];
+  q.sint = xsqrt(1.f - q.cost * q.cost);
+  q.phi = (float)kR2p * u[2];
+  q.cosp = xcos(q.phi);
+  q.sinp = xsin(q.phi);
+  d.u = u[3];
+  q.nub = lucy_freq_mixed(m, c, s, d);
+  opacset<float, false>(m, dv, q, q.nub, a);
+  q.ux = q.sint * q.cosp; q.uy = q.sint * q.sinp; q.uz = q.cost;
+  const float opac = opacity(q, rho);
+  const float rin = __ldg(m.rarrf + p.ir - 1), rout = __ldg(m.rarrf + p.ir);
+  constexpr float kLong = 3.402823466e38f;  // a step that needs the wall search
+  float ds = -xlog(u[4]) / opac;
+  if (!(opac > 0.f && ds < 0.5f * (rout - rin))) ds = kLong;
+  d.u = u[5];
+  const int sel = select_dust<float>(m, q, rho, d);
+  const float alb = pick4(q.albedo, max(sel, 0));
+  // how far the chain holds
+  const float alb_before = __shfl_up_sync(0xffffffffu, alb, 1);
+  const int sel_before = __shfl_up_sync(0xffffffffu, sel, 1);
+  const bool holds = lane < kAhead && thermal && (lane == 0 || (sel_before == s && u[0] > alb_before));
+  const unsigned broken = __ballot_sync(0xffffffffu, !holds);
+  int chain = __ffs(broken) - 1;
+  int last = min(chain, most);
+  // a packet that reaches a cap is killed in walk()
+  last = min(last, a.iintmax - f.iint);
+  if (a.max_interactions > 0) last = (int)min((int64_t)last, a.max_interactions - f.ntot - 1);
+  last = max(last, 0);
+  float op = 0.f;
+  int inub = 0;
+  if constexpr (kPeel) {
+    op = peel_opacity(m, q, c);
+    inub = nu_bin<float>(a, q.nub);
+    q.sip = 1.f; q.sqp = q.sup = q.svp = 0.f;
+    q.ir = p.ir; q.it = p.it; q.ip = p.ip;
+    q.on_wall = 0;
+    q.i_orig = ((m.disk_mask >> s) & 1u) ? 2 : 3;
+  }
+  // the way, event by event
+  auto record = [&](int k) {  // the peel-off record of event k, unless its rays end in the cell
+    if constexpr (kPeel) {
+      const float opk = __shfl_sync(0xffffffffu, op, k);
+      if (p.safe > 0.f && deep_peel_at(p, p.safe, opk)) return;
+      if (slot == slot_end) {
+        if (lane == 0) slot = atomicAdd(qcount, (unsigned long long)a.qchunk);
+        slot = __shfl_sync(0xffffffffu, slot, 0);
+        slot_end = slot + (unsigned long long)a.qchunk;
+      }
+      if (lane == k) {
+        q.x = p.x; q.y = p.y; q.z = p.z;
+        make_rec<float>(queue[slot], q, inub, 0, s, 0);
+      }
+      ++slot;
+    }
+  };
+  const int on_wall = p.on_wall;
+  int k = 0;
+  bool far = on_wall != 0;  // (a pending event is never on a wall)
+  for (; k < last && !far; ++k) {
+    const float dsk = __shfl_sync(0xffffffffu, ds, k);
+    const float ux = __shfl_sync(0xffffffffu, q.ux, k), uy = __shfl_sync(0xffffffffu, q.uy, k),
+                uz = __shfl_sync(0xffffffffu, q.uz, k);
+    record(k);
+    if (!(dsk < p.safe)) {
+      if (dsk < kLong) p.safe = safe_dist(m, p.x.hi, p.y.hi, p.z.hi, p.ir, p.it, p.ip);
+      if (!(dsk < p.safe)) {
+        far = true;
+        break;
+      }
+    }
+    p.safe = __fsub_rn(p.safe, dsk);
+    const PathLen S{dsk, 0.f};
+    p.x = pos_step(p.x, S, ux);
+    p.y = pos_step(p.y, S, uy);
+    p.z = pos_step(p.z, S, uz);
+  }
+  b.n = k;
+  b.far = far;
+  b.wall = far || (k < chain && k < most);  // stopped by a long step or by a cap
+  if (b.wall && !far) record(k);
+  const int done = b.n + (b.wall ? 1 : 0);
+  if (done == 0) return b;
+  // the tallies of each event by its lane
+  if (lane < done) {
+    atomicAdd(t.dbig + c, 1u);
+    atomicAdd(t.nabs + (int64_t)s * m.ncell + c, 1ull);
+  }
+  if (lane < b.n) tally_path<float>(m, t, q, rho, c, ds, rout);
+  L.events += done;
+  L.cross += b.n;
+  f.ntot += done;
+  f.iint += done;
+  f.iflag = 0;
+  rng.at += 6 * b.n + (b.wall ? 4 : 0);
+  // the packet as its last event left it
+  const int l = done - 1;
+  p.i_orig = ((m.disk_mask >> __shfl_sync(0xffffffffu, s, l)) & 1u) ? 2 : 3;
+  p.sip = 1.f; p.sqp = p.sup = p.svp = 0.f;
+  auto from = [&](float v) { return __shfl_sync(0xffffffffu, v, l); };
+  p.cost = from(q.cost); p.sint = from(q.sint); p.phi = from(q.phi);
+  p.cosp = from(q.cosp); p.sinp = from(q.sinp); p.nub = from(q.nub);
+#pragma unroll
+  for (int j = 0; j < kSlots; ++j) {
+    p.kapd[j] = from(q.kapd[j]);
+    p.albedo[j] = from(q.albedo[j]);
+    p.g[j] = from(q.g[j]);
+    p.pl[j] = from(q.pl[j]);
+  }
+  if (!b.wall) f.idust2 = __shfl_sync(0xffffffffu, sel, l);
+  return b;
+}
+
+// The packets that k_wave left, one per warp: every lane holds the packet, and
+// the parts of its events that a lane alone would do one after another are
+// shared between the lanes.  The mixed form runs absorptions up to sixteen at
+// once (tail_batch), the tries of a scattering angle ten at once (scat_draw),
+// the walls of a cell side by side (next_wall_warp) and the tallies of a step
+// in one instruction (tauint_warp); the FP64 form reads its logarithms, sines
+// and cosines from a table 32 lanes formed (DrawTable) and shares the tries
+// and the tallies.  What bounds it is the latency of one packet's chain of
+// events: in the plain model's disk 5.0 us an event for a lane of k_wave, 3.0
+// us here with one event after another, 1.2 us with the absorptions side by
+// side.  The arithmetic is that of k_wave, bit for bit.
 template <class R, bool kPeel>
 __global__ void __launch_bounds__(128, 4) k_tail(DevModel m, DevTallies t, TallyDims d, RunArgs a, Slot<R>* pool,
                                                  const unsigned int* nlive, const unsigned int* live,
@@ -2962,18 +3393,32 @@ __global__ void __launch_bounds__(128, 4) k_tail(DevModel m, DevTallies t, Tally
     Slot<R> s = pool[gid];
     WarpRng<R> rng;
     rng_init(rng, draws + (threadIdx.x >> 5), a.key0, a.key1, s.pid, s.c0, s.left);
+    Rho<R> rho = load_rho<R>(m, cidx(m, s.p.ir, s.p.it, s.p.ip));
     unsigned long long slot = 0ull, slot_end = 0ull;
-    for (int nrec = 0; !kPeel || nrec < E; ++nrec) {
-      ensure(rng, 8);  // an event draws at most 7 beside the tries of a scattering
-      PeelRec<R> none;
-      if (kPeel && slot == slot_end) {
-        if (lane == 0) slot = atomicAdd(qcount, (unsigned long long)a.qchunk);
-        slot = __shfl_sync(0xffffffffu, slot, 0);
-        slot_end = slot + (unsigned long long)a.qchunk;
+    for (int nrec = 0; !kPeel || nrec < E;) {
+      bool tried = false, pending = true;
+      if constexpr (sizeof(R) == 4) {
+        ensure(rng, 6 * kAhead);
+        const Batch b = tail_batch<kPeel>(m, dv, t, a, s.p, rng, s.f, rho, L, queue, qcount, slot, slot_end,
+                                          kPeel ? E - nrec : kAhead);
+        nrec += b.n + (b.wall ? 1 : 0);
+        if (b.n > 0 && !b.wall) continue;
+        tried = b.far;
+        pending = !b.wall;
       }
-      if (interact<R>(m, dv, t, a, s.p, rng, s.f, L, tr, kPeel ? queue[slot] : none)) ++slot;
+      if (pending) {
+        ensure(rng, 8);  // an event draws at most 7 beside the tries of a scattering
+        PeelRec<R> none;
+        if (kPeel && slot == slot_end) {
+          if (lane == 0) slot = atomicAdd(qcount, (unsigned long long)a.qchunk);
+          slot = __shfl_sync(0xffffffffu, slot, 0);
+          slot_end = slot + (unsigned long long)a.qchunk;
+        }
+        if (interact<R>(m, dv, t, a, s.p, rng, s.f, L, tr, kPeel ? queue[slot] : none)) ++slot;
+        ++nrec;
+      }
       ensure(rng, 8);
-      if (walk<R, kPeel>(m, t, d, a, s.p, rng, s.f, L, tr, false) != ST_INTERACT) {
+      if (walk<R, kPeel>(m, t, d, a, s.p, rng, s.f, rho, L, tr, false, tried) != ST_INTERACT) {
         s.stage = 0;
         break;
       }
