@@ -188,8 +188,8 @@ struct LucyArgs {
   int nslots;
 };
 
-__device__ double dusttemp_dev(const LucyArgs& a, double na, double T0, int s, double massarr) {
-  return lucy_dusttemp(a.lTint, a.nT, a.kappap + (size_t)s * a.nT, a.kappav[s], a.ltot, a.nphot, na, T0, massarr);
+__device__ double dusttemp_dev(const LucyTables& q, const LucyArgs& a, double na, double T0, int s, double massarr) {
+  return lucy_dusttemp(q, a.lTint, a.nT, a.kappap + (size_t)s * a.nT, a.kappav[s], a.ltot, a.nphot, na, T0, massarr);
 }
 
 // The peel-off walk of the mixed form reads one row per cell with the peel
@@ -221,13 +221,15 @@ __device__ __forceinline__ int2 lucy_row(const LucyRows& q, float T0, int s) {
 __global__ void k_lucy(LucyArgs a, LucyRows rows, const unsigned long long* dtauabs, const double* rho4d, const double* massarr,
                        double* tdust, float* tdustf, unsigned char* peelmask, unsigned long long* maxrel,
                        const float4* rho4f, float4* rho4p) {
+  __shared__ LucyTables tab;
+  lucy_tables(tab, a.lTint, a.nT);
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < a.ncell; c += (int64_t)gridDim.x * blockDim.x) {
     unsigned mask = 0;
     for (int s = 0; s < kSlots; ++s) {
       double T = tdust[4 * c + s];
       if (s < a.nslots && rho4d[4 * c + s] > 0.0) {
         const double na = (double)(long long)dtauabs[(int64_t)s * a.ncell + c] / a.path_scale;
-        const double Td = dusttemp_dev(a, na, T, s, massarr[4 * c + s]);
+        const double Td = dusttemp_dev(tab, a, na, T, s, massarr[4 * c + s]);
         if (na >= a.na_min) {
           const double rel = fabs(Td - T) / Td;
           atomicMax(maxrel, (unsigned long long)__double_as_longlong(rel));
@@ -578,14 +580,15 @@ int ensure_tail(hc3d_ctx* c, int64_t threads) {
 
 // Launch the packets of an unpeeled run on the context's stream (after
 // ensure_tail; allocates nothing, so it can be captured).
-cudaError_t launch_packets(hc3d_ctx* c, RunArgs a, const LaunchCfg& cfg, int tail_blocks) {
+cudaError_t launch_packets(hc3d_ctx* c, RunArgs a, const LaunchCfg& cfg, int tail_blocks, bool fused) {
   const int64_t warps = (int64_t)cfg.blocks * (cfg.threads / 32);
   a.lanes = (int)std::min<int64_t>(32, (a.np + warps - 1) / warps);
   a.dump = kTailLanes;
   const cudaError_t e = cudaMemsetAsync(c->tail.count, 0, 2 * sizeof(unsigned int), cfg.stream);
   if (e != cudaSuccess) return e;
-  return c->precision == HC3D_PREC_FP64 ? launch_packets_fp64(c->dm, c->dt, c->dims, a, c->tail, cfg, tail_blocks)
-                                        : launch_packets_mixed(c->dm, c->dt, c->dims, a, c->tail, cfg, tail_blocks);
+  return c->precision == HC3D_PREC_FP64 ? launch_packets_fp64(c->dm, c->dt, c->dims, a, c->tail, cfg, tail_blocks, fused)
+                                        : launch_packets_mixed(c->dm, c->dt, c->dims, a, c->tail, cfg, tail_blocks,
+                                                               fused);
 }
 
 // the events of wave w (created on first use, kept with the context)
@@ -1433,12 +1436,12 @@ extern "C" int hc3d_zero_tallies(hc3d_ctx* c) {
 
 // Launch shape of an unpeeled run: a persistent grid of the resident blocks, or
 // fewer when the batch has fewer packets than they have warps.
-LaunchCfg transport_cfg(hc3d_ctx* c, int64_t np) {
+LaunchCfg transport_cfg(hc3d_ctx* c, int64_t np, int threads, int grid_blocks) {
   LaunchCfg cfg;
-  cfg.threads = c->block_size;
+  cfg.threads = threads;
   cfg.stream = c->stream;
-  if (c->grid_blocks > 0) {
-    cfg.blocks = c->grid_blocks;
+  if (grid_blocks > 0) {
+    cfg.blocks = grid_blocks;
     return cfg;
   }
   int per_sm = 0;
@@ -1472,10 +1475,10 @@ extern "C" int hc3d_run_iteration(hc3d_ctx* c, const hc3d_run_params* p) {
     c->epoch_np += p->np;
     return HC3D_OK;
   }
-  const LaunchCfg cfg = transport_cfg(c, p->np);
+  const LaunchCfg cfg = transport_cfg(c, p->np, c->block_size, c->grid_blocks);
   if ((r = ensure_tail(c, (int64_t)cfg.blocks * cfg.threads))) return r;
   CK(cudaEventRecord(c->ev0, c->stream));
-  cudaError_t e = launch_packets(c, a, cfg, tail_blocks_for(c, false, p->np));
+  cudaError_t e = launch_packets(c, a, cfg, tail_blocks_for(c, false, p->np), false);
   if (e != cudaSuccess) return fail(c, HC3D_ERR_CUDA, std::string("transport launch: ") + cudaGetErrorString(e));
   CK(cudaEventRecord(c->ev1, c->stream));
   if ((r = finish_run(c))) return r;
@@ -1521,10 +1524,63 @@ extern "C" int hc3d_run_chunk(hc3d_ctx* c, const hc3d_run_params* p, int64_t np_
   return HC3D_OK;
 }
 
-// Several models' packets in one persistent launch (k_transport_batch): the
-// Lucy iterations of a model grid run as one launch per iteration, the
-// small models' long-history tails beside the bulk of the others.  Each
-// context keeps its own tallies, which equal those of hc3d_run_iteration.
+// The unpeeled packet loops of several models at once: each model's kernels on
+// its own stream, between a fork from the first context's stream and a join
+// with it, so that the device runs the long histories of some models beside
+// the bulk of the others.
+static int run_batch_unpeeled(hc3d_ctx* const* ctxs, const hc3d_run_params* params, int n) {
+  hc3d_ctx* c = ctxs[0];
+  std::vector<RunArgs> args((size_t)n);
+  for (int j = 0; j < n; ++j) {
+    hc3d_ctx* cj = ctxs[j];
+    int r = prepare_run(cj, &params[j], &args[(size_t)j]);
+    const LaunchCfg cfg = transport_cfg(cj, params[j].np, 128, 0);
+    if (!r) r = ensure_tail(cj, (int64_t)cfg.blocks * cfg.threads);
+    if (r) {
+      if (cj != c) c->err = "model " + std::to_string(j) + ": " + cj->err;
+      return r;
+    }
+  }
+  CK(cudaEventRecord(c->ev0, c->stream));
+  cudaError_t e = cudaSuccess;
+  for (int j = 0; j < n && e == cudaSuccess; ++j) {
+    hc3d_ctx* cj = ctxs[j];
+    if (params[j].np == 0) continue;
+    if (cj != c) e = cudaStreamWaitEvent(cj->stream, c->ev0, 0);
+    if (e == cudaSuccess) e = cudaMemsetAsync(cj->d_work, 0, sizeof(unsigned long long), cj->stream);
+    if (e == cudaSuccess)
+      e = launch_packets(cj, args[(size_t)j], transport_cfg(cj, params[j].np, 128, 0),
+                         tail_blocks_for(cj, false, params[j].np), true);
+    if (e == cudaSuccess && cj != c) {
+      e = cudaEventRecord(cj->join, cj->stream);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, cj->join, 0);
+    }
+  }
+  if (e == cudaSuccess) e = cudaEventRecord(c->ev1, c->stream);
+  for (int j = 0; j < n; ++j) {  // also after a failed launch: nothing of the batch is left in flight
+    const cudaError_t es = cudaStreamSynchronize(ctxs[j]->stream);
+    if (e == cudaSuccess) e = es;
+  }
+  if (e != cudaSuccess) return fail(c, HC3D_ERR_CUDA, std::string("batched transport: ") + cudaGetErrorString(e));
+  float ms = 0.f;
+  CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
+  for (int j = 0; j < n; ++j) {
+    hc3d_ctx* cj = ctxs[j];
+    const int r = finish_run(cj);
+    if (r) return r;
+    cj->epoch_np += params[j].np;
+    cj->last_ms = cj->last_transport_ms = ms;
+    cj->last_peel_ms = 0.0;
+    cj->last_launches = 1;
+  }
+  return HC3D_OK;
+}
+
+// Several models' packets at once: unpeeled ones by run_batch_unpeeled; with a
+// peeled one among them in one persistent launch (k_transport_batch), which
+// walks each event's peel-off rays in the thread that made it.  Each context
+// keeps its own tallies, which equal those of hc3d_run_iteration (in the mixed
+// form up to the rounding of the walk).
 extern "C" int hc3d_run_batch(hc3d_ctx* const* ctxs, const hc3d_run_params* params, int n) {
   if (!ctxs || !params || n < 1 || n > kMaxBatch) return HC3D_ERR_INVALID;
   hc3d_ctx* c = ctxs[0];
@@ -1537,6 +1593,9 @@ extern "C" int hc3d_run_batch(hc3d_ctx* const* ctxs, const hc3d_run_params* para
       if (ctxs[i] == ctxs[j]) return fail(c, HC3D_ERR_INVALID, "a context appears twice in the batch");
   }
   CK(cudaSetDevice(c->device));
+  bool peeled = false;
+  for (int j = 0; j < n; ++j) peeled = peeled || params[j].ipeel;
+  if (!peeled) return run_batch_unpeeled(ctxs, params, n);
   std::vector<BatchItem> items((size_t)n);
   std::vector<int64_t> first((size_t)n + 1, 0);
   for (int j = 0; j < n; ++j) {
@@ -1962,7 +2021,7 @@ extern "C" int hc3d_lucy_iterations(hc3d_ctx* c, const hc3d_run_params* p, int n
   unsigned long long* d_rel = nullptr;
   int r = dalloc(c, tmp, &d_rel, (size_t)n_iter);
   if (r) return r;
-  const LaunchCfg cfg = transport_cfg(c, p->np);
+  const LaunchCfg cfg = transport_cfg(c, p->np, c->block_size, c->grid_blocks);
   if ((r = ensure_tail(c, (int64_t)cfg.blocks * cfg.threads))) {
     free_all(c, tmp);
     return r;
@@ -1989,7 +2048,7 @@ extern "C" int hc3d_lucy_iterations(hc3d_ctx* c, const hc3d_run_params* p, int n
     if (e == cudaSuccess) e = cudaMemsetAsync(c->dt.sed, 0, sizeof(unsigned long long) * 9 * c->dims.nsed, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->dt.counters, 0, sizeof(unsigned long long) * 16, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->d_work, 0, sizeof(unsigned long long), st);
-    if (e == cudaSuccess) e = launch_packets(c, args[(size_t)k], cfg, tail_blocks);
+    if (e == cudaSuccess) e = launch_packets(c, args[(size_t)k], cfg, tail_blocks, false);
     if (e == cudaSuccess) {
       k_lucy<<<grid_blocks_for(c, la.ncell), 256, 0, st>>>(la, lucy_rows(c), c->dt.dtauabs, c->dm.rho4d, c->d_massarr, c->d_tdust,
                                                            c->d_tdustf, c->d_peelmask, d_rel + k, c->dm.rho4f,

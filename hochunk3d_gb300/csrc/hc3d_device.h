@@ -208,11 +208,12 @@ cudaError_t launch_wave_tail_mixed(const DevModel& m, const DevTallies& t, const
 cudaError_t launch_wave_tail_fp64(const DevModel& m, const DevTallies& t, const TallyDims& d, const RunArgs& a,
                                   const WaveBufs& w, int q, int E, const LaunchCfg& cfg);
 // An unpeeled batch: k_wave without a queue, then k_tail for the packets it
-// leaves.  b.count is zero before it.
+// leaves.  b.count is zero before it.  fused: the rounding of the mixed-form
+// wall search (next_wall_ray).
 cudaError_t launch_packets_mixed(const DevModel& m, const DevTallies& t, const TallyDims& d, const RunArgs& a,
-                                 const TailBufs& b, const LaunchCfg& cfg, int tail_blocks);
+                                 const TailBufs& b, const LaunchCfg& cfg, int tail_blocks, bool fused);
 cudaError_t launch_packets_fp64(const DevModel& m, const DevTallies& t, const TallyDims& d, const RunArgs& a,
-                                const TailBufs& b, const LaunchCfg& cfg, int tail_blocks);
+                                const TailBufs& b, const LaunchCfg& cfg, int tail_blocks, bool fused);
 const void* packets_fn_mixed();
 const void* packets_fn_fp64();
 const void* tail_fn_mixed(bool peel);

@@ -41,7 +41,7 @@ static DevModel tail_model_fp64(const DevModel& m) {
 
 cudaError_t launch_wave_transport_fp64(const DevModel& m, const DevTallies& t, const TallyDims& d, const RunArgs& a,
                                         const WaveBufs& w, int q, int E, const LaunchCfg& cfg) {
-  dev::k_wave<double, true><<<cfg.blocks, cfg.threads, m.dust_smem, cfg.stream>>>(
+  dev::k_wave<double, true, true><<<cfg.blocks, cfg.threads, m.dust_smem, cfg.stream>>>(
       m, t, d, a, static_cast<dev::Slot<double>*>(w.pool), static_cast<dev::PeelRec<double>*>(w.queue[q]), w.qcount[q], E,
       w.alive[q], w.live[q]);
   return cudaGetLastError();
@@ -50,29 +50,29 @@ cudaError_t launch_wave_transport_fp64(const DevModel& m, const DevTallies& t, c
 cudaError_t launch_wave_tail_fp64(const DevModel& m, const DevTallies& t, const TallyDims& d, const RunArgs& a,
                                    const WaveBufs& w, int q, int E, const LaunchCfg& cfg) {
   const DevModel tm = tail_model_fp64(m);
-  dev::k_tail<double, true><<<cfg.blocks, 128, tm.dust_smem, cfg.stream>>>(
+  dev::k_tail<double, true, true><<<cfg.blocks, 128, tm.dust_smem, cfg.stream>>>(
       tm, t, d, a, static_cast<dev::Slot<double>*>(w.pool), w.alive[1 - q], w.live[1 - q], w.next_live,
       static_cast<dev::PeelRec<double>*>(w.queue[q]), w.qcount[q], E, w.alive[q], w.live[q]);
   return cudaGetLastError();
 }
 
 cudaError_t launch_packets_fp64(const DevModel& m, const DevTallies& t, const TallyDims& d, const RunArgs& a,
-                                 const TailBufs& b, const LaunchCfg& cfg, int tail_blocks) {
+                                 const TailBufs& b, const LaunchCfg& cfg, int tail_blocks, bool) {
   auto* pool = static_cast<dev::Slot<double>*>(b.pool);
-  dev::k_wave<double, false><<<cfg.blocks, cfg.threads, m.dust_smem, cfg.stream>>>(m, t, d, a, pool, nullptr, nullptr, 0,
+  dev::k_wave<double, false, false><<<cfg.blocks, cfg.threads, m.dust_smem, cfg.stream>>>(m, t, d, a, pool, nullptr, nullptr, 0,
                                                                              b.count, nullptr);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   const DevModel tm = tail_model_fp64(m);
-  dev::k_tail<double, false><<<tail_blocks, 128, tm.dust_smem, cfg.stream>>>(tm, t, d, a, pool, b.count, nullptr,
+  dev::k_tail<double, false, false><<<tail_blocks, 128, tm.dust_smem, cfg.stream>>>(tm, t, d, a, pool, b.count, nullptr,
                                                                        b.count + 1, nullptr, nullptr, 0, nullptr,
                                                                        nullptr);
   return cudaGetLastError();
 }
 
-const void* packets_fn_fp64() { return (const void*)dev::k_wave<double, false>; }
+const void* packets_fn_fp64() { return (const void*)dev::k_wave<double, false, false>; }
 const void* tail_fn_fp64(bool peel) {
-  return peel ? (const void*)dev::k_tail<double, true> : (const void*)dev::k_tail<double, false>;
+  return peel ? (const void*)dev::k_tail<double, true, true> : (const void*)dev::k_tail<double, false, false>;
 }
 int tail_smem_fp64(const DevModel& m) { return tail_model_fp64(m).dust_smem; }
 
@@ -85,7 +85,7 @@ cudaError_t launch_wave_peel_fp64(const DevModel& m, const DevTallies& t, const 
 
 size_t slot_bytes_fp64() { return sizeof(dev::Slot<double>); }
 size_t rec_bytes_fp64() { return sizeof(dev::PeelRec<double>); }
-const void* wave_fn_fp64() { return (const void*)dev::k_wave<double, true>; }
+const void* wave_fn_fp64() { return (const void*)dev::k_wave<double, true, true>; }
 const void* peel_fn_fp64() { return (const void*)dev::k_peel<double>; }
 
 }  // namespace hc3d

@@ -41,7 +41,7 @@ static DevModel tail_model_mixed(const DevModel& m) {
 
 cudaError_t launch_wave_transport_mixed(const DevModel& m, const DevTallies& t, const TallyDims& d, const RunArgs& a,
                                         const WaveBufs& w, int q, int E, const LaunchCfg& cfg) {
-  dev::k_wave<float, true><<<cfg.blocks, cfg.threads, m.dust_smem, cfg.stream>>>(
+  dev::k_wave<float, true, true><<<cfg.blocks, cfg.threads, m.dust_smem, cfg.stream>>>(
       m, t, d, a, static_cast<dev::Slot<float>*>(w.pool), static_cast<dev::PeelRec<float>*>(w.queue[q]), w.qcount[q], E,
       w.alive[q], w.live[q]);
   return cudaGetLastError();
@@ -50,29 +50,36 @@ cudaError_t launch_wave_transport_mixed(const DevModel& m, const DevTallies& t, 
 cudaError_t launch_wave_tail_mixed(const DevModel& m, const DevTallies& t, const TallyDims& d, const RunArgs& a,
                                    const WaveBufs& w, int q, int E, const LaunchCfg& cfg) {
   const DevModel tm = tail_model_mixed(m);
-  dev::k_tail<float, true><<<cfg.blocks, 128, tm.dust_smem, cfg.stream>>>(
+  dev::k_tail<float, true, true><<<cfg.blocks, 128, tm.dust_smem, cfg.stream>>>(
       tm, t, d, a, static_cast<dev::Slot<float>*>(w.pool), w.alive[1 - q], w.live[1 - q], w.next_live,
       static_cast<dev::PeelRec<float>*>(w.queue[q]), w.qcount[q], E, w.alive[q], w.live[q]);
   return cudaGetLastError();
 }
 
-cudaError_t launch_packets_mixed(const DevModel& m, const DevTallies& t, const TallyDims& d, const RunArgs& a,
+template <bool kFused>
+static cudaError_t launch_packets_as(const DevModel& m, const DevTallies& t, const TallyDims& d, const RunArgs& a,
                                  const TailBufs& b, const LaunchCfg& cfg, int tail_blocks) {
   auto* pool = static_cast<dev::Slot<float>*>(b.pool);
-  dev::k_wave<float, false><<<cfg.blocks, cfg.threads, m.dust_smem, cfg.stream>>>(m, t, d, a, pool, nullptr, nullptr, 0,
+  dev::k_wave<float, false, kFused><<<cfg.blocks, cfg.threads, m.dust_smem, cfg.stream>>>(m, t, d, a, pool, nullptr, nullptr, 0,
                                                                              b.count, nullptr);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   const DevModel tm = tail_model_mixed(m);
-  dev::k_tail<float, false><<<tail_blocks, 128, tm.dust_smem, cfg.stream>>>(tm, t, d, a, pool, b.count, nullptr,
+  dev::k_tail<float, false, kFused><<<tail_blocks, 128, tm.dust_smem, cfg.stream>>>(tm, t, d, a, pool, b.count, nullptr,
                                                                        b.count + 1, nullptr, nullptr, 0, nullptr,
                                                                        nullptr);
   return cudaGetLastError();
 }
 
-const void* packets_fn_mixed() { return (const void*)dev::k_wave<float, false>; }
+cudaError_t launch_packets_mixed(const DevModel& m, const DevTallies& t, const TallyDims& d, const RunArgs& a,
+                                 const TailBufs& b, const LaunchCfg& cfg, int tail_blocks, bool fused) {
+  return fused ? launch_packets_as<true>(m, t, d, a, b, cfg, tail_blocks)
+               : launch_packets_as<false>(m, t, d, a, b, cfg, tail_blocks);
+}
+
+const void* packets_fn_mixed() { return (const void*)dev::k_wave<float, false, false>; }
 const void* tail_fn_mixed(bool peel) {
-  return peel ? (const void*)dev::k_tail<float, true> : (const void*)dev::k_tail<float, false>;
+  return peel ? (const void*)dev::k_tail<float, true, true> : (const void*)dev::k_tail<float, false, false>;
 }
 int tail_smem_mixed(const DevModel& m) { return tail_model_mixed(m).dust_smem; }
 
@@ -96,7 +103,7 @@ int peel_threads_mixed(int variant) { return kPeelShapes[variant < 0 || variant 
 
 size_t slot_bytes_mixed() { return sizeof(dev::Slot<float>); }
 size_t rec_bytes_mixed() { return sizeof(dev::PeelRec<float>); }
-const void* wave_fn_mixed() { return (const void*)dev::k_wave<float, true>; }
+const void* wave_fn_mixed() { return (const void*)dev::k_wave<float, true, true>; }
 const void* peel_fn_mixed(int variant) {
   switch (variant) {
     case 1: return (const void*)dev::k_peel_mixed<float, 192, 3>;

@@ -50,6 +50,8 @@ struct Args {
 __global__ void __launch_bounds__(kThreads) k_lucy_noalloc(Args a, unsigned long long* scratch) {
   __shared__ unsigned long long smax[kThreads / 32];
   __shared__ bool last;
+  __shared__ hc3d::LucyTables tab;
+  hc3d::lucy_tables(tab, a.lTint, a.nT);
   unsigned long long mx = 0;
   const long long n4 = (long long)a.nrg * a.ntg * a.npg;
   const long long base = (long long)blockIdx.x * kThreads * kPerThread;
@@ -66,7 +68,7 @@ __global__ void __launch_bounds__(kThreads) k_lucy_noalloc(Args a, unsigned long
     double T = T0;
     if (ir < a.nrg - 1 && it < a.ntg - 1 && ip < a.npg - 1 && a.densarr[k] > 0.0) {
       const double na = (double)a.dtauabs[k] / a.path_scale;
-      T = hc3d::lucy_dusttemp(a.lTint, a.nT, a.kappap + (size_t)s * a.nT, a.kappav[s], a.ltot, a.nphot, na, T0,
+      T = hc3d::lucy_dusttemp(tab, a.lTint, a.nT, a.kappap + (size_t)s * a.nT, a.kappav[s], a.ltot, a.nphot, na, T0,
                               a.massarr[k]);
       if (na >= a.na_min) {
         const unsigned long long bits = (unsigned long long)__double_as_longlong(fabs(T - T0) / T);

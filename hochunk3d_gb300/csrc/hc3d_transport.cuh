@@ -540,10 +540,10 @@ __device__ __forceinline__ float fsqrt_pos(float x) { return x * rsqrtf(x); }
 // only their far root, and the next wall is the smallest non-negative root
 // of the rest, a minimum over at most six candidates.  FP32, except the
 // near-sphere and grazing sphere roots (FP64).
-// kFused: how |x|^2 and x.u take their z term: by an FMA (the peeled runs) or
-// by a separate product and sum (the unpeeled ones).  The two round
-// differently in the last bit; each kind of run keeps the one that its
-// results have always had.
+// kFused: how |x|^2 and x.u take their z term: by an FMA (the peeled runs and
+// the batched ones) or by a separate product and sum (the unpeeled runs of one
+// model).  The two round differently in the last bit; each kind of run keeps
+// the one that its results have always had.
 template <bool kFused>
 __device__ __forceinline__ bool next_wall_ray(const DevModel& m, Ray& r, const PathLen& S, int ir, int it, int ip,
                                               int own, float& dt, int& iface) {
@@ -3100,7 +3100,7 @@ struct Slot {
 // instructions, 5 us.  Once the batch has no packet left, a warp with fewer
 // than a.dump busy lanes therefore stops and leaves its packets to k_tail:
 // in their pool slots (kPeel), or as the first *alive slots of the pool.
-template <class R, bool kPeel>
+template <class R, bool kPeel, bool kFused>
 __global__ void __launch_bounds__(128, 3) k_wave(DevModel m, DevTallies t, TallyDims d, RunArgs a, Slot<R>* pool,
                                                PeelRec<R>* queue, unsigned long long* qcount, int E,
                                                unsigned int* alive, unsigned int* live) {
@@ -3178,7 +3178,7 @@ __global__ void __launch_bounds__(128, 3) k_wave(DevModel m, DevTallies t, Tally
       }
       if (emitted) {
         Rho<R> rho;
-        const int st = walk<R, kPeel>(m, t, d, a, s.p, rng, s.f, rho, L, tr, s.stage == 2);
+        const int st = walk<R, kFused>(m, t, d, a, s.p, rng, s.f, rho, L, tr, s.stage == 2);
         s.stage = st == ST_INTERACT ? 1 : 0;
         if (!kPeel && s.stage == 0) L.settle();
       }
@@ -3368,7 +3368,7 @@ __device__ __forceinline__ Batch tail_batch(const DevModel& m, const DustView<fl
 // events: in the plain model's disk 5.0 us an event for a lane of k_wave, 3.0
 // us here with one event after another, 1.2 us with the absorptions side by
 // side.  The arithmetic is that of k_wave, bit for bit.
-template <class R, bool kPeel>
+template <class R, bool kPeel, bool kFused>
 __global__ void __launch_bounds__(128, 4) k_tail(DevModel m, DevTallies t, TallyDims d, RunArgs a, Slot<R>* pool,
                                                  const unsigned int* nlive, const unsigned int* live,
                                                  unsigned int* next, PeelRec<R>* queue, unsigned long long* qcount,
@@ -3418,7 +3418,7 @@ __global__ void __launch_bounds__(128, 4) k_tail(DevModel m, DevTallies t, Tally
         ++nrec;
       }
       ensure(rng, 8);
-      if (walk<R, kPeel>(m, t, d, a, s.p, rng, s.f, rho, L, tr, false, tried) != ST_INTERACT) {
+      if (walk<R, kFused>(m, t, d, a, s.p, rng, s.f, rho, L, tr, false, tried) != ST_INTERACT) {
         s.stage = 0;
         break;
       }

@@ -341,13 +341,15 @@ int hc3d_lucy_update(hc3d_ctx *ctx, double ltot, int64_t np, double *tdust_out,
  * scales. */
 int hc3d_set_lucy_tally(hc3d_ctx *ctx, const int64_t *dtauabs);
 
-/* The packet loops of n models (1..256) in one persistent launch: ctxs[j]
- * runs params[j] with its own tables, grid and tallies.  Peeled runs
- * (ipeel = 1) walk each event's peel-off rays in the thread that made the
- * event, with the same walk as the wavefront form, so the tallies equal
- * those of hc3d_run_iteration(ctxs[j], &params[j]) bit for bit in the FP64
- * form and within FP32 rounding in the mixed form.  All contexts share one
- * device and precision; the launch runs on the stream of ctxs[0].  No
+/* The packet loops of n models (1..256) at once: ctxs[j] runs params[j] with
+ * its own tables, grid and tallies.  Unpeeled models run on their contexts'
+ * own streams, between a fork from the stream of ctxs[0] and a join with it.
+ * With a peeled model (ipeel = 1) among them all run in one persistent
+ * launch on the stream of ctxs[0], which walks each event's peel-off rays in
+ * the thread that made the event, with the same walk as the wavefront form.
+ * The tallies equal those of hc3d_run_iteration(ctxs[j], &params[j]) bit for
+ * bit in the FP64 form and within FP32 rounding in the mixed form.  All
+ * contexts share one device and precision.  No
  * counterpart in the reference (one model per run). */
 int hc3d_run_batch(hc3d_ctx *const *ctxs, const hc3d_run_params *params, int n);
 
