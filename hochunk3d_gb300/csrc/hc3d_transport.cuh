@@ -140,7 +140,7 @@ template <class R> __device__ __forceinline__ void draw_phi(Rng& r, R& phi, R& c
 // stream, formed 32 lanes at a time in shared memory.  The FP64 form keeps the
 // functions above of each beside them -- a lone FP64 logarithm is a chain of
 // 2100 cycles -- and reads them instead; the mixed form runs its events side by
-// side in the lanes (tail_batch), which form what they need.  Every lane holds
+// side in the lanes (tail_window), which form what they need.  Every lane holds
 // the same position; ensure() is called by the whole warp.
 template <class R> struct DrawTable;
 template <> struct DrawTable<float> {
@@ -242,7 +242,7 @@ template <class R> __device__ __forceinline__ void draw_phi(WarpRng<R>& r, R& ph
     sphi = r.t->sphi[r.at++];
   }
 }
-// one draw, of a lane that works ahead (tail_batch)
+// one draw, of a lane that works ahead (tail_window)
 struct OneDraw {
   float u;
 };
@@ -3197,170 +3197,218 @@ __global__ void __launch_bounds__(128, 3) k_wave(DevModel m, DevTallies t, Tally
   flush(t, L);
 }
 
-// Up to kAhead events of one packet side by side in the lanes of its warp.
+// The events of one packet in one cell, their absorptions formed ahead side by
+// side in the lanes of its warp.
 //
 // An absorption re-emits the packet with a frequency drawn from the cell's
 // temperature, in an isotropic direction: what it leaves depends on its draws
-// and on the cell, and not on the packet that was absorbed.  In an optically
-// thick cell most events are absorptions that end in the cell (safe steps), so
-// their frequencies, opacities, directions and step lengths are formed at once:
-// lane k takes the k-th event from here, on the draws it has if all before it
-// are absorptions (six each: albedo, mu, phi, frequency, tau, species).  The
-// chain holds as far as the albedo draw of each event absorbs it, by the
-// albedo its predecessor left, and the species it assumed is the one its
-// predecessor's last draw selects.  What depends on the packet's way -- the
-// position, and whether a step is safe -- is then followed event by event, in
-// the order and rounding of the walk, and the events up to the first one that
-// needs the wall search are tallied by their lanes.  That one (`wall`) is left
-// re-emitted, for the caller to walk; a scattering is left to interact().
+// and on the cell, and not on the packet that was absorbed.  It takes six draws
+// (albedo, mu, phi, frequency, tau, species), a scattering of t tries 3 + 3 t.
+// So the n-th event from here starts a multiple of three draws on, and lane j <
+// 16 forms the absorption that would start 6 j draws on, lane 16 + j the one 6
+// j + 3 draws on: frequency, opacities, direction and step.  The packet's way is
+// then followed event by event, in the order and rounding of the walk: whether
+// its albedo draw absorbs the packet, by the albedo the event before left;
+// whether the species it assumed is the one that event's last draw selected;
+// whether the step ends within the safe distance.  Where all hold, the event
+// costs its position and a few shuffles; a scattering and a step that needs the
+// wall search are run by the whole warp (interact, walk), and while the packet
+// stays in its cell the lanes' events after them still hold.  What the lanes'
+// events tally they tally at the end, each its own.
 //
-// One event after another took 5700 cycles each, nearly all of them in the
-// part that the lanes share here.
-constexpr int kAhead = 16;
+// One event after another took 5700 cycles each; side by side up to the first
+// scattering or wall search, 4.4 events of the plain model's disk at a time,
+// 2300.
+constexpr int kAhead = 16;  // events a lane set looks ahead
 
-struct Batch {
-  int n;      // events done, walked and tallied
-  bool wall;  // and one more absorbed and re-emitted, to be walked
-  bool far;   // whose step is longer than the safe distance
+// what the lanes' events leave, in shared memory (a field's 32 values side by
+// side): any lane's is read by the whole warp, and the packet keeps its registers
+enum AheadField {
+  A_COST, A_SINT, A_PHI, A_COSP, A_SINP, A_NUB, A_UX, A_UY, A_UZ, A_DS, A_ALB, A_WHAT, A_OP, A_INUB,
+  A_KAPD, A_ALBEDO = A_KAPD + kSlots, A_G = A_ALBEDO + kSlots, A_PL = A_G + kSlots, A_FIELDS = A_PL + kSlots
+};
+struct Ahead {
+  float v[A_FIELDS][32];
 };
 
-template <bool kPeel>
-__device__ __forceinline__ Batch tail_batch(const DevModel& m, const DustView<float>& dv, const DevTallies& t,
-                                            const RunArgs& a, Pkt<float>& p, WarpRng<float>& rng, Flow<float>& f,
-                                            const Rho<float>& rho, Local& L, PeelRec<float>* queue,
-                                            unsigned long long* qcount, unsigned long long& slot,
-                                            unsigned long long& slot_end, int most) {
-  Batch b{0, false, false};
+// Runs events until the packet leaves the cell, ends or has run `most` of them
+// (nrec counts them); whether it goes on.
+template <bool kPeel, bool kFused>
+__device__ __forceinline__ bool tail_window(const DevModel& m, const DustView<float>& dv, const DevTallies& t,
+                                            const TallyDims& td, const RunArgs& a, Pkt<float>& p, WarpRng<float>& rng,
+                                            Flow<float>& f, Rho<float>& rho, Ahead& ah, Local& L, Tracer& tr,
+                                            PeelRec<float>* queue, unsigned long long* qcount,
+                                            unsigned long long& slot, unsigned long long& slot_end, int& nrec, int E) {
   const int lane = threadIdx.x & 31;
   const int64_t c = cidx(m, p.ir, p.it, p.ip);
-  const int at = rng.at + 6 * min(lane, kAhead - 1);
-  const float* u = rng.t->u + at;
-  // the species each event is assumed to meet: the pending one's is known,
-  // the later ones' as the packet's present opacities select it
+  const int ir0 = p.ir;
+  ensure(rng, 6 * kAhead + 8);
+  const int off0 = 6 * (lane & (kAhead - 1)) + (lane >= kAhead ? 3 : 0);
+  const float* u = rng.t->u + rng.at + off0;
+  const uint32_t from = 4u * rng.block + (uint32_t)rng.at;  // the draw the window starts at
+  // the species a lane's event is assumed to meet: the pending event's is
+  // known, the others' as the packet's present opacities select it
   OneDraw d{u[lane == 0 ? 0 : -1]};
   int s = select_dust<float>(m, p, rho, d);
   if (lane == 0) s = f.idust2;
   const bool thermal = s >= 0 && !((m.sg_mask >> s) & 1u);
-  // lane 0: is the pending event an absorption at all?
-  if (__shfl_sync(0xffffffffu, (int)(thermal && u[0] > pick4(p.albedo, f.idust2)), 0) == 0) return b;
-  if (!thermal) s = f.idust2;
-  Pkt<float> q;
-  q.cost = 1.f - 2.f * u[1];
-  q.sint = xsqrt(1.f - q.cost * q.cost);
-  q.phi = (float)kR2p * u[2];
-  q.cosp = xcos(q.phi);
-  q.sinp = xsin(q.phi);
-  d.u = u[3];
-  q.nub = lucy_freq_mixed(m, c, s, d);
-  opacset<float, false>(m, dv, q, q.nub, a);
-  q.ux = q.sint * q.cosp; q.uy = q.sint * q.sinp; q.uz = q.cost;
-  const float opac = opacity(q, rho);
-  const float rin = __ldg(m.rarrf + p.ir - 1), rout = __ldg(m.rarrf + p.ir);
+  if (!thermal) s = 0;
   constexpr float kLong = 3.402823466e38f;  // a step that needs the wall search
-  float ds = -xlog(u[4]) / opac;
-  if (!(opac > 0.f && ds < 0.5f * (rout - rin))) ds = kLong;
-  d.u = u[5];
-  const int sel = select_dust<float>(m, q, rho, d);
-  const float alb = pick4(q.albedo, max(sel, 0));
-  // how far the chain holds
-  const float alb_before = __shfl_up_sync(0xffffffffu, alb, 1);
-  const int sel_before = __shfl_up_sync(0xffffffffu, sel, 1);
-  const bool holds = lane < kAhead && thermal && (lane == 0 || (sel_before == s && u[0] > alb_before));
-  const unsigned broken = __ballot_sync(0xffffffffu, !holds);
-  int chain = __ffs(broken) - 1;
-  int last = min(chain, most);
-  // a packet that reaches a cap is killed in walk()
-  last = min(last, a.iintmax - f.iint);
-  if (a.max_interactions > 0) last = (int)min((int64_t)last, a.max_interactions - f.ntot - 1);
-  last = max(last, 0);
-  float op = 0.f;
-  int inub = 0;
-  if constexpr (kPeel) {
-    op = peel_opacity(m, q, c);
-    inub = nu_bin<float>(a, q.nub);
-    q.sip = 1.f; q.sqp = q.sup = q.svp = 0.f;
-    q.ir = p.ir; q.it = p.it; q.ip = p.ip;
-    q.on_wall = 0;
-    q.i_orig = ((m.disk_mask >> s) & 1u) ? 2 : 3;
-  }
-  // the way, event by event
-  auto record = [&](int k) {  // the peel-off record of event k, unless its rays end in the cell
+  __syncwarp();  // the last window's values have been read
+  {
+    Pkt<float> q;
+    q.cost = 1.f - 2.f * u[1];
+    q.sint = xsqrt(1.f - q.cost * q.cost);
+    q.phi = (float)kR2p * u[2];
+    q.cosp = xcos(q.phi);
+    q.sinp = xsin(q.phi);
+    d.u = u[3];
+    q.nub = lucy_freq_mixed(m, c, s, d);
+    opacset<float, false>(m, dv, q, q.nub, a);
+    const float opac = opacity(q, rho);
+    float ds = -xlog(u[4]) / opac;
+    if (!(opac > 0.f && ds < 0.5f * (__ldg(m.rarrf + p.ir) - __ldg(m.rarrf + p.ir - 1)))) ds = kLong;
+    d.u = u[5];
+    const int sel = select_dust<float>(m, q, rho, d);
+    auto put = [&](int k, float v) { ah.v[k][lane] = v; };
+    put(A_COST, q.cost); put(A_SINT, q.sint); put(A_PHI, q.phi); put(A_COSP, q.cosp); put(A_SINP, q.sinp);
+    put(A_NUB, q.nub);
+    put(A_UX, q.sint * q.cosp); put(A_UY, q.sint * q.sinp); put(A_UZ, q.cost);
+    put(A_DS, ds);
+    put(A_ALB, pick4(q.albedo, max(sel, 0)));
+    put(A_WHAT, __int_as_float((thermal ? s : 7) | ((sel < 0 ? 7 : sel) << 4)));
     if constexpr (kPeel) {
-      const float opk = __shfl_sync(0xffffffffu, op, k);
-      if (p.safe > 0.f && deep_peel_at(p, p.safe, opk)) return;
-      if (slot == slot_end) {
-        if (lane == 0) slot = atomicAdd(qcount, (unsigned long long)a.qchunk);
-        slot = __shfl_sync(0xffffffffu, slot, 0);
-        slot_end = slot + (unsigned long long)a.qchunk;
-      }
-      if (lane == k) {
-        q.x = p.x; q.y = p.y; q.z = p.z;
-        make_rec<float>(queue[slot], q, inub, 0, s, 0);
-      }
-      ++slot;
+      put(A_OP, peel_opacity(m, q, c));
+      put(A_INUB, __int_as_float(nu_bin<float>(a, q.nub)));
+    }
+#pragma unroll
+    for (int k = 0; k < kSlots; ++k) {
+      put(A_KAPD + k, q.kapd[k]);
+      put(A_ALBEDO + k, q.albedo[k]);
+      put(A_G + k, q.g[k]);
+      put(A_PL + k, q.pl[k]);
+    }
+  }
+  __syncwarp();
+  // the packet as the event of lane l left it
+  auto adopt = [&](int l) {
+    p.cost = ah.v[A_COST][l]; p.sint = ah.v[A_SINT][l]; p.phi = ah.v[A_PHI][l];
+    p.cosp = ah.v[A_COSP][l]; p.sinp = ah.v[A_SINP][l]; p.nub = ah.v[A_NUB][l];
+#pragma unroll
+    for (int j = 0; j < kSlots; ++j) {
+      p.kapd[j] = ah.v[A_KAPD + j][l];
+      p.albedo[j] = ah.v[A_ALBEDO + j][l];
+      p.g[j] = ah.v[A_G + j][l];
+      p.pl[j] = ah.v[A_PL + j][l];
+    }
+    p.i_orig = ((m.disk_mask >> (__float_as_int(ah.v[A_WHAT][l]) & 15)) & 1u) ? 2 : 3;
+    p.sip = 1.f; p.sqp = p.sup = p.svp = 0.f;
+  };
+  auto reserve = [&]() {  // a queue slot for the next record
+    if (kPeel && slot == slot_end) {
+      if (lane == 0) slot = atomicAdd(qcount, (unsigned long long)a.qchunk);
+      slot = __shfl_sync(0xffffffffu, slot, 0);
+      slot_end = slot + (unsigned long long)a.qchunk;
     }
   };
-  const int on_wall = p.on_wall;
-  int k = 0;
-  bool far = on_wall != 0;  // (a pending event is never on a wall)
-  for (; k < last && !far; ++k) {
-    const float dsk = __shfl_sync(0xffffffffu, ds, k);
-    const float ux = __shfl_sync(0xffffffffu, q.ux, k), uy = __shfl_sync(0xffffffffu, q.uy, k),
-                uz = __shfl_sync(0xffffffffu, q.uz, k);
-    record(k);
-    if (!(dsk < p.safe)) {
-      if (dsk < kLong) p.safe = safe_dist(m, p.x.hi, p.y.hi, p.z.hi, p.ir, p.it, p.ip);
-      if (!(dsk < p.safe)) {
-        far = true;
-        break;
+  unsigned absorbed = 0u, stepped = 0u;  // the lanes whose event was an absorption, a step within the cell
+  int left = -1;                         // the lane whose event left the packet, where p does not have it yet
+  float alb_now = pick4(p.albedo, f.idust2);
+  bool live = true, here = true;
+  while (here && (!kPeel || nrec < E)) {
+    const int off = (int)(4u * rng.block + (uint32_t)rng.at - from);
+    if (off > 6 * kAhead - 3) break;
+    ensure(rng, 8);
+    const int h = off / 3, l = (h >> 1) + ((h & 1) ? kAhead : 0);
+    const int wl = __float_as_int(ah.v[A_WHAT][l]);
+    ++nrec;
+    bool tried = false;
+    if (rng.t->u[rng.at] > alb_now && (wl & 15) == f.idust2) {
+      // absorbed and re-emitted as lane l has it
+      if constexpr (kPeel) {
+        if (!(p.safe > 0.f && deep_peel_at(p, p.safe, ah.v[A_OP][l]))) {
+          reserve();
+          if (lane == 0) {
+            PeelRec<float>& e = queue[slot];
+            const int sl = wl & 15;
+            e.x = p.x; e.y = p.y; e.z = p.z;
+            e.ir = p.ir; e.it = p.it; e.ip = p.ip;
+            e.flags = (((m.disk_mask >> sl) & 1u ? 2 : 3) << 2) | (sl << 5);
+            e.inub = __float_as_int(ah.v[A_INUB][l]);
+            e.sip = 1.f; e.sqp = e.sup = e.svp = 0.f;
+            e.d0 = ah.v[A_COST][l]; e.d1 = ah.v[A_SINT][l]; e.d2 = ah.v[A_PHI][l]; e.d3 = ah.v[A_COSP][l];
+            e.d4 = ah.v[A_SINP][l];
+            e.g = ah.v[A_G + sl][l]; e.pl = ah.v[A_PL + sl][l];
+#pragma unroll
+            for (int k = 0; k < kSlots; ++k) e.kapd[k] = ah.v[A_KAPD + k][l];
+          }
+          ++slot;
+        }
       }
+      const float dsl = ah.v[A_DS][l];
+      L.events++;
+      f.ntot++;
+      f.iint++;
+      f.iflag = 0;
+      absorbed |= 1u << l;
+      // a packet that reaches a cap is killed in walk()
+      const bool capped = f.iint > a.iintmax || (a.max_interactions > 0 && f.ntot >= a.max_interactions);
+      if (!capped && wl < 0x70) {
+        if (!(dsl < p.safe) && dsl < kLong) p.safe = safe_dist(m, p.x.hi, p.y.hi, p.z.hi, p.ir, p.it, p.ip);
+        if (dsl < p.safe) {
+          p.safe = __fsub_rn(p.safe, dsl);
+          const PathLen S{dsl, 0.f};
+          p.x = pos_step(p.x, S, ah.v[A_UX][l]);
+          p.y = pos_step(p.y, S, ah.v[A_UY][l]);
+          p.z = pos_step(p.z, S, ah.v[A_UZ][l]);
+          L.cross++;
+          stepped |= 1u << l;
+          rng.at += 6;
+          f.idust2 = wl >> 4;
+          alb_now = ah.v[A_ALB][l];
+          left = l;
+          continue;
+        }
+        tried = true;
+      }
+      adopt(l);
+      left = -1;
+      rng.at += 4;
+    } else {
+      if (left >= 0) adopt(left);
+      left = -1;
+      PeelRec<float> none;
+      reserve();
+      if (interact<float>(m, dv, t, a, p, rng, f, L, tr, kPeel ? queue[slot] : none)) ++slot;
+      ensure(rng, 8);
     }
-    p.safe = __fsub_rn(p.safe, dsk);
-    const PathLen S{dsk, 0.f};
-    p.x = pos_step(p.x, S, ux);
-    p.y = pos_step(p.y, S, uy);
-    p.z = pos_step(p.z, S, uz);
+    const int ir = p.ir, it = p.it, ip = p.ip;
+    live = walk<float, kFused>(m, t, td, a, p, rng, f, rho, L, tr, false, tried) == ST_INTERACT;
+    here = live && p.ir == ir && p.it == it && p.ip == ip;
+    if (live) alb_now = pick4(p.albedo, f.idust2);
   }
-  b.n = k;
-  b.far = far;
-  b.wall = far || (k < chain && k < most);  // stopped by a long step or by a cap
-  if (b.wall && !far) record(k);
-  const int done = b.n + (b.wall ? 1 : 0);
-  if (done == 0) return b;
-  // the tallies of each event by its lane
-  if (lane < done) {
+  if (left >= 0) adopt(left);
+  const float rout = __ldg(m.rarrf + ir0);
+  if ((absorbed >> lane) & 1u) {
     atomicAdd(t.dbig + c, 1u);
     atomicAdd(t.nabs + (int64_t)s * m.ncell + c, 1ull);
   }
-  if (lane < b.n) tally_path<float>(m, t, q, rho, c, ds, rout);
-  L.events += done;
-  L.cross += b.n;
-  f.ntot += done;
-  f.iint += done;
-  f.iflag = 0;
-  rng.at += 6 * b.n + (b.wall ? 4 : 0);
-  // the packet as its last event left it
-  const int l = done - 1;
-  p.i_orig = ((m.disk_mask >> __shfl_sync(0xffffffffu, s, l)) & 1u) ? 2 : 3;
-  p.sip = 1.f; p.sqp = p.sup = p.svp = 0.f;
-  auto from = [&](float v) { return __shfl_sync(0xffffffffu, v, l); };
-  p.cost = from(q.cost); p.sint = from(q.sint); p.phi = from(q.phi);
-  p.cosp = from(q.cosp); p.sinp = from(q.sinp); p.nub = from(q.nub);
+  if ((stepped >> lane) & 1u) {
+    Pkt<float> q;
 #pragma unroll
-  for (int j = 0; j < kSlots; ++j) {
-    p.kapd[j] = from(q.kapd[j]);
-    p.albedo[j] = from(q.albedo[j]);
-    p.g[j] = from(q.g[j]);
-    p.pl[j] = from(q.pl[j]);
+    for (int k = 0; k < kSlots; ++k) {
+      q.kapd[k] = ah.v[A_KAPD + k][lane];
+      q.albedo[k] = ah.v[A_ALBEDO + k][lane];
+    }
+    tally_path<float>(m, t, q, load_rho<float>(m, c), c, ah.v[A_DS][lane], rout);
   }
-  if (!b.wall) f.idust2 = __shfl_sync(0xffffffffu, sel, l);
-  return b;
+  return live;
 }
 
 // The packets that k_wave left, one per warp: every lane holds the packet, and
 // the parts of its events that a lane alone would do one after another are
-// shared between the lanes.  The mixed form runs absorptions up to sixteen at
-// once (tail_batch), the tries of a scattering angle ten at once (scat_draw),
+// shared between the lanes.  The mixed form forms the absorptions of a cell
+// side by side (tail_window), the tries of a scattering angle ten at once (scat_draw),
 // the walls of a cell side by side (next_wall_warp) and the tallies of a step
 // in one instruction (tauint_warp); the FP64 form reads its logarithms, sines
 // and cosines from a table 32 lanes formed (DrawTable) and shares the tries
@@ -3378,6 +3426,7 @@ __global__ void __launch_bounds__(128, 4) k_tail(DevModel m, DevTallies t, Tally
   dust_view<R>(m, reinterpret_cast<R*>(dust_smem), dv);
   __shared__ unsigned long long block_counters[16];
   __shared__ DrawTable<R> draws[4];
+  __shared__ Ahead ahead[sizeof(R) == 4 ? 4 : 1];
   Local L;
   local_init(L, block_counters);
   const int lane = threadIdx.x & 31;
@@ -3396,17 +3445,11 @@ __global__ void __launch_bounds__(128, 4) k_tail(DevModel m, DevTallies t, Tally
     Rho<R> rho = load_rho<R>(m, cidx(m, s.p.ir, s.p.it, s.p.ip));
     unsigned long long slot = 0ull, slot_end = 0ull;
     for (int nrec = 0; !kPeel || nrec < E;) {
-      bool tried = false, pending = true;
       if constexpr (sizeof(R) == 4) {
-        ensure(rng, 6 * kAhead);
-        const Batch b = tail_batch<kPeel>(m, dv, t, a, s.p, rng, s.f, rho, L, queue, qcount, slot, slot_end,
-                                          kPeel ? E - nrec : kAhead);
-        nrec += b.n + (b.wall ? 1 : 0);
-        if (b.n > 0 && !b.wall) continue;
-        tried = b.far;
-        pending = !b.wall;
-      }
-      if (pending) {
+        if (tail_window<kPeel, kFused>(m, dv, t, d, a, s.p, rng, s.f, rho, ahead[threadIdx.x >> 5], L, tr, queue, qcount, slot, slot_end, nrec,
+                                       E))
+          continue;
+      } else {
         ensure(rng, 8);  // an event draws at most 7 beside the tries of a scattering
         PeelRec<R> none;
         if (kPeel && slot == slot_end) {
@@ -3416,12 +3459,11 @@ __global__ void __launch_bounds__(128, 4) k_tail(DevModel m, DevTallies t, Tally
         }
         if (interact<R>(m, dv, t, a, s.p, rng, s.f, L, tr, kPeel ? queue[slot] : none)) ++slot;
         ++nrec;
+        ensure(rng, 8);
+        if (walk<R, kFused>(m, t, d, a, s.p, rng, s.f, rho, L, tr, false) == ST_INTERACT) continue;
       }
-      ensure(rng, 8);
-      if (walk<R, kFused>(m, t, d, a, s.p, rng, s.f, rho, L, tr, false, tried) != ST_INTERACT) {
-        s.stage = 0;
-        break;
-      }
+      s.stage = 0;
+      break;
     }
     L.settle();
     if constexpr (kPeel) {
