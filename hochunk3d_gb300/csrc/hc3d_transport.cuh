@@ -42,9 +42,17 @@ constexpr double kTauMax = 25.0;  // peeloff_3d.f90:40
 // ---- math overloads ---------------------------------------------------------
 __device__ __forceinline__ float xsqrt(float x) { return sqrtf(x); }
 __device__ __forceinline__ double xsqrt(double x) { return sqrt(x); }
-__device__ __forceinline__ float xcos(float x) { return cosf(x); }
+// every angle here lies within a few turns: the assumption drops the reduction
+// of large arguments, 2 KB of code at each call
+__device__ __forceinline__ float xcos(float x) {
+  __builtin_assume(fabsf(x) < 1024.f);
+  return cosf(x);
+}
 __device__ __forceinline__ double xcos(double x) { return cos(x); }
-__device__ __forceinline__ float xsin(float x) { return sinf(x); }
+__device__ __forceinline__ float xsin(float x) {
+  __builtin_assume(fabsf(x) < 1024.f);
+  return sinf(x);
+}
 __device__ __forceinline__ double xsin(double x) { return sin(x); }
 __device__ __forceinline__ float xacos(float x) { return acosf(x); }
 __device__ __forceinline__ double xacos(double x) { return acos(x); }
@@ -161,43 +169,42 @@ struct WarpRng {
 
 template <class G> struct IsWarp { static constexpr bool value = false; };
 template <class R> struct IsWarp<WarpRng<R>> { static constexpr bool value = true; };
-// whether the caller of select_dust has the density of the cell at hand
-struct OneDraw;
-template <class G> struct KnowsRho { static constexpr bool value = IsWarp<G>::value; };
-template <> struct KnowsRho<OneDraw> { static constexpr bool value = true; };
-
-template <class R> __device__ __forceinline__ void fill_draws(WarpRng<R>& r) {
-  r.block += (uint32_t)(r.at >> 2);
-  r.at &= 3;
+// the draws of Philox blocks block .. of a stream into a table (not inlined: a
+// warp that runs one packet keeps its code small, see k_tail)
+template <class R>
+static __device__ __noinline__ void fill_table(DrawTable<R>* t, uint32_t block, uint32_t c2, uint32_t c3, uint32_t k0,
+                                               uint32_t k1) {
   const int lane = threadIdx.x & 31;
   __syncwarp();  // the lanes have read what they need of the old table
-  if constexpr (sizeof(R) == 4) {
-#pragma unroll
-    for (int h = 0; h < DrawTable<R>::kDraws / 128; ++h) {
-      uint32_t b[4];
-      philox(r.block + (uint32_t)(32 * h + lane), 0u, r.c2, r.c3, r.k0, r.k1, b);
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        r.t->u[128 * h + 4 * lane + j] = ((float)(b[j] >> 8) + 0.5f) * (1.0f / 16777216.0f);
-    }
-  } else {
-    uint32_t b[4];
-    philox(r.block + (uint32_t)lane, 0u, r.c2, r.c3, r.k0, r.k1, b);
 #pragma unroll 1
-    for (int j = 0; j < 4; ++j) {
-      const R u = ((double)pick4(b, j) + 0.5) * (1.0 / 4294967296.0);
-      const int k = 4 * lane + j;
-      r.t->u[k] = u;
-      r.t->nl[k] = -xlog(u);
-      const R mu = R(1) - R(2) * u;
-      r.t->mu[k] = mu;
-      r.t->smu[k] = xsqrt(R(1) - mu * mu);
-      const R phi = (R)kR2p * u;
-      r.t->cphi[k] = xcos(phi);
-      r.t->sphi[k] = xsin(phi);
+  for (int h = 0; h < DrawTable<R>::kDraws / 128; ++h) {
+    uint32_t b[4];
+    philox(block + (uint32_t)(32 * h + lane), 0u, c2, c3, k0, k1, b);
+    const int k = 128 * h + 4 * lane;
+    if constexpr (sizeof(R) == 4) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) t->u[k + j] = ((float)(b[j] >> 8) + 0.5f) * (1.0f / 16777216.0f);
+    } else {
+#pragma unroll 1
+      for (int j = 0; j < 4; ++j) {
+        const R u = ((double)pick4(b, j) + 0.5) * (1.0 / 4294967296.0);
+        t->u[k + j] = u;
+        t->nl[k + j] = -xlog(u);
+        const R mu = R(1) - R(2) * u;
+        t->mu[k + j] = mu;
+        t->smu[k + j] = xsqrt(R(1) - mu * mu);
+        const R phi = (R)kR2p * u;
+        t->cphi[k + j] = xcos(phi);
+        t->sphi[k + j] = xsin(phi);
+      }
     }
   }
   __syncwarp();
+}
+template <class R> __device__ __forceinline__ void fill_draws(WarpRng<R>& r) {
+  r.block += (uint32_t)(r.at >> 2);
+  r.at &= 3;
+  fill_table<R>(r.t, r.block, r.c2, r.c3, r.k0, r.k1);
 }
 template <class R> __device__ __forceinline__ void ensure(WarpRng<R>& r, int n) {
   if (r.at + n > DrawTable<R>::kDraws) fill_draws(r);
@@ -218,29 +225,15 @@ template <class R> __device__ __forceinline__ void rng_save(const WarpRng<R>& r,
   left = (4 - (r.at & 3)) & 3;
 }
 template <class R> __device__ __forceinline__ R ran(WarpRng<R>& r) { return r.t->u[r.at++]; }
-template <class R> __device__ __forceinline__ R neg_log(WarpRng<R>& r) {
-  if constexpr (sizeof(R) == 4) return -xlog(r.t->u[r.at++]);
-  else return r.t->nl[r.at++];
-}
+template <class R> __device__ __forceinline__ R neg_log(WarpRng<R>& r) { return r.t->nl[r.at++]; }
 template <class R> __device__ __forceinline__ void draw_mu(WarpRng<R>& r, R& mu, R& smu) {
-  if constexpr (sizeof(R) == 4) {
-    mu = R(1) - R(2) * r.t->u[r.at++];
-    smu = xsqrt(R(1) - mu * mu);
-  } else {
-    mu = r.t->mu[r.at];
-    smu = r.t->smu[r.at++];
-  }
+  mu = r.t->mu[r.at];
+  smu = r.t->smu[r.at++];
 }
 template <class R> __device__ __forceinline__ void draw_phi(WarpRng<R>& r, R& phi, R& cphi, R& sphi) {
   phi = (R)kR2p * r.t->u[r.at];
-  if constexpr (sizeof(R) == 4) {
-    cphi = xcos(phi);
-    sphi = xsin(phi);
-    r.at++;
-  } else {
-    cphi = r.t->cphi[r.at];
-    sphi = r.t->sphi[r.at++];
-  }
+  cphi = r.t->cphi[r.at];
+  sphi = r.t->sphi[r.at++];
 }
 // one draw, of a lane that works ahead (tail_window)
 struct OneDraw {
@@ -825,9 +818,7 @@ __device__ __forceinline__ void dust_view(const DevModel& m, R* smem, DustView<R
 // Computed once per unique table; species slots sharing a dust file share
 // the result (only kappa_V differs), which is what the per-slot loop of the
 // reference computes for them.
-// kWarp: a whole warp forms the opacities of one packet, and searches the
-// table two levels of 32 rows deep by ballots.
-template <class R, bool kWarp>
+template <class R>
 __device__ __forceinline__ void opacset(const DevModel& m, const DustView<R>& v, Pkt<R>& p, R nu, const RunArgs& a) {
   if constexpr (sizeof(R) == 4) {
     // mixed form: the same bracket from the ln(nu) guide of each table, then
@@ -844,13 +835,6 @@ __device__ __forceinline__ void opacset(const DevModel& m, const DustView<R>& v,
         i0 = i1 = 1;
       } else if (nu <= nud[nl - 1]) {
         i0 = i1 = nl;
-      } else if (kWarp && nl <= 1024) {
-        const int lane = threadIdx.x & 31, st = (nl + 31) >> 5;
-        const int k1 = lane * st;
-        const int base = (__popc(__ballot_sync(0xffffffffu, k1 < nl && nud[min(k1, nl - 1)] >= nu)) - 1) * st;
-        const int k2 = base + lane;
-        i0 = base + __popc(__ballot_sync(0xffffffffu, lane < st && k2 < nl && nud[min(k2, nl - 1)] >= nu));
-        i1 = i0 + 1;
       } else {
         const int b = min(max((int)((logf(nu) - m.dlnlo[u]) * m.dginv[u]), 0), kDustGuide - 1);
         const short2 gb = __ldg(m.dguide + u * kDustGuide + b);
@@ -1183,18 +1167,15 @@ static __device__ __forceinline__ int tauint_mixed(const DevModel& m, const DevT
   }
 }
 
-// tauint_mixed of a packet that a whole warp runs (k_tail), every lane holding
-// the same state.  rho: the density of the packet's cell, kept from one call
-// to the next, so that the next event's step starts without its load.  The
-// safe distance is formed only where it can be larger than the step: it is at
-// most half the cell's radial depth, less a margin above FP32 rounding.
-// tried: the caller has found the step to be longer than it.
+// The wall walk of tauint_mixed for a packet that a whole warp runs (k_tail),
+// every lane holding the same state, from a point whose step is longer than its
+// safe distance.  rho: the density of the packet's cell.
 template <bool kFused>
-static __device__ __forceinline__ int tauint_warp(const DevModel& m, const DevTallies& t, Pkt<float>& p, float tau,
-                                                  Rho<float>& rho, bool tried, Local& L) {
+static __device__ __forceinline__ int wall_walk(const DevModel& m, const DevTallies& t, Pkt<float>& p, float tau,
+                                                Rho<float>& rho, Local& L) {
   const int lane = threadIdx.x & 31;
   const int cap = 4 * (m.nrg + m.ntg + m.npg) + 64;
-  int nreloc = 0, ntiny = 0;
+  int nreloc = 0, ntiny = 0, st;
   Ray ray;
   ray_init(ray, p.x, p.y, p.z, p.ux, p.uy, p.uz);
   PathLen S{0.f, 0.f};
@@ -1202,65 +1183,40 @@ static __device__ __forceinline__ int tauint_warp(const DevModel& m, const DevTa
   // s, lane 4 the path, lane 5 the small grains' path
   const float ps = (float)t.path_scale;
   const float kabs = pick4(p.kapd, lane & 3) * (1.f - pick4(p.albedo, lane & 3));
-  const float ksg = m.sg_on ? pick4(p.kapd, m.sg_slot) * (1.f - pick4(p.albedo, m.sg_slot)) * m.sg_jfac : 0.f;
   unsigned long long* const base = lane < 4 ? t.dtauabs + (int64_t)lane * m.ncell : (lane == 4 ? t.jmean : t.jsg);
-  auto tally = [&](int64_t c, float ds, float rout) {
-    const float r = pick4(rho.v, lane & 3);
-    float q = ds / rout;
-    if (m.sg_on && lane == 5) q = ds * ksg / rout;
-    const float v = lane < 4 ? kabs * r * ds : q;
-    if (lane < 4 ? r > 0.f : (lane == 4 || (lane == 5 && m.sg_on))) atomicAdd(base + c, fxf(v, ps));
-  };
-  int64_t c = cidx(m, p.ir, p.it, p.ip);
-  if (!tried && p.on_wall == 0 && p.ir >= 1 && p.ir <= m.nrg - 1 && p.it >= 1 && p.it <= m.ntg - 1) {
-    const float opac = opacity(p, rho);
-    const float ds = tau / opac;
-    const float rin = __ldg(m.rarrf + p.ir - 1), rout = __ldg(m.rarrf + p.ir);
-    if (opac > 0.f && ds < 0.5f * (rout - rin)) {
-      if (!(ds < p.safe)) p.safe = safe_dist(m, p.x.hi, p.y.hi, p.z.hi, p.ir, p.it, p.ip);
-      if (ds < p.safe) {
-        p.safe = __fsub_rn(p.safe, ds);
-        L.cross++;
-        tally(c, ds, rout);
-        path_add(S, ds);
-        ray_pos(ray, S, p.x, p.y, p.z);
-        return TI_INTERACT;
-      }
-    }
-  }
+  const bool mine = lane <= 4 || (lane == 5 && m.sg_on);
   p.safe = 0.f;
   float tsum = 0.f;
-  auto at = [&]() { ray_pos(ray, S, p.x, p.y, p.z); };
-  auto reloc = [&]() {
-    double x, y, z;
-    ray_at(ray, S, x, y, z);
-    int jr = p.ir, jt = p.it, jp = p.ip;
-    const int where = relocate(m, x, y, z, jr, jt, jp);
-    p.ir = jr; p.it = jt; p.ip = jp;
-    c = cidx(m, p.ir, p.it, p.ip);
-    if (where == 0) rho = load_rho<float>(m, c);
-    return where;
-  };
+  bool locate = false;  // re-derive the cell first
   for (int n = 0;; ++n) {
+    if (locate) {
+      locate = false;
+      ++nreloc;
+      double x, y, z;
+      ray_at(ray, S, x, y, z);
+      int jr = p.ir, jt = p.it, jp = p.ip;
+      const int where = relocate(m, x, y, z, jr, jt, jp);
+      p.ir = jr; p.it = jt; p.ip = jp;
+      if (where == 1) { p.ir = m.nrg; st = TI_ESCAPE; break; }
+      if (where == 2) { p.ir = 0; st = TI_STAR; break; }
+      p.on_wall = 0;
+      rho = load_rho<float>(m, cidx(m, p.ir, p.it, p.ip));
+    }
     if (n > cap || p.it < 1 || p.it > m.ntg - 1 || p.ir < 1 || p.ir > m.nrg - 1) {
       L.fault = n > cap ? F_CAP : F_RANGE;
-      at();
-      return TI_FAULT;
+      st = TI_FAULT;
+      break;
     }
     float dt;
     int iface;
     if (!next_wall_warp<kFused>(m, ray, S, p.ir, p.it, p.ip, p.on_wall, dt, iface)) {
-      at();
       if (nreloc < 4) {
-        ++nreloc;
-        const int where = reloc();
-        if (where == 1) { p.ir = m.nrg; return TI_ESCAPE; }
-        if (where == 2) { p.ir = 0; return TI_STAR; }
-        p.on_wall = 0;
+        locate = true;
         continue;
       }
       L.fault = F_NOWALL;
-      return TI_FAULT;
+      st = TI_FAULT;
+      break;
     }
     const float opac = opacity(p, rho);
     const float tnext = fmaf(opac, dt, tsum);  // the optical depth at the wall
@@ -1269,51 +1225,45 @@ static __device__ __forceinline__ int tauint_warp(const DevModel& m, const DevTa
     const bool stop = tnext > tau;
     float ds = dt;
     if (stop) ds = (tau - tsum) / opac;
-    if (stop) {
-      tally(c, ds, rout);
-      path_add(S, ds);
-      at();
-      p.on_wall = 0;
-      return TI_INTERACT;
+    {
+      const float r = pick4(rho.v, lane & 3);
+      float v = ds / rout;
+      if (lane < 4) v = kabs * r * ds;
+      if (m.sg_on && lane == 5)
+        v = ds * (pick4(p.kapd, m.sg_slot) * (1.f - pick4(p.albedo, m.sg_slot)) * m.sg_jfac) / rout;
+      if (mine && (lane >= 4 || r > 0.f)) atomicAdd(base + cidx(m, p.ir, p.it, p.ip), fxf(v, ps));
     }
-    const int64_t c0 = c;
+    path_add(S, ds);
+    if (stop) {
+      p.on_wall = 0;
+      st = TI_INTERACT;
+      break;
+    }
     tsum = tnext;
     step_index(m.npg, iface, p.ir, p.it, p.ip);
-    // the next cell's density, loaded before the tally of this one
-    Rho<float> next = rho;
-    if (p.ir >= 1 && p.ir <= m.nrg - 1 && p.it >= 1 && p.it <= m.ntg - 1) {
-      c = cidx(m, p.ir, p.it, p.ip);
-      next = load_rho<float>(m, c);
-    }
-    tally(c0, ds, rout);
-    rho = next;
-    path_add(S, dt);
     p.on_wall = 1 << own_after(iface);
-    if (p.ir == m.nrg) { at(); return TI_ESCAPE; }
-    if (p.ir == 0) { at(); return TI_STAR; }
+    if (p.ir == m.nrg) { st = TI_ESCAPE; break; }
+    if (p.ir == 0) { st = TI_STAR; break; }
+    if (p.it >= 1 && p.it <= m.ntg - 1) rho = load_rho<float>(m, cidx(m, p.ir, p.it, p.ip));
     if (!tiny_step(m, dt, p.ir)) {
       ntiny = 0;
     } else if (++ntiny > 6 && nreloc < 4) {
-      ++nreloc;
       ntiny = 0;
-      at();
-      const int where = reloc();
-      if (where == 1) { p.ir = m.nrg; return TI_ESCAPE; }
-      if (where == 2) { p.ir = 0; return TI_STAR; }
-      p.on_wall = 0;
+      locate = true;
     }
   }
+  ray_pos(ray, S, p.x, p.y, p.z);
+  return st;
 }
 
 // tauint in either form: the FP64 form walks with the reference's wall
 // machinery (closest_wall rule), the mixed form with tauint_mixed.
-// kWarp: a whole warp runs the packet; rho is then the density of its cell.
+// kWarp: a whole warp runs the packet (FP64 form).
 template <class R, bool kFused, bool kWarp>
-__device__ __forceinline__ int tauint(const DevModel& m, const DevTallies& t, Pkt<R>& p, R tau, Rho<R>& rho_, bool tried,
-                                      Local& L, Tracer& tr) {
+__device__ __forceinline__ int tauint(const DevModel& m, const DevTallies& t, Pkt<R>& p, R tau, Local& L, Tracer& tr) {
   if constexpr (sizeof(R) == 4) {
-    if constexpr (kWarp) return tauint_warp<kFused>(m, t, p, tau, rho_, tried, L);
-    else return tauint_mixed<kFused>(m, t, p, tau, L, tr);
+    static_assert(!kWarp, "the mixed form's is wall_walk");
+    return tauint_mixed<kFused>(m, t, p, tau, L, tr);
   } else {
     R tsum = R(0);
     const int cap = 4 * (m.nrg + m.ntg + m.npg) + 64;
@@ -1366,37 +1316,45 @@ __device__ __forceinline__ int tauint(const DevModel& m, const DevTallies& t, Pk
 }
 
 // ---- select_dust.f90:16-42 ---------------------------------------------------
-template <class R, class G>
-__device__ __forceinline__ int select_dust(const DevModel& m, const Pkt<R>& p, const Rho<R>& rho_, G& rng) {
-  const R xran = ran<R>(rng);
-  Rho<R> rho;
-  if constexpr (KnowsRho<G>::value && sizeof(R) == 4) {
-    rho = rho_;
-    // one species with opacity takes every draw (the draw past the rounded
-    // sum of the fractions too, see below)
-    unsigned some = 0u;
-#pragma unroll
-    for (int s = 0; s < kSlots; ++s) some |= p.kapd[s] * rho.v[s] > 0.f ? 1u << s : 0u;
-    if (some != 0u && (some & (some - 1u)) == 0u) return __ffs(some) - 1;
-  } else {
-    rho = load_rho<R>(m, cidx(m, p.ir, p.it, p.ip));
-  }
+template <class R>
+__device__ __forceinline__ int select_species(const R (&kapd)[kSlots], const R (&rho)[kSlots], R xran) {
   R opac = R(0), frac = R(0);
 #pragma unroll
-  for (int s = 0; s < kSlots; ++s) opac += p.kapd[s] * rho.v[s];
+  for (int s = 0; s < kSlots; ++s) opac += kapd[s] * rho[s];
   if (opac == R(0)) return -1;
   int last = -1;
   const R inv = R(1) / opac;  // mixed form: one division
 #pragma unroll
   for (int s = 0; s < kSlots; ++s) {
-    if constexpr (sizeof(R) == 4) frac += p.kapd[s] * rho.v[s] * inv;
-    else frac += p.kapd[s] * rho.v[s] / opac;
-    if (p.kapd[s] * rho.v[s] > R(0)) last = s;
+    if constexpr (sizeof(R) == 4) frac += kapd[s] * rho[s] * inv;
+    else frac += kapd[s] * rho[s] / opac;
+    if (kapd[s] * rho[s] > R(0)) last = s;
     if (xran <= frac + (R)(double)1.e-10f) return s;
   }
   // FP32 fractions can sum to just below 1; the draw then belongs to the
   // last species with opacity (the FP64 form keeps the reference's stop)
   return sizeof(R) == 4 ? last : -1;
+}
+
+template <class R, class G>
+__device__ __forceinline__ int select_dust(const DevModel& m, const Pkt<R>& p, G& rng) {
+  const R xran = ran<R>(rng);
+  return select_species<R>(p.kapd, load_rho<R>(m, cidx(m, p.ir, p.it, p.ip)).v, xran);
+}
+
+// the same for a warp that runs one packet: one species with opacity takes
+// every draw (the draw past the rounded sum of the fractions too, see above)
+static __device__ __noinline__ int select_known(float k0, float k1, float k2, float k3, float r0, float r1, float r2,
+                                                float r3, float xran) {
+  const float kapd[kSlots] = {k0, k1, k2, k3}, rho[kSlots] = {r0, r1, r2, r3};
+  unsigned some = 0u;
+#pragma unroll
+  for (int s = 0; s < kSlots; ++s) some |= kapd[s] * rho[s] > 0.f ? 1u << s : 0u;
+  if (some != 0u && (some & (some - 1u)) == 0u) return __ffs(some) - 1;
+  return select_species<float>(kapd, rho, xran);
+}
+__device__ __forceinline__ int select_known(const Pkt<float>& p, const Rho<float>& rho, float xran) {
+  return select_known(p.kapd[0], p.kapd[1], p.kapd[2], p.kapd[3], rho.v[0], rho.v[1], rho.v[2], rho.v[3], xran);
 }
 
 // ---- dustmat.f90:40-65 -----------------------------------------------------------
@@ -2209,8 +2167,7 @@ __device__ __forceinline__ void peel_all(const DevModel& m, const DevTallies& t,
 // once per temperature update (lucy_row) and read here, 8 bytes.  The frequency
 // index is the same bracket of the interpolated CDF as the reference's
 // bisection (the CDF is non-decreasing, so the bracket is unique), found
-// from the guide table and a short bisection over the interleaved rows; a
-// warp that runs one packet reads the guide's whole bracket at once.
+// from the guide table and a short bisection over the interleaved rows.
 template <class G>
 __device__ __forceinline__ float lucy_freq_mixed(const DevModel& m, int64_t c, int id, G& rng) {
   const int nnu = m.nnu;
@@ -2234,48 +2191,23 @@ __device__ __forceinline__ float lucy_freq_mixed(const DevModel& m, int64_t c, i
     return T0 * __ldg(nuint + nnu - 1);
   }
   int i0 = g.x, i1 = g.y;
-  bool found = false;
-  float2 nn;  // the frequency of row i0 and its ratio to the next
-  if constexpr (IsWarp<G>::value) {
-    // lane j has P(i0 + j); the CDF does not decrease, so the last value <= xi
-    // and the first > xi are neighbours
-    const int i = min(i0 + (int)(threadIdx.x & 31), i1);
+  const float Pa = P(i0), Pb = P(i1);
+  if (Pa <= xi) P0 = Pa; else i0 = 1;
+  if (Pb > xi) P1 = Pb; else i1 = nnu;
+  if (i1 <= i0) { i0 = 1; i1 = nnu; P0 = Pf; P1 = Pl; }
+  while (i1 - i0 > 1) {
+    const int i = (i0 + i1) / 2;
     const float v = P(i);
-    const float2 nv = __ldg(m.nuratio + i - 1);
-    const unsigned above = __ballot_sync(0xffffffffu, v > xi);
-    if (above != 0u && (above & 1u) == 0u) {
-      const int w1 = __ffs(above) - 1;
-      P0 = __shfl_sync(0xffffffffu, v, w1 - 1);
-      P1 = __shfl_sync(0xffffffffu, v, w1);
-      nn.x = __shfl_sync(0xffffffffu, nv.x, w1 - 1);
-      nn.y = __shfl_sync(0xffffffffu, nv.y, w1 - 1);
-      found = true;
-    }
+    if (v > xi) { i1 = i; P1 = v; }
+    else { i0 = i; P0 = v; }
   }
-  if (!found) {
-    const float Pa = P(i0), Pb = P(i1);
-    if (Pa <= xi) P0 = Pa; else i0 = 1;
-    if (Pb > xi) P1 = Pb; else i1 = nnu;
-    if (i1 <= i0) { i0 = 1; i1 = nnu; P0 = Pf; P1 = Pl; }
-    while (i1 - i0 > 1) {
-      const int i = (i0 + i1) / 2;
-      const float v = P(i);
-      if (v > xi) { i1 = i; P1 = v; }
-      else { i0 = i; P0 = v; }
-    }
-    nn = __ldg(m.nuratio + i0 - 1);
-  }
+  const float2 nn = __ldg(m.nuratio + i0 - 1);  // the frequency of row i0 and its ratio to the next
   float w;
   if (xi < P0) w = 0.f;
   else if (xi > P1) w = 1.f;
   else if (P0 <= 0.f) w = 0.5f;
   else if (P1 <= 0.f || xi <= 0.f) w = f;
-  else if constexpr (IsWarp<G>::value) {
-    const float l = logf(((threadIdx.x & 31) == 0 ? xi : P1) / P0);  // lane 0 the numerator, the others the denominator
-    w = __shfl_sync(0xffffffffu, l, 0) / __shfl_sync(0xffffffffu, l, 1);
-  } else {
-    w = logf(xi / P0) / logf(P1 / P0);
-  }
+  else w = logf(xi / P0) / logf(P1 / P0);
   return T0 * nn.x * powf(nn.y, w);
 }
 
@@ -2602,7 +2534,7 @@ __device__ bool emit_star(const DevModel& m, const DustView<R>& dv, const RunArg
     p.nub = atmosfreq<R>(m, rng);
   }
   p.i_orig = 1;
-  opacset<R, false>(m, dv, p, p.nub, a);
+  opacset<R>(m, dv, p, p.nub, a);
   const R coslp = xcos(p.lp), sinlp = xsin(p.lp);
   const double rp_ = (double)p.sinb;
   set_pos(p.z, (double)p.cosb);
@@ -2659,7 +2591,7 @@ __device__ void emit_external(const DevModel& m, const DustView<R>& dv, const Ru
   initp_transform<R>(p);
   p.nub = rep_isrf<R>(m, rng);
   p.i_orig = 4;
-  opacset<R, false>(m, dv, p, p.nub, a);
+  opacset<R>(m, dv, p, p.nub, a);
   const R coslp = xcos(p.lp), sinlp = xsin(p.lp);
   const double zp = (double)p.cosb * a.rmax * 0.999999, rp_ = (double)p.sinb * a.rmax * 0.999999;
   set_pos(p.z, zp);
@@ -2812,7 +2744,7 @@ __device__ __forceinline__ bool emit_acc(const DevModel& m, const DustView<R>& d
   }
   p.ux = p.sint * p.cosp; p.uy = p.sint * p.sinp; p.uz = p.cost;
   p.i_orig = 2;
-  opacset<R, false>(m, dv, p, p.nub, a);
+  opacset<R>(m, dv, p, p.nub, a);
   tr.add(0, p.ir, p.it, p.ip, 0, 0.0, dval(p.x), dval(p.y), dval(p.z));
   make_rec<R>(rec, p, a, 0, idust2 < 0 ? 0 : idust2);
   return true;
@@ -2845,15 +2777,14 @@ __device__ __forceinline__ bool emit(const DevModel& m, const DustView<R>& dv, c
 // G: the packet's draws, one lane's (Rng) or a warp's (WarpRng, k_tail).
 template <class R, bool kFused, class G>
 __device__ __forceinline__ int walk(const DevModel& m, const DevTallies& t, const TallyDims& d, const RunArgs& a, Pkt<R>& p, G& rng,
-                    Flow<R>& f, Rho<R>& rho, Local& L, Tracer& tr, bool first,
-                    bool tried = false) {
+                    Flow<R>& f, Local& L, Tracer& tr, bool first) {
   const R tau = neg_log<R>(rng);
   if (!first) {
     f.xpold = p.x; f.ypold = p.y; f.zpold = p.z;
     p.ux = p.sint * p.cosp; p.uy = p.sint * p.sinp; p.uz = p.cost;
   }
   const int pir = p.ir, pit = p.it, pip = p.ip;
-  const int st = tauint<R, kFused, IsWarp<G>::value>(m, t, p, tau, rho, tried, L, tr);
+  const int st = tauint<R, kFused, IsWarp<G>::value>(m, t, p, tau, L, tr);
   if (st == TI_ESCAPE) {
     tr.add(3, p.ir, p.it, p.ip, 0, 0.0, dval(p.x), dval(p.y), dval(p.z));
     if (L.on) bin_escape<R>(t, d, a, p, dval(f.xpold), dval(f.ypold), dval(f.zpold), f.iflag, f.iscat, L);
@@ -2881,7 +2812,7 @@ __device__ __forceinline__ int walk(const DevModel& m, const DevTallies& t, cons
       return ST_DONE;
     }
   }
-  f.idust2 = select_dust<R>(m, p, rho, rng);
+  f.idust2 = select_dust<R>(m, p, rng);
   if (f.idust2 < 0) {
     L.add(HC3D_CNT_STUCK);
     if (L.on) {
@@ -2962,7 +2893,7 @@ __device__ __forceinline__ bool interact(const DevModel& m, const DustView<R>& d
       else p.nub = lucydustfreq<R>(m, tave, idust2, rng);
     }
     f.iflag = 0;
-    opacset<R, IsWarp<G>::value>(m, dv, p, p.nub, a);
+    opacset<R>(m, dv, p, p.nub, a);
     keep = a.ipeel == 1 && !deep_peel<R>(m, p, c);
     if (keep && L.on) make_rec<R>(rec, p, a, 0, idust2);
     f.iint++;
@@ -2991,11 +2922,10 @@ __device__ void run_packet(const DevModel& m, const DustView<R>& dv, const DevTa
   Flow<R> f;
   f.xpold = p.x; f.ypold = p.y; f.zpold = p.z;
   f.iflag = 0; f.iscat = 0; f.iint = 0; f.idust2 = 0; f.ntot = 0;
-  Rho<R> rho;
-  int st = walk<R, kFused>(m, t, d, a, p, rng, f, rho, L, tr, true);
+  int st = walk<R, kFused>(m, t, d, a, p, rng, f, L, tr, true);
   while (st == ST_INTERACT) {
     if (interact<R>(m, dv, t, a, p, rng, f, L, tr, rec)) peel_all<R>(m, t, d, a, rec, L);
-    st = walk<R, kFused>(m, t, d, a, p, rng, f, rho, L, tr, false);
+    st = walk<R, kFused>(m, t, d, a, p, rng, f, L, tr, false);
   }
 }
 
@@ -3177,8 +3107,7 @@ __global__ void __launch_bounds__(128, 3) k_wave(DevModel m, DevTallies t, Tally
         ++slot;  // the slot is kept only when the event made a record
       }
       if (emitted) {
-        Rho<R> rho;
-        const int st = walk<R, kFused>(m, t, d, a, s.p, rng, s.f, rho, L, tr, s.stage == 2);
+        const int st = walk<R, kFused>(m, t, d, a, s.p, rng, s.f, L, tr, s.stage == 2);
         s.stage = st == ST_INTERACT ? 1 : 0;
         if (!kPeel && s.stage == 0) L.settle();
       }
@@ -3224,59 +3153,69 @@ constexpr int kAhead = 16;  // events a lane set looks ahead
 // what the lanes' events leave, in shared memory (a field's 32 values side by
 // side): any lane's is read by the whole warp, and the packet keeps its registers
 enum AheadField {
-  A_COST, A_SINT, A_PHI, A_COSP, A_SINP, A_NUB, A_UX, A_UY, A_UZ, A_DS, A_ALB, A_WHAT, A_OP, A_INUB,
+  A_COST, A_SINT, A_PHI, A_COSP, A_SINP, A_NUB, A_UX, A_UY, A_UZ, A_TAU, A_DS, A_ALB, A_WHAT, A_OP, A_INUB,
   A_KAPD, A_ALBEDO = A_KAPD + kSlots, A_G = A_ALBEDO + kSlots, A_PL = A_G + kSlots, A_FIELDS = A_PL + kSlots
 };
 struct Ahead {
   float v[A_FIELDS][32];
 };
 
-// Runs events until the packet leaves the cell, ends or has run `most` of them
-// (nrec counts them); whether it goes on.
+// Runs events until the packet leaves the cell, ends or has run E of them (nrec
+// counts them); whether it goes on.  Each part has one place in the code: 16
+// warps of an SM are anywhere in it, and at 184 KB, with the parts inlined
+// wherever they were used, 10 of 15 cycles of an instruction were spent waiting
+// for its fetch.
 template <bool kPeel, bool kFused>
 __device__ __forceinline__ bool tail_window(const DevModel& m, const DustView<float>& dv, const DevTallies& t,
                                             const TallyDims& td, const RunArgs& a, Pkt<float>& p, WarpRng<float>& rng,
-                                            Flow<float>& f, Rho<float>& rho, Ahead& ah, Local& L, Tracer& tr,
-                                            PeelRec<float>* queue, unsigned long long* qcount,
-                                            unsigned long long& slot, unsigned long long& slot_end, int& nrec, int E) {
+                                            Flow<float>& f, Ahead& ah, Local& L, PeelRec<float>* queue,
+                                            unsigned long long* qcount, unsigned long long& slot,
+                                            unsigned long long& slot_end, int& nrec, int E) {
   const int lane = threadIdx.x & 31;
-  const int64_t c = cidx(m, p.ir, p.it, p.ip);
-  const int ir0 = p.ir;
-  ensure(rng, 6 * kAhead + 8);
-  const int off0 = 6 * (lane & (kAhead - 1)) + (lane >= kAhead ? 3 : 0);
-  const float* u = rng.t->u + rng.at + off0;
-  const uint32_t from = 4u * rng.block + (uint32_t)rng.at;  // the draw the window starts at
-  // the species a lane's event is assumed to meet: the pending event's is
-  // known, the others' as the packet's present opacities select it
-  OneDraw d{u[lane == 0 ? 0 : -1]};
-  int s = select_dust<float>(m, p, rho, d);
-  if (lane == 0) s = f.idust2;
-  const bool thermal = s >= 0 && !((m.sg_mask >> s) & 1u);
-  if (!thermal) s = 0;
+  const int c = (int)cidx(m, p.ir, p.it, p.ip), ir0 = p.ir, it0 = p.it, ip0 = p.ip;
   constexpr float kLong = 3.402823466e38f;  // a step that needs the wall search
-  __syncwarp();  // the last window's values have been read
+  ensure(rng, 6 * kAhead + 8);
+  const uint32_t from = 4u * rng.block + (uint32_t)rng.at;  // the draw the window starts at
+  Rho<float> rho = load_rho<float>(m, c);
+  const float reach = 0.5f * (__ldg(m.rarrf + ir0) - __ldg(m.rarrf + ir0 - 1));  // no safe distance is longer
+  int s;  // the species this lane's event is assumed to meet
   {
+    const float* u = rng.t->u + rng.at + 6 * (lane & (kAhead - 1)) + (lane >= kAhead ? 3 : 0);
+    // the pending event's is known, the others' as the packet's present
+    // opacities select it
+    s = select_known(p, rho, u[lane == 0 ? 0 : -1]);
+    if (lane == 0) s = f.idust2;
+    const bool none = s < 0;
+    if (none) s = 0;
+    // a small grain's frequency is drawn before its direction (emit_sg.f90)
+    const bool sg = (m.sg_mask >> s) & 1u;
     Pkt<float> q;
-    q.cost = 1.f - 2.f * u[1];
+    OneDraw d{sg ? u[1] : u[3]};
+    if (sg) {
+      const int im = a.iter1 ? 2 : __ldg(m.imean + c);
+      q.nub = (float)rep_draine<float>(m, im, a.iter1 ? 0.0 : __ldg(m.imfract + c), d);
+    } else {
+      q.nub = lucy_freq_mixed(m, c, s, d);
+    }
+    q.cost = 1.f - 2.f * (sg ? u[2] : u[1]);
     q.sint = xsqrt(1.f - q.cost * q.cost);
-    q.phi = (float)kR2p * u[2];
+    q.phi = (float)kR2p * (sg ? u[3] : u[2]);
     q.cosp = xcos(q.phi);
     q.sinp = xsin(q.phi);
-    d.u = u[3];
-    q.nub = lucy_freq_mixed(m, c, s, d);
-    opacset<float, false>(m, dv, q, q.nub, a);
-    const float opac = opacity(q, rho);
-    float ds = -xlog(u[4]) / opac;
-    if (!(opac > 0.f && ds < 0.5f * (__ldg(m.rarrf + p.ir) - __ldg(m.rarrf + p.ir - 1)))) ds = kLong;
-    d.u = u[5];
-    const int sel = select_dust<float>(m, q, rho, d);
+    opacset<float>(m, dv, q, q.nub, a);
+    const float tau = -xlog(u[4]), opac = opacity(q, rho);
+    float ds = tau / opac;
+    if (!(opac > 0.f && ds < reach)) ds = kLong;
+    const int sel = select_known(q, rho, u[5]);
+    __syncwarp();  // the last window's values have been read
     auto put = [&](int k, float v) { ah.v[k][lane] = v; };
     put(A_COST, q.cost); put(A_SINT, q.sint); put(A_PHI, q.phi); put(A_COSP, q.cosp); put(A_SINP, q.sinp);
     put(A_NUB, q.nub);
     put(A_UX, q.sint * q.cosp); put(A_UY, q.sint * q.sinp); put(A_UZ, q.cost);
+    put(A_TAU, tau);
     put(A_DS, ds);
     put(A_ALB, pick4(q.albedo, max(sel, 0)));
-    put(A_WHAT, __int_as_float((thermal ? s : 7) | ((sel < 0 ? 7 : sel) << 4)));
+    put(A_WHAT, __int_as_float((none ? 7 : s) | ((sel < 0 ? 7 : sel) << 4)));
     if constexpr (kPeel) {
       put(A_OP, peel_opacity(m, q, c));
       put(A_INUB, __int_as_float(nu_bin<float>(a, q.nub)));
@@ -3288,29 +3227,8 @@ __device__ __forceinline__ bool tail_window(const DevModel& m, const DustView<fl
       put(A_G + k, q.g[k]);
       put(A_PL + k, q.pl[k]);
     }
+    __syncwarp();
   }
-  __syncwarp();
-  // the packet as the event of lane l left it
-  auto adopt = [&](int l) {
-    p.cost = ah.v[A_COST][l]; p.sint = ah.v[A_SINT][l]; p.phi = ah.v[A_PHI][l];
-    p.cosp = ah.v[A_COSP][l]; p.sinp = ah.v[A_SINP][l]; p.nub = ah.v[A_NUB][l];
-#pragma unroll
-    for (int j = 0; j < kSlots; ++j) {
-      p.kapd[j] = ah.v[A_KAPD + j][l];
-      p.albedo[j] = ah.v[A_ALBEDO + j][l];
-      p.g[j] = ah.v[A_G + j][l];
-      p.pl[j] = ah.v[A_PL + j][l];
-    }
-    p.i_orig = ((m.disk_mask >> (__float_as_int(ah.v[A_WHAT][l]) & 15)) & 1u) ? 2 : 3;
-    p.sip = 1.f; p.sqp = p.sup = p.svp = 0.f;
-  };
-  auto reserve = [&]() {  // a queue slot for the next record
-    if (kPeel && slot == slot_end) {
-      if (lane == 0) slot = atomicAdd(qcount, (unsigned long long)a.qchunk);
-      slot = __shfl_sync(0xffffffffu, slot, 0);
-      slot_end = slot + (unsigned long long)a.qchunk;
-    }
-  };
   unsigned absorbed = 0u, stepped = 0u;  // the lanes whose event was an absorption, a step within the cell
   int left = -1;                         // the lane whose event left the packet, where p does not have it yet
   float alb_now = pick4(p.albedo, f.idust2);
@@ -3321,15 +3239,43 @@ __device__ __forceinline__ bool tail_window(const DevModel& m, const DustView<fl
     ensure(rng, 8);
     const int h = off / 3, l = (h >> 1) + ((h & 1) ? kAhead : 0);
     const int wl = __float_as_int(ah.v[A_WHAT][l]);
+    const bool scat = rng.t->u[rng.at] <= alb_now;
+    if (!scat && (wl & 15) != f.idust2) break;  // lane l assumed another species (never the pending event's)
+    // the packet as the event of a lane left it, for a scattering or a wall search
+    const int src = scat ? left : l;
+    auto adopt = [&]() {
+      p.cost = ah.v[A_COST][src]; p.sint = ah.v[A_SINT][src]; p.phi = ah.v[A_PHI][src];
+      p.cosp = ah.v[A_COSP][src]; p.sinp = ah.v[A_SINP][src]; p.nub = ah.v[A_NUB][src];
+#pragma unroll
+      for (int j = 0; j < kSlots; ++j) {
+        p.kapd[j] = ah.v[A_KAPD + j][src];
+        p.albedo[j] = ah.v[A_ALBEDO + j][src];
+        p.g[j] = ah.v[A_G + j][src];
+        p.pl[j] = ah.v[A_PL + j][src];
+      }
+      p.i_orig = ((m.disk_mask >> (__float_as_int(ah.v[A_WHAT][src]) & 15)) & 1u) ? 2 : 3;
+      p.sip = 1.f; p.sqp = p.sup = p.svp = 0.f;
+      left = -1;
+    };
     ++nrec;
-    bool tried = false;
-    if (rng.t->u[rng.at] > alb_now && (wl & 15) == f.idust2) {
-      // absorbed and re-emitted as lane l has it
-      if constexpr (kPeel) {
-        if (!(p.safe > 0.f && deep_peel_at(p, p.safe, ah.v[A_OP][l]))) {
-          reserve();
-          if (lane == 0) {
-            PeelRec<float>& e = queue[slot];
+    L.events++;
+    f.ntot++;
+    f.iint++;
+    f.iflag = scat ? 1 : 0;
+    if (scat && left >= 0) adopt();
+    if constexpr (kPeel) {  // the event's peel-off record, unless its rays end in the cell
+      const float op = scat ? (p.safe > 0.f ? peel_opacity(m, p, c) : 0.f) : ah.v[A_OP][l];
+      if (!(p.safe > 0.f && deep_peel_at(p, p.safe, op))) {
+        if (slot == slot_end) {
+          if (lane == 0) slot = atomicAdd(qcount, (unsigned long long)a.qchunk);
+          slot = __shfl_sync(0xffffffffu, slot, 0);
+          slot_end = slot + (unsigned long long)a.qchunk;
+        }
+        if (lane == 0) {
+          PeelRec<float>& e = queue[slot];
+          if (scat) {
+            make_rec<float>(e, p, a, 1, f.idust2);
+          } else {
             const int sl = wl & 15;
             e.x = p.x; e.y = p.y; e.z = p.z;
             e.ir = p.ir; e.it = p.it; e.ip = p.ip;
@@ -3342,55 +3288,109 @@ __device__ __forceinline__ bool tail_window(const DevModel& m, const DustView<fl
 #pragma unroll
             for (int k = 0; k < kSlots; ++k) e.kapd[k] = ah.v[A_KAPD + k][l];
           }
-          ++slot;
         }
+        ++slot;
       }
-      const float dsl = ah.v[A_DS][l];
-      L.events++;
-      f.ntot++;
-      f.iint++;
-      f.iflag = 0;
-      absorbed |= 1u << l;
-      // a packet that reaches a cap is killed in walk()
-      const bool capped = f.iint > a.iintmax || (a.max_interactions > 0 && f.ntot >= a.max_interactions);
-      if (!capped && wl < 0x70) {
-        if (!(dsl < p.safe) && dsl < kLong) p.safe = safe_dist(m, p.x.hi, p.y.hi, p.z.hi, p.ir, p.it, p.ip);
-        if (dsl < p.safe) {
-          p.safe = __fsub_rn(p.safe, dsl);
-          const PathLen S{dsl, 0.f};
-          p.x = pos_step(p.x, S, ah.v[A_UX][l]);
-          p.y = pos_step(p.y, S, ah.v[A_UY][l]);
-          p.z = pos_step(p.z, S, ah.v[A_UZ][l]);
-          L.cross++;
-          stepped |= 1u << l;
-          rng.at += 6;
-          f.idust2 = wl >> 4;
-          alb_now = ah.v[A_ALB][l];
-          left = l;
-          continue;
-        }
-        tried = true;
-      }
-      adopt(l);
-      left = -1;
-      rng.at += 4;
-    } else {
-      if (left >= 0) adopt(left);
-      left = -1;
-      PeelRec<float> none;
-      reserve();
-      if (interact<float>(m, dv, t, a, p, rng, f, L, tr, kPeel ? queue[slot] : none)) ++slot;
-      ensure(rng, 8);
     }
-    const int ir = p.ir, it = p.it, ip = p.ip;
-    live = walk<float, kFused>(m, t, td, a, p, rng, f, rho, L, tr, false, tried) == ST_INTERACT;
-    here = live && p.ir == ir && p.it == it && p.ip == ip;
-    if (live) alb_now = pick4(p.albedo, f.idust2);
+    float tau, ds;
+    if (scat) {
+      f.iscat++;
+      rng.at++;
+      stokes<float>(p, f.idust2, rng);
+      ensure(rng, 2);
+      tau = -xlog(rng.t->u[rng.at++]);
+      const float opac = opacity(p, rho);
+      ds = tau / opac;
+      if (!(opac > 0.f && ds < reach)) ds = kLong;
+      p.ux = p.sint * p.cosp; p.uy = p.sint * p.sinp; p.uz = p.cost;
+      if (lane == l) {  // the step's tally is this lane's to make, whose own event did not happen
+#pragma unroll
+        for (int k = 0; k < kSlots; ++k) {
+          ah.v[A_KAPD + k][l] = p.kapd[k];
+          ah.v[A_ALBEDO + k][l] = p.albedo[k];
+        }
+        ah.v[A_DS][l] = ds;
+      }
+    } else {
+      absorbed |= 1u << l;
+      rng.at += 5;
+      tau = ah.v[A_TAU][l];
+      ds = ah.v[A_DS][l];
+      p.ux = ah.v[A_UX][l]; p.uy = ah.v[A_UY][l]; p.uz = ah.v[A_UZ][l];
+    }
+    if (!(ds < p.safe) && ds < kLong) p.safe = safe_dist(m, p.x.hi, p.y.hi, p.z.hi, p.ir, p.it, p.ip);
+    if (ds < p.safe) {
+      p.safe = __fsub_rn(p.safe, ds);
+      const PathLen S{ds, 0.f};
+      p.x = pos_step(p.x, S, p.ux);
+      p.y = pos_step(p.y, S, p.uy);
+      p.z = pos_step(p.z, S, p.uz);
+      L.cross++;
+      stepped |= 1u << l;
+      if (!scat) left = l;
+    } else {
+      if (!scat) adopt();
+      f.xpold = p.x; f.ypold = p.y; f.zpold = p.z;
+      const int st = wall_walk<kFused>(m, t, p, tau, rho, L);
+      if (st != TI_INTERACT) {
+        if (st == TI_ESCAPE) {
+          if (lane == 0)
+            bin_escape<float>(t, td, a, p, dval(f.xpold), dval(f.ypold), dval(f.zpold), f.iflag, f.iscat, L);
+        } else if (st == TI_STAR) {
+          L.add(HC3D_CNT_AFLUX);
+        } else {
+          L.add(HC3D_CNT_STUCK);
+          if (lane == 0) {
+            set_status(a, 1);
+            log_fault(t, rng, L.fault);
+          }
+        }
+        live = false;
+        break;
+      }
+      here = p.ir == ir0 && p.it == it0 && p.ip == ip0;
+      if (!here) f.iint = 0;
+    }
+    if (f.iint > a.iintmax || (a.max_interactions > 0 && f.ntot >= a.max_interactions)) {
+      if (lane == 0) atomicAdd(t.killed + cidx(m, p.ir, p.it, p.ip), 1u);
+      L.add(HC3D_CNT_ABFLUX);
+      live = false;
+      break;
+    }
+    // the species that the next event meets
+    if (left >= 0 && left == l) {
+      rng.at++;
+      f.idust2 = wl >> 4;
+      alb_now = ah.v[A_ALB][l];
+    } else {
+      f.idust2 = select_known(p, rho, rng.t->u[rng.at++]);
+      alb_now = pick4(p.albedo, max(f.idust2, 0));
+    }
+    if (f.idust2 < 0 || f.idust2 > kSlots) {
+      L.add(HC3D_CNT_STUCK);
+      if (lane == 0) {
+        set_status(a, 2);
+        log_fault(t, rng, F_SELECT);
+      }
+      live = false;
+      break;
+    }
   }
-  if (left >= 0) adopt(left);
-  const float rout = __ldg(m.rarrf + ir0);
+  if (live && left >= 0) {  // the packet as its last event left it, for the next window
+    p.cost = ah.v[A_COST][left]; p.sint = ah.v[A_SINT][left]; p.phi = ah.v[A_PHI][left];
+    p.cosp = ah.v[A_COSP][left]; p.sinp = ah.v[A_SINP][left]; p.nub = ah.v[A_NUB][left];
+#pragma unroll
+    for (int j = 0; j < kSlots; ++j) {
+      p.kapd[j] = ah.v[A_KAPD + j][left];
+      p.albedo[j] = ah.v[A_ALBEDO + j][left];
+      p.g[j] = ah.v[A_G + j][left];
+      p.pl[j] = ah.v[A_PL + j][left];
+    }
+    p.i_orig = ((m.disk_mask >> (__float_as_int(ah.v[A_WHAT][left]) & 15)) & 1u) ? 2 : 3;
+    p.sip = 1.f; p.sqp = p.sup = p.svp = 0.f;
+  }
   if ((absorbed >> lane) & 1u) {
-    atomicAdd(t.dbig + c, 1u);
+    atomicAdd(((m.sg_mask >> s) & 1u ? t.dsg : t.dbig) + c, 1u);
     atomicAdd(t.nabs + (int64_t)s * m.ncell + c, 1ull);
   }
   if ((stepped >> lane) & 1u) {
@@ -3400,7 +3400,7 @@ __device__ __forceinline__ bool tail_window(const DevModel& m, const DustView<fl
       q.kapd[k] = ah.v[A_KAPD + k][lane];
       q.albedo[k] = ah.v[A_ALBEDO + k][lane];
     }
-    tally_path<float>(m, t, q, load_rho<float>(m, c), c, ah.v[A_DS][lane], rout);
+    tally_path<float>(m, t, q, load_rho<float>(m, c), c, ah.v[A_DS][lane], __ldg(m.rarrf + ir0));
   }
   return live;
 }
@@ -3442,11 +3442,10 @@ __global__ void __launch_bounds__(128, 4) k_tail(DevModel m, DevTallies t, Tally
     Slot<R> s = pool[gid];
     WarpRng<R> rng;
     rng_init(rng, draws + (threadIdx.x >> 5), a.key0, a.key1, s.pid, s.c0, s.left);
-    Rho<R> rho = load_rho<R>(m, cidx(m, s.p.ir, s.p.it, s.p.ip));
     unsigned long long slot = 0ull, slot_end = 0ull;
     for (int nrec = 0; !kPeel || nrec < E;) {
       if constexpr (sizeof(R) == 4) {
-        if (tail_window<kPeel, kFused>(m, dv, t, d, a, s.p, rng, s.f, rho, ahead[threadIdx.x >> 5], L, tr, queue, qcount, slot, slot_end, nrec,
+        if (tail_window<kPeel, kFused>(m, dv, t, d, a, s.p, rng, s.f, ahead[threadIdx.x >> 5], L, queue, qcount, slot, slot_end, nrec,
                                        E))
           continue;
       } else {
@@ -3460,7 +3459,7 @@ __global__ void __launch_bounds__(128, 4) k_tail(DevModel m, DevTallies t, Tally
         if (interact<R>(m, dv, t, a, s.p, rng, s.f, L, tr, kPeel ? queue[slot] : none)) ++slot;
         ++nrec;
         ensure(rng, 8);
-        if (walk<R, kFused>(m, t, d, a, s.p, rng, s.f, rho, L, tr, false) == ST_INTERACT) continue;
+        if (walk<R, kFused>(m, t, d, a, s.p, rng, s.f, L, tr, false) == ST_INTERACT) continue;
       }
       s.stage = 0;
       break;
