@@ -497,15 +497,24 @@ __device__ __forceinline__ void ray_at(const Ray& r, const PathLen& S, double& x
   z = fma(s, (double)r.uz, dval(r.zs));
 }
 
-// x + S u as a pair: x a pair, S a pair, u FP32 (error-free product and sum)
-__device__ __forceinline__ Pos2 pos_step(const Pos2& x, const PathLen& S, float u) {
-  const float pr = __fmul_rn(S.hi, u);
-  const float pe = fmaf(S.lo, u, fmaf(S.hi, u, -pr));
+// x + S u as a pair, x and S pairs, u FP32: an error-free product and sum. In
+// two, since the rounded product S u and its rest do not depend on the point.
+__device__ __forceinline__ void step_terms(const PathLen& S, float u, float& pr, float& pe) {
+  pr = __fmul_rn(S.hi, u);
+  pe = fmaf(S.lo, u, fmaf(S.hi, u, -pr));
+}
+__device__ __forceinline__ Pos2 pos_add(const Pos2& x, float pr, float pe) {
   const float sm = __fadd_rn(x.hi, pr);
   const float bp = __fsub_rn(sm, x.hi);
   const float e = __fadd_rn(__fadd_rn(__fsub_rn(x.hi, __fsub_rn(sm, bp)), __fsub_rn(pr, bp)), __fadd_rn(x.lo, pe));
   const float hi = __fadd_rn(sm, e);
   return Pos2{hi, __fsub_rn(e, __fsub_rn(hi, sm))};
+}
+
+__device__ __forceinline__ Pos2 pos_step(const Pos2& x, const PathLen& S, float u) {
+  float pr, pe;
+  step_terms(S, u, pr, pe);
+  return pos_add(x, pr, pe);
 }
 
 // the point of the ray at path length S, as pairs
@@ -3153,7 +3162,8 @@ constexpr int kAhead = 16;  // events a lane set looks ahead
 // what the lanes' events leave, in shared memory (a field's 32 values side by
 // side): any lane's is read by the whole warp, and the packet keeps its registers
 enum AheadField {
-  A_COST, A_SINT, A_PHI, A_COSP, A_SINP, A_NUB, A_UX, A_UY, A_UZ, A_TAU, A_DS, A_ALB, A_WHAT, A_OP, A_INUB,
+  A_COST, A_SINT, A_PHI, A_COSP, A_SINP, A_NUB, A_TAU, A_DS, A_ALB, A_WHAT, A_OP, A_INUB,
+  A_PX, A_EX, A_PY, A_EY, A_PZ, A_EZ,  // step_terms of the three coordinates
   A_KAPD, A_ALBEDO = A_KAPD + kSlots, A_G = A_ALBEDO + kSlots, A_PL = A_G + kSlots, A_FIELDS = A_PL + kSlots
 };
 struct Ahead {
@@ -3179,6 +3189,8 @@ __device__ __forceinline__ bool tail_window(const DevModel& m, const DustView<fl
   Rho<float> rho = load_rho<float>(m, c);
   const float reach = 0.5f * (__ldg(m.rarrf + ir0) - __ldg(m.rarrf + ir0 - 1));  // no safe distance is longer
   int s;  // the species this lane's event is assumed to meet
+  unsigned follows, sound;  // the lanes whose event is an absorption of the assumed species after that of the lane
+                            // before, and those whose event leaves a species to meet
   {
     const float* u = rng.t->u + rng.at + 6 * (lane & (kAhead - 1)) + (lane >= kAhead ? 3 : 0);
     // the pending event's is known, the others' as the packet's present
@@ -3211,10 +3223,21 @@ __device__ __forceinline__ bool tail_window(const DevModel& m, const DustView<fl
     auto put = [&](int k, float v) { ah.v[k][lane] = v; };
     put(A_COST, q.cost); put(A_SINT, q.sint); put(A_PHI, q.phi); put(A_COSP, q.cosp); put(A_SINP, q.sinp);
     put(A_NUB, q.nub);
-    put(A_UX, q.sint * q.cosp); put(A_UY, q.sint * q.sinp); put(A_UZ, q.cost);
+    float pr, pe;
+    step_terms(PathLen{ds, 0.f}, q.sint * q.cosp, pr, pe);
+    put(A_PX, pr); put(A_EX, pe);
+    step_terms(PathLen{ds, 0.f}, q.sint * q.sinp, pr, pe);
+    put(A_PY, pr); put(A_EY, pe);
+    step_terms(PathLen{ds, 0.f}, q.cost, pr, pe);
+    put(A_PZ, pr); put(A_EZ, pe);
     put(A_TAU, tau);
     put(A_DS, ds);
-    put(A_ALB, pick4(q.albedo, max(sel, 0)));
+    const float alb = pick4(q.albedo, max(sel, 0));
+    put(A_ALB, alb);
+    const float alb_before = __shfl_up_sync(0xffffffffu, alb, 1);
+    const int sel_before = __shfl_up_sync(0xffffffffu, sel, 1);
+    follows = __ballot_sync(0xffffffffu, (lane & (kAhead - 1)) != 0 && !none && sel_before == s && u[0] > alb_before);
+    sound = __ballot_sync(0xffffffffu, sel >= 0);
     put(A_WHAT, __int_as_float((none ? 7 : s) | ((sel < 0 ? 7 : sel) << 4)));
     if constexpr (kPeel) {
       put(A_OP, peel_opacity(m, q, c));
@@ -3231,67 +3254,113 @@ __device__ __forceinline__ bool tail_window(const DevModel& m, const DustView<fl
   }
   unsigned absorbed = 0u, stepped = 0u;  // the lanes whose event was an absorption, a step within the cell
   int left = -1;                         // the lane whose event left the packet, where p does not have it yet
+  auto adopt = [&](int l) {              // the packet as the event of lane l left it
+    p.cost = ah.v[A_COST][l]; p.sint = ah.v[A_SINT][l]; p.phi = ah.v[A_PHI][l];
+    p.cosp = ah.v[A_COSP][l]; p.sinp = ah.v[A_SINP][l]; p.nub = ah.v[A_NUB][l];
+#pragma unroll
+    for (int j = 0; j < kSlots; ++j) {
+      p.kapd[j] = ah.v[A_KAPD + j][l];
+      p.albedo[j] = ah.v[A_ALBEDO + j][l];
+      p.g[j] = ah.v[A_G + j][l];
+      p.pl[j] = ah.v[A_PL + j][l];
+    }
+    p.i_orig = ((m.disk_mask >> (__float_as_int(ah.v[A_WHAT][l]) & 15)) & 1u) ? 2 : 3;
+    p.sip = 1.f; p.sqp = p.sup = p.svp = 0.f;
+    left = -1;
+  };
+  // the peel-off record of an event, the absorption of lane l or a scattering
+  // (l < 0) of p, unless its rays end in the cell
+  auto record = [&](int l) {
+    if constexpr (kPeel) {
+      const float op = l >= 0 ? ah.v[A_OP][l] : (p.safe > 0.f ? peel_opacity(m, p, c) : 0.f);
+      if (p.safe > 0.f && deep_peel_at(p, p.safe, op)) return;
+      if (slot == slot_end) {
+        if (lane == 0) slot = atomicAdd(qcount, (unsigned long long)a.qchunk);
+        slot = __shfl_sync(0xffffffffu, slot, 0);
+        slot_end = slot + (unsigned long long)a.qchunk;
+      }
+      if (lane == 0) {
+        PeelRec<float>& e = queue[slot];
+        if (l < 0) {
+          make_rec<float>(e, p, a, 1, f.idust2);
+        } else {
+          const int sl = __float_as_int(ah.v[A_WHAT][l]) & 15;
+          e.x = p.x; e.y = p.y; e.z = p.z;
+          e.ir = p.ir; e.it = p.it; e.ip = p.ip;
+          e.flags = (((m.disk_mask >> sl) & 1u ? 2 : 3) << 2) | (sl << 5);
+          e.inub = __float_as_int(ah.v[A_INUB][l]);
+          e.sip = 1.f; e.sqp = e.sup = e.svp = 0.f;
+          e.d0 = ah.v[A_COST][l]; e.d1 = ah.v[A_SINT][l]; e.d2 = ah.v[A_PHI][l]; e.d3 = ah.v[A_COSP][l];
+          e.d4 = ah.v[A_SINP][l];
+          e.g = ah.v[A_G + sl][l]; e.pl = ah.v[A_PL + sl][l];
+#pragma unroll
+          for (int k = 0; k < kSlots; ++k) e.kapd[k] = ah.v[A_KAPD + k][l];
+        }
+      }
+      ++slot;
+    }
+  };
   float alb_now = pick4(p.albedo, f.idust2);
   bool live = true, here = true;
   while (here && (!kPeel || nrec < E)) {
     const int off = (int)(4u * rng.block + (uint32_t)rng.at - from);
     if (off > 6 * kAhead - 3) break;
     ensure(rng, 8);
-    const int h = off / 3, l = (h >> 1) + ((h & 1) ? kAhead : 0);
-    const int wl = __float_as_int(ah.v[A_WHAT][l]);
+    const int h = off / 3;
+    int l = (h >> 1) + ((h & 1) ? kAhead : 0);
     const bool scat = rng.t->u[rng.at] <= alb_now;
-    if (!scat && (wl & 15) != f.idust2) break;  // lane l assumed another species (never the pending event's)
-    // the packet as the event of a lane left it, for a scattering or a wall search
-    const int src = scat ? left : l;
-    auto adopt = [&]() {
-      p.cost = ah.v[A_COST][src]; p.sint = ah.v[A_SINT][src]; p.phi = ah.v[A_PHI][src];
-      p.cosp = ah.v[A_COSP][src]; p.sinp = ah.v[A_SINP][src]; p.nub = ah.v[A_NUB][src];
-#pragma unroll
-      for (int j = 0; j < kSlots; ++j) {
-        p.kapd[j] = ah.v[A_KAPD + j][src];
-        p.albedo[j] = ah.v[A_ALBEDO + j][src];
-        p.g[j] = ah.v[A_G + j][src];
-        p.pl[j] = ah.v[A_PL + j][src];
+    bool far = false;
+    if (!scat) {
+      if ((__float_as_int(ah.v[A_WHAT][l]) & 15) != f.idust2) break;  // it assumed another species (not the pending event's)
+      // the run of absorptions from here, as far as their steps are safe and no cap is reached
+      int len = min(__ffs(~(follows >> 1 >> l)), __ffs(~(sound >> l) | 1u << kAhead) - 1);
+      len = min(len, a.iintmax - f.iint);
+      if (a.max_interactions > 0) len = (int)min((int64_t)len, a.max_interactions - f.ntot - 1);
+      if (kPeel) len = min(len, E - nrec);
+      int k = 0;
+      for (; k < len; ++k) {
+        const float ds = ah.v[A_DS][l + k];
+        float safe = p.safe;
+        if (!(ds < safe)) {
+          if (ds < kLong) safe = safe_dist(m, p.x.hi, p.y.hi, p.z.hi, p.ir, p.it, p.ip);
+          if (!(ds < safe)) {
+            far = true;
+            break;
+          }
+        }
+        record(l + k);
+        p.safe = __fsub_rn(safe, ds);
+        p.x = pos_add(p.x, ah.v[A_PX][l + k], ah.v[A_EX][l + k]);
+        p.y = pos_add(p.y, ah.v[A_PY][l + k], ah.v[A_EY][l + k]);
+        p.z = pos_add(p.z, ah.v[A_PZ][l + k], ah.v[A_EZ][l + k]);
       }
-      p.i_orig = ((m.disk_mask >> (__float_as_int(ah.v[A_WHAT][src]) & 15)) & 1u) ? 2 : 3;
-      p.sip = 1.f; p.sqp = p.sup = p.svp = 0.f;
-      left = -1;
-    };
+      if (k > 0) {
+        const unsigned bits = ((1u << k) - 1u) << l;
+        absorbed |= bits;
+        stepped |= bits;
+        L.events += k;
+        L.cross += k;
+        f.ntot += k;
+        f.iint += k;
+        f.iflag = 0;
+        nrec += k;
+        rng.at += 6 * k;
+        l += k;
+        left = l - 1;
+        f.idust2 = __float_as_int(ah.v[A_WHAT][left]) >> 4;
+        alb_now = ah.v[A_ALB][left];
+        if (!far) continue;  // a scattering, another species or a cap is next
+        if (kPeel && nrec >= E) break;
+      }
+    }
     ++nrec;
     L.events++;
     f.ntot++;
     f.iint++;
     f.iflag = scat ? 1 : 0;
-    if (scat && left >= 0) adopt();
-    if constexpr (kPeel) {  // the event's peel-off record, unless its rays end in the cell
-      const float op = scat ? (p.safe > 0.f ? peel_opacity(m, p, c) : 0.f) : ah.v[A_OP][l];
-      if (!(p.safe > 0.f && deep_peel_at(p, p.safe, op))) {
-        if (slot == slot_end) {
-          if (lane == 0) slot = atomicAdd(qcount, (unsigned long long)a.qchunk);
-          slot = __shfl_sync(0xffffffffu, slot, 0);
-          slot_end = slot + (unsigned long long)a.qchunk;
-        }
-        if (lane == 0) {
-          PeelRec<float>& e = queue[slot];
-          if (scat) {
-            make_rec<float>(e, p, a, 1, f.idust2);
-          } else {
-            const int sl = wl & 15;
-            e.x = p.x; e.y = p.y; e.z = p.z;
-            e.ir = p.ir; e.it = p.it; e.ip = p.ip;
-            e.flags = (((m.disk_mask >> sl) & 1u ? 2 : 3) << 2) | (sl << 5);
-            e.inub = __float_as_int(ah.v[A_INUB][l]);
-            e.sip = 1.f; e.sqp = e.sup = e.svp = 0.f;
-            e.d0 = ah.v[A_COST][l]; e.d1 = ah.v[A_SINT][l]; e.d2 = ah.v[A_PHI][l]; e.d3 = ah.v[A_COSP][l];
-            e.d4 = ah.v[A_SINP][l];
-            e.g = ah.v[A_G + sl][l]; e.pl = ah.v[A_PL + sl][l];
-#pragma unroll
-            for (int k = 0; k < kSlots; ++k) e.kapd[k] = ah.v[A_KAPD + k][l];
-          }
-        }
-        ++slot;
-      }
-    }
+    const int src = scat ? left : l;
+    if (scat && src >= 0) adopt(src);
+    record(scat ? -1 : l);
     float tau, ds;
     if (scat) {
       f.iscat++;
@@ -3302,7 +3371,6 @@ __device__ __forceinline__ bool tail_window(const DevModel& m, const DustView<fl
       const float opac = opacity(p, rho);
       ds = tau / opac;
       if (!(opac > 0.f && ds < reach)) ds = kLong;
-      p.ux = p.sint * p.cosp; p.uy = p.sint * p.sinp; p.uz = p.cost;
       if (lane == l) {  // the step's tally is this lane's to make, whose own event did not happen
 #pragma unroll
         for (int k = 0; k < kSlots; ++k) {
@@ -3312,14 +3380,15 @@ __device__ __forceinline__ bool tail_window(const DevModel& m, const DustView<fl
         ah.v[A_DS][l] = ds;
       }
     } else {
+      adopt(src);
       absorbed |= 1u << l;
       rng.at += 5;
       tau = ah.v[A_TAU][l];
       ds = ah.v[A_DS][l];
-      p.ux = ah.v[A_UX][l]; p.uy = ah.v[A_UY][l]; p.uz = ah.v[A_UZ][l];
     }
-    if (!(ds < p.safe) && ds < kLong) p.safe = safe_dist(m, p.x.hi, p.y.hi, p.z.hi, p.ir, p.it, p.ip);
-    if (ds < p.safe) {
+    p.ux = p.sint * p.cosp; p.uy = p.sint * p.sinp; p.uz = p.cost;
+    if (!far && !(ds < p.safe) && ds < kLong) p.safe = safe_dist(m, p.x.hi, p.y.hi, p.z.hi, p.ir, p.it, p.ip);
+    if (!far && ds < p.safe) {
       p.safe = __fsub_rn(p.safe, ds);
       const PathLen S{ds, 0.f};
       p.x = pos_step(p.x, S, p.ux);
@@ -3327,9 +3396,7 @@ __device__ __forceinline__ bool tail_window(const DevModel& m, const DustView<fl
       p.z = pos_step(p.z, S, p.uz);
       L.cross++;
       stepped |= 1u << l;
-      if (!scat) left = l;
     } else {
-      if (!scat) adopt();
       f.xpold = p.x; f.ypold = p.y; f.zpold = p.z;
       const int st = wall_walk<kFused>(m, t, p, tau, rho, L);
       if (st != TI_INTERACT) {
@@ -3357,16 +3424,8 @@ __device__ __forceinline__ bool tail_window(const DevModel& m, const DustView<fl
       live = false;
       break;
     }
-    // the species that the next event meets
-    if (left >= 0 && left == l) {
-      rng.at++;
-      f.idust2 = wl >> 4;
-      alb_now = ah.v[A_ALB][l];
-    } else {
-      f.idust2 = select_known(p, rho, rng.t->u[rng.at++]);
-      alb_now = pick4(p.albedo, max(f.idust2, 0));
-    }
-    if (f.idust2 < 0 || f.idust2 > kSlots) {
+    f.idust2 = select_known(p, rho, rng.t->u[rng.at++]);  // the species that the next event meets
+    if (f.idust2 < 0) {
       L.add(HC3D_CNT_STUCK);
       if (lane == 0) {
         set_status(a, 2);
@@ -3375,20 +3434,9 @@ __device__ __forceinline__ bool tail_window(const DevModel& m, const DustView<fl
       live = false;
       break;
     }
+    alb_now = pick4(p.albedo, f.idust2);
   }
-  if (live && left >= 0) {  // the packet as its last event left it, for the next window
-    p.cost = ah.v[A_COST][left]; p.sint = ah.v[A_SINT][left]; p.phi = ah.v[A_PHI][left];
-    p.cosp = ah.v[A_COSP][left]; p.sinp = ah.v[A_SINP][left]; p.nub = ah.v[A_NUB][left];
-#pragma unroll
-    for (int j = 0; j < kSlots; ++j) {
-      p.kapd[j] = ah.v[A_KAPD + j][left];
-      p.albedo[j] = ah.v[A_ALBEDO + j][left];
-      p.g[j] = ah.v[A_G + j][left];
-      p.pl[j] = ah.v[A_PL + j][left];
-    }
-    p.i_orig = ((m.disk_mask >> (__float_as_int(ah.v[A_WHAT][left]) & 15)) & 1u) ? 2 : 3;
-    p.sip = 1.f; p.sqp = p.sup = p.svp = 0.f;
-  }
+  if (live && left >= 0) adopt(left);
   if ((absorbed >> lane) & 1u) {
     atomicAdd(((m.sg_mask >> s) & 1u ? t.dsg : t.dbig) + c, 1u);
     atomicAdd(t.nabs + (int64_t)s * m.ncell + c, 1ull);
