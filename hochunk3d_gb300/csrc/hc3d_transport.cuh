@@ -99,9 +99,18 @@ __device__ __forceinline__ T pick4(const T (&a)[4], int i) {
   return i == 0 ? a[0] : (i == 1 ? a[1] : (i == 2 ? a[2] : a[3]));
 }
 
+// one Philox block, out of line: a packet's draws are taken at some forty places
+// of a kernel, and 1.3 KB at each had the kernels wait for their instructions
+static __device__ __noinline__ uint4 philox_block(uint32_t c0, uint32_t c2, uint32_t c3, uint32_t k0, uint32_t k1) {
+  uint32_t b[4];
+  philox(c0, 0u, c2, c3, k0, k1, b);
+  return make_uint4(b[0], b[1], b[2], b[3]);
+}
+
 __device__ __forceinline__ uint32_t next_u32(Rng& r) {
   if (r.left == 0) {
-    philox(r.c0, 0u, r.c2, r.c3, r.k0, r.k1, r.b);
+    const uint4 q = philox_block(r.c0, r.c2, r.c3, r.k0, r.k1);
+    r.b[0] = q.x; r.b[1] = q.y; r.b[2] = q.z; r.b[3] = q.w;
     r.c0++;
     r.left = 4;
   }
@@ -827,60 +836,64 @@ __device__ __forceinline__ void dust_view(const DevModel& m, R* smem, DustView<R
 // Computed once per unique table; species slots sharing a dust file share
 // the result (only kappa_V differs), which is what the per-slot loop of the
 // reference computes for them.
+// One table at nu, mixed form: the same bracket as the reference's bisection,
+// from the ln(nu) guide of the table and a short bisection inside it.
+struct OpacRow {
+  float g, pl, kap, alb;
+};
+__device__ __forceinline__ OpacRow opac_row(const float* nud, const float* kap, const float* alb, const float* g,
+                                            const float* pl, int nl, const short2* guide, float lnlo, float inv,
+                                            float nu) {
+  int i0 = 1, i1 = nl;
+  if (nu >= nud[0]) {
+    i0 = i1 = 1;
+  } else if (nu <= nud[nl - 1]) {
+    i0 = i1 = nl;
+  } else {
+    const int b = min(max((int)((logf(nu) - lnlo) * inv), 0), kDustGuide - 1);
+    const short2 gb = __ldg(guide + b);
+    if (nud[gb.x - 1] >= nu && nu > nud[gb.y]) { i0 = gb.x; i1 = gb.y + 1; }
+    while (i1 - i0 > 1) {
+      const int i = (i1 + i0) / 2;
+      if (nu <= nud[i - 1]) i0 = i; else i1 = i;
+    }
+  }
+  if (i0 == i1) return OpacRow{g[i0 - 1], pl[i0 - 1], kap[i0 - 1], alb[i0 - 1]};
+  const float n1 = nud[i1 - 1], n0 = nud[i0 - 1];
+  const float f = (nu - n1) / (n0 - n1), fm1 = 1.f - f;
+  return OpacRow{fmaf(fm1, g[i1 - 1], __fmul_rn(f, g[i0 - 1])), fmaf(fm1, pl[i1 - 1], __fmul_rn(f, pl[i0 - 1])),
+                 fmaf(fm1, kap[i1 - 1], __fmul_rn(f, kap[i0 - 1])), fmaf(fm1, alb[i1 - 1], __fmul_rn(f, alb[i0 - 1]))};
+}
+
+// the tables after the first, out of line (most models' slots share one file)
+static __device__ __noinline__ OpacRow opac_row_of(const float* nud, const float* kap, const float* alb, const float* g,
+                                                   const float* pl, int nl, const short2* guide, float lnlo, float inv,
+                                                   float nu) {
+  return opac_row(nud, kap, alb, g, pl, nl, guide, lnlo, inv, nu);
+}
+
 template <class R>
 __device__ __forceinline__ void opacset(const DevModel& m, const DustView<R>& v, Pkt<R>& p, R nu, const RunArgs& a) {
   if constexpr (sizeof(R) == 4) {
-    // mixed form: the same bracket from the ln(nu) guide of each table, then
-    // a short bisection inside it; values kept in registers
-    float gt[kSlots], plt[kSlots], kt[kSlots], at[kSlots];
-#pragma unroll
-    for (int u = 0; u < kSlots; ++u) {
-      gt[u] = plt[u] = kt[u] = at[u] = 0.f;
-      if (u >= m.ntab) continue;
-      const int nl = m.tab_nl[u];
-      const float* nud = v.nud[u];
-      int i0 = 1, i1 = nl;
-      if (nu >= nud[0]) {
-        i0 = i1 = 1;
-      } else if (nu <= nud[nl - 1]) {
-        i0 = i1 = nl;
-      } else {
-        const int b = min(max((int)((logf(nu) - m.dlnlo[u]) * m.dginv[u]), 0), kDustGuide - 1);
-        const short2 gb = __ldg(m.dguide + u * kDustGuide + b);
-        if (nud[gb.x - 1] >= nu && nu > nud[gb.y]) { i0 = gb.x; i1 = gb.y + 1; }
-        while (i1 - i0 > 1) {
-          const int i = (i1 + i0) / 2;
-          if (nu <= nud[i - 1]) i0 = i; else i1 = i;
-        }
-      }
-      if (i0 == i1) {
-        gt[u] = v.g[u][i0 - 1]; plt[u] = v.pl[u][i0 - 1]; kt[u] = v.kap[u][i0 - 1]; at[u] = v.alb[u][i0 - 1];
-      } else {
-        const float n1 = nud[i1 - 1], n0 = nud[i0 - 1];
-        const float f = (nu - n1) / (n0 - n1), fm1 = 1.f - f;
-        gt[u] = fmaf(fm1, v.g[u][i1 - 1], __fmul_rn(f, v.g[u][i0 - 1]));
-        plt[u] = fmaf(fm1, v.pl[u][i1 - 1], __fmul_rn(f, v.pl[u][i0 - 1]));
-        kt[u] = fmaf(fm1, v.kap[u][i1 - 1], __fmul_rn(f, v.kap[u][i0 - 1]));
-        at[u] = fmaf(fm1, v.alb[u][i1 - 1], __fmul_rn(f, v.alb[u][i0 - 1]));
-      }
-    }
-    if (m.ntab == 1) {  // every slot reads one table
-#pragma unroll
-      for (int id = 0; id < kSlots; ++id) {
-        p.g[id] = gt[0]; p.pl[id] = plt[0]; p.albedo[id] = at[0];
-        p.kapd[id] = kt[0] * a.kapfac[id];
-      }
-      return;
-    }
+    const OpacRow r0 = opac_row(v.nud[0], v.kap[0], v.alb[0], v.g[0], v.pl[0], m.tab_nl[0], m.dguide, m.dlnlo[0],
+                                m.dginv[0], nu);
 #pragma unroll
     for (int id = 0; id < kSlots; ++id) {
-      const int u = m.table_of[id];
-      float g_ = gt[0], pl_ = plt[0], k_ = kt[0], a_ = at[0];
+      p.g[id] = r0.g; p.pl[id] = r0.pl; p.albedo[id] = r0.alb;
+      p.kapd[id] = r0.kap * a.kapfac[id];
+    }
+    if (m.ntab == 1) return;
 #pragma unroll
-      for (int q = 1; q < kSlots; ++q)
-        if (u == q) { g_ = gt[q]; pl_ = plt[q]; k_ = kt[q]; a_ = at[q]; }
-      p.g[id] = g_; p.pl[id] = pl_; p.albedo[id] = a_;
-      p.kapd[id] = k_ * a.kapfac[id];
+    for (int u = 1; u < kSlots; ++u) {
+      if (u >= m.ntab) continue;
+      const OpacRow r = opac_row_of(v.nud[u], v.kap[u], v.alb[u], v.g[u], v.pl[u], m.tab_nl[u],
+                                    m.dguide + u * kDustGuide, m.dlnlo[u], m.dginv[u], nu);
+#pragma unroll
+      for (int id = 0; id < kSlots; ++id)
+        if (m.table_of[id] == u) {
+          p.g[id] = r.g; p.pl[id] = r.pl; p.albedo[id] = r.alb;
+          p.kapd[id] = r.kap * a.kapfac[id];
+        }
     }
     return;
   }
@@ -1078,102 +1091,94 @@ __device__ __forceinline__ float opacity(const Pkt<float>& p, const Rho<float>& 
 template <bool kFused>
 static __device__ __forceinline__ int tauint_mixed(const DevModel& m, const DevTallies& t, Pkt<float>& p, float tau, Local& L,
                                    Tracer& tr) {
-  float tsum = 0.f;
   const int cap = 4 * (m.nrg + m.ntg + m.npg) + 64;
-  int nreloc = 0, ntiny = 0;
+  int nreloc = 0, ntiny = 0, st;
   Ray ray;
   ray_init(ray, p.x, p.y, p.z, p.ux, p.uy, p.uz);
   PathLen S{0.f, 0.f};
+  float ds = 0.f, tsum = 0.f;
+  bool inside = false;  // the step ends in the cell, without a wall search
   if (p.on_wall == 0 && p.ir >= 1 && p.ir <= m.nrg - 1 && p.it >= 1 && p.it <= m.ntg - 1) {
     // From a point inside the cell, a step shorter than the safe distance
     // ends in the cell: the interaction the walk would find, without the
     // wall search.  The safe distance holds for a ball around the point
     // where it was formed; each such step uses up its length.
-    const int64_t c = cidx(m, p.ir, p.it, p.ip);
-    const Rho<float> rho = load_rho<float>(m, c);
-    const float opac = opacity(p, rho);
-    const float ds = tau / opac;
+    const float opac = opacity(p, load_rho<float>(m, cidx(m, p.ir, p.it, p.ip)));
+    ds = tau / opac;
     if (opac > 0.f && !(ds < p.safe)) p.safe = safe_dist(m, p.x.hi, p.y.hi, p.z.hi, p.ir, p.it, p.ip);
-    if (opac > 0.f && ds < p.safe) {
-      p.safe = __fsub_rn(p.safe, ds);
-      L.cross++;
-      tally_path<float>(m, t, p, rho, c, ds, __ldg(m.rarrf + p.ir));
-      path_add(S, ds);
-      ray_pos(ray, S, p.x, p.y, p.z);
-      tr.add(2, p.ir, p.it, p.ip, 0, (double)tau, dval(p.x), dval(p.y), dval(p.z));
-      return TI_INTERACT;
-    }
+    inside = opac > 0.f && ds < p.safe;
   }
-  p.safe = 0.f;
-  auto at = [&]() { ray_pos(ray, S, p.x, p.y, p.z); };
-  auto reloc = [&]() {
-    double x, y, z;
-    ray_at(ray, S, x, y, z);
-    int jr = p.ir, jt = p.it, jp = p.ip;
-    const int where = relocate(m, x, y, z, jr, jt, jp);
-    p.ir = jr; p.it = jt; p.ip = jp;
-    return where;
-  };
+  p.safe = inside ? __fsub_rn(p.safe, ds) : 0.f;
+  bool locate = false;  // re-derive the cell first
   for (int n = 0;; ++n) {
-    if (n > cap || p.it < 1 || p.it > m.ntg - 1 || p.ir < 1 || p.ir > m.nrg - 1) {
-      L.fault = n > cap ? F_CAP : F_RANGE;
-      at();
-      return TI_FAULT;
+    int iface = 0;
+    float dt = 0.f;
+    if (!inside) {
+      if (locate) {
+        locate = false;
+        ++nreloc;
+        double x, y, z;
+        ray_at(ray, S, x, y, z);
+        int jr = p.ir, jt = p.it, jp = p.ip;
+        const int where = relocate(m, x, y, z, jr, jt, jp);
+        p.ir = jr; p.it = jt; p.ip = jp;
+        if (where == 1) { p.ir = m.nrg; st = TI_ESCAPE; break; }
+        if (where == 2) { p.ir = 0; st = TI_STAR; break; }
+        p.on_wall = 0;
+      }
+      if (n > cap || p.it < 1 || p.it > m.ntg - 1 || p.ir < 1 || p.ir > m.nrg - 1) {
+        L.fault = n > cap ? F_CAP : F_RANGE;
+        st = TI_FAULT;
+        break;
+      }
     }
     // the cell's density, loaded before the wall search (latency overlap)
     const int64_t c = cidx(m, p.ir, p.it, p.ip);
     const Rho<float> rho = load_rho<float>(m, c);
-    float dt;
-    int iface;
-    if (!next_wall_ray<kFused>(m, ray, S, p.ir, p.it, p.ip, p.on_wall, dt, iface)) {
-      at();
+    if (!inside && !next_wall_ray<kFused>(m, ray, S, p.ir, p.it, p.ip, p.on_wall, dt, iface)) {
       if (nreloc < 4) {
-        ++nreloc;
-        const int where = reloc();
-        if (where == 1) { p.ir = m.nrg; return TI_ESCAPE; }
-        if (where == 2) { p.ir = 0; return TI_STAR; }
-        p.on_wall = 0;
+        locate = true;
         continue;
       }
       L.fault = F_NOWALL;
-      return TI_FAULT;
+      st = TI_FAULT;
+      break;
     }
-    const float opac = opacity(p, rho);
-    const float tnext = fmaf(opac, dt, tsum);  // the optical depth at the wall
-    const float rout = __ldg(m.rarrf + p.ir);
+    bool stop = inside;
+    float tnext = 0.f;
+    if (!inside) {
+      const float opac = opacity(p, rho);
+      tnext = fmaf(opac, dt, tsum);  // the optical depth at the wall
+      stop = tnext > tau;
+      ds = stop ? (tau - tsum) / opac : dt;
+    }
     L.cross++;
-    const bool stop = tnext > tau;
-    const float ds = stop ? (tau - tsum) / opac : dt;
-    tally_path<float>(m, t, p, rho, c, ds, rout);
+    tally_path<float>(m, t, p, rho, c, ds, __ldg(m.rarrf + p.ir));
+    path_add(S, ds);
     if (stop) {
-      path_add(S, ds);
-      at();
       p.on_wall = 0;
-      tr.add(2, p.ir, p.it, p.ip, 0, (double)tau, dval(p.x), dval(p.y), dval(p.z));
-      return TI_INTERACT;
+      st = TI_INTERACT;
+      break;
     }
     tsum = tnext;
     step_index(m.npg, iface, p.ir, p.it, p.ip);
-    path_add(S, dt);
     p.on_wall = 1 << own_after(iface);
     if (tr.recs) {
-      at();
+      ray_pos(ray, S, p.x, p.y, p.z);
       tr.add(1, p.ir, p.it, p.ip, iface, (double)tsum, dval(p.x), dval(p.y), dval(p.z));
     }
-    if (p.ir == m.nrg) { at(); return TI_ESCAPE; }
-    if (p.ir == 0) { at(); return TI_STAR; }
+    if (p.ir == m.nrg) { st = TI_ESCAPE; break; }
+    if (p.ir == 0) { st = TI_STAR; break; }
     if (!tiny_step(m, dt, p.ir)) {
       ntiny = 0;
     } else if (++ntiny > 6 && nreloc < 4) {
-      ++nreloc;
       ntiny = 0;
-      at();
-      const int where = reloc();
-      if (where == 1) { p.ir = m.nrg; return TI_ESCAPE; }
-      if (where == 2) { p.ir = 0; return TI_STAR; }
-      p.on_wall = 0;
+      locate = true;
     }
   }
+  ray_pos(ray, S, p.x, p.y, p.z);
+  if (st == TI_INTERACT) tr.add(2, p.ir, p.it, p.ip, 0, (double)tau, dval(p.x), dval(p.y), dval(p.z));
+  return st;
 }
 
 // The wall walk of tauint_mixed for a packet that a whole warp runs (k_tail),
@@ -2782,6 +2787,28 @@ __device__ __forceinline__ bool emit(const DevModel& m, const DustView<R>& dv, c
 }
 
 
+// emit out of line: the sources' code, run once a packet, stays out of the way
+// of the events'.  Its references are copies, so that the packet itself keeps its
+// registers.
+template <class R>
+static __device__ __noinline__ bool emit_cold(const DevModel& m, const DustView<R>& dv, const DevTallies& t,
+                                              const RunArgs& a, Pkt<R>& p, Rng& rng, PeelRec<R>& rec, Local& L) {
+  Tracer tr{nullptr, 0, 0};
+  return emit<R>(m, dv, t, a, p, rng, rec, tr, L);
+}
+template <class R>
+__device__ __forceinline__ bool emit_packet(const DevModel& m, const DustView<R>& dv, const DevTallies& t,
+                                            const RunArgs& a, Pkt<R>& p, Rng& rng, PeelRec<R>& rec, Local& L) {
+  DustView<R> v = dv;
+  Pkt<R> q;
+  Rng r = rng;
+  Local l = L;
+  const bool ok = emit_cold<R>(m, v, t, a, q, r, rec, l);
+  p = q;
+  rng = r;
+  return ok;
+}
+
 // tau sample + tauint + outcome, propagate.f90:46-62 (first) and 169-202.
 // G: the packet's draws, one lane's (Rng) or a warp's (WarpRng, k_tail).
 template <class R, bool kFused, class G>
@@ -3106,7 +3133,7 @@ __global__ void __launch_bounds__(128, 3) k_wave(DevModel m, DevTallies t, Tally
       bool emitted = true;
       if (s.stage == 0) {
         ++slot;
-        emitted = emit<R>(m, dv, t, a, s.p, rng, rec, tr, L);  // else dropped: the lane takes the next packet
+        emitted = emit_packet<R>(m, dv, t, a, s.p, rng, rec, L);  // else dropped: the lane takes the next packet
         if (emitted) {
           s.f.xpold = s.p.x; s.f.ypold = s.p.y; s.f.zpold = s.p.z;
           s.f.iflag = 0; s.f.iscat = 0; s.f.iint = 0; s.f.idust2 = 0; s.f.ntot = 0;
