@@ -35,7 +35,7 @@ namespace hc3d {
 // fit beside them (48 KB a block) are read from global memory
 static DevModel tail_model_fp64(const DevModel& m) {
   DevModel q = m;
-  if (m.dust_smem + 4 * (int)(sizeof(dev::DrawTable<double>) + sizeof(dev::Ahead)) + 256 > 48 * 1024) q.dust_smem = 0;
+  if (m.dust_smem + 4 * (int)(sizeof(dev::DrawTable<double>) + sizeof(dev::Ahead<double>)) + 256 > 48 * 1024) q.dust_smem = 0;
   return q;
 }
 

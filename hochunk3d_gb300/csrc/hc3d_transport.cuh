@@ -154,19 +154,12 @@ template <class R> __device__ __forceinline__ void draw_phi(Rng& r, R& phi, R& c
 }
 
 // Draws of a packet that a whole warp runs (k_tail): the next draws of its
-// stream, formed 32 lanes at a time in shared memory.  The FP64 form keeps the
-// functions above of each beside them -- a lone FP64 logarithm is a chain of
-// 2100 cycles -- and reads them instead; the mixed form runs its events side by
-// side in the lanes (tail_window), which form what they need.  Every lane holds
-// the same position; ensure() is called by the whole warp.
-template <class R> struct DrawTable;
-template <> struct DrawTable<float> {
+// stream, formed 32 lanes at a time in shared memory.  Every lane holds the same
+// position; ensure() is called by the whole warp.
+template <class R>
+struct DrawTable {
   static constexpr int kDraws = 256;
-  float u[kDraws];
-};
-template <> struct DrawTable<double> {
-  static constexpr int kDraws = 128;
-  double u[kDraws], nl[kDraws], mu[kDraws], smu[kDraws], cphi[kDraws], sphi[kDraws];
+  R u[kDraws];
 };
 template <class R>
 struct WarpRng {
@@ -176,8 +169,6 @@ struct WarpRng {
   int at;          // next draw of the table
 };
 
-template <class G> struct IsWarp { static constexpr bool value = false; };
-template <class R> struct IsWarp<WarpRng<R>> { static constexpr bool value = true; };
 // the draws of Philox blocks block .. of a stream into a table (not inlined: a
 // warp that runs one packet keeps its code small, see k_tail)
 template <class R>
@@ -190,22 +181,10 @@ static __device__ __noinline__ void fill_table(DrawTable<R>* t, uint32_t block, 
     uint32_t b[4];
     philox(block + (uint32_t)(32 * h + lane), 0u, c2, c3, k0, k1, b);
     const int k = 128 * h + 4 * lane;
-    if constexpr (sizeof(R) == 4) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) t->u[k + j] = ((float)(b[j] >> 8) + 0.5f) * (1.0f / 16777216.0f);
-    } else {
-#pragma unroll 1
-      for (int j = 0; j < 4; ++j) {
-        const R u = ((double)pick4(b, j) + 0.5) * (1.0 / 4294967296.0);
-        t->u[k + j] = u;
-        t->nl[k + j] = -xlog(u);
-        const R mu = R(1) - R(2) * u;
-        t->mu[k + j] = mu;
-        t->smu[k + j] = xsqrt(R(1) - mu * mu);
-        const R phi = (R)kR2p * u;
-        t->cphi[k + j] = xcos(phi);
-        t->sphi[k + j] = xsin(phi);
-      }
+    for (int j = 0; j < 4; ++j) {
+      if constexpr (sizeof(R) == 4) t->u[k + j] = ((float)(b[j] >> 8) + 0.5f) * (1.0f / 16777216.0f);
+      else t->u[k + j] = ((double)b[j] + 0.5) * (1.0 / 4294967296.0);
     }
   }
   __syncwarp();
@@ -233,22 +212,12 @@ template <class R> __device__ __forceinline__ void rng_save(const WarpRng<R>& r,
   c0 = r.block + (uint32_t)((r.at + 3) >> 2);
   left = (4 - (r.at & 3)) & 3;
 }
-template <class R> __device__ __forceinline__ R ran(WarpRng<R>& r) { return r.t->u[r.at++]; }
-template <class R> __device__ __forceinline__ R neg_log(WarpRng<R>& r) { return r.t->nl[r.at++]; }
-template <class R> __device__ __forceinline__ void draw_mu(WarpRng<R>& r, R& mu, R& smu) {
-  mu = r.t->mu[r.at];
-  smu = r.t->smu[r.at++];
-}
-template <class R> __device__ __forceinline__ void draw_phi(WarpRng<R>& r, R& phi, R& cphi, R& sphi) {
-  phi = (R)kR2p * r.t->u[r.at];
-  cphi = r.t->cphi[r.at];
-  sphi = r.t->sphi[r.at++];
-}
 // one draw, of a lane that works ahead (tail_window)
+template <class R>
 struct OneDraw {
-  float u;
+  R u;
 };
-template <class R> __device__ __forceinline__ R ran(OneDraw& r) { return r.u; }
+template <class R> __device__ __forceinline__ R ran(OneDraw<R>& r) { return r.u; }
 
 // ---- packet state: the tts_mod/stokesvar_mod globals of one packet ------------
 // Positions: FP64 in the FP64 form.  The mixed form carries each coordinate
@@ -446,6 +415,71 @@ __device__ __forceinline__ bool next_wall(const DevModel& m, R ux, R uy, R uz, d
     }
   }
   return w.next(on_wall != 0, dt, iface);
+}
+
+// The same search by the lanes of a warp that runs one packet (k_tail): lane 2 w
+// + j holds the j-th root that wall w + 1 inserts above, so that lane order is
+// insertion order.  One quadratic serves spheres and cones: with tan2 = -1 and a
+// = 1 the cone's terms are the sphere's, rounding included (a product with -1,
+// a division by 2), and the planes share its division.  A lone FP64 square root
+// is a chain of 690 cycles and a division of 650; one after another the walls
+// took three of each and more, some 6500 cycles, side by side 2200.
+__device__ __forceinline__ bool next_wall_warp64(const DevModel& m, double ux, double uy, double uz, double x, double y,
+                                                 double z, int ir, int it, int ip, int on_wall, double& dt,
+                                                 int& iface) {
+  const int lane = threadIdx.x & 31, w = min(lane >> 1, 5), j = lane & 1;
+  const bool sphere = w < 2, cone = w == 2 || w == 3, plane = w >= 4;
+  const double* p1 = sphere ? m.r2arr + ir - 1 + w : (cone ? m.tan2d + it - 1 + (w - 2) : m.aarrd + ip - 1 + (w - 4));
+  const double v = __ldg(p1);
+  const double B = __ldg(m.barrd + ip - 1 + (plane ? w - 4 : 0));
+  const double hemi = (double)__ldg(m.hemi + it - 1 + (w == 3 ? 1 : 0));
+  const double tz = sphere ? -1.0 : v;
+  const double tzz = tz * z;
+  const double b = 2.0 * (x * ux + y * uy - tzz * uz);
+  const double c = (x * x + y * y - tzz * z) - (sphere ? v : 0.0);
+  const double a = sphere ? 1.0 : ux * ux + uy * uy - tz * uz * uz;
+  const double descr = b * b - 4.0 * a * c;
+  const double s = sqrt(descr);
+  const bool mid = cone && v < 0.0, lin = cone && a == 0.0;
+  double num = j ? -b - s : -b + s, den = 2.0 * a;
+  bool ok = descr > 0.0;
+  if (mid) {
+    num = -z; den = uz;
+    ok = j == 0 && uz != 0.0;
+  } else if (lin) {
+    num = -c; den = b;
+    ok = j == 0 && b != 0.0;
+  } else if (plane) {
+    num = -(v * x + B * y);
+    den = v * ux + B * uy;
+    ok = j == 0 && den != 0.0 && m.npg > 2;
+  }
+  const double t = num / den + 0.0;  // -0 becomes +0
+  if (cone && !mid) ok = ok && (z + t * uz) * hemi > 0.0;
+  ok = ok && lane < 12 && !(cone && v == 0.0) && (sphere || m.ntg > 2);
+  const unsigned long long bits = (unsigned long long)__double_as_longlong(t);
+  constexpr unsigned long long kHuge = 0x7fefffffffffffffull;  // of the largest double: a root must lie below it
+  const unsigned long long mag = bits & 0x7fffffffffffffffull;
+  const bool neg = (bits >> 63) != 0ull;
+  ok = ok && mag < kHuge;
+  auto least = [&](bool in, unsigned long long& val) {  // the least of the lanes' magnitudes and its first lane (-1: none)
+    const unsigned hi = in ? (unsigned)(mag >> 32) : 0xffffffffu;
+    const unsigned mh = __reduce_min_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_min_sync(0xffffffffu, in && hi == mh ? (unsigned)mag : 0xffffffffu);
+    const unsigned who = __ballot_sync(0xffffffffu, in && hi == mh && (unsigned)mag == ml);
+    val = who ? (unsigned long long)mh << 32 | ml : kHuge;
+    return __ffs(who) - 1;
+  };
+  unsigned long long tp;
+  int win = least(ok && !neg, tp);
+  if (on_wall) {
+    unsigned long long tn;
+    least(ok && neg, tn);
+    if (!(tn < tp)) win = least(ok && !neg && lane != win, tp);
+  }
+  dt = __longlong_as_double((long long)tp);
+  iface = (win >> 1) + 1;
+  return tp != kHuge;
 }
 
 // A straight ray of the mixed form, parametrised by its path length S from
@@ -1270,22 +1304,55 @@ static __device__ __forceinline__ int wall_walk(const DevModel& m, const DevTall
   return st;
 }
 
+// tauint of the FP64 form for a packet that a whole warp runs (k_tail)
+static __device__ __forceinline__ int wall_walk64(const DevModel& m, const DevTallies& t, Pkt<double>& p, double tau,
+                                                  Rho<double>& rho, Local& L) {
+  double tsum = 0.0;
+  const int cap = 4 * (m.nrg + m.ntg + m.npg) + 64;
+  for (int n = 0;; ++n) {
+    double dt;
+    int iface;
+    const bool in = n <= cap && p.it >= 1 && p.it <= m.ntg - 1 && p.ir >= 1 && p.ir <= m.nrg - 1;
+    if (!in || !next_wall_warp64(m, p.ux, p.uy, p.uz, p.x, p.y, p.z, p.ir, p.it, p.ip, p.on_wall, dt, iface)) {
+      L.fault = n > cap ? F_CAP : (in ? F_NOWALL : F_RANGE);
+      return TI_FAULT;
+    }
+    const int64_t c = cidx(m, p.ir, p.it, p.ip);
+    double opac = 0.0;
+#pragma unroll
+    for (int s = 0; s < kSlots; ++s) opac += p.kapd[s] * rho.v[s];
+    const double dtau = opac * dt;
+    L.cross++;
+    const bool stop = tsum + dtau > tau;
+    double ds = dt;
+    if (stop) ds = (tau - tsum) / opac;
+    p.x += ds * p.ux;
+    p.y += ds * p.uy;
+    p.z += ds * p.uz;
+    tally_path_warp<double>(m, t, p, rho, c, ds, __ldg(m.rarr + p.ir));
+    if (stop) {
+      p.on_wall = 0;
+      return TI_INTERACT;
+    }
+    tsum += dtau;
+    step_index(m.npg, iface, p.ir, p.it, p.ip);
+    p.on_wall = 1 << own_after(iface);
+    if (p.ir == m.nrg) return TI_ESCAPE;
+    if (p.ir == 0) return TI_STAR;
+    if (p.it >= 1 && p.it <= m.ntg - 1) rho = load_rho<double>(m, cidx(m, p.ir, p.it, p.ip));
+  }
+}
+
 // tauint in either form: the FP64 form walks with the reference's wall
 // machinery (closest_wall rule), the mixed form with tauint_mixed.
-// kWarp: a whole warp runs the packet (FP64 form).
-template <class R, bool kFused, bool kWarp>
+template <class R, bool kFused>
 __device__ __forceinline__ int tauint(const DevModel& m, const DevTallies& t, Pkt<R>& p, R tau, Local& L, Tracer& tr) {
   if constexpr (sizeof(R) == 4) {
-    static_assert(!kWarp, "the mixed form's is wall_walk");
     return tauint_mixed<kFused>(m, t, p, tau, L, tr);
   } else {
     R tsum = R(0);
     const int cap = 4 * (m.nrg + m.ntg + m.npg) + 64;
     const double uxd = (double)p.ux, uyd = (double)p.uy, uzd = (double)p.uz;
-    auto tally = [&](const Rho<R>& rho, int64_t c, R ds, R rout) {
-      if constexpr (kWarp) tally_path_warp<R>(m, t, p, rho, c, ds, rout);
-      else tally_path<R>(m, t, p, rho, c, ds, rout);
-    };
     for (int n = 0;; ++n) {
       if (n > cap || p.it < 1 || p.it > m.ntg - 1 || p.ir < 1 || p.ir > m.nrg - 1) {
         L.fault = n > cap ? F_CAP : F_RANGE;
@@ -1311,11 +1378,11 @@ __device__ __forceinline__ int tauint(const DevModel& m, const DevTallies& t, Pk
         p.y += (double)ds * uyd;
         p.z += (double)ds * uzd;
         p.on_wall = 0;
-        tally(rho, c, ds, (R)rout);
+        tally_path<R>(m, t, p, rho, c, ds, (R)rout);
         tr.add(2, p.ir, p.it, p.ip, 0, (double)tau, p.x, p.y, p.z);
         return TI_INTERACT;
       }
-      tally(rho, c, dt, (R)rout);
+      tally_path<R>(m, t, p, rho, c, dt, (R)rout);
       tsum += dtau;
       step_index(m.npg, iface, p.ir, p.it, p.ip);
       p.x += (double)dt * uxd;
@@ -1369,6 +1436,21 @@ static __device__ __noinline__ int select_known(float k0, float k1, float k2, fl
 }
 __device__ __forceinline__ int select_known(const Pkt<float>& p, const Rho<float>& rho, float xran) {
   return select_known(p.kapd[0], p.kapd[1], p.kapd[2], p.kapd[3], rho.v[0], rho.v[1], rho.v[2], rho.v[3], xran);
+}
+
+static __device__ __noinline__ int select_known64(double k0, double k1, double k2, double k3, double r0, double r1,
+                                                  double r2, double r3, double xran) {
+  const double kapd[kSlots] = {k0, k1, k2, k3}, rho[kSlots] = {r0, r1, r2, r3};
+  unsigned some = 0u;
+#pragma unroll
+  for (int s = 0; s < kSlots; ++s) some |= kapd[s] * rho[s] > 0.0 ? 1u << s : 0u;
+  // its fraction is exactly 1 (an infinite opacity has none and is left to the loop)
+  if (some != 0u && (some & (some - 1u)) == 0u && kapd[0] * rho[0] + kapd[1] * rho[1] + kapd[2] * rho[2] + kapd[3] * rho[3] <= 1.7e308)
+    return __ffs(some) - 1;
+  return select_species<double>(kapd, rho, xran);
+}
+__device__ __forceinline__ int select_known(const Pkt<double>& p, const Rho<double>& rho, double xran) {
+  return select_known64(p.kapd[0], p.kapd[1], p.kapd[2], p.kapd[3], rho.v[0], rho.v[1], rho.v[2], rho.v[3], xran);
 }
 
 // ---- dustmat.f90:40-65 -----------------------------------------------------------
@@ -2810,7 +2892,6 @@ __device__ __forceinline__ bool emit_packet(const DevModel& m, const DustView<R>
 }
 
 // tau sample + tauint + outcome, propagate.f90:46-62 (first) and 169-202.
-// G: the packet's draws, one lane's (Rng) or a warp's (WarpRng, k_tail).
 template <class R, bool kFused, class G>
 __device__ __forceinline__ int walk(const DevModel& m, const DevTallies& t, const TallyDims& d, const RunArgs& a, Pkt<R>& p, G& rng,
                     Flow<R>& f, Local& L, Tracer& tr, bool first) {
@@ -2820,7 +2901,7 @@ __device__ __forceinline__ int walk(const DevModel& m, const DevTallies& t, cons
     p.ux = p.sint * p.cosp; p.uy = p.sint * p.sinp; p.uz = p.cost;
   }
   const int pir = p.ir, pit = p.it, pip = p.ip;
-  const int st = tauint<R, kFused, IsWarp<G>::value>(m, t, p, tau, L, tr);
+  const int st = tauint<R, kFused>(m, t, p, tau, L, tr);
   if (st == TI_ESCAPE) {
     tr.add(3, p.ir, p.it, p.ip, 0, 0.0, dval(p.x), dval(p.y), dval(p.z));
     if (L.on) bin_escape<R>(t, d, a, p, dval(f.xpold), dval(f.ypold), dval(f.zpold), f.iflag, f.iscat, L);
@@ -3189,12 +3270,15 @@ constexpr int kAhead = 16;  // events a lane set looks ahead
 // what the lanes' events leave, in shared memory (a field's 32 values side by
 // side): any lane's is read by the whole warp, and the packet keeps its registers
 enum AheadField {
-  A_COST, A_SINT, A_PHI, A_COSP, A_SINP, A_NUB, A_TAU, A_DS, A_ALB, A_WHAT, A_OP, A_INUB,
+  A_COST, A_SINT, A_PHI, A_COSP, A_SINP, A_NUB, A_TAU, A_ALB, A_KAPD, A_ALBEDO = A_KAPD + kSlots, A_G = A_ALBEDO + kSlots, A_PL = A_G + kSlots, A_DS = A_PL + kSlots, A_OP,
   A_PX, A_EX, A_PY, A_EY, A_PZ, A_EZ,  // step_terms of the three coordinates
-  A_KAPD, A_ALBEDO = A_KAPD + kSlots, A_G = A_ALBEDO + kSlots, A_PL = A_G + kSlots, A_FIELDS = A_PL + kSlots
+  A_FIELDS, A_FIELDS64 = A_DS  // the FP64 form has no steps within the safe distance
 };
+template <class R>
 struct Ahead {
-  float v[A_FIELDS][32];
+  R v[sizeof(R) == 4 ? A_FIELDS : A_FIELDS64][32];
+  int what[32];  // the species assumed, and << 4 the species selected (7: none)
+  int inub[32];
 };
 
 // Runs events until the packet leaves the cell, ends or has run E of them (nrec
@@ -3202,24 +3286,25 @@ struct Ahead {
 // warps of an SM are anywhere in it, and at 184 KB, with the parts inlined
 // wherever they were used, 10 of 15 cycles of an instruction were spent waiting
 // for its fetch.
-template <bool kPeel, bool kFused>
-__device__ __forceinline__ bool tail_window(const DevModel& m, const DustView<float>& dv, const DevTallies& t,
-                                            const TallyDims& td, const RunArgs& a, Pkt<float>& p, WarpRng<float>& rng,
-                                            Flow<float>& f, Ahead& ah, Local& L, PeelRec<float>* queue,
+template <class R, bool kPeel, bool kFused>
+__device__ __forceinline__ bool tail_window(const DevModel& m, const DustView<R>& dv, const DevTallies& t,
+                                            const TallyDims& td, const RunArgs& a, Pkt<R>& p, WarpRng<R>& rng,
+                                            Flow<R>& f, Ahead<R>& ah, Local& L, PeelRec<R>* queue,
                                             unsigned long long* qcount, unsigned long long& slot,
                                             unsigned long long& slot_end, int& nrec, int E) {
   const int lane = threadIdx.x & 31;
   const int c = (int)cidx(m, p.ir, p.it, p.ip), ir0 = p.ir, it0 = p.it, ip0 = p.ip;
   constexpr float kLong = 3.402823466e38f;  // a step that needs the wall search
+  constexpr bool kMixed = sizeof(R) == 4;
   ensure(rng, 6 * kAhead + 8);
   const uint32_t from = 4u * rng.block + (uint32_t)rng.at;  // the draw the window starts at
-  Rho<float> rho = load_rho<float>(m, c);
+  Rho<R> rho = load_rho<R>(m, c);
   const float reach = 0.5f * (__ldg(m.rarrf + ir0) - __ldg(m.rarrf + ir0 - 1));  // no safe distance is longer
   int s;  // the species this lane's event is assumed to meet
   unsigned follows, sound;  // the lanes whose event is an absorption of the assumed species after that of the lane
                             // before, and those whose event leaves a species to meet
   {
-    const float* u = rng.t->u + rng.at + 6 * (lane & (kAhead - 1)) + (lane >= kAhead ? 3 : 0);
+    const R* u = rng.t->u + rng.at + 6 * (lane & (kAhead - 1)) + (lane >= kAhead ? 3 : 0);
     // the pending event's is known, the others' as the packet's present
     // opacities select it
     s = select_known(p, rho, u[lane == 0 ? 0 : -1]);
@@ -3228,48 +3313,49 @@ __device__ __forceinline__ bool tail_window(const DevModel& m, const DustView<fl
     if (none) s = 0;
     // a small grain's frequency is drawn before its direction (emit_sg.f90)
     const bool sg = (m.sg_mask >> s) & 1u;
-    Pkt<float> q;
-    OneDraw d{sg ? u[1] : u[3]};
+    Pkt<R> q;
+    OneDraw<R> d{sg ? u[1] : u[3]};
     if (sg) {
       const int im = a.iter1 ? 2 : __ldg(m.imean + c);
-      q.nub = (float)rep_draine<float>(m, im, a.iter1 ? 0.0 : __ldg(m.imfract + c), d);
+      q.nub = (R)rep_draine<R>(m, im, a.iter1 ? 0.0 : __ldg(m.imfract + c), d);
     } else {
-      q.nub = lucy_freq_mixed(m, c, s, d);
+      if constexpr (kMixed) q.nub = lucy_freq_mixed(m, c, s, d);
+      else q.nub = lucydustfreq<R>(m, __ldg(m.tdust + 4 * (int64_t)c + s), s, d);
     }
-    q.cost = 1.f - 2.f * (sg ? u[2] : u[1]);
-    q.sint = xsqrt(1.f - q.cost * q.cost);
-    q.phi = (float)kR2p * (sg ? u[3] : u[2]);
+    q.cost = R(1) - R(2) * (sg ? u[2] : u[1]);
+    q.sint = xsqrt(R(1) - q.cost * q.cost);
+    q.phi = (R)kR2p * (sg ? u[3] : u[2]);
     q.cosp = xcos(q.phi);
     q.sinp = xsin(q.phi);
-    opacset<float>(m, dv, q, q.nub, a);
-    const float tau = -xlog(u[4]), opac = opacity(q, rho);
-    float ds = tau / opac;
-    if (!(opac > 0.f && ds < reach)) ds = kLong;
+    opacset<R>(m, dv, q, q.nub, a);
+    const R tau = -xlog(u[4]);
     const int sel = select_known(q, rho, u[5]);
     __syncwarp();  // the last window's values have been read
-    auto put = [&](int k, float v) { ah.v[k][lane] = v; };
+    auto put = [&](int k, R v) { ah.v[k][lane] = v; };
     put(A_COST, q.cost); put(A_SINT, q.sint); put(A_PHI, q.phi); put(A_COSP, q.cosp); put(A_SINP, q.sinp);
     put(A_NUB, q.nub);
-    float pr, pe;
-    step_terms(PathLen{ds, 0.f}, q.sint * q.cosp, pr, pe);
-    put(A_PX, pr); put(A_EX, pe);
-    step_terms(PathLen{ds, 0.f}, q.sint * q.sinp, pr, pe);
-    put(A_PY, pr); put(A_EY, pe);
-    step_terms(PathLen{ds, 0.f}, q.cost, pr, pe);
-    put(A_PZ, pr); put(A_EZ, pe);
     put(A_TAU, tau);
-    put(A_DS, ds);
-    const float alb = pick4(q.albedo, max(sel, 0));
+    if constexpr (kMixed) {
+      const float opac = opacity(q, rho);
+      float ds = tau / opac, pr, pe;
+      if (!(opac > 0.f && ds < reach)) ds = kLong;
+      put(A_DS, ds);
+      step_terms(PathLen{ds, 0.f}, q.sint * q.cosp, pr, pe);
+      put(A_PX, pr); put(A_EX, pe);
+      step_terms(PathLen{ds, 0.f}, q.sint * q.sinp, pr, pe);
+      put(A_PY, pr); put(A_EY, pe);
+      step_terms(PathLen{ds, 0.f}, q.cost, pr, pe);
+      put(A_PZ, pr); put(A_EZ, pe);
+      if constexpr (kPeel) put(A_OP, peel_opacity(m, q, c));
+    }
+    const R alb = pick4(q.albedo, max(sel, 0));
     put(A_ALB, alb);
-    const float alb_before = __shfl_up_sync(0xffffffffu, alb, 1);
+    const R alb_before = __shfl_up_sync(0xffffffffu, alb, 1);
     const int sel_before = __shfl_up_sync(0xffffffffu, sel, 1);
     follows = __ballot_sync(0xffffffffu, (lane & (kAhead - 1)) != 0 && !none && sel_before == s && u[0] > alb_before);
     sound = __ballot_sync(0xffffffffu, sel >= 0);
-    put(A_WHAT, __int_as_float((none ? 7 : s) | ((sel < 0 ? 7 : sel) << 4)));
-    if constexpr (kPeel) {
-      put(A_OP, peel_opacity(m, q, c));
-      put(A_INUB, __int_as_float(nu_bin<float>(a, q.nub)));
-    }
+    ah.what[lane] = (none ? 7 : s) | ((sel < 0 ? 7 : sel) << 4);
+    if constexpr (kPeel) ah.inub[lane] = nu_bin<R>(a, q.nub);
 #pragma unroll
     for (int k = 0; k < kSlots; ++k) {
       put(A_KAPD + k, q.kapd[k]);
@@ -3291,32 +3377,34 @@ __device__ __forceinline__ bool tail_window(const DevModel& m, const DustView<fl
       p.g[j] = ah.v[A_G + j][l];
       p.pl[j] = ah.v[A_PL + j][l];
     }
-    p.i_orig = ((m.disk_mask >> (__float_as_int(ah.v[A_WHAT][l]) & 15)) & 1u) ? 2 : 3;
-    p.sip = 1.f; p.sqp = p.sup = p.svp = 0.f;
+    p.i_orig = ((m.disk_mask >> (ah.what[l] & 15)) & 1u) ? 2 : 3;
+    p.sip = R(1); p.sqp = p.sup = p.svp = R(0);
     left = -1;
   };
   // the peel-off record of an event, the absorption of lane l or a scattering
   // (l < 0) of p, unless its rays end in the cell
   auto record = [&](int l) {
     if constexpr (kPeel) {
-      const float op = l >= 0 ? ah.v[A_OP][l] : (p.safe > 0.f ? peel_opacity(m, p, c) : 0.f);
-      if (p.safe > 0.f && deep_peel_at(p, p.safe, op)) return;
+      if constexpr (kMixed) {
+        const float op = l >= 0 ? ah.v[A_OP][l] : (p.safe > 0.f ? peel_opacity(m, p, c) : 0.f);
+        if (p.safe > 0.f && deep_peel_at(p, p.safe, op)) return;
+      }
       if (slot == slot_end) {
         if (lane == 0) slot = atomicAdd(qcount, (unsigned long long)a.qchunk);
         slot = __shfl_sync(0xffffffffu, slot, 0);
         slot_end = slot + (unsigned long long)a.qchunk;
       }
       if (lane == 0) {
-        PeelRec<float>& e = queue[slot];
+        PeelRec<R>& e = queue[slot];
         if (l < 0) {
-          make_rec<float>(e, p, a, 1, f.idust2);
+          make_rec<R>(e, p, a, 1, f.idust2);
         } else {
-          const int sl = __float_as_int(ah.v[A_WHAT][l]) & 15;
+          const int sl = ah.what[l] & 15;
           e.x = p.x; e.y = p.y; e.z = p.z;
           e.ir = p.ir; e.it = p.it; e.ip = p.ip;
           e.flags = (((m.disk_mask >> sl) & 1u ? 2 : 3) << 2) | (sl << 5);
-          e.inub = __float_as_int(ah.v[A_INUB][l]);
-          e.sip = 1.f; e.sqp = e.sup = e.svp = 0.f;
+          e.inub = ah.inub[l];
+          e.sip = R(1); e.sqp = e.sup = e.svp = R(0);
           e.d0 = ah.v[A_COST][l]; e.d1 = ah.v[A_SINT][l]; e.d2 = ah.v[A_PHI][l]; e.d3 = ah.v[A_COSP][l];
           e.d4 = ah.v[A_SINP][l];
           e.g = ah.v[A_G + sl][l]; e.pl = ah.v[A_PL + sl][l];
@@ -3327,7 +3415,7 @@ __device__ __forceinline__ bool tail_window(const DevModel& m, const DustView<fl
       ++slot;
     }
   };
-  float alb_now = pick4(p.albedo, f.idust2);
+  R alb_now = pick4(p.albedo, f.idust2);
   bool live = true, here = true;
   while (here && (!kPeel || nrec < E)) {
     const int off = (int)(4u * rng.block + (uint32_t)rng.at - from);
@@ -3336,48 +3424,50 @@ __device__ __forceinline__ bool tail_window(const DevModel& m, const DustView<fl
     const int h = off / 3;
     int l = (h >> 1) + ((h & 1) ? kAhead : 0);
     const bool scat = rng.t->u[rng.at] <= alb_now;
-    bool far = false;
-    if (!scat) {
-      if ((__float_as_int(ah.v[A_WHAT][l]) & 15) != f.idust2) break;  // it assumed another species (not the pending event's)
-      // the run of absorptions from here, as far as their steps are safe and no cap is reached
-      int len = min(__ffs(~(follows >> 1 >> l)), __ffs(~(sound >> l) | 1u << kAhead) - 1);
-      len = min(len, a.iintmax - f.iint);
-      if (a.max_interactions > 0) len = (int)min((int64_t)len, a.max_interactions - f.ntot - 1);
-      if (kPeel) len = min(len, E - nrec);
-      int k = 0;
-      for (; k < len; ++k) {
-        const float ds = ah.v[A_DS][l + k];
-        float safe = p.safe;
-        if (!(ds < safe)) {
-          if (ds < kLong) safe = safe_dist(m, p.x.hi, p.y.hi, p.z.hi, p.ir, p.it, p.ip);
+    bool far = !kMixed;
+    if (!scat && (ah.what[l] & 15) != f.idust2) break;  // it assumed another species (not the pending event's)
+    if constexpr (kMixed) {
+      if (!scat) {
+        // the run of absorptions from here, as far as their steps are safe and no cap is reached
+        int len = min(__ffs(~(follows >> 1 >> l)), __ffs(~(sound >> l) | 1u << kAhead) - 1);
+        len = min(len, a.iintmax - f.iint);
+        if (a.max_interactions > 0) len = (int)min((int64_t)len, a.max_interactions - f.ntot - 1);
+        if (kPeel) len = min(len, E - nrec);
+        int k = 0;
+        for (; k < len; ++k) {
+          const float ds = ah.v[A_DS][l + k];
+          float safe = p.safe;
           if (!(ds < safe)) {
-            far = true;
-            break;
+            if (ds < kLong) safe = safe_dist(m, p.x.hi, p.y.hi, p.z.hi, p.ir, p.it, p.ip);
+            if (!(ds < safe)) {
+              far = true;
+              break;
+            }
           }
+          record(l + k);
+          p.safe = __fsub_rn(safe, ds);
+          p.x = pos_add(p.x, ah.v[A_PX][l + k], ah.v[A_EX][l + k]);
+          p.y = pos_add(p.y, ah.v[A_PY][l + k], ah.v[A_EY][l + k]);
+          p.z = pos_add(p.z, ah.v[A_PZ][l + k], ah.v[A_EZ][l + k]);
         }
-        record(l + k);
-        p.safe = __fsub_rn(safe, ds);
-        p.x = pos_add(p.x, ah.v[A_PX][l + k], ah.v[A_EX][l + k]);
-        p.y = pos_add(p.y, ah.v[A_PY][l + k], ah.v[A_EY][l + k]);
-        p.z = pos_add(p.z, ah.v[A_PZ][l + k], ah.v[A_EZ][l + k]);
-      }
-      if (k > 0) {
-        const unsigned bits = ((1u << k) - 1u) << l;
-        absorbed |= bits;
-        stepped |= bits;
-        L.events += k;
-        L.cross += k;
-        f.ntot += k;
-        f.iint += k;
-        f.iflag = 0;
-        nrec += k;
-        rng.at += 6 * k;
-        l += k;
-        left = l - 1;
-        f.idust2 = __float_as_int(ah.v[A_WHAT][left]) >> 4;
-        alb_now = ah.v[A_ALB][left];
-        if (!far) continue;  // a scattering, another species or a cap is next
-        if (kPeel && nrec >= E) break;
+        if (k > 0) {
+          const unsigned bits = ((1u << k) - 1u) << l;
+          absorbed |= bits;
+          stepped |= bits;
+          L.events += k;
+          L.cross += k;
+          f.ntot += k;
+          f.iint += k;
+          f.iflag = 0;
+          nrec += k;
+          rng.at += 6 * k;
+          l += k;
+          left = l - 1;
+          f.idust2 = ah.what[left] >> 4;
+          alb_now = ah.v[A_ALB][left];
+          if (!far) continue;  // a scattering, another species or a cap is next
+          if (kPeel && nrec >= E) break;
+        }
       }
     }
     ++nrec;
@@ -3388,48 +3478,58 @@ __device__ __forceinline__ bool tail_window(const DevModel& m, const DustView<fl
     const int src = scat ? left : l;
     if (scat && src >= 0) adopt(src);
     record(scat ? -1 : l);
-    float tau, ds;
+    R tau;
+    float ds = kLong;
     if (scat) {
       f.iscat++;
       rng.at++;
-      stokes<float>(p, f.idust2, rng);
+      stokes<R>(p, f.idust2, rng);
       ensure(rng, 2);
       tau = -xlog(rng.t->u[rng.at++]);
-      const float opac = opacity(p, rho);
-      ds = tau / opac;
-      if (!(opac > 0.f && ds < reach)) ds = kLong;
-      if (lane == l) {  // the step's tally is this lane's to make, whose own event did not happen
+      if constexpr (kMixed) {
+        const float opac = opacity(p, rho);
+        ds = tau / opac;
+        if (!(opac > 0.f && ds < reach)) ds = kLong;
+        if (lane == l) {  // the step's tally is this lane's to make, whose own event did not happen
 #pragma unroll
-        for (int k = 0; k < kSlots; ++k) {
-          ah.v[A_KAPD + k][l] = p.kapd[k];
-          ah.v[A_ALBEDO + k][l] = p.albedo[k];
+          for (int k = 0; k < kSlots; ++k) {
+            ah.v[A_KAPD + k][l] = p.kapd[k];
+            ah.v[A_ALBEDO + k][l] = p.albedo[k];
+          }
+          ah.v[A_DS][l] = ds;
         }
-        ah.v[A_DS][l] = ds;
       }
     } else {
       adopt(src);
       absorbed |= 1u << l;
       rng.at += 5;
       tau = ah.v[A_TAU][l];
-      ds = ah.v[A_DS][l];
+      if constexpr (kMixed) ds = ah.v[A_DS][l];
     }
     p.ux = p.sint * p.cosp; p.uy = p.sint * p.sinp; p.uz = p.cost;
-    if (!far && !(ds < p.safe) && ds < kLong) p.safe = safe_dist(m, p.x.hi, p.y.hi, p.z.hi, p.ir, p.it, p.ip);
-    if (!far && ds < p.safe) {
-      p.safe = __fsub_rn(p.safe, ds);
-      const PathLen S{ds, 0.f};
-      p.x = pos_step(p.x, S, p.ux);
-      p.y = pos_step(p.y, S, p.uy);
-      p.z = pos_step(p.z, S, p.uz);
-      L.cross++;
-      stepped |= 1u << l;
-    } else {
+    bool inside = false;
+    if constexpr (kMixed) {
+      if (!far && !(ds < p.safe) && ds < kLong) p.safe = safe_dist(m, p.x.hi, p.y.hi, p.z.hi, p.ir, p.it, p.ip);
+      inside = !far && ds < p.safe;
+      if (inside) {
+        p.safe = __fsub_rn(p.safe, ds);
+        const PathLen S{ds, 0.f};
+        p.x = pos_step(p.x, S, p.ux);
+        p.y = pos_step(p.y, S, p.uy);
+        p.z = pos_step(p.z, S, p.uz);
+        L.cross++;
+        stepped |= 1u << l;
+      }
+    }
+    if (!inside) {
       f.xpold = p.x; f.ypold = p.y; f.zpold = p.z;
-      const int st = wall_walk<kFused>(m, t, p, tau, rho, L);
+      int st;
+      if constexpr (kMixed) st = wall_walk<kFused>(m, t, p, tau, rho, L);
+      else st = wall_walk64(m, t, p, tau, rho, L);
       if (st != TI_INTERACT) {
         if (st == TI_ESCAPE) {
           if (lane == 0)
-            bin_escape<float>(t, td, a, p, dval(f.xpold), dval(f.ypold), dval(f.zpold), f.iflag, f.iscat, L);
+            bin_escape<R>(t, td, a, p, dval(f.xpold), dval(f.ypold), dval(f.zpold), f.iflag, f.iscat, L);
         } else if (st == TI_STAR) {
           L.add(HC3D_CNT_AFLUX);
         } else {
@@ -3468,31 +3568,32 @@ __device__ __forceinline__ bool tail_window(const DevModel& m, const DustView<fl
     atomicAdd(((m.sg_mask >> s) & 1u ? t.dsg : t.dbig) + c, 1u);
     atomicAdd(t.nabs + (int64_t)s * m.ncell + c, 1ull);
   }
-  if ((stepped >> lane) & 1u) {
-    Pkt<float> q;
+  if constexpr (kMixed) {
+    if ((stepped >> lane) & 1u) {
+      Pkt<float> q;
 #pragma unroll
-    for (int k = 0; k < kSlots; ++k) {
-      q.kapd[k] = ah.v[A_KAPD + k][lane];
-      q.albedo[k] = ah.v[A_ALBEDO + k][lane];
+      for (int k = 0; k < kSlots; ++k) {
+        q.kapd[k] = ah.v[A_KAPD + k][lane];
+        q.albedo[k] = ah.v[A_ALBEDO + k][lane];
+      }
+      tally_path<float>(m, t, q, load_rho<float>(m, c), c, ah.v[A_DS][lane], __ldg(m.rarrf + ir0));
     }
-    tally_path<float>(m, t, q, load_rho<float>(m, c), c, ah.v[A_DS][lane], __ldg(m.rarrf + ir0));
   }
   return live;
 }
 
 // The packets that k_wave left, one per warp: every lane holds the packet, and
 // the parts of its events that a lane alone would do one after another are
-// shared between the lanes.  The mixed form forms the absorptions of a cell
-// side by side (tail_window), the tries of a scattering angle ten at once (scat_draw),
-// the walls of a cell side by side (next_wall_warp) and the tallies of a step
-// in one instruction (tauint_warp); the FP64 form reads its logarithms, sines
-// and cosines from a table 32 lanes formed (DrawTable) and shares the tries
-// and the tallies.  What bounds it is the latency of one packet's chain of
-// events: in the plain model's disk 5.0 us an event for a lane of k_wave, 3.0
-// us here with one event after another, 1.2 us with the absorptions side by
-// side.  The arithmetic is that of k_wave, bit for bit.
+// shared between the lanes: the absorptions of a cell are formed side by side
+// (tail_window), the tries of a scattering angle ten at once (scat_draw), the
+// walls of a cell by a lane each (next_wall_warp, next_wall_warp64) and the
+// tallies of a step in one instruction.  What bounds it is the latency of one
+// packet's chain of events, and with many packets in flight the fetch of its
+// instructions.  In the plain model's disk a lone packet took 5.0 us an event in
+// a lane of k_wave, and takes 0.95 us here; 13 and 5.6 us in the FP64 form.  The
+// arithmetic is that of k_wave, bit for bit.
 template <class R, bool kPeel, bool kFused>
-__global__ void __launch_bounds__(128, 4) k_tail(DevModel m, DevTallies t, TallyDims d, RunArgs a, Slot<R>* pool,
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 3) k_tail(DevModel m, DevTallies t, TallyDims d, RunArgs a, Slot<R>* pool,
                                                  const unsigned int* nlive, const unsigned int* live,
                                                  unsigned int* next, PeelRec<R>* queue, unsigned long long* qcount,
                                                  int E, unsigned int* alive_out, unsigned int* live_out) {
@@ -3501,13 +3602,12 @@ __global__ void __launch_bounds__(128, 4) k_tail(DevModel m, DevTallies t, Tally
   dust_view<R>(m, reinterpret_cast<R*>(dust_smem), dv);
   __shared__ unsigned long long block_counters[16];
   __shared__ DrawTable<R> draws[4];
-  __shared__ Ahead ahead[sizeof(R) == 4 ? 4 : 1];
+  __shared__ Ahead<R> ahead[4];
   Local L;
   local_init(L, block_counters);
   const int lane = threadIdx.x & 31;
   L.on = lane == 0;
   const unsigned n = *nlive;
-  Tracer tr{nullptr, 0, 0};
   for (;;) {
     unsigned k = 0;
     if (lane == 0) k = atomicAdd(next, 1u);
@@ -3519,25 +3619,11 @@ __global__ void __launch_bounds__(128, 4) k_tail(DevModel m, DevTallies t, Tally
     rng_init(rng, draws + (threadIdx.x >> 5), a.key0, a.key1, s.pid, s.c0, s.left);
     unsigned long long slot = 0ull, slot_end = 0ull;
     for (int nrec = 0; !kPeel || nrec < E;) {
-      if constexpr (sizeof(R) == 4) {
-        if (tail_window<kPeel, kFused>(m, dv, t, d, a, s.p, rng, s.f, ahead[threadIdx.x >> 5], L, queue, qcount, slot, slot_end, nrec,
-                                       E))
-          continue;
-      } else {
-        ensure(rng, 8);  // an event draws at most 7 beside the tries of a scattering
-        PeelRec<R> none;
-        if (kPeel && slot == slot_end) {
-          if (lane == 0) slot = atomicAdd(qcount, (unsigned long long)a.qchunk);
-          slot = __shfl_sync(0xffffffffu, slot, 0);
-          slot_end = slot + (unsigned long long)a.qchunk;
-        }
-        if (interact<R>(m, dv, t, a, s.p, rng, s.f, L, tr, kPeel ? queue[slot] : none)) ++slot;
-        ++nrec;
-        ensure(rng, 8);
-        if (walk<R, kFused>(m, t, d, a, s.p, rng, s.f, L, tr, false) == ST_INTERACT) continue;
+      if (!tail_window<R, kPeel, kFused>(m, dv, t, d, a, s.p, rng, s.f, ahead[threadIdx.x >> 5], L, queue, qcount, slot,
+                                         slot_end, nrec, E)) {
+        s.stage = 0;
+        break;
       }
-      s.stage = 0;
-      break;
     }
     L.settle();
     if constexpr (kPeel) {
