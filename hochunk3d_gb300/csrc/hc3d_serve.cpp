@@ -95,7 +95,7 @@ int64_t footprint_bytes(const hc3d::Model& m, int npeel) {
   const int64_t grid = ncell * (4 * 4 /*rho f32*/ + 4 * 8 /*rho f64*/ + 2 * 4 * 8 /*tdust, massarr*/ + 4 * 4 /*tdust f32*/ + 4 * 8 /*Lucy rows*/ +
                                 1 /*peel mask*/ + 2 * 4 * 8 /*nabs, dtauabs*/ + 8 /*jmean*/ + 2 * 4 /*killed, dbig*/) +
                        sg;
-  const int64_t walls = (int64_t)(m.nrg + m.ntg + m.npg) * 64 + n4 * 8 /*vcell*/;
+  const int64_t walls = (int64_t)(m.nrg + m.ntg + m.npg) * 64 + n4 * (8 /*vcell*/ + 4 * 8 /*planes in the callers' layout*/);
   const int64_t tables = (int64_t)m.nT * m.nnu * 4 * 12 + (int64_t)m.nlammax * 4 * 5 * 12 + (1 << 20);
   const int64_t sed = (int64_t)m.nfreq * m.nmu * m.nph * m.nap * 8 * 9 * 8;
   const int64_t psed = (int64_t)m.nfreq * npeel * m.nap * 8 * 9 * 8;
