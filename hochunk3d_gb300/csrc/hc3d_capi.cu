@@ -1311,6 +1311,7 @@ extern "C" int hc3d_load_grid(hc3d_ctx* c, const hc3d_grid* g) {
   }
   DevModel& m = c->dm;
   m.nrg = nrg; m.ntg = ntg; m.npg = npg; m.ncell = ncell;
+  m.nr1 = nrg - 1; m.nt1 = ntg - 1; m.np1 = npg - 1; m.nplane = m.nr1 * m.nt1;
   m.rarr = d_r; m.r2arr = d_r2; m.thetarr = d_th; m.costarr = d_ct; m.phiarr = d_ph; m.tan2d = d_t2; m.tan2f = d_t2f; m.hemi = d_hemi;
   {
     std::vector<float> rf32(g->rarr, g->rarr + nrg), r2f32(g->r2arr, g->r2arr + nrg);
@@ -1325,24 +1326,26 @@ extern "C" int hc3d_load_grid(hc3d_ctx* c, const hc3d_grid* g) {
     float2* d_cs = nullptr;
     if ((r = dupload(c, own, &d_cs, cs.data(), cs.size()))) return r;
     m.thcs = d_cs;
-    std::vector<float2> r2p(nrg - 1), cf(ntg), pf(npg), cc(ntg);
+    std::vector<float2> r2p(nrg - 1), cf(ntg), pf(npg), pw;
     for (int i = 0; i < nrg - 1; ++i) r2p[i] = make_float2(r2f32[i], r2f32[i + 1]);
     for (int i = 0; i < ntg; ++i) cf[i] = make_float2(tan2f[i], hemi[i]);
+    for (int i = 0; i < nrg - 1; ++i) pw.push_back(make_float2(rf32[i], rf32[i + 1]));
     for (int i = 0; i < ntg; ++i) {
       // cos^2 theta of the wall; the midplane (tan2arr = -1) and the poles (tan2arr = 0) are marked
       const double cth = std::cos(g->thetarr[i]);
-      if (g->tan2arr[i] < 0.0) cc[i] = make_float2(-1.f, 0.f);
-      else if (g->tan2arr[i] == 0.0) cc[i] = make_float2(1.f, 0.f);
-      else cc[i] = make_float2((float)(cth * cth), hemi[i]);
+      if (g->tan2arr[i] < 0.0) pw.push_back(make_float2(-1.f, 0.f));
+      else if (g->tan2arr[i] == 0.0) pw.push_back(make_float2(1.f, 0.f));
+      else pw.push_back(make_float2((float)(cth * cth), hemi[i]));
     }
     for (int i = 0; i < npg; ++i) pf[i] = make_float2(af[i], bf[i]);
-    float2 *d_r2p = nullptr, *d_cf = nullptr, *d_pf = nullptr, *d_cc = nullptr;
+    pw.insert(pw.end(), pf.begin(), pf.end());
+    float2 *d_r2p = nullptr, *d_cf = nullptr, *d_pf = nullptr, *d_pw = nullptr;
     if ((r = dupload(c, own, &d_r2p, r2p.data(), r2p.size())) || (r = dupload(c, own, &d_cf, cf.data(), cf.size())) ||
-        (r = dupload(c, own, &d_pf, pf.data(), pf.size())) || (r = dupload(c, own, &d_cc, cc.data(), cc.size())))
+        (r = dupload(c, own, &d_pf, pf.data(), pf.size())) || (r = dupload(c, own, &d_pw, pw.data(), pw.size())))
       return r;
     m.r2pair = d_r2p;
     m.conef = d_cf;
-    m.conec = d_cc;
+    m.peelw = d_pw;
     m.planef = d_pf;
   }
   m.aarrd = d_a; m.barrd = d_b; m.aarrf = d_af; m.barrf = d_bf; m.rho4f = d_rf; m.rho4d = d_rd;

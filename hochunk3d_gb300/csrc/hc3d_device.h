@@ -50,6 +50,7 @@ struct DevTallies {
 struct DevModel {
   // grid
   int nrg, ntg, npg;
+  int nr1, nt1, np1, nplane;  // cells along each axis and in one azimuthal plane: nrg-1, ntg-1, npg-1, nr1*nt1
   int64_t ncell;
   const double* rarr;     // (nrg)
   const float* rarrf;     // (nrg)
@@ -65,8 +66,11 @@ struct DevModel {
   // interleaved FP32 wall data of the mixed-form wall search (one load per family)
   const float2* r2pair;   // (nrg-1) squared inner and outer radius of radial cell ir (index ir-1)
   const float2* conef;    // (ntg) tan^2 and hemisphere sign of polar wall it (index it-1)
-  const float2* conec;    // (ntg) cos^2 theta and hemisphere sign of polar wall it: C < 0 marks the
-                          // midplane, a hemisphere sign of 0 a pole (mixed-form peel-off walk)
+  // walls of the mixed-form peel-off walk: the inner and outer radius of the nr1 radial cells, then
+  // cos^2 theta and hemisphere sign of the ntg polar walls (cos^2 theta < 0 marks the midplane, a
+  // hemisphere sign of 0 a pole), then planef.  In one table, so that the lanes of a warp that cross
+  // different kinds of wall read the next one with one load.
+  const float2* peelw;
   const float2* planef;   // (npg) A = sin(phi), B = -cos(phi) of azimuthal wall ip (index ip-1)
   const double* aarrd; const double* barrd;  // (npg)
   const float* aarrf; const float* barrf;    // (npg)

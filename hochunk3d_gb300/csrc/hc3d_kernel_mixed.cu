@@ -91,10 +91,10 @@ cudaError_t launch_wave_peel_mixed(const DevModel& m, const DevTallies& t, const
   const auto* qu = static_cast<const dev::PeelRec<float>*>(w.queue[q]);
   switch (cfg.variant) {
     case 1:
-      dev::k_peel_mixed<float, 192, 3><<<cfg.blocks, 192, 0, cfg.stream>>>(m, t, d, a, qu, w.qcount[q], w.next_ray[q]);
+      dev::k_peel_mixed<float, 192, 3><<<cfg.blocks, 192, a.npeel * sizeof(dev::PeelDir), cfg.stream>>>(m, t, d, a, qu, w.qcount[q], w.next_ray[q]);
       break;
     default:
-      dev::k_peel_mixed<float, 128, 5><<<cfg.blocks, 128, 0, cfg.stream>>>(m, t, d, a, qu, w.qcount[q], w.next_ray[q]);
+      dev::k_peel_mixed<float, 128, 5><<<cfg.blocks, 128, a.npeel * sizeof(dev::PeelDir), cfg.stream>>>(m, t, d, a, qu, w.qcount[q], w.next_ray[q]);
   }
   return cudaGetLastError();
 }

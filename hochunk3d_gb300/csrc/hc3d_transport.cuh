@@ -578,6 +578,19 @@ constexpr float kGrazeSphere = 1.0f / 1024.0f;
 // square root of a positive FP32 value by the reciprocal square root (the
 // wall searches take it of discriminants already tested > 0)
 __device__ __forceinline__ float fsqrt_pos(float x) { return x * rsqrtf(x); }
+// rsqrtf and __fdividef for operands and results that are never subnormal
+// (the lengths and roots of a ray that crosses a grid): the same values without
+// the scaling that subnormals would need, four instructions less each.
+__device__ __forceinline__ float rsqrt_n(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float fdiv_n(float x, float y) {
+  float r;
+  asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(x), "f"(y));
+  return r;
+}
 
 // The mixed-form wall search on a Ray at path length S.  The reference keeps
 // the roots of every wall in closest_wall and skips the root of the wall it
@@ -1863,9 +1876,9 @@ struct PeelDir {
 };
 
 struct PeelEsc {
-  unsigned long long e;
-  float tsum, xf, yf, zf;
+  unsigned e;
   int k;
+  float tsum, xf, yf, zf;
 };
 
 constexpr int kPeelThreads = 256;
@@ -1979,7 +1992,9 @@ struct PeelWalk {
   float tr;                      // next sphere crossing: the inner sphere when tr < 0, else the outer
   float lo1, lo2, hi1, hi2;      // roots ahead on the lower and upper polar wall of the cell
   float tp;                      // next azimuthal crossing
-  int ir, it, ip, nstep;
+  int ir, it, ip;
+  int left;                      // crossings left before the ray counts as stuck
+  int c;                         // compact index of the cell
   bool up;                       // azimuth increases along the ray
   float kap[kSlots];
   float4 rho;                    // peel-masked densities of the current cell, loaded when the ray entered it
@@ -1989,57 +2004,64 @@ struct PeelWalk {
 
   enum { GOING = 0, OUT = 1, ENDED = 2 };  // OUT: left the grid, to be tallied
 
-  // Issue the load of the current cell's densities.  Called as soon as the
-  // ray enters a cell, before the next crossings of the walls are formed,
-  // so that the load's latency overlaps that arithmetic instead of stalling
-  // the next step.  An index out of range is caught by the next step.
-  __device__ __forceinline__ void fetch_rho(const DevModel& m) {
-    if (ir >= 1 && ir <= m.nrg - 1 && it >= 1 && it <= m.ntg - 1 && ip >= 1 && ip <= m.npg - 1)
-      rho = __ldg(m.rho4p + (ir - 1) + (m.nrg - 1) * ((it - 1) + (m.ntg - 1) * (ip - 1)));
+  // The first cell's index and densities.  A ray that starts outside the grid
+  // has no crossings left; from there on step() keeps the index in it.
+  // The row is loaded as soon as the ray enters a cell, before the next
+  // crossings of the walls are formed, so that the load's latency overlaps
+  // that arithmetic instead of stalling the next step.
+  __device__ __forceinline__ void first_cell(const DevModel& m, int cap) {
+    left = 0;
+    if (ir >= 1 && ir <= m.nr1 && it >= 1 && it <= m.nt1 && ip >= 1 && ip <= m.np1) {
+      left = cap + 1;
+      c = (ir - 1) + m.nr1 * (it - 1) + m.nplane * (ip - 1);
+      rho = __ldg(m.rho4p + c);
+    }
   }
 
-  // the sphere bounding cell ir in the direction of travel at parameter t
-  __device__ __forceinline__ void next_sphere(const DevModel& m) {
-    const float rin = __ldg(m.rarrf + ir - 1);
-    if (t < 0.f && rin > p) {
-      const float ti = -fsqrt_pos((rin - p) * (rin + p));
-      if (ti >= t) {
-        tr = ti;
+  // the sphere bounding the cell (inner and outer radius) in the direction of travel at parameter t
+  __device__ __forceinline__ void next_sphere(float2 radii) {
+    const float rin = radii.x, rout = radii.y;
+    const bool in = t < 0.f && rin > p;  // the inner sphere lies ahead
+    const float r = in ? rin : rout;
+    const float q = (r - p) * (r + p);
+    float x = q > 0.f ? q * rsqrt_n(q) : 0.f;
+    if (in) {
+      if (-x >= t) {
+        tr = -x;
         return;
       }
+      x = ((rout - p) * (rout + p)) * rsqrt_n((rout - p) * (rout + p));
     }
-    const float rout = __ldg(m.rarrf + ir);
-    const float q = (rout - p) * (rout + p);
-    tr = fmaxf(fmaxf(q > 0.f ? fsqrt_pos(q) : 0.f, t), 0.f);
+    tr = fmaxf(fmaxf(x, t), 0.f);
   }
 
-  // The roots r1 <= r2 at or after t of polar wall w (index into conec) on
+  // The roots r1 <= r2 at or after t of a polar wall (cos^2 theta, hemisphere sign) on
   // the nappe of its hemisphere, kInf where there are none; own: the ray
   // starts on this wall, so the root nearest t is not taken.  The cone is
   // C rho^2 - (1 - C) z^2 = 0 with C = cos^2 theta, so no coefficient grows
   // like tan^2 theta near the midplane; with |u| = 1 and c.u = 0 the terms
   // are a = C - uz^2, h = -cz uz, q = C p^2 - cz^2, and the discriminant
   // h^2 - a q = C (cz^2 - a p^2) has no cancelling terms.
-  __device__ __forceinline__ void cone_roots(const DevModel& m, int w, bool own, float& r1, float& r2) const {
+  __device__ __forceinline__ void cone_roots(float2 cw, bool own, float& r1, float& r2) const {
     r1 = r2 = kInf;
-    const float2 cw = __ldg(m.conec + w);
     const float C = cw.x, hemi = cw.y;
-    if (C < 0.f) {  // the midplane z = 0
-      if (!own && uz != 0.f) {
-        const float r = __fdividef(-cz, uz);
+    if (C < 0.f || hemi == 0.f) {
+      // C < 0: the midplane z = 0; otherwise a pole, which is not crossed
+      if (C < 0.f && !own && uz != 0.f) {
+        const float r = fdiv_n(-cz, uz);
         if (r >= t) r1 = r;
       }
       return;
     }
-    if (hemi == 0.f) return;  // a pole: no crossing
     const float a = fmaf(-uz, uz, C);
     const float h = -cz * uz;
     const float q = fmaf(C, p2, -cz * cz);
     const float D = C * fmaf(-a, p2, cz * cz);
     if (!(D > 0.f)) return;
-    const float w_ = -(h + copysignf(fsqrt_pos(D), h));  // |w_| >= sqrt(D) > 0
-    const float ra = a != 0.f ? __fdividef(w_, a) : kInf, rb = __fdividef(q, w_);
+    const float w_ = -(h + copysignf(D * rsqrt_n(D), h));  // |w_| >= sqrt(D) > 0
+    const float ra = a != 0.f ? fdiv_n(w_, a) : kInf, rb = fdiv_n(q, w_);
     const float x1 = fminf(ra, rb), x2 = fmaxf(ra, rb);
+    // on the nappe z hemi > 0: the sign of a product that does not underflow
     bool v1 = fmaf(x1, uz, cz) * hemi > 0.f;
     bool v2 = x2 < kInf && fmaf(x2, uz, cz) * hemi > 0.f;
     if (own) {
@@ -2052,14 +2074,13 @@ struct PeelWalk {
     r2 = v1 && v2 ? x2 : kInf;
   }
 
-  // the crossing at or after t of azimuthal wall w (index into planef) on its
+  // the crossing at or after t of an azimuthal wall (sin phi, -cos phi) on its
   // half-plane, kInf where there is none
-  __device__ __forceinline__ float plane_root(const DevModel& m, int w) const {
-    const float2 ab = __ldg(m.planef + w);
+  __device__ __forceinline__ float plane_root(float2 ab) const {
     const float A = ab.x, B = ab.y;
     const float den = fmaf(A, ux, B * uy);
     if (den == 0.f) return kInf;
-    const float r = __fdividef(-fmaf(A, cx, B * cy), den);
+    const float r = fdiv_n(-fmaf(A, cx, B * cy), den);
     if (!(r >= t)) return kInf;
     // (x, y) . (cos phi, sin phi) > 0 with cos phi = -B, sin phi = A
     if (fmaf(A, fmaf(r, uy, cy), -B * fmaf(r, ux, cx)) <= 0.f) return kInf;
@@ -2101,73 +2122,111 @@ struct PeelWalk {
     tsum = 0.0;
     tpart = 0.f;
     tf = 0.f;
-    nstep = 0;
     lo1 = lo2 = hi1 = hi2 = tp = kInf;
     tr = fmaxf(t, 0.f);
     up = x * uyd - y * uxd > 0.0;  // z component of x cross u, constant along the line
     if (!go || ir < 1 || ir > m.nrg - 1) return go;
-    next_sphere(m);
+    const float2 *cones = m.peelw + m.nr1, *planes = cones + m.ntg;
+    next_sphere(__ldg(m.peelw + ir - 1));
     if (m.ntg > 2) {
-      cone_roots(m, it - 1, (own >> 3) & 1, lo1, lo2);
-      cone_roots(m, it, (own >> 4) & 1, hi1, hi2);
+      cone_roots(__ldg(cones + it - 1), (own >> 3) & 1, lo1, lo2);
+      cone_roots(__ldg(cones + it), (own >> 4) & 1, hi1, hi2);
       if (m.npg > 2) {
         const bool mine = up ? ((own >> 6) & 1) : ((own >> 5) & 1);
-        tp = mine ? kInf : plane_root(m, up ? ip : ip - 1);
+        tp = mine ? kInf : plane_root(__ldg(planes + (up ? ip : ip - 1)));
       }
     }
     return go;
   }
 
-  __device__ __forceinline__ int step(const DevModel& m, int cap, PeelCount& pc) {
-    if (nstep > cap || it < 1 || it > m.ntg - 1 || ir < 1 || ir > m.nrg - 1) {
-      pc.stuck++;
-      return ENDED;
-    }
-    ++nstep;
+  // One crossing.  Issue slots and the latency between them bound the walk
+  // (58 % of the slots, 20 warps on an SM): of 27 lanes that go on, 20 cross a
+  // sphere, 6 a cone and 1 or 2 a plane, and the warp runs the three sections
+  // in turn.  So the lanes move their index and load the next wall, whatever
+  // its kind, and the next row together; each then recomputes the roots of
+  // the one family that it crossed, the walls below and above (inwards and
+  // outwards) through the same code.  The row is used late, after the next
+  // index is known, and the wall is asked for before it, so that neither waits
+  // for the other.  On the full three-dimensional model (982 million rays,
+  // 5.6e10 crossings) the walk took 622 ms with a section and its own loads for
+  // each side of each kind and takes 446 ms.  Holding the lanes together at
+  // each crossing (a vote, one exit) cost 6 to 8 %; letting cones and planes
+  // wait for more lanes gains nothing, since the lanes that wait are missed
+  // in the part that all run.
+  __device__ __forceinline__ int step(const DevModel& m, PeelCount& pc) {
     const float th = fminf(lo1, hi1);
     const float tn = fminf(tr, fminf(th, tp));
     const float ds = tn - t;
     t = tn;
+    const bool sph = tn == tr, pol = tn == th;
+    const bool below = lo1 <= hi1;
+    bool out = false;
+    int w;  // the wall that comes next, in peelw
+    if (sph || pol) {  // one index moves by one: selects, no branches
+      const int d = (sph ? tr < 0.f : below) ? -1 : 1;
+      const int v = (sph ? ir : it) + d;
+      c += sph ? d : d * m.nr1;
+      out = (unsigned)(v - 1) >= (unsigned)(sph ? m.nr1 : m.nt1);
+      ir = sph ? v : ir;
+      it = sph ? it : v;
+      w = sph ? v - 1 : m.nr1 + (below ? v - 1 : v);
+    } else {  // with the wrap at 0 / 2 pi
+      int q = up ? ip + 1 : ip - 1;
+      if (q > m.np1) q = 1;
+      if (q < 1) q = m.np1;
+      c += (q - ip) * m.nplane;
+      ip = q;
+      w = m.nr1 + m.ntg + (up ? q : q - 1);
+    }
+    float2 wall;
+    if (!out) wall = __ldg(m.peelw + w);
     const float opac = fmaf(kap[0], rho.x, fmaf(kap[1], rho.y, fmaf(kap[2], rho.z, kap[3] * rho.w)));
     const float dtau = opac * ds;
     tpart += dtau;
     tf += dtau;
-    pc.cross++;
     if (tf > (float)kTauMax) return ENDED;
-    if (tn == tr) {
-      ir += tr < 0.f ? -1 : 1;
-      if (ir == m.nrg) return OUT;
-      if (ir == 0) return ENDED;
-      fetch_rho(m);
-      next_sphere(m);
-    } else if (tn == th) {
-      if (lo1 <= hi1) {  // the lower polar wall: into cell it - 1
-        hi1 = lo2;
-        hi2 = kInf;
-        --it;
-        if (it < 1) return GOING;  // caught by the range check of the next step
-        fetch_rho(m);
-        cone_roots(m, it - 1, false, lo1, lo2);
-      } else {           // the upper polar wall: into cell it + 1
-        lo1 = hi2;
-        lo2 = kInf;
-        ++it;
-        if (it > m.ntg - 1) return GOING;
-        fetch_rho(m);
-        cone_roots(m, it, false, hi1, hi2);
-      }
-    } else {  // the azimuthal wall, with the wrap at 0 / 2 pi
-      if (up) {
-        ip = ip == m.npg - 1 ? 1 : ip + 1;
-        fetch_rho(m);
-        tp = plane_root(m, ip);
-      } else {
-        ip = ip == 1 ? m.npg - 1 : ip - 1;
-        fetch_rho(m);
-        tp = plane_root(m, ip - 1);
-      }
+    if (out) {
+      if (sph) return ir == 0 ? ENDED : OUT;
+      pc.stuck++;  // past the last polar wall
+      return ENDED;
+    }
+    rho = __ldg(m.rho4p + c);
+    if (sph) {
+      next_sphere(wall);
+    } else if (pol) {  // the wall behind is the one ahead no more; its second root may be
+      float r1, r2;
+      cone_roots(wall, false, r1, r2);
+      const float back = below ? lo2 : hi2;
+      lo1 = below ? r1 : back;
+      lo2 = below ? r2 : kInf;
+      hi1 = below ? back : r1;
+      hi2 = below ? kInf : r2;
+    } else {
+      tp = plane_root(wall);
     }
     return GOING;
+  }
+
+  // Up to n crossings, then the FP32 partial escape tau goes to the FP64 sum.
+  // The crossings are counted once, not in each.
+  __device__ __forceinline__ int round(const DevModel& m, int n, PeelCount& pc) {
+    n = min(n, left);
+    int st = GOING, k = 0;
+#pragma unroll 1
+    while (k < n) {
+      ++k;
+      st = step(m, pc);
+      if (st != GOING) break;
+    }
+    pc.cross += k;
+    left -= k;
+    if (st == GOING && left == 0) {
+      pc.stuck++;
+      st = ENDED;
+    }
+    tsum += (double)tpart;
+    tpart = 0.f;
+    return st;
   }
 
   // the set-up state of a ray that start() accepted, for a lane to take later
@@ -2182,7 +2241,7 @@ struct PeelWalk {
     q.k = k;
   }
 
-  __device__ __forceinline__ void load(const DevModel& m, const PeelStart& q, const PeelDir& dd) {
+  __device__ __forceinline__ void load(const DevModel& m, const PeelStart& q, const PeelDir& dd, int cap) {
     cx = q.cx; cy = q.cy; cz = q.cz; p = q.p; p2 = q.p2; t = q.t; tr = q.tr;
     lo1 = q.lo1; lo2 = q.lo2; hi1 = q.hi1; hi2 = q.hi2; tp = q.tp;
 #pragma unroll
@@ -2193,14 +2252,7 @@ struct PeelWalk {
     tsum = 0.0;
     tpart = 0.f;
     tf = 0.f;
-    nstep = 0;
-    fetch_rho(m);
-  }
-
-  // add the FP32 partial escape tau of the last round to the FP64 sum
-  __device__ __forceinline__ void flush_tau() {
-    tsum += (double)tpart;
-    tpart = 0.f;
+    first_cell(m, cap);
   }
 
   // FP32 point of the ray where it left the grid
@@ -2227,14 +2279,11 @@ __device__ __forceinline__ void peel_ray_mixed(const DevModel& m, const DevTalli
   const PeelDir dd = peel_dir(a, k);
   PeelWalk w;
   if (!w.start(m, e, dd)) return;
-  w.fetch_rho(m);
   PeelCount pc{1u, 0u, 0u};
   const int cap = 4 * (m.nrg + m.ntg + m.npg) + 64;
+  w.first_cell(m, cap);
   int st;
-  while ((st = w.step(m, cap, pc)) == PeelWalk::GOING) {
-    if ((w.nstep & 7) == 0) w.flush_tau();  // the rounds of k_peel_mixed
-  }
-  w.flush_tau();
+  while ((st = w.round(m, 8, pc)) == PeelWalk::GOING) {}
   L.add(HC3D_CNT_PEELS);
   L.add(HC3D_CNT_CROSS_PEEL, pc.cross);
   if (pc.stuck) L.add(HC3D_CNT_PEEL_STUCK, pc.stuck);
@@ -3690,17 +3739,21 @@ static __device__ __noinline__ int prep_rays(const DevModel& m, const PeelRec<fl
 // Instantiated for two block shapes, between which the autotuner picks:
 // 128 threads x 5 blocks per SM and 192 x 3, both held to 96 registers (the
 // walk state of a lane, the set-up stack and the 32-ray tally would take
-// about 118; the spills are outside the crossing loop).  With one register
+// about 120; the spills are outside the crossing loop).  With one register
 // budget the two compile to the same arithmetic, so their tallies agree bit
-// for bit.  128 x 5 (20 warps per SM) ran 2 % faster than 256 x 2 at 118
-// registers (16 warps); 256 x 3 at 80 registers ran slower.
+// for bit.  On the full three-dimensional model 128 x 5 (20 warps per SM) took
+// 446 ms, 128 x 4 at 122 registers 456, 256 x 2 458, 64 x 9 442 (within the
+// runs of one shape), 128 x 6 at 80 registers 512.  The directions lie in
+// dynamic shared memory, as many as there are: a block holds 20 KB instead of
+// 27 and leaves the rows of the cells 124 KB of L1 instead of 92 (498 -> 466 ms
+// before the loads were moved).
 template <class R, int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB) k_peel_mixed(DevModel m, DevTallies t, TallyDims d, RunArgs a,
                                                               const PeelRec<R>* queue,
                                                               const unsigned long long* qcount,
                                                               unsigned long long* next_ray) {
   static_assert(sizeof(R) == 4, "the warp-synchronous ray pool is the mixed form");
-  __shared__ PeelDir dirs[kMaxPeel];
+  extern __shared__ PeelDir dirs[];  // npeel of them
   __shared__ PeelEsc esc[THREADS / 32][kPeelBuf];
   __shared__ PeelRec<float> stage[THREADS / 32][kPeelStage];
   __shared__ PeelStart prep[THREADS / 32][32];
@@ -3767,7 +3820,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_peel_mixed(DevModel m, DevTal
         const PeelStart& q = pbuf[nprep - 1 - idx];
         e = q.e;
         k = q.k;
-        w.load(m, q, dirs[k]);
+        w.load(m, q, dirs[k], cap);
         have = true;
         pc.peels++;
       }
@@ -3780,16 +3833,9 @@ __global__ void __launch_bounds__(THREADS, MINB) k_peel_mixed(DevModel m, DevTal
       // up to kPeelSub crossings between refills: the warp-wide refill and
       // parking steps run once per kPeelSub crossings, at the cost of a lane
       // whose ray ends idling for the rest of the round
-#pragma unroll 1
-      for (int sub = 0; sub < kPeelSub; ++sub) {
-        const int s = w.step(m, cap, pc);
-        if (s != PeelWalk::GOING) {
-          out = s == PeelWalk::OUT;
-          have = false;
-          break;
-        }
-      }
-      w.flush_tau();  // one FP64 add per round of up to kPeelSub crossings
+      const int s = w.round(m, kPeelSub, pc);
+      out = s == PeelWalk::OUT;
+      have = s == PeelWalk::GOING;
     }
     // park the rays that left the grid; tally them 32 at a time
     const unsigned outm = __ballot_sync(0xffffffffu, out);
