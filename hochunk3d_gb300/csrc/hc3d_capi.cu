@@ -1392,13 +1392,18 @@ extern "C" int hc3d_load_grid(hc3d_ctx* c, const hc3d_grid* g) {
     }
     for (int i = 0; i < npg; ++i) pf[i] = make_float2(af[i], bf[i]);
     pw.insert(pw.end(), pf.begin(), pf.end());
-    float2 *d_r2p = nullptr, *d_cf = nullptr, *d_pf = nullptr, *d_pw = nullptr;
+    std::vector<float2> ww(r2p);
+    ww.insert(ww.end(), cf.begin(), cf.end());
+    ww.insert(ww.end(), pf.begin(), pf.end());
+    float2 *d_ww = nullptr, *d_r2p = nullptr, *d_cf = nullptr, *d_pf = nullptr, *d_pw = nullptr;
     if ((r = dupload(c, own, &d_r2p, r2p.data(), r2p.size())) || (r = dupload(c, own, &d_cf, cf.data(), cf.size())) ||
-        (r = dupload(c, own, &d_pf, pf.data(), pf.size())) || (r = dupload(c, own, &d_pw, pw.data(), pw.size())))
+        (r = dupload(c, own, &d_pf, pf.data(), pf.size())) || (r = dupload(c, own, &d_pw, pw.data(), pw.size())) ||
+        (r = dupload(c, own, &d_ww, ww.data(), ww.size())))
       return r;
     m.r2pair = d_r2p;
     m.conef = d_cf;
     m.peelw = d_pw;
+    m.wallw = d_ww;
     m.planef = d_pf;
   }
   m.aarrd = d_a; m.barrd = d_b; m.aarrf = d_af; m.barrf = d_bf; m.rho4f = d_rf; m.rho4d = d_rd;

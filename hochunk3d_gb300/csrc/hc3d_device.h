@@ -71,6 +71,8 @@ struct DevModel {
   // hemisphere sign of 0 a pole), then planef.  In one table, so that the lanes of a warp that cross
   // different kinds of wall read the next one with one load.
   const float2* peelw;
+  // walls of k_tail's search in one table: r2pair, conef, planef
+  const float2* wallw;
   const float2* planef;   // (npg) A = sin(phi), B = -cos(phi) of azimuthal wall ip (index ip-1)
   const double* aarrd; const double* barrd;  // (npg)
   const float* aarrf; const float* barrf;    // (npg)

@@ -717,20 +717,18 @@ __device__ __forceinline__ bool next_wall_ray(const DevModel& m, Ray& r, const P
 // cycles against 900 for the walls one after another.
 template <bool kFused>
 __device__ __forceinline__ bool next_wall_warp(const DevModel& m, Ray& r, const PathLen& S, int ir, int it, int ip,
-                                               int own, float& dt, int& iface) {
+                                               int own, float& dt, int& win, int& side) {
   const int lane = threadIdx.x & 31;
   const float ux = r.ux, uy = r.uy, uz = r.uz;
   const float xr = fmaf(S.hi, ux, fmaf(S.lo, ux, r.x0));
   const float yr = fmaf(S.hi, uy, fmaf(S.lo, uy, r.y0));
   const float zr = fmaf(S.hi, uz, fmaf(S.lo, uz, r.z0));
-  const int side = fmaf(xr, uy, -__fmul_rn(yr, ux)) > 0.f ? 1 : 0;
-  const float2* wp = m.r2pair + ir - 1;
-  if (lane == 2) wp = m.conef + it - 1;
-  if (lane == 3) wp = m.conef + it;
-  if (lane == 4) wp = m.planef + ip - 1 + side;
-  const float2 w = __ldg(wp);
-  const int id = lane + 1 + (lane == 4 ? side : 0);
-  const bool mine = (own >> min(id, 7)) & 1;
+  side = fmaf(xr, uy, -__fmul_rn(yr, ux)) > 0.f ? 1 : 0;
+  // the place of the lane's wall in wallw, and its bit in `own`
+  const int turn = lane == 4 ? side : 0;
+  const int at = lane < 2 ? ir - 1 : (lane < 4 ? m.nr1 + it + (lane - 3) : m.nr1 + m.ntg + ip - 1 + turn);
+  const float2 w = __ldg(m.wallw + at);
+  const bool mine = (own >> (min(lane, 6) + 1 + turn)) & 1;
   const float pxy = fmaf(xr, ux, __fmul_rn(yr, uy)), pz = __fmul_rn(zr, uz);
   const float rho2 = fmaf(xr, xr, __fmul_rn(yr, yr)), z2 = __fmul_rn(zr, zr);
   constexpr float kNone = 3.402823466e38f;
@@ -740,11 +738,11 @@ __device__ __forceinline__ bool next_wall_warp(const DevModel& m, Ray& r, const 
   const float b = 2.f * fmaf(-tan2, pz, pxy);
   const float cq = fmaf(-tan2, z2, rho2);
   const float disc = fmaf(b, b, -__fmul_rn(4.f * a, cq));
-  const float rs = rsqrtf(disc), inv = __fdividef(0.5f, a);
+  const float rs = rsqrt_n(disc), inv = fdiv_n(0.5f, a);
   const float t1 = __fmul_rn(fmaf(disc, rs, -b), inv), t2 = __fmul_rn(fmaf(-disc, rs, -b), inv);
   // the midplane; the far root on one's own cone; a ray along the cone: one root
   const bool mid = tan2 < 0.f;
-  const float ts = __fdividef(mid ? -zr : (mine ? -b : -cq), mid ? uz : (mine ? a : b));
+  const float ts = fdiv_n(mid ? -zr : (mine ? -b : -cq), mid ? uz : (mine ? a : b));
   auto ahead = [&](float t) { return t >= 0.f && fmaf(t, uz, zr) * hemi > 0.f; };
   float tc = kNone;
   if (mid) {
@@ -757,9 +755,12 @@ __device__ __forceinline__ bool next_wall_warp(const DevModel& m, Ray& r, const 
   }
   if (tan2 == 0.f) tc = kNone;  // a pole
   // planes
-  const float d = fmaf(w.x, ux, __fmul_rn(w.y, uy));
-  const float tq = __fdividef(-fmaf(w.x, xr, __fmul_rn(w.y, yr)), d);
-  const float tp = m.npg > 2 && !mine && d != 0.f && tq >= 0.f ? tq : kNone;
+  float tp = kNone;
+  if (m.np1 > 1) {
+    const float d = fmaf(w.x, ux, __fmul_rn(w.y, uy));
+    const float tq = fdiv_n(-fmaf(w.x, xr, __fmul_rn(w.y, yr)), d);
+    if (!mine && d != 0.f && tq >= 0.f) tp = tq;
+  }
   // spheres
   const float r2 = lane == 0 ? w.x : w.y;
   float hb = kFused ? fmaf(zr, uz, pxy) : __fadd_rn(pxy, pz);
@@ -777,8 +778,8 @@ __device__ __forceinline__ bool next_wall_warp(const DevModel& m, Ray& r, const 
     c = (float)cd;
     ds = (float)fma(hbd, hbd, -cd);
   }
-  const float rd = rsqrtf(ds), sq = __fmul_rn(ds, rd);
-  const float tn = __fdividef(fmaxf(lane == 0 ? c : -c, 0.f), lane == 0 ? fmaf(ds, rd, -hb) : __fadd_rn(hb, sq));
+  const float rd = rsqrt_n(ds), sq = __fmul_rn(ds, rd);
+  const float tn = fdiv_n(fmaxf(lane == 0 ? c : -c, 0.f), lane == 0 ? fmaf(ds, rd, -hb) : __fadd_rn(hb, sq));
   float tr = lane == 0 || hb > 0.f ? tn : __fsub_rn(sq, hb);
   bool ok = ds > 0.f && (lane == 1 || hb < 0.f);
   if (mine) {
@@ -789,9 +790,8 @@ __device__ __forceinline__ bool next_wall_warp(const DevModel& m, Ray& r, const 
   const float t = lane < 2 ? tr : (lane < 4 ? tc : (lane == 4 ? tp : kNone));
   const unsigned bits = __float_as_uint(__fadd_rn(t, 0.f));  // t >= 0: ordered as unsigned (-0 becomes +0)
   const unsigned best = __reduce_min_sync(0xffffffffu, bits);
-  const int win = __ffs(__ballot_sync(0xffffffffu, bits == best)) - 1;
+  win = __ffs(__ballot_sync(0xffffffffu, bits == best)) - 1;
   dt = __uint_as_float(best);
-  iface = win + 1 + (win == 4 ? side : 0);
   return best != __float_as_uint(kNone);
 }
 
@@ -1230,7 +1230,12 @@ static __device__ __forceinline__ int tauint_mixed(const DevModel& m, const DevT
 
 // The wall walk of tauint_mixed for a packet that a whole warp runs (k_tail),
 // every lane holding the same state, from a point whose step is longer than its
-// safe distance.  rho: the density of the packet's cell.
+// safe distance.  rho: the density of the packet's cell.  Two thirds of the
+// warps' cycles are spent here while many packets are in flight, bound by the
+// instructions of a crossing: the lanes' walls come from one table, the cell's
+// index, outer radius and this lane's density are carried along, and one
+// division serves the path and the small grains' path (plain model, 200000
+// packets peeled: 183 -> 176 ms; four models of the grid in a batch 62 -> 59).
 template <bool kFused>
 static __device__ __forceinline__ int wall_walk(const DevModel& m, const DevTallies& t, Pkt<float>& p, float tau,
                                                 Rho<float>& rho, Local& L) {
@@ -1241,14 +1246,29 @@ static __device__ __forceinline__ int wall_walk(const DevModel& m, const DevTall
   ray_init(ray, p.x, p.y, p.z, p.ux, p.uy, p.uz);
   PathLen S{0.f, 0.f};
   // what this lane tallies of a step: lane s < 4 the absorbed path of species
-  // s, lane 4 the path, lane 5 the small grains' path
+  // s, lane 4 the path, lane 5 the small grains' path (its share of the path
+  // is one factor for the whole walk)
   const float ps = (float)t.path_scale;
   const float kabs = pick4(p.kapd, lane & 3) * (1.f - pick4(p.albedo, lane & 3));
   unsigned long long* const base = lane < 4 ? t.dtauabs + (int64_t)lane * m.ncell : (lane == 4 ? t.jmean : t.jsg);
   const bool mine = lane <= 4 || (lane == 5 && m.sg_on);
+  float share = 1.f;
+  if (m.sg_on && lane == 5) share = pick4(p.kapd, m.sg_slot) * (1.f - pick4(p.albedo, m.sg_slot)) * m.sg_jfac;
   p.safe = 0.f;
   float tsum = 0.f;
   bool locate = false;  // re-derive the cell first
+  int c = 0;            // the cell, its density to this lane's species and its outer radius
+  float rl = 0.f, rout = 0.f;
+  auto enter = [&](bool row) {
+    if (row) rho = load_rho<float>(m, c);
+    rl = __ldg(reinterpret_cast<const float*>(m.rho4f + c) + (lane & 3));
+    rout = __ldg(m.rarrf + p.ir);
+  };
+  auto in_grid = [&] { return (unsigned)(p.it - 1) < (unsigned)m.nt1 && (unsigned)(p.ir - 1) < (unsigned)m.nr1; };
+  if (in_grid()) {
+    c = (int)cidx(m, p.ir, p.it, p.ip);
+    enter(false);
+  }
   for (int n = 0;; ++n) {
     if (locate) {
       locate = false;
@@ -1261,16 +1281,17 @@ static __device__ __forceinline__ int wall_walk(const DevModel& m, const DevTall
       if (where == 1) { p.ir = m.nrg; st = TI_ESCAPE; break; }
       if (where == 2) { p.ir = 0; st = TI_STAR; break; }
       p.on_wall = 0;
-      rho = load_rho<float>(m, cidx(m, p.ir, p.it, p.ip));
+      c = (int)cidx(m, p.ir, p.it, p.ip);
+      enter(true);
     }
-    if (n > cap || p.it < 1 || p.it > m.ntg - 1 || p.ir < 1 || p.ir > m.nrg - 1) {
+    if (n > cap || !in_grid()) {
       L.fault = n > cap ? F_CAP : F_RANGE;
       st = TI_FAULT;
       break;
     }
     float dt;
-    int iface;
-    if (!next_wall_warp<kFused>(m, ray, S, p.ir, p.it, p.ip, p.on_wall, dt, iface)) {
+    int win, side;
+    if (!next_wall_warp<kFused>(m, ray, S, p.ir, p.it, p.ip, p.on_wall, dt, win, side)) {
       if (nreloc < 4) {
         locate = true;
         continue;
@@ -1281,18 +1302,14 @@ static __device__ __forceinline__ int wall_walk(const DevModel& m, const DevTall
     }
     const float opac = opacity(p, rho);
     const float tnext = fmaf(opac, dt, tsum);  // the optical depth at the wall
-    const float rout = __ldg(m.rarrf + p.ir);
     L.cross++;
     const bool stop = tnext > tau;
     float ds = dt;
     if (stop) ds = (tau - tsum) / opac;
     {
-      const float r = pick4(rho.v, lane & 3);
-      float v = ds / rout;
-      if (lane < 4) v = kabs * r * ds;
-      if (m.sg_on && lane == 5)
-        v = ds * (pick4(p.kapd, m.sg_slot) * (1.f - pick4(p.albedo, m.sg_slot)) * m.sg_jfac) / rout;
-      if (mine && (lane >= 4 || r > 0.f)) atomicAdd(base + cidx(m, p.ir, p.it, p.ip), fxf(v, ps));
+      float v = (lane == 5 ? ds * share : ds) / rout;
+      if (lane < 4) v = kabs * rl * ds;
+      if (mine && (lane >= 4 || rl > 0.f)) atomicAdd(base + c, fxf(v, ps));
     }
     path_add(S, ds);
     if (stop) {
@@ -1301,12 +1318,25 @@ static __device__ __forceinline__ int wall_walk(const DevModel& m, const DevTall
       break;
     }
     tsum = tnext;
-    step_index(m.npg, iface, p.ir, p.it, p.ip);
-    p.on_wall = 1 << own_after(iface);
-    if (p.ir == m.nrg) { st = TI_ESCAPE; break; }
-    if (p.ir == 0) { st = TI_STAR; break; }
-    if (p.it >= 1 && p.it <= m.ntg - 1) rho = load_rho<float>(m, cidx(m, p.ir, p.it, p.ip));
-    if (!tiny_step(m, dt, p.ir)) {
+    // the wall crossed: lane 0 the inner sphere, 1 the outer, 2 and 3 the polar
+    // walls, 4 the azimuthal one (bits 5 and 6 of on_wall, with the wrap)
+    if (win < 4) {
+      const int d = win & 1 ? 1 : -1;
+      if (win < 2) p.ir += d;
+      else p.it += d;
+      c += win < 2 ? d : d * m.nr1;
+      p.on_wall = 2 << (win ^ 1);
+      if (p.ir == m.nrg) { st = TI_ESCAPE; break; }
+      if (p.ir == 0) { st = TI_STAR; break; }
+    } else {
+      int q = side ? p.ip + 1 : p.ip - 1;
+      q = q == 0 ? m.np1 : (q == m.npg ? 1 : q);
+      c += (q - p.ip) * m.nplane;
+      p.ip = q;
+      p.on_wall = side ? 1 << 5 : 1 << 6;
+    }
+    if ((unsigned)(p.it - 1) < (unsigned)m.nt1) enter(true);
+    if (!(dt <= 1.0e-6f * rout)) {
       ntiny = 0;
     } else if (++ntiny > 6 && nreloc < 4) {
       ntiny = 0;
