@@ -254,9 +254,4 @@ cudaError_t launch_transport_batch_fp64(const BatchItem* items, const int64_t* f
 const void* transport_batch_fn_mixed();
 const void* transport_batch_fn_fp64();
 
-int transport_regs_mixed();
-int transport_regs_fp64();
-const void* transport_fn_mixed();
-const void* transport_fn_fp64();
-
 }  // namespace hc3d

@@ -11,14 +11,6 @@ cudaError_t launch_transport_fp64(const DevModel& m, const DevTallies& t, const 
   return cudaGetLastError();
 }
 
-int transport_regs_fp64() {
-  cudaFuncAttributes attr;
-  if (cudaFuncGetAttributes(&attr, dev::k_transport<double>) != cudaSuccess) return -1;
-  return attr.numRegs;
-}
-
-const void* transport_fn_fp64() { return (const void*)dev::k_transport<double>; }
-
 cudaError_t launch_transport_batch_fp64(const BatchItem* items, const int64_t* first, int n, unsigned long long* work,
                                          int64_t total, const LaunchCfg& cfg) {
   dev::k_transport_batch<double><<<cfg.blocks, cfg.threads, 0, cfg.stream>>>(items, first, n, work, total);

@@ -11,14 +11,6 @@ cudaError_t launch_transport_mixed(const DevModel& m, const DevTallies& t, const
   return cudaGetLastError();
 }
 
-int transport_regs_mixed() {
-  cudaFuncAttributes attr;
-  if (cudaFuncGetAttributes(&attr, dev::k_transport<float>) != cudaSuccess) return -1;
-  return attr.numRegs;
-}
-
-const void* transport_fn_mixed() { return (const void*)dev::k_transport<float>; }
-
 cudaError_t launch_transport_batch_mixed(const BatchItem* items, const int64_t* first, int n, unsigned long long* work,
                                          int64_t total, const LaunchCfg& cfg) {
   dev::k_transport_batch<float><<<cfg.blocks, cfg.threads, 0, cfg.stream>>>(items, first, n, work, total);

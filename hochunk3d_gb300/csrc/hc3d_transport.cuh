@@ -1068,35 +1068,28 @@ __device__ __forceinline__ void tally_path(const DevModel& m, const DevTallies& 
 }
 
 // The same by the lanes of a warp that runs one packet (FP64 form; the mixed
-// form's is in tauint_warp): lane s < 4 tallies species s, lane 4 the path,
+// form's is in wall_walk): lane s < 4 tallies species s, lane 4 the path,
 // lane 5 the small grains' path -- one fixed-point conversion and one atomic
 // instruction instead of up to six.
-template <class R>
-__device__ __forceinline__ void tally_path_warp(const DevModel& m, const DevTallies& t, const Pkt<R>& p,
-                                                const Rho<R>& rho, int64_t c, R ds, R rout) {
+__device__ __forceinline__ void tally_path_warp(const DevModel& m, const DevTallies& t, const Pkt<double>& p,
+                                                const Rho<double>& rho, int64_t c, double ds, double rout) {
   const int lane = threadIdx.x & 31;
   unsigned long long* q = nullptr;
-  R v = R(0);
+  double v = 0.0;
   if (lane < kSlots) {
-    const R r = pick4(rho.v, lane);
-    if (r > R(0)) {
+    const double r = pick4(rho.v, lane);
+    if (r > 0.0) {
       q = t.dtauabs + (int64_t)lane * m.ncell + c;
-      v = pick4(p.kapd, lane) * (R(1) - pick4(p.albedo, lane)) * r * ds;
+      v = pick4(p.kapd, lane) * (1.0 - pick4(p.albedo, lane)) * r * ds;
     }
   } else if (lane == 4) {
     q = t.jmean + c;
     v = ds / rout;
   } else if (lane == 5 && m.sg_on) {
     q = t.jsg + c;
-    if constexpr (sizeof(R) == 4)
-      v = ds * (pick4(p.kapd, m.sg_slot) * (1.f - pick4(p.albedo, m.sg_slot)) * m.sg_jfac) / rout;
-    else
-      v = ds * (pick4(p.kapd, m.sg_slot) * (1.0 - pick4(p.albedo, m.sg_slot)) * m.sg_jfacd) / rout;
+    v = ds * (pick4(p.kapd, m.sg_slot) * (1.0 - pick4(p.albedo, m.sg_slot)) * m.sg_jfacd) / rout;
   }
-  if (q) {
-    if constexpr (sizeof(R) == 4) atomicAdd(q, fxf(v, (float)t.path_scale));
-    else atomicAdd(q, fx(v, t.path_scale));
-  }
+  if (q) atomicAdd(q, fx(v, t.path_scale));
 }
 
 // A lower bound on the distance from a point inside cell (ir, it, ip) to
@@ -1372,7 +1365,7 @@ static __device__ __forceinline__ int wall_walk64(const DevModel& m, const DevTa
     p.x += ds * p.ux;
     p.y += ds * p.uy;
     p.z += ds * p.uz;
-    tally_path_warp<double>(m, t, p, rho, c, ds, __ldg(m.rarr + p.ir));
+    tally_path_warp(m, t, p, rho, c, ds, __ldg(m.rarr + p.ir));
     if (stop) {
       p.on_wall = 0;
       return TI_INTERACT;
@@ -2303,7 +2296,7 @@ __device__ __forceinline__ PeelDir peel_dir(const RunArgs& a, int k) {
 }
 
 // One peel-off ray of the mixed form walked by one thread (the per-packet
-// loop of k_transport: trace harness and unwaved runs)
+// loops of k_transport, the trace harness, and of k_transport_batch)
 __device__ __forceinline__ void peel_ray_mixed(const DevModel& m, const DevTallies& t, const TallyDims& d,
                                                const RunArgs& a, const PeelRec<float>& e, int k, Local& L) {
   const PeelDir dd = peel_dir(a, k);
@@ -2325,7 +2318,7 @@ __device__ __forceinline__ void peel_ray_mixed(const DevModel& m, const DevTalli
 }
 
 // The peel-off rays of one event walked by the thread that made it (the
-// per-packet loop of k_transport)
+// per-packet loops)
 template <class R>
 __device__ __forceinline__ void peel_all(const DevModel& m, const DevTallies& t, const TallyDims& d,
                                          const RunArgs& a, const PeelRec<R>& rec, Local& L) {
@@ -3106,8 +3099,7 @@ __device__ __forceinline__ void flush(const DevTallies& t, Local& L) {
 }
 
 // ---- per-thread form: one packet at a time, its peel-off rays inline --------------
-// Used for the trace harness and for runs without peel-off (the Lucy
-// iterations), where a packet's history is its only work.
+// Used for the trace harness and for batches that hold a peeled model.
 template <class R, bool kFused>
 __device__ void run_packet(const DevModel& m, const DustView<R>& dv, const DevTallies& t, const TallyDims& d, const RunArgs& a, Rng& rng,
                            Local& L, Tracer& tr) {
@@ -3125,6 +3117,7 @@ __device__ void run_packet(const DevModel& m, const DustView<R>& dv, const DevTa
   }
 }
 
+// the trace harness
 template <class R>
 __global__ void __launch_bounds__(128) k_transport(DevModel m, DevTallies t, TallyDims d, RunArgs a) {
   extern __shared__ double dust_smem[];
@@ -3133,28 +3126,16 @@ __global__ void __launch_bounds__(128) k_transport(DevModel m, DevTallies t, Tal
   __shared__ unsigned long long block_counters[16];
   Local L;
   local_init(L, block_counters);
-  if (a.inj) {
-    // trace harness: one thread per traced packet, draws from the injected list
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < a.np) {
-      Rng rng;
-      rng_init(rng, a.key0, a.key1, (uint64_t)(a.packet_offset + k));
-      rng.inj = a.inj + (size_t)k * a.ninj;
-      rng.ninj = a.ninj;
-      Tracer tr{reinterpret_cast<TraceRec*>(a.trace) + (size_t)k * a.max_rec, a.max_rec, 0};
-      run_packet<R, false>(m, dv, t, d, a, rng, L, tr);
-      a.nrec[k] = tr.n;
-    }
-  } else {
-    Tracer tr{nullptr, 0, 0};
-    for (;;) {
-      const unsigned long long pid = atomicAdd(a.work, 1ull);
-      if (pid >= (unsigned long long)a.np) break;
-      Rng rng;
-      rng_init(rng, a.key0, a.key1, (uint64_t)(a.packet_offset + (int64_t)pid));
-      run_packet<R, false>(m, dv, t, d, a, rng, L, tr);
-      L.settle();
-    }
+  // one thread per traced packet, draws from the injected list
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < a.np) {
+    Rng rng;
+    rng_init(rng, a.key0, a.key1, (uint64_t)(a.packet_offset + k));
+    rng.inj = a.inj + (size_t)k * a.ninj;
+    rng.ninj = a.ninj;
+    Tracer tr{reinterpret_cast<TraceRec*>(a.trace) + (size_t)k * a.max_rec, a.max_rec, 0};
+    run_packet<R, false>(m, dv, t, d, a, rng, L, tr);
+    a.nrec[k] = tr.n;
   }
   flush(t, L);
 }
@@ -3162,7 +3143,8 @@ __global__ void __launch_bounds__(128) k_transport(DevModel m, DevTallies t, Tal
 // ---- batched form: the packets of several models in one persistent launch ------------
 // Every thread takes the next packet of the whole batch from one counter,
 // finds its model by bisection in the packet ranges, and runs it with that
-// model's tables, grid, tallies and run arguments.  Dust tables are read
+// model's tables, grid, tallies and run arguments; batches without peel-off
+// run k_wave and k_tail per model, side by side.  Dust tables are read
 // from global memory (each model has its own), and the event counters go
 // straight to the model's global counters.  A model's packets keep their
 // global ids and streams, so a batched run gives the tallies of the model
