@@ -184,13 +184,13 @@ struct LucyArgs {
   int nT;
   const double* lTint;
   const double* kappap;  // (nT, kSlots)
-  double kappav[kSlots];
-  double ltot, nphot, path_scale, tsub, na_min;
+  double factor[kSlots];        // lucy_factor of the slots' species
+  double path_rcp, tsub, na_min;  // path_rcp: 1 / path_scale, a power of two
   int nslots;
 };
 
 __device__ double dusttemp_dev(const LucyTables& q, const LucyArgs& a, double na, double T0, int s, double massarr) {
-  return lucy_dusttemp(q, a.lTint, a.nT, a.kappap + (size_t)s * a.nT, a.kappav[s], a.ltot, a.nphot, na, T0, massarr);
+  return lucy_dusttemp(q, a.lTint, a.nT, a.kappap + (size_t)s * a.nT, a.factor[s], na, T0, massarr);
 }
 
 // The peel-off walk of the mixed form reads one row per cell with the peel
@@ -223,18 +223,18 @@ __global__ void k_lucy(LucyArgs a, LucyRows rows, const unsigned long long* dtau
                        double* tdust, float* tdustf, unsigned char* peelmask, unsigned long long* maxrel,
                        const float4* rho4f, float4* rho4p) {
   __shared__ LucyTables tab;
+  __shared__ unsigned long long most;  // the block's largest relative change, as ordered bits
+  if (threadIdx.x == 0) most = 0ull;
   lucy_tables(tab, a.lTint, a.nT);
+  double mx = 0.0;
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < a.ncell; c += (int64_t)gridDim.x * blockDim.x) {
     unsigned mask = 0;
     for (int s = 0; s < kSlots; ++s) {
       double T = tdust[4 * c + s];
       if (s < a.nslots && rho4d[4 * c + s] > 0.0) {
-        const double na = (double)(long long)dtauabs[(int64_t)s * a.ncell + c] / a.path_scale;
+        const double na = (double)(long long)dtauabs[(int64_t)s * a.ncell + c] * a.path_rcp;
         const double Td = dusttemp_dev(tab, a, na, T, s, massarr[4 * c + s]);
-        if (na >= a.na_min) {
-          const double rel = fabs(Td - T) / Td;
-          atomicMax(maxrel, (unsigned long long)__double_as_longlong(rel));
-        }
+        if (na >= a.na_min) mx = lucy_change(mx, Td, T);
         T = Td;
         tdust[4 * c + s] = Td;
         tdustf[4 * c + s] = (float)Td;
@@ -245,6 +245,9 @@ __global__ void k_lucy(LucyArgs a, LucyRows rows, const unsigned long long* dtau
     peelmask[c] = (unsigned char)mask;
     rho4p[c] = masked_rho(rho4f[c], mask);
   }
+  if (mx != 0.0) atomicMax(&most, (unsigned long long)__double_as_longlong(mx));
+  __syncthreads();
+  if (threadIdx.x == 0 && most) atomicMax(maxrel, most);
 }
 
 // What follows from the temperatures of a loaded grid: the peel mask, the
@@ -1652,7 +1655,7 @@ extern "C" int hc3d_run_iteration(hc3d_ctx* c, const hc3d_run_params* p) {
   c->last_ms = ms;
   c->last_transport_ms = ms;
   c->last_peel_ms = 0.0;
-  c->last_launches = 1;
+  c->last_launches = 2;  // k_wave, k_tail
   c->epoch_np += p->np;
   return HC3D_OK;
 }
@@ -1736,7 +1739,7 @@ static int run_batch_unpeeled(hc3d_ctx* const* ctxs, const hc3d_run_params* para
     cj->epoch_np += params[j].np;
     cj->last_ms = cj->last_transport_ms = ms;
     cj->last_peel_ms = 0.0;
-    cj->last_launches = 1;
+    cj->last_launches = 2;  // k_wave, k_tail
   }
   return HC3D_OK;
 }
@@ -2009,10 +2012,8 @@ LucyArgs lucy_args(hc3d_ctx* c, double ltot, int64_t np) {
   a.nT = c->dm.nT;
   a.lTint = c->dm.lTint;
   a.kappap = c->d_kappap;
-  for (int s = 0; s < kSlots; ++s) a.kappav[s] = c->kappav[s];
-  a.ltot = ltot;
-  a.nphot = (double)np;
-  a.path_scale = c->dt.path_scale;
+  for (int s = 0; s < kSlots; ++s) a.factor[s] = lucy_factor(ltot, (double)np, c->kappav[s]);
+  a.path_rcp = 1.0 / c->dt.path_scale;
   a.tsub = c->tsub;
   a.na_min = 1.0e4;
   a.nslots = 0;  // the slots the host arrays describe (a prefix: the species ascend)
@@ -2183,7 +2184,7 @@ extern "C" int hc3d_lucy_iterations(hc3d_ctx* c, const hc3d_run_params* p, int n
   c->last_ms = ms;
   c->last_transport_ms = ms;
   c->last_peel_ms = 0.0;
-  c->last_launches = 2 * n_iter;
+  c->last_launches = 3 * n_iter;  // k_wave, k_tail, k_lucy
   std::vector<unsigned long long> bits((size_t)n_iter);
   r = d2h(c, bits.data(), d_rel, sizeof(unsigned long long) * n_iter);
   free_all(c, tmp);

@@ -9,20 +9,23 @@
 namespace hc3d {
 
 // What bounds the solve is the FP64 pipe (1/64 of the FP32 rate on this GPU):
-// some eight steps per cell, each a logarithm for the opacity's row and a fourth
-// root. log(), pow() and the divisions made 190 FP64 instructions of a step.
-// The fourth root of a cell's constant factor is formed once and that of the
-// opacity by a cubic correction of an FP32 root, the rows' reciprocal spacings
-// are kept in shared memory, and the logarithm is table-driven: about 35, and
-// 18.3 ms against 71.0 for the 20.7 million (cell, species) pairs of the
-// full-3D grid (hc3d_lucy_update_noalloc), 0.83 GB of inputs and outputs.
+// some seven steps per cell, each a logarithm for the opacity's row and a fourth
+// root. log(), pow() and the divisions made 190 FP64 instructions of a step,
+// 71.0 ms for the 20.7 million (cell, species) pairs of the full-3D grid
+// (hc3d_lucy_update_noalloc; 0.83 GB of inputs and outputs). The cell's constants
+// are one factor w, so that a step is T = (kappa_P(T) w)^(-1/4): a table-driven
+// logarithm, a row, and a cubic correction of an FP32 root; what only orders
+// positive numbers is compared as integers, off that pipe. 26 instructions a
+// step, and some 30 a cell besides, 13.7 ms (18.3 with the factor's two roots and
+// divisions, 128 intervals and the tables formed in each of 20000 blocks).
 //
 // The logarithm: P.T.P. Tang, "Table-driven implementation of the logarithm
 // function in IEEE floating-point arithmetic", ACM TOMS 16 (1990) 378. x = 2^e
-// m, m in [1, 2); with F the mid-point of m's interval of 1/128 and r = m/F - 1
-// (|r| < 1/256), log x = e ln 2 + log F + log(1 + r), the last by its series up
-// to r^7 (the next term is below 2^-67).
-constexpr int kLucyLog = 128;   // intervals of the logarithm's table
+// m, m in [1, 2); with F the mid-point of m's interval of 1/1024 and r = m/F - 1
+// (|r| < 1/2048), log x = e ln 2 + log F + log(1 + r), the last by its series up
+// to r^4 (the next term is below 2^-57, and |log x| above 1.9 over the range of
+// temperatures).
+constexpr int kLucyLog = 1024;  // intervals of the logarithm's table
 constexpr int kLucyRows = 1024; // opacity rows whose reciprocal spacing is kept in shared memory
 
 struct LucyTables {
@@ -44,62 +47,77 @@ __device__ __forceinline__ void lucy_tables(LucyTables& q, const double* lTint, 
 // log of a positive normal x
 __device__ __forceinline__ double lucy_log(const LucyTables& q, double x) {
   const unsigned hi = (unsigned)__double2hiint(x);
-  const int e = (int)(hi >> 20) - 1023, i = (int)(hi >> 13) & (kLucyLog - 1);
+  const int e = (int)(hi >> 20) - 1023, i = (int)(hi >> 10) & (kLucyLog - 1);
   const double m = __hiloint2double((int)((hi & 0xfffffu) | 0x3ff00000u), __double2loint(x));
   const double r = fma(m, q.rcp[i], -1.0);
-  double s = fma(r, 1.0 / 7.0, -1.0 / 6.0);
-  s = fma(s, r, 1.0 / 5.0);
-  s = fma(s, r, -1.0 / 4.0);
-  s = fma(s, r, 1.0 / 3.0);
+  double s = fma(r, -1.0 / 4.0, 1.0 / 3.0);
   s = fma(s, r, -1.0 / 2.0);
   s = fma(s * r, r, r);
   return fma((double)e, 0.693147180559945309417232121458, q.logf[i] + s);
 }
 
-// KapP: Planck-mean kappa/kappa_V at T (K/11605), linear in log T.
+// KapP: Planck-mean kappa/kappa_V at T (K/11605), linear in log T; row0 = -lTint(1) rl
 __device__ __forceinline__ double lucy_kapp(const LucyTables& q, const double* lTint, int nT, const double* kp,
-                                            double l1, double rl, double T) {
+                                            double row0, double rl, double T) {
   const double lT = lucy_log(q, T);
-  const int k = (int)((lT - l1) * rl) + 1;
+  const int k = (int)fma(lT, rl, row0) + 1;
   if (k < 1) return kp[0];
   if (k > nT - 1) return kp[nT - 1];
-  const double d = lT - lTint[k - 1];
+  const double d = lT - lTint[k - 1], k0 = kp[k - 1];
   const double f = k <= kLucyRows ? d * q.rdl[k - 1] : d / (lTint[k] - lTint[k - 1]);
-  return (1.0 - f) * kp[k - 1] + f * kp[k];
+  return fma(f, kp[k] - k0, k0);
 }
 
-// x^(-1/4): an FP32 root, then one step of third order. With x y^4 = 1 - h, h
-// about 1e-6 of FP32 rounding, x^(-1/4) = y (1 + h/4 + 5 h^2/32 + O(h^3)).
-__device__ __forceinline__ double lucy_root4_inv(double x) {
-  if (!(x > 1e-30 && x < 1e30)) return 1.0 / sqrt(sqrt(x));  // outside FP32
-  const double y = (double)rsqrtf(sqrtf((float)x));
-  const double y2 = y * y;
-  const double h = fma(-x, y2 * y2, 1.0);
-  return fma(y * h, fma(h, 5.0 / 32.0, 0.25), y);
+// ltot / (4 sigma N kappa_V): the factor of the absorbed path in the balance
+inline double lucy_factor(double ltot, double nphot, double kappav) {
+  return ltot / (4.0 * 5.670400e-5 * nphot * kappav);
 }
 
 // Energy balance 4 sigma T^4 kappa_V kappa_P(T) (rho V) = na L / N, iterated
-// from T0 to 1e-5 relative (at most 1000 steps), clamped to [0.1, 1600] K.
+// from T0 to 1e-5 relative (at most 1000 steps), clamped to [0.1, 1600] K;
+// factor: lucy_factor of the species.
+//
+// x^(-1/4): an FP32 root, then one step of third order. With x y^4 = 1 - h, h
+// about 1e-6 of FP32 rounding, x^(-1/4) = y (1 + h/4 + 5 h^2/32 + O(h^3)).
 __device__ __forceinline__ double lucy_dusttemp(const LucyTables& q, const double* lTint, int nT, const double* kp,
-                                                double kappav, double ltot, double nphot, double na, double T0,
-                                                double massarr) {
-  const double eps = 1.e-5, sigt = 5.670400e-5, lo = 0.1 / 11605.0, hi = 1600.0 / 11605.0;
-  const double l1 = lTint[0], rl = (double)(nT - 1) / (lTint[nT - 1] - l1);
-  const double c = (na * ltot) / (4.0 * sigt * nphot * kappav);
-  const double g = sqrt(sqrt(c)) / (11605.0 * massarr);
+                                                double factor, double na, double T0, double massarr) {
+  const double eps = 1.e-5, lo = 0.1 / 11605.0, hi = 1600.0 / 11605.0;
   double Td = T0 != 0.0 ? T0 : lo;
   if (Td < 0.0) return __longlong_as_double(0x7ff8000000000000ll);  // its logarithm
-  double Told = 0.5 * Td;
-  int it = 0;
-  while (fabs(Td - Told) > eps * Td && it < 1000) {
-    ++it;
-    Told = Td;
-    const double r = lucy_root4_inv(lucy_kapp(q, lTint, nT, kp, l1, rl, Td));
-    Td = massarr > 0.0 ? r * g : lo;  // no mass: the floor
-    if (Td > hi) Td = hi;
-    if (Td < lo) Td = lo;
+  if (!(Td < 1.0 / 0.0)) return Td;
+  const double rl = (double)(nT - 1) / (lTint[nT - 1] - lTint[0]), row0 = -lTint[0] * rl;
+  const double m = 11605.0 * massarr, m2 = m * m;
+  const double w = (m2 * m2) / (na * factor);
+  for (int it = 0; it < 1000; ++it) {
+    const double Told = Td;
+    const double x = lucy_kapp(q, lTint, nT, kp, row0, rl, Td) * w;
+    if (!(massarr > 0.0)) {
+      Td = lo;  // no mass: the floor
+    } else if ((unsigned)(__double2hiint(x) - 0x39c00000) < 0x0c600000u) {  // 2^-99 <= x < 2^99: positive, and FP32's
+      const double y = (double)rsqrtf(sqrtf((float)x));
+      const double y2 = y * y;
+      const double h = fma(-x, y2 * y2, 1.0);
+      Td = fma(y * h, fma(h, 5.0 / 32.0, 0.25), y);
+      if (__double_as_longlong(Td) > __double_as_longlong(hi)) Td = hi;
+      if (__double_as_longlong(Td) < __double_as_longlong(lo)) Td = lo;
+    } else {
+      Td = 1.0 / sqrt(sqrt(x));
+      if (!(Td == Td)) return Td;
+      if (Td > hi) Td = hi;
+      if (Td < lo) Td = lo;
+    }
+    if (__double_as_longlong(fabs(Td - Told)) <= __double_as_longlong(eps * Td)) break;
   }
   return Td;
+}
+
+// the larger of mx and the relative change |T - T0| / T (bits of NaN are larger
+// than any number's); the division only where the change may be the larger
+__device__ __forceinline__ double lucy_change(double mx, double T, double T0) {
+  const double d = fabs(T - T0);
+  if (d <= mx * T) return mx;
+  const double v = fabs(d / T);
+  return __double_as_longlong(v) > __double_as_longlong(mx) ? v : mx;
 }
 
 }  // namespace hc3d

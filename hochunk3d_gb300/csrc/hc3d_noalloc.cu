@@ -17,6 +17,7 @@
 // overlap on the GPU (different streams, or different host threads without
 // ordering) race on it.
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 
@@ -26,8 +27,8 @@
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kPerThread = 4;
-constexpr long long kMaxBlocks = HC3D_NOALLOC_MAX_ELEMENTS / (kThreads * kPerThread);
+constexpr int kPerSm = 8;           // resident blocks: the tables are formed once in each
+constexpr long long kMaxBlocks = 4096;
 
 // [0, kMaxBlocks): per-block maxima of |T_new - T_old| / T_new (as ordered
 // bits of non-negative doubles); [kMaxBlocks]: blocks finished;
@@ -38,13 +39,13 @@ struct Args {
   int nrg, ntg, npg, ndg;
   long long n;  // nrg*ntg*npg*ndg
   const long long* dtauabs;
-  double path_scale;
+  double path_scale, path_rcp;  // path_rcp: its reciprocal where that is exact, else 0
   const double *densarr, *massarr, *tdust_in;
   double* tdust_out;
   int nT;
   const double *lTint, *kappap;
-  double kappav[HC3D_NDG];
-  double ltot, nphot, na_min;
+  double factor[HC3D_NDG];
+  double na_min;
 };
 
 __global__ void __launch_bounds__(kThreads) k_lucy_noalloc(Args a, unsigned long long* scratch) {
@@ -52,31 +53,22 @@ __global__ void __launch_bounds__(kThreads) k_lucy_noalloc(Args a, unsigned long
   __shared__ bool last;
   __shared__ hc3d::LucyTables tab;
   hc3d::lucy_tables(tab, a.lTint, a.nT);
-  unsigned long long mx = 0;
-  const long long n4 = (long long)a.nrg * a.ntg * a.npg;
-  const long long base = (long long)blockIdx.x * kThreads * kPerThread;
-#pragma unroll
-  for (int j = 0; j < kPerThread; ++j) {
-    const long long k = base + (long long)j * kThreads + threadIdx.x;
-    if (k >= a.n) break;
-    const int s = (int)(k / n4);
-    const long long c4 = k - (long long)s * n4;
-    const int ir = (int)(c4 % a.nrg);
-    const int it = (int)((c4 / a.nrg) % a.ntg);
-    const int ip = (int)(c4 / ((long long)a.nrg * a.ntg));
+  double most = 0.0;
+  // at most 2^27 elements
+  const unsigned n = (unsigned)a.n, nrg = (unsigned)a.nrg, ntg = (unsigned)a.ntg, n4 = nrg * ntg * (unsigned)a.npg;
+  for (unsigned k = blockIdx.x * kThreads + threadIdx.x; k < n; k += gridDim.x * kThreads) {
+    const unsigned s = k / n4, c4 = k - s * n4, col = c4 / nrg, ip = col / ntg;
+    const int ir = (int)(c4 - col * nrg), it = (int)(col - ip * ntg);
     const double T0 = a.tdust_in[k];
     double T = T0;
-    if (ir < a.nrg - 1 && it < a.ntg - 1 && ip < a.npg - 1 && a.densarr[k] > 0.0) {
-      const double na = (double)a.dtauabs[k] / a.path_scale;
-      T = hc3d::lucy_dusttemp(tab, a.lTint, a.nT, a.kappap + (size_t)s * a.nT, a.kappav[s], a.ltot, a.nphot, na, T0,
-                              a.massarr[k]);
-      if (na >= a.na_min) {
-        const unsigned long long bits = (unsigned long long)__double_as_longlong(fabs(T - T0) / T);
-        mx = bits > mx ? bits : mx;
-      }
+    if (ir < a.nrg - 1 && it < a.ntg - 1 && (int)ip < a.npg - 1 && a.densarr[k] > 0.0) {
+      const double t = (double)a.dtauabs[k], na = a.path_rcp != 0.0 ? t * a.path_rcp : t / a.path_scale;
+      T = hc3d::lucy_dusttemp(tab, a.lTint, a.nT, a.kappap + (size_t)s * a.nT, a.factor[s], na, T0, a.massarr[k]);
+      if (na >= a.na_min) most = hc3d::lucy_change(most, T, T0);
     }
     a.tdust_out[k] = T;
   }
+  unsigned long long mx = (unsigned long long)__double_as_longlong(most);
   // block maximum, then the last block to finish reduces the block maxima
   for (int o = 16; o > 0; o >>= 1) {
     const unsigned long long v = __shfl_down_sync(0xffffffffu, mx, o);
@@ -145,11 +137,13 @@ extern "C" int hc3d_lucy_update_noalloc(const hc3d_lucy_buffers* b, double* max_
   a.path_scale = b->path_scale;
   a.densarr = b->densarr; a.massarr = b->massarr; a.tdust_in = b->tdust_in; a.tdust_out = b->tdust_out;
   a.nT = b->nT; a.lTint = b->lTint; a.kappap = b->kappap;
-  for (int s = 0; s < b->ndg; ++s) a.kappav[s] = b->kappav[s];
-  a.ltot = b->ltot;
-  a.nphot = (double)b->np;
+  for (int s = 0; s < b->ndg; ++s) a.factor[s] = hc3d::lucy_factor(b->ltot, (double)b->np, b->kappav[s]);
+  int ex = 0;
+  a.path_rcp = std::frexp(b->path_scale, &ex) == 0.5 && ex > -1000 && ex < 1000 ? 1.0 / b->path_scale : 0.0;
   a.na_min = 1.0e4;
-  const long long blocks = (n + (long long)kThreads * kPerThread - 1) / ((long long)kThreads * kPerThread);
+  int sms = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device) != cudaSuccess) return HC3D_ERR_CUDA;
+  const long long blocks = std::min({(n + kThreads - 1) / kThreads, (long long)sms * kPerSm, kMaxBlocks});
   k_lucy_noalloc<<<(unsigned)blocks, kThreads, 0, st>>>(a, scratch);
   if (cudaGetLastError() != cudaSuccess) return HC3D_ERR_CUDA;
   unsigned long long bits = 0;
