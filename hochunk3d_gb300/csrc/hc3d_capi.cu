@@ -93,8 +93,9 @@ namespace {
 
 // Busy lanes of a warp below which k_wave leaves its packets to k_tail, once
 // the batch has no packet left.  Measured on the plain model, 1e5 packets with
-// at most 6e4 interactions: 4 lanes 220 ms, 8 217, 16 215, 24 215, all 211;
-// the accretion model 103, 60, 61, 60, 59 ms: flat from 8 on.
+// at most 6e4 interactions: 4 lanes 105 ms, 8 94, 16 96, 24 94, all 94; the
+// three-dimensional grid 114, 99, 98, 97, 98; the accretion model 69, 21, 21,
+// 21, 21 ms: flat from 8 on.
 constexpr int kTailLanes = 16;
 
 int fail(hc3d_ctx* c, int code, const std::string& msg) {
