@@ -3210,8 +3210,15 @@ struct Slot {
 // instructions, 5 us.  Once the batch has no packet left, a warp with fewer
 // than a.dump busy lanes therefore stops and leaves its packets to k_tail:
 // in their pool slots (kPeel), or as the first *alive slots of the pool.
+//
+// While a batch lasts the fetch and the latency of its instructions bound it, so
+// more warps pay: 4 blocks per SM at 128 registers against 3 at 168 took 28.2
+// against 32.6 ms for 1e6 packets of at most 3 events on 200x199x33 walls, 19.1
+// against 21.5 on 200x199x2, and 1.95 against 2.07 s for 1e6 packets of the full
+// three-dimensional iteration; 5 and 6 blocks took no less. The FP64 form, 121
+// against 116 ms, keeps 3.
 template <class R, bool kPeel, bool kFused>
-__global__ void __launch_bounds__(128, 3) k_wave(DevModel m, DevTallies t, TallyDims d, RunArgs a, Slot<R>* pool,
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 3) k_wave(DevModel m, DevTallies t, TallyDims d, RunArgs a, Slot<R>* pool,
                                                PeelRec<R>* queue, unsigned long long* qcount, int E,
                                                unsigned int* alive, unsigned int* live) {
   extern __shared__ double dust_smem[];
