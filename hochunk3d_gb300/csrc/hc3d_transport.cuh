@@ -256,12 +256,16 @@ struct Pkt {
 // ones live in the block's shared memory, so they take no registers on the
 // packet's chain of events; local_init() clears them, flush() adds them to the
 // device counters once per block.  The counts of every crossing and every
-// interaction are kept in registers (cross, events) and settled into
-// the shared counters when a packet ends: a 64-bit shared add is a
-// compare-and-swap loop, which the lanes of a warp that cross a wall together
-// run one after another.  32 bits hold one packet's counts: at most
-// max_interactions walks of at most 4 (nrg + ntg + npg) crossings, or one
-// event's peel-off rays.
+// interaction are kept in registers (cross, events) and settled into the
+// shared counters when a packet ends, in the peeled form of k_wave at the end
+// of a wave, and wherever a walk leaves kSettle crossings or more: a 64-bit
+// shared add is a compare-and-swap loop, which the lanes of a warp that cross a
+// wall together run one after another.  A walk crosses at most 4 (nrg + ntg +
+// npg) + 65 walls (its cap), below 2^30 + 2^5 on a grid of fewer than 2^29
+// cells in two hemispheres, and an event without a walk counts one crossing:
+// 32 bits hold what comes between two looks, whatever the cap on interactions.
+constexpr unsigned kSettle = 1u << 30;
+static_assert(kSettle + 4ull * ((1ull << 28) + 8) + 65 + 32 < (1ull << 32), "a walk and a window's events from below kSettle");
 struct Local {
   unsigned long long* sc;  // the block's 16 counters
   int fault;
@@ -3116,6 +3120,7 @@ __device__ void run_packet(const DevModel& m, const DustView<R>& dv, const DevTa
   while (st == ST_INTERACT) {
     if (interact<R>(m, dv, t, a, p, rng, f, L, tr, rec)) peel_all<R>(m, t, d, a, rec, L);
     st = walk<R, kFused>(m, t, d, a, p, rng, f, L, tr, false);
+    if (L.cross >= kSettle) L.settle();
   }
 }
 
@@ -3296,7 +3301,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 3) k_wave(DevModel m
       if (emitted) {
         const int st = walk<R, kFused>(m, t, d, a, s.p, rng, s.f, L, tr, s.stage == 2);
         s.stage = st == ST_INTERACT ? 1 : 0;
-        if (!kPeel && s.stage == 0) L.settle();
+        if ((!kPeel && s.stage == 0) || L.cross >= kSettle) L.settle();
       }
     }
     exhausted = __any_sync(0xffffffffu, taken >= (unsigned long long)a.np);
@@ -3596,6 +3601,7 @@ __device__ __forceinline__ bool tail_window(const DevModel& m, const DustView<R>
       int st;
       if constexpr (kMixed) st = wall_walk<kFused>(m, t, p, tau, rho, L);
       else st = wall_walk64(m, t, p, tau, rho, L);
+      if (L.cross >= kSettle) L.settle();
       if (st != TI_INTERACT) {
         if (st == TI_ESCAPE) {
           if (lane == 0)
