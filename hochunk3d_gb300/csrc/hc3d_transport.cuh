@@ -716,8 +716,10 @@ __device__ __forceinline__ bool next_wall_ray(const DevModel& m, Ray& r, const P
 // on the side the ray turns towards.  Every lane forms all three kinds of root
 // from its own wall's parameters without a branch, so that their latencies
 // overlap, and keeps the one of its wall; the next wall is the minimum over
-// the lanes, the lowest lane of equal ones as in the search above.  About 300
-// cycles against 900 for the walls one after another.
+// the lanes, the lowest lane of equal ones as in the search above.  The roots are
+// formed by the functions of that search, for subnormal operands too: a packet
+// may pass from one search to the other anywhere.  About 300 cycles against 900
+// for the walls one after another.
 template <bool kFused>
 __device__ __forceinline__ bool next_wall_warp(const DevModel& m, Ray& r, const PathLen& S, int ir, int it, int ip,
                                                int own, float& dt, int& win, int& side) {
@@ -741,11 +743,11 @@ __device__ __forceinline__ bool next_wall_warp(const DevModel& m, Ray& r, const 
   const float b = 2.f * fmaf(-tan2, pz, pxy);
   const float cq = fmaf(-tan2, z2, rho2);
   const float disc = fmaf(b, b, -__fmul_rn(4.f * a, cq));
-  const float rs = rsqrt_n(disc), inv = fdiv_n(0.5f, a);
+  const float rs = rsqrtf(disc), inv = __fdividef(0.5f, a);
   const float t1 = __fmul_rn(fmaf(disc, rs, -b), inv), t2 = __fmul_rn(fmaf(-disc, rs, -b), inv);
   // the midplane; the far root on one's own cone; a ray along the cone: one root
   const bool mid = tan2 < 0.f;
-  const float ts = fdiv_n(mid ? -zr : (mine ? -b : -cq), mid ? uz : (mine ? a : b));
+  const float ts = __fdividef(mid ? -zr : (mine ? -b : -cq), mid ? uz : (mine ? a : b));
   auto ahead = [&](float t) { return t >= 0.f && fmaf(t, uz, zr) * hemi > 0.f; };
   float tc = kNone;
   if (mid) {
@@ -761,7 +763,7 @@ __device__ __forceinline__ bool next_wall_warp(const DevModel& m, Ray& r, const 
   float tp = kNone;
   if (m.np1 > 1) {
     const float d = fmaf(w.x, ux, __fmul_rn(w.y, uy));
-    const float tq = fdiv_n(-fmaf(w.x, xr, __fmul_rn(w.y, yr)), d);
+    const float tq = __fdividef(-fmaf(w.x, xr, __fmul_rn(w.y, yr)), d);
     if (!mine && d != 0.f && tq >= 0.f) tp = tq;
   }
   // spheres
@@ -781,8 +783,8 @@ __device__ __forceinline__ bool next_wall_warp(const DevModel& m, Ray& r, const 
     c = (float)cd;
     ds = (float)fma(hbd, hbd, -cd);
   }
-  const float rd = rsqrt_n(ds), sq = __fmul_rn(ds, rd);
-  const float tn = fdiv_n(fmaxf(lane == 0 ? c : -c, 0.f), lane == 0 ? fmaf(ds, rd, -hb) : __fadd_rn(hb, sq));
+  const float rd = rsqrtf(ds), sq = __fmul_rn(ds, rd);
+  const float tn = __fdividef(fmaxf(lane == 0 ? c : -c, 0.f), lane == 0 ? fmaf(ds, rd, -hb) : __fadd_rn(hb, sq));
   float tr = lane == 0 || hb > 0.f ? tn : __fsub_rn(sq, hb);
   bool ok = ds > 0.f && (lane == 1 || hb < 0.f);
   if (mine) {
