@@ -581,9 +581,12 @@ constexpr float kGrazeSphere = 1.0f / 1024.0f;
 // square root of a positive FP32 value by the reciprocal square root (the
 // wall searches take it of discriminants already tested > 0)
 __device__ __forceinline__ float fsqrt_pos(float x) { return x * rsqrtf(x); }
-// rsqrtf and __fdividef for operands and results that are never subnormal
-// (the lengths and roots of a ray that crosses a grid): the same values without
-// the scaling that subnormals would need, four instructions less each.
+// rsqrtf and __fdividef without the scaling that subnormal operands would need,
+// four instructions less each: the same values for all others, and a subnormal
+// counts as zero.  For the peel-off walk, whose lengths are the radii of the grid
+// or differences of them; where a difference can be smaller (the discriminant of
+// a cone), it is tested against kLeast.
+constexpr float kLeast = 1.17549435e-38f;  // the least normal number
 __device__ __forceinline__ float rsqrt_n(float x) {
   float r;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -2088,7 +2091,7 @@ struct PeelWalk {
     const float h = -cz * uz;
     const float q = fmaf(C, p2, -cz * cz);
     const float D = C * fmaf(-a, p2, cz * cz);
-    if (!(D > 0.f)) return;
+    if (!(D >= kLeast)) return;  // a cone touched, not crossed
     const float w_ = -(h + copysignf(D * rsqrt_n(D), h));  // |w_| >= sqrt(D) > 0
     const float ra = a != 0.f ? fdiv_n(w_, a) : kInf, rb = fdiv_n(q, w_);
     const float x1 = fminf(ra, rb), x2 = fmaxf(ra, rb);

@@ -3,7 +3,8 @@
 A packet's history may pass from one thread (``next_wall_ray``) to a warp
 (``next_wall_warp``) anywhere, so the two searches have to return the same
 wall and the same distance, bit for bit, for every operand -- subnormal ones
-included.  ``tests/wall_search.cu`` calls both on the same rays."""
+included.  ``tests/wall_search.cu`` calls both on the same rays, and the
+peel-off walk's roots of a cone."""
 from __future__ import annotations
 
 import ctypes as C
@@ -16,6 +17,7 @@ from hochunk3d_gb300 import build as B
 
 pytestmark = pytest.mark.gpu
 RAY = np.dtype([(k, "f4") for k in ("x", "y", "z", "ux", "uy", "uz")] + [(k, "i4") for k in ("ir", "it", "ip", "own")])
+CONE = np.dtype([(k, "f4") for k in ("c2", "hemi", "p2", "cz", "uz", "t")])
 FOUND = np.dtype([("ok", "i4"), ("dt", "f4"), ("iface", "i4")])
 
 
@@ -92,3 +94,34 @@ def test_a_thread_and_a_warp_find_the_same_wall(searches, scale, fused):
     assert one["ok"].mean() > 0.9
     differ = (one["ok"] != many["ok"]) | (one["dt"] != many["dt"]) | (one["iface"] != many["iface"])
     assert not differ.any(), (int(differ.sum()), q[differ][:3], one[differ][:3], many[differ][:3])
+
+
+def test_cone_that_is_grazed_within_a_subnormal_discriminant(searches):
+    """The discriminant C (cz^2 - a p^2) of rays that touch a cone next to the
+    origin is subnormal; what the walk then takes for roots are roots: each
+    satisfies |root - root in 64 bits| <= sqrt(2^-126) / |a|, the distance of
+    the two roots where the discriminant leaves the normal range."""
+    import torch
+
+    rng = np.random.default_rng(3)
+    n = 20000
+    q = np.zeros(n, CONE)
+    q["c2"], q["uz"], q["hemi"] = rng.uniform(0.3, 0.9, n), rng.uniform(-0.5, 0.5, n), rng.choice([-1.0, 1.0], n)
+    q["cz"] = rng.choice([-1.0, 1.0], n) * 10.0 ** rng.uniform(-19.4, -18.5, n)
+    a = q["c2"].astype(float) - q["uz"].astype(float) ** 2
+    q["p2"] = q["cz"].astype(float) ** 2 / a * (1.0 - 10.0 ** rng.uniform(-6, -1, n))
+    q["t"] = -1.0
+    D = q["c2"].astype(float) * (q["cz"].astype(float) ** 2 - a * q["p2"].astype(float))
+    sub = (a > 0.01) & (D > 0.0) & (D < 2.0 ** -127)
+    assert sub.sum() > 1000
+    d_q = _dev(q)
+    out = torch.zeros(2 * n, dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    assert searches.cone_search(C.c_void_p(d_q.data_ptr()), n, C.c_void_p(out.data_ptr())) == 0
+    roots = out.cpu().numpy().reshape(n, 2)[sub].astype(float)
+    h = -(q["cz"].astype(float) * q["uz"].astype(float))[sub]
+    mid = -h / a[sub]
+    got = roots < 1e30
+    off = np.abs(roots - mid[:, None])
+    bound = 2.0 ** -63 / a[sub][:, None]
+    assert (off[got] <= np.broadcast_to(bound, off.shape)[got]).all(), (off[got].max(), bound.max())

@@ -1,6 +1,6 @@
 // The mixed form's wall searches beside each other, for test_gpu_wall_search.py:
 // the search of one thread (next_wall_ray) and that of a warp (next_wall_warp)
-// on the same rays.
+// on the same rays, and the roots that the peel-off walk finds on a cone.
 #include <cstdint>
 
 #include "hc3d_transport.cuh"
@@ -16,6 +16,9 @@ struct Found {
   int ok;       // a wall was found
   float dt;
   int iface;    // 1..6
+};
+struct ConeIn {
+  float c2, hemi, p2, cz, uz, t;
 };
 
 namespace {
@@ -41,6 +44,19 @@ __global__ void k_search(DevModel m, const RayIn* in, int n, Found* lone, Found*
   }
 }
 
+__global__ void k_cone(const ConeIn* in, int n, float2* roots) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  PeelWalk w;
+  w.p2 = in[k].p2;
+  w.cz = in[k].cz;
+  w.uz = in[k].uz;
+  w.t = in[k].t;
+  float r1, r2;
+  w.cone_roots(make_float2(in[k].c2, in[k].hemi), false, r1, r2);
+  roots[k] = make_float2(r1, r2);
+}
+
 }  // namespace
 
 // walls: r2arr (nrg) FP64, then the FP32 pairs of DevModel::wallw (nr1 spheres, ntg cones, npg planes)
@@ -57,6 +73,12 @@ extern "C" int wall_search(int nrg, int ntg, int npg, const double* r2arr, const
   const int blocks = (n + 3) / 4;
   if (fused) k_search<true><<<blocks, 128>>>(m, in, n, lone, warp);
   else k_search<false><<<blocks, 128>>>(m, in, n, lone, warp);
+  if (cudaGetLastError() != cudaSuccess) return 1;
+  return cudaDeviceSynchronize() != cudaSuccess;
+}
+
+extern "C" int cone_search(const ConeIn* in, int n, float2* roots) {
+  k_cone<<<(n + 127) / 128, 128>>>(in, n, roots);
   if (cudaGetLastError() != cudaSuccess) return 1;
   return cudaDeviceSynchronize() != cudaSuccess;
 }
