@@ -565,9 +565,14 @@ int tail_blocks_for(hc3d_ctx* c, bool peel, int64_t n) {
   return (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)c->sm_count * per_sm, (n + 3) / 4));
 }
 
-// Room for the packets an unpeeled run of `threads` threads leaves to k_tail.
-int ensure_tail(hc3d_ctx* c, int64_t threads) {
-  if (c->tail.pool && c->tail_slots >= threads) return HC3D_OK;
+// Room for the packets that an unpeeled run leaves to k_tail: fewer than
+// kTailLanes of each warp, and no more than the batch has.  (8 MB for the
+// resident blocks, where a place per thread took 18; 100000 blocks asked for by
+// the caller took 2.9 GB for 3000 packets.)
+int ensure_tail(hc3d_ctx* c, const LaunchCfg& cfg, int64_t np) {
+  const int64_t slots = std::max<int64_t>(
+      1, std::min<int64_t>(np, (int64_t)cfg.blocks * (cfg.threads / 32) * (kTailLanes - 1)));
+  if (c->tail.pool && c->tail_slots >= slots) return HC3D_OK;
   free_all(c, c->tail_allocs);
   c->tail = TailBufs{};
   c->tail_slots = 0;
@@ -575,11 +580,11 @@ int ensure_tail(hc3d_ctx* c, int64_t threads) {
   unsigned char* pool;
   unsigned int* count;
   int r;
-  if ((r = dalloc(c, c->tail_allocs, &pool, slot * (size_t)threads)) || (r = dalloc(c, c->tail_allocs, &count, 2)))
+  if ((r = dalloc(c, c->tail_allocs, &pool, slot * (size_t)slots)) || (r = dalloc(c, c->tail_allocs, &count, 2)))
     return r;
   c->tail.pool = pool;
   c->tail.count = count;
-  c->tail_slots = threads;
+  c->tail_slots = slots;
   return HC3D_OK;
 }
 
@@ -1655,7 +1660,7 @@ extern "C" int hc3d_run_iteration(hc3d_ctx* c, const hc3d_run_params* p) {
     return HC3D_OK;
   }
   const LaunchCfg cfg = transport_cfg(c, p->np, c->block_size, c->grid_blocks);
-  if ((r = ensure_tail(c, (int64_t)cfg.blocks * cfg.threads))) return r;
+  if ((r = ensure_tail(c, cfg, p->np))) return r;
   CK(cudaEventRecord(c->ev0, c->stream));
   cudaError_t e = launch_packets(c, a, cfg, tail_blocks_for(c, false, p->np), false);
   if (e != cudaSuccess) return fail(c, HC3D_ERR_CUDA, std::string("transport launch: ") + cudaGetErrorString(e));
@@ -1714,7 +1719,7 @@ static int run_batch_unpeeled(hc3d_ctx* const* ctxs, const hc3d_run_params* para
     hc3d_ctx* cj = ctxs[j];
     int r = prepare_run(cj, &params[j], &args[(size_t)j]);
     const LaunchCfg cfg = transport_cfg(cj, params[j].np, 128, 0);
-    if (!r) r = ensure_tail(cj, (int64_t)cfg.blocks * cfg.threads);
+    if (!r) r = ensure_tail(cj, cfg, params[j].np);
     if (r) {
       if (cj != c) c->err = "model " + std::to_string(j) + ": " + cj->err;
       return r;
@@ -2138,7 +2143,7 @@ extern "C" int hc3d_lucy_iterations(hc3d_ctx* c, const hc3d_run_params* p, int n
   int r = dalloc(c, tmp, &d_rel, (size_t)n_iter);
   if (r) return r;
   const LaunchCfg cfg = transport_cfg(c, p->np, c->block_size, c->grid_blocks);
-  if ((r = ensure_tail(c, (int64_t)cfg.blocks * cfg.threads))) {
+  if ((r = ensure_tail(c, cfg, p->np))) {
     free_all(c, tmp);
     return r;
   }
