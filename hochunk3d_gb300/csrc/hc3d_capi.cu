@@ -1123,7 +1123,8 @@ extern "C" int hc3d_load_tables(hc3d_ctx* c, const hc3d_dust_tables* t) {
       c->dm.table_of[s] = found;
     }
     c->dm.ntab = ntab;
-    c->dm.dust_smem = smem <= 48 * 1024 ? (int)smem : 0;
+    // beside the block's event counters; larger tables are read from global memory
+    c->dm.dust_smem = smem + 16 * sizeof(unsigned long long) <= 48 * 1024 ? (int)smem : 0;
     un.resize(L * ntab); uk.resize(un.size()); ua.resize(un.size()); ug.resize(un.size()); up.resize(un.size());
     nud.swap(un); kap.swap(uk); alb.swap(ua); gg.swap(ug); pl.swap(up);
   }
