@@ -83,8 +83,8 @@ __device__ __forceinline__ double lucy_dusttemp(const LucyTables& q, const doubl
                                                 double factor, double na, double T0, double massarr) {
   const double eps = 1.e-5, lo = 0.1 / 11605.0, hi = 1600.0 / 11605.0;
   double Td = T0 != 0.0 ? T0 : lo;
-  if (Td < 0.0) return __longlong_as_double(0x7ff8000000000000ll);  // its logarithm
-  if (!(Td < 1.0 / 0.0)) return Td;
+  if (!(fabs(Td) < 1.0 / 0.0)) return Td;
+  if (Td < 0.0) Td = 2.2250738585072014e-308;  // below the table, as any start under its first row
   const double rl = (double)(nT - 1) / (lTint[nT - 1] - lTint[0]), row0 = -lTint[0] * rl;
   const double m = 11605.0 * massarr, m2 = m * m;
   const double w = (m2 * m2) / (na * factor);
