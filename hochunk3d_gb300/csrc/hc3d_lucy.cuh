@@ -87,7 +87,7 @@ __device__ __forceinline__ double lucy_dusttemp(const LucyTables& q, const doubl
   if (Td < 0.0) Td = 2.2250738585072014e-308;  // below the table, as any start under its first row
   const double rl = (double)(nT - 1) / (lTint[nT - 1] - lTint[0]), row0 = -lTint[0] * rl;
   const double m = 11605.0 * massarr, m2 = m * m;
-  const double w = (m2 * m2) / (na * factor);
+  const double w = na != 0.0 ? (m2 * m2) / (na * factor) : 1.0 / 0.0;  // without a tally the floor, however small m
   for (int it = 0; it < 1000; ++it) {
     const double Told = Td;
     const double x = lucy_kapp(q, lTint, nT, kp, row0, rl, Td) * w;

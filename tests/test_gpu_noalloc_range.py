@@ -58,3 +58,12 @@ def test_negative_starting_temperature(built):
     assert LO < want[0] < HI
     np.testing.assert_allclose(got, want, rtol=1e-12)  # the iterates agree to a few ulp
     assert np.isfinite(rel)
+
+
+def test_masses_of_any_size(built):
+    """A cell that absorbed nothing is at the floor and one that absorbed is
+    where its mass puts it, however small or large the mass."""
+    mass = np.array([1e-300, 1e-90, 1e-82, 1e-3, 1e5, 1e73, 1e90, 1e300, 5e-324])
+    for tally in (0, 1 << 40):
+        got, want, _ = _solve(np.full(len(mass), tally), mass, np.full(len(mass), 0.01))
+        np.testing.assert_allclose(got, want, rtol=1e-12, err_msg=str(tally))
