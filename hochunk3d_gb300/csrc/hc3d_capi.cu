@@ -33,7 +33,7 @@ struct hc3d_ctx {
   double* d_tdust = nullptr;   // (ncell*4), also dm.tdust
   float* d_tdustf = nullptr;   // (ncell*4) FP32 copy, also dm.tdustf
   unsigned char* d_peelmask = nullptr;
-  int2* d_lucyrow = nullptr;  // (ncell*4) weight and CDF row pair of each temperature, also dm.lucyrow
+  int2* d_lucyrow = nullptr;  // (ncell*4) weight and CDF row pair of each temperature, also dm.lucyrow (mixed form only)
   float4* d_rho4p = nullptr;  // (ncell) peel-masked FP32 densities, also dm.rho4p
   int ndg_in = 0;
   // species (1..8, reference numbering) of the four device slots (hc3d_set_species)
@@ -207,7 +207,7 @@ __device__ __forceinline__ float4 masked_rho(float4 r, unsigned mask) {
 struct LucyRows {
   const float* lT;  // (nT) FP32
   int nT;
-  int2* rows;       // NULL: no tables loaded yet
+  int2* rows;       // NULL: no tables loaded yet, or the FP64 form, which does not read them
 };
 
 __device__ __forceinline__ int2 lucy_row(const LucyRows& q, float T0, int s) {
@@ -239,7 +239,7 @@ __global__ void k_lucy(LucyArgs a, LucyRows rows, const unsigned long long* dtau
         T = Td;
         tdust[4 * c + s] = Td;
         tdustf[4 * c + s] = (float)Td;
-        rows.rows[4 * c + s] = lucy_row(rows, (float)Td, s);
+        if (rows.rows) rows.rows[4 * c + s] = lucy_row(rows, (float)Td, s);
       }
       if (T < a.tsub / 11605.0) mask |= 1u << s;
     }
@@ -1353,7 +1353,8 @@ extern "C" int hc3d_load_grid(hc3d_ctx* c, const hc3d_grid* g) {
   {
     const std::vector<float> tdf(td.begin(), td.end());
     if ((r = dupload(c, own, &c->d_tdustf, tdf.data(), tdf.size()))) return r;
-    if ((r = dalloc(c, own, &c->d_lucyrow, (size_t)4 * ncell))) return r;
+    c->d_lucyrow = nullptr;
+    if (c->precision == HC3D_PREC_MIXED && (r = dalloc(c, own, &c->d_lucyrow, (size_t)4 * ncell))) return r;
   }
   DevTallies& t = c->dt;
   if ((r = dalloc(c, own, &t.nabs, (size_t)kSlots * ncell)) || (r = dalloc(c, own, &t.dtauabs, (size_t)kSlots * ncell)) ||

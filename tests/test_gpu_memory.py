@@ -1,0 +1,38 @@
+"""Device memory that a loaded model holds, from the allocator's own count."""
+from __future__ import annotations
+
+import ctypes as C
+
+import pytest
+
+from hochunk3d_gb300 import hc3d
+from tests.helpers import make_model
+
+pytestmark = pytest.mark.gpu
+
+
+def _used():
+    """Bytes in use of the device's default pool (cudaMemPoolAttrUsedMemCurrent)."""
+    import torch
+
+    torch.cuda.synchronize()
+    rt = C.CDLL("libcudart.so.%s" % torch.version.cuda.split(".")[0])
+    pool, n = C.c_void_p(), C.c_uint64()
+    assert rt.cudaDeviceGetDefaultMemPool(C.byref(pool), 0) == 0
+    assert rt.cudaMemPoolGetAttribute(pool, 7, C.byref(n)) == 0
+    return n.value
+
+
+def test_rows_of_the_mixed_form_are_not_kept_in_fp64(tmp_path, built):
+    """The rows of the Lucy CDF (8 bytes per cell and species slot), which only
+    the mixed form reads."""
+    m = make_model(tmp_path, "plain")
+    held = {}
+    for prec in (hc3d.PREC_MIXED, hc3d.PREC_FP64):
+        ctx = hc3d.Context(prec)
+        before = _used()
+        ctx.load(m)
+        held[prec] = _used() - before
+        ctx.close()
+    rows = 4 * 8 * m.info.ncells
+    assert held[hc3d.PREC_FP64] <= held[hc3d.PREC_MIXED] - rows, held
