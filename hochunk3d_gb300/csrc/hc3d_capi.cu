@@ -1237,7 +1237,7 @@ extern "C" int hc3d_load_tables(hc3d_ctx* c, const hc3d_dust_tables* t) {
     short2* d_guide = nullptr;
     int* d_last = nullptr;
     std::vector<void*> tmp;
-    if ((r = dalloc(c, own, &d_kf, kbn * kSlots)) || (r = dalloc(c, own, &d_pair, (size_t)kSlots * (nT - 1) * nnu)) ||
+    if ((r = dalloc(c, tmp, &d_kf, kbn * kSlots)) || (r = dalloc(c, own, &d_pair, (size_t)kSlots * (nT - 1) * nnu)) ||
         (r = dalloc(c, own, &d_guide, (size_t)kSlots * (nT - 1) * kGuide)) ||
         (r = dalloc(c, tmp, &d_last, (size_t)kSlots * nT * (kGuide + 1)))) {
       free_all(c, tmp);
@@ -1250,7 +1250,6 @@ extern "C" int hc3d_load_tables(hc3d_ctx* c, const hc3d_dust_tables* t) {
     k_cdf_guide<<<grid_blocks_for(c, ng), 256, 0, c->stream>>>(nT, nnu, ng, d_last, d_guide);
     free_all(c, tmp);
     CK(cudaGetLastError());
-    c->dm.kapBintf = d_kf;
     std::vector<float2> ratio(nnu);
     for (int i = 0; i < nnu; ++i) {
       const float n0 = (float)t->nuint[i], n1 = (float)t->nuint[std::min(i + 1, nnu - 1)];

@@ -102,7 +102,7 @@ struct DevModel {
   const double* limb_xmu; const double* limb_prob;
   // FP32 copies of the per-event tables, read by the mixed form
   const float* nudustf; const float* kappadf; const float* adustf; const float* gdustf; const float* pldustf;
-  const float* lTintf; const float* nuintf; const float* kapBintf;
+  const float* lTintf; const float* nuintf;
   const float* hnuintf; const float* atmosnuf; const float* lognuf; const float* loghnuf;
   // Lucy CDF of the mixed form: kpairf[(slot*(nT-1) + j-1)*nnu + i-1] = (K(j,i), K(j+1,i)) of the
   // FP32 kapBint rows j and j+1; kguide[(slot*(nT-1) + j-1)*kGuide + b] = (lo, hi) brackets the

@@ -578,9 +578,6 @@ __device__ __forceinline__ void ray_pos(const Ray& r, const PathLen& S, Pos2& x,
 constexpr float kNearSphere = 1.0f / 4096.0f;
 constexpr float kGrazeSphere = 1.0f / 1024.0f;
 
-// square root of a positive FP32 value by the reciprocal square root (the
-// wall searches take it of discriminants already tested > 0)
-__device__ __forceinline__ float fsqrt_pos(float x) { return x * rsqrtf(x); }
 // rsqrtf and __fdividef without the scaling that subnormal operands would need,
 // four instructions less each: the same values for all others, and a subnormal
 // counts as zero.  For the peel-off walk, whose lengths are the radii of the grid
@@ -1915,7 +1912,6 @@ struct PeelEsc {
   float tsum, xf, yf, zf;
 };
 
-constexpr int kPeelThreads = 256;
 constexpr int kPeelBuf = 64;
 constexpr int kPeelChunk = 256;  // rays a warp reserves per atomic, at most
 constexpr int kPeelStage = 4;    // records a warp stages in shared memory
@@ -2402,7 +2398,7 @@ __device__ __forceinline__ R lucydustfreq(const DevModel& m, R T0, int id, G& rn
   const int nT = m.nT, nnu = m.nnu;
   const R* lTint = tab<R>(m.lTint, m.lTintf);
   const R* nuint = tab<R>(m.nuint, m.nuintf);
-  const R* K = tab<R>(m.kapBint, m.kapBintf) + (size_t)id * nT * nnu;
+  const R* K = m.kapBint + (size_t)id * nT * nnu;
   const R lT0 = xlog(T0);
   const R xi = ran<R>(rng);
   const R l1 = __ldg(lTint), lN = __ldg(lTint + nT - 1);

@@ -36,3 +36,15 @@ def test_rows_of_the_mixed_form_are_not_kept_in_fp64(tmp_path, built):
         ctx.close()
     rows = 4 * 8 * m.info.ncells
     assert held[hc3d.PREC_FP64] <= held[hc3d.PREC_MIXED] - rows, held
+
+
+def test_tables_are_kept_once(tmp_path, built):
+    """Of the Lucy CDF: the FP64 tables and, of the same size, the pairs of FP32
+    rows that the mixed form draws from; 300 bytes a cell and 8 MB hold the rest."""
+    m = make_model(tmp_path, "plain")
+    ctx = hc3d.Context(hc3d.PREC_MIXED)
+    before = _used()
+    ctx.load(m)
+    held = _used() - before
+    ctx.close()
+    assert held <= 2 * 4 * 8 * m.nT * m.nnu + 300 * m.info.ncells + (8 << 20), held
