@@ -82,7 +82,6 @@ struct hc3d_ctx {
   int64_t carry_alive = 0;
   uint32_t chunk_key0 = 0, chunk_key1 = 0;
   int qchunk = 8;                   // k_wave queue slots reserved per atomic
-  bool use_waves = true;            // peeled runs use the wavefront form
   // unpeeled runs: the packets that k_wave leaves to k_tail (grown on demand, kept with the context)
   TailBufs tail{};
   std::vector<void*> tail_allocs;
@@ -1654,7 +1653,7 @@ extern "C" int hc3d_run_iteration(hc3d_ctx* c, const hc3d_run_params* p) {
   if (r) return r;
   if (p->np == 0) return HC3D_OK;
   CK(cudaMemsetAsync(c->d_work, 0, sizeof(unsigned long long), c->stream));
-  if (p->ipeel && c->use_waves) {
+  if (p->ipeel) {
     if ((r = run_waves(c, p, a))) return r;
     if ((r = finish_run(c))) return r;
     c->epoch_np += p->np;
@@ -1679,8 +1678,8 @@ extern "C" int hc3d_run_iteration(hc3d_ctx* c, const hc3d_run_params* p) {
 
 extern "C" int hc3d_run_chunk(hc3d_ctx* c, const hc3d_run_params* p, int64_t np_iteration, int final) {
   if (!c || !p) return HC3D_ERR_INVALID;
-  if (!p->ipeel || !c->use_waves) {
-    // the per-thread form finishes every packet it starts: a chunk is a run
+  if (!p->ipeel) {
+    // an unpeeled run finishes every packet it starts: a chunk is a run
     if (np_iteration < p->np) return fail(c, HC3D_ERR_INVALID, "np_iteration < np");
     if (!c->scales_set && c->grid && c->tables) set_scales(c, np_iteration);
     return hc3d_run_iteration(c, p);
@@ -1851,7 +1850,7 @@ extern "C" int hc3d_autotune(hc3d_ctx* c, const hc3d_run_params* sample, hc3d_tu
   if (!c->tables || !c->grid) return fail(c, HC3D_ERR_STATE, "load tables and grid first");
   if (c->chunk_open) return fail(c, HC3D_ERR_STATE, "a chunked iteration has packets in flight");
   std::memset(out, 0, sizeof *out);
-  const bool waves = sample->ipeel && c->use_waves;
+  const bool waves = sample->ipeel != 0;
   const int64_t q0 = c->queue_records;
   const int b0 = c->block_size, g0 = c->regen, v0 = c->peel_variant;
   // time the sample under the context's current settings as candidate k.
