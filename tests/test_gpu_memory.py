@@ -48,3 +48,21 @@ def test_tables_are_kept_once(tmp_path, built):
     held = _used() - before
     ctx.close()
     assert held <= 2 * 4 * 8 * m.nT * m.nnu + 300 * m.info.ncells + (8 << 20), held
+
+
+@pytest.mark.parametrize("name,over", [("tiny", {}), ("tiny_sg", {}), ("plain", {}), ("plain", {"NPG": 17})])
+def test_footprint_covers_what_a_model_holds(tmp_path, built, name, over):
+    """The server's admission size is at least the loaded model and the peeled
+    iteration's SED and image tallies."""
+    m = make_model(tmp_path, name, **over)
+    ctx = hc3d.Context(hc3d.PREC_MIXED)
+    before = _used()
+    ctx.load(m)
+    held = _used() - before
+    p = m.run_params(np=100, iter=1, ipeel=1)
+    ctx.zero()
+    ctx.run(p)
+    t = ctx.tallies(p, grid=False)
+    ctx.close()
+    tallies = sum(t[k].nbytes for k in t if k.startswith(("image", "s", "t", "num")) and hasattr(t[k], "nbytes"))
+    assert int(hc3d.lib().hc3d_model_footprint(m._h)) >= held + tallies, (held, tallies)
