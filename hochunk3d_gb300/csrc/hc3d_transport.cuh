@@ -60,6 +60,20 @@ __device__ __forceinline__ float xlog(float x) { return logf(x); }
 __device__ __forceinline__ double xlog(double x) { return log(x); }
 __device__ __forceinline__ float xabs(float x) { return fabsf(x); }
 __device__ __forceinline__ double xabs(double x) { return fabs(x); }
+// A product, and a product and sum, that are rounded as they stand here: the
+// mixed form rounds the sum once, the FP64 form both (its unit is compiled
+// without contraction).  The compiler may fuse a plain product with any sum it
+// feeds, and differently in each kernel: what forms a packet's history in more
+// than one kernel is written with these.
+__device__ __forceinline__ float xmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double xmul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float xmad(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double xmad(double a, double b, double c) { return __dadd_rn(__dmul_rn(a, b), c); }
+// the FP64 sums of either form
+template <class R> __device__ __forceinline__ double dmad(double a, double b, double c) {
+  if constexpr (sizeof(R) == 4) return fma(a, b, c);
+  else return xmad(a, b, c);
+}
 template <class R> __device__ __forceinline__ R rhuge();
 template <> __device__ __forceinline__ float rhuge<float>() { return 3.402823466e38f; }
 template <> __device__ __forceinline__ double rhuge<double>() { return 1.7976931348623157e308; }
@@ -143,12 +157,13 @@ template <> __device__ __forceinline__ float ran<float>(Rng& r) {
 // the optical depth -ln u, and an isotropic direction (cos theta = 1 - 2u, sin
 // theta; cos phi and sin phi of phi = 2 pi u).
 template <class R> __device__ __forceinline__ R neg_log(Rng& r) { return -xlog(ran<R>(r)); }
+template <class R> __device__ __forceinline__ R sin_of(R mu) { return xsqrt(xmad(-mu, mu, R(1))); }
 template <class R> __device__ __forceinline__ void draw_mu(Rng& r, R& mu, R& smu) {
   mu = R(1) - R(2) * ran<R>(r);
-  smu = xsqrt(R(1) - mu * mu);
+  smu = sin_of(mu);
 }
 template <class R> __device__ __forceinline__ void draw_phi(Rng& r, R& phi, R& cphi, R& sphi) {
-  phi = (R)kR2p * ran<R>(r);
+  phi = xmul((R)kR2p, ran<R>(r));
   cphi = xcos(phi);
   sphi = xsin(phi);
 }
@@ -1442,13 +1457,13 @@ template <class R>
 __device__ __forceinline__ int select_species(const R (&kapd)[kSlots], const R (&rho)[kSlots], R xran) {
   R opac = R(0), frac = R(0);
 #pragma unroll
-  for (int s = 0; s < kSlots; ++s) opac += kapd[s] * rho[s];
+  for (int s = 0; s < kSlots; ++s) opac += xmul(kapd[s], rho[s]);
   if (opac == R(0)) return -1;
   int last = -1;
   const R inv = R(1) / opac;  // mixed form: one division
 #pragma unroll
   for (int s = 0; s < kSlots; ++s) {
-    if constexpr (sizeof(R) == 4) frac += kapd[s] * rho[s] * inv;
+    if constexpr (sizeof(R) == 4) frac = xmad(xmul(kapd[s], rho[s]), inv, frac);
     else frac += kapd[s] * rho[s] / opac;
     if (kapd[s] * rho[s] > R(0)) last = s;
     if (xran <= frac + (R)(double)1.e-10f) return s;
@@ -1495,10 +1510,13 @@ __device__ __forceinline__ int select_known(const Pkt<double>& p, const Rho<doub
 }
 
 // ---- dustmat.f90:40-65 -----------------------------------------------------------
-template <class R>
+// kNamed: rounded as xmul and xmad say (a packet's scattering); otherwise, here
+// and in mueller, as the compiler contracts it (the peel-off rays, which end
+// where they are formed)
+template <bool kNamed, class R>
 __device__ __forceinline__ void dustmat(R g, R pl, R cost, R cost2, R& p1, R& p2, R& p3) {
-  const R g2 = g * g;
-  const R temp = (g2 + R(1)) - (R(2) * g) * cost;
+  const R g2 = kNamed ? xmul(g, g) : g * g;
+  const R temp = kNamed ? xmad(-(R(2) * g), cost, g2 + R(1)) : (g2 + R(1)) - (R(2) * g) * cost;
   p1 = R(1.5) * (R(1) - g2) / (R(2) + g2) * (R(1) + cost2) / (temp * xsqrt(temp));
   p2 = -pl * p1 * (R(1) - cost2) / (R(1) + cost2);
   p3 = p1 * R(2) * cost / (R(1) + cost2);
@@ -1506,7 +1524,7 @@ __device__ __forceinline__ void dustmat(R g, R pl, R cost, R cost2, R& p1, R& p2
 
 template <class R>
 __device__ __forceinline__ R peak_of(R g) {
-  const R g2 = g * g;
+  const R g2 = xmul(g, g);
   R temp;
   if (g > R(0)) temp = (g2 + R(1)) - R(2) * g;
   else temp = (g2 + R(1)) + R(2) * g;
@@ -1516,12 +1534,26 @@ __device__ __forceinline__ R peak_of(R g) {
 
 // Mueller rotation of a Stokes vector (the a21..a44 blocks of stokes.f90 and
 // stokespeel.f90); s2x/c2x: double angle of i1 (or i3), sin2i2/cos2i2 of i2.
-template <class R>
+template <bool kNamed, class R>
 __device__ __forceinline__ void mueller(bool upper, R p1, R p2, R p3, R s2x, R c2x, R sini2, R cosi2, R& si, R& sq,
                                         R& su, R& sv) {
-  const R sin2i2 = R(2) * sini2 * cosi2, cos2i2 = R(2) * cosi2 * cosi2 - R(1);
+  const R sin2i2 = R(2) * sini2 * cosi2;
+  const R cos2i2 = kNamed ? xmad(R(2) * cosi2, cosi2, R(-1)) : R(2) * cosi2 * cosi2 - R(1);
   const R sin2 = sin2i2 * s2x, cos2 = cos2i2 * c2x;
   const R sin2cos1 = sin2i2 * c2x, cos2sin1 = cos2i2 * s2x;
+  if constexpr (kNamed) {
+    // the same elements; those of the lower half differ in sign
+    const R p = upper ? p2 : -p2;
+    const R b23 = xmad(p1, cos2sin1, xmul(p3, sin2cos1)), b32 = xmad(p1, sin2cos1, xmul(p3, cos2sin1));
+    const R a12 = p2 * c2x, a13 = p * s2x;
+    const R a21 = p2 * cos2i2, a22 = xmad(p1, cos2, -xmul(p3, sin2)), a23 = upper ? b23 : -b23;
+    const R a31 = -p * sin2i2, a32 = upper ? -b32 : b32, a33 = xmad(p3, cos2, -xmul(p1, sin2));
+    const R i = xmad(a13, su, xmad(p1, si, xmul(a12, sq)));
+    const R q = xmad(a23, su, xmad(a21, si, xmul(a22, sq)));
+    const R u = xmad(a33, su, xmad(a31, si, xmul(a32, sq)));
+    si = i; sq = q; su = u; sv = xmul(p3, sv);
+    return;
+  }
   R a11, a12, a13, a21, a22, a23, a31, a32, a33, a44;
   if (upper) {
     a11 = p1; a12 = p2 * c2x; a13 = p2 * s2x;
@@ -1554,18 +1586,18 @@ struct ScatTry {
 template <class R>
 __device__ __forceinline__ void scat_try(const Pkt<R>& p, R g, R pl, R u0, R u1, ScatTry<R>& q) {
   q.bmu = R(1) - R(2) * u0;
-  R cosb2 = q.bmu * q.bmu;
-  dustmat<R>(g, pl, q.bmu, cosb2, q.p1, q.p2, q.p3);
+  R cosb2 = xmul(q.bmu, q.bmu);
+  dustmat<true>(g, pl, q.bmu, cosb2, q.p1, q.p2, q.p3);
   if (xabs(q.bmu) > R(1)) { q.bmu = q.bmu > R(1) ? R(1) : R(-1); cosb2 = R(1); }
   q.sinbt = xsqrt(R(1) - cosb2);
-  const R ri1 = (R)kR2p * u1;
+  const R ri1 = xmul((R)kR2p, u1);
   q.upper = ri1 > (R)kPi;
   const R ang = q.upper ? (R)kR2p - ri1 : ri1;
   q.ci = xcos(ang);
   q.si = xsin(ang);
-  const R s2 = R(2) * q.si * q.ci, c2 = R(2) * q.ci * q.ci - R(1);
+  const R s2 = R(2) * q.si * q.ci, c2 = xmad(R(2) * q.ci, q.ci, R(-1));
   const R a12 = q.p2 * c2, a13 = q.upper ? q.p2 * s2 : -q.p2 * s2;
-  q.rprob = (q.p1 * p.sip + a12 * p.sqp + a13 * p.sup) / p.sip;
+  q.rprob = xmad(a13, p.sup, xmad(q.p1, p.sip, xmul(a12, p.sqp))) / p.sip;
 }
 
 // the rejection loop, its tries one after another
@@ -1634,15 +1666,15 @@ __device__ __forceinline__ void stokes(Pkt<R>& p, int id, G& rng) {
   const bool upper = q.upper;
   const R a = rprob;
   if (bmu == R(1)) return;
-  const R s2x = R(2) * si_ * ci, c2x = R(2) * ci * ci - R(1);
+  const R s2x = R(2) * si_ * ci, c2x = xmad(R(2) * ci, ci, R(-1));
   R cosi2 = R(0), sini2 = R(0);
   if (bmu == R(-1)) {
     si_ = R(1); sini2 = R(1); ci = R(0); cosi2 = R(0);
     p.cost = -costp; p.sint = sintp;
   } else {
-    p.cost = costp * bmu + sintp * sinbt * ci;
+    p.cost = xmad(costp, bmu, xmul(xmul(sintp, sinbt), ci));
     if (xabs(p.cost) < R(1)) {
-      p.sint = xabs(xsqrt(R(1) - p.cost * p.cost));
+      p.sint = sin_of(p.cost);
       sini2 = si_ * sintp / p.sint;
       const R bott = p.sint * sinbt;
       cosi2 = costp / bott - p.cost * bmu / bott;
@@ -1654,13 +1686,13 @@ __device__ __forceinline__ void stokes(Pkt<R>& p, int id, G& rng) {
       p.sint = R(0); sini2 = R(0);
     }
   }
-  R cosdph = upper ? -cosi2 * ci + sini2 * si_ * bmu : -ci * cosi2 + si_ * sini2 * bmu;
+  R cosdph = xmad(xmul(sini2, si_), bmu, -xmul(cosi2, ci));
   if (xabs(cosdph) > R(1)) cosdph = cosdph > R(1) ? R(1) : R(-1);
   p.phi = upper ? phip + xacos(cosdph) : phip - xacos(cosdph);
   if (p.phi > (R)kR2p) p.phi -= (R)kR2p;
   if (p.phi < R(0)) p.phi += (R)kR2p;
   R si = p.sip, sq = p.sqp, su = p.sup, sv = p.svp;
-  mueller<R>(upper, p1, p2, p3, s2x, c2x, sini2, cosi2, si, sq, su, sv);
+  mueller<true>(upper, p1, p2, p3, s2x, c2x, sini2, cosi2, si, sq, su, sv);
   p.sip = si / a; p.sqp = sq / a; p.sup = su / a; p.svp = sv / a;
   p.cosp = xcos(p.phi);
   p.sinp = xsin(p.phi);
@@ -1690,7 +1722,7 @@ __device__ __forceinline__ void stokespeel(R g, R pl, R& sip, R& sqp, R& sup, R&
                                            R costp, R sintp) {
   R cosb2 = bmu * bmu;
   R p1, p2, p3;
-  dustmat<R>(g, pl, bmu, cosb2, p1, p2, p3);
+  dustmat<false>(g, pl, bmu, cosb2, p1, p2, p3);
   if (xabs(bmu) > R(1)) { bmu = bmu > R(1) ? R(1) : R(-1); cosb2 = R(1); }
   const R sinbt = xsqrt(R(1) - cosb2);
   const bool upper = ri1 > (R)kPi;
@@ -1712,7 +1744,7 @@ __device__ __forceinline__ void stokespeel(R g, R pl, R& sip, R& sqp, R& sup, R&
     if (cost <= R(-1)) cosi2 = R(1);
     sini2 = R(0);
   }
-  mueller<R>(upper, p1, p2, p3, s2x, c2x, sini2, cosi2, sip, sqp, sup, svp);
+  mueller<false>(upper, p1, p2, p3, s2x, c2x, sini2, cosi2, sip, sqp, sup, svp);
 }
 
 // ---- peel-off events -------------------------------------------------------------------
@@ -2488,6 +2520,7 @@ __device__ __forceinline__ int locate3_dev(const double* xx, int n, double x) {
   return jl;
 }
 
+template <class R>
 __device__ __forceinline__ double draine_logfreq(const DevModel& m, int j, double xran, double lx) {
   const int nd = m.sg_nd;
   int i = locate3_dev(m.sg_cdf + (size_t)(j - 1) * nd, nd, xran);
@@ -2496,16 +2529,16 @@ __device__ __forceinline__ double draine_logfreq(const DevModel& m, int j, doubl
   const double* lc = m.sg_logcdf + (size_t)(j - 1) * nd;
   const double l0 = __ldg(lc + i - 1), l1 = __ldg(lc + i);
   const double f0 = __ldg(m.sg_logfreq + i - 1), f1 = __ldg(m.sg_logfreq + i);
-  return (lx - l0) / (l1 - l0) * (f1 - f0) + f0;
+  return dmad<R>((lx - l0) / (l1 - l0), f1 - f0, f0);
 }
 
 template <class R, class G>
 __device__ __forceinline__ double rep_draine(const DevModel& m, int im, double jmf, G& rng) {
   const double xran = (double)ran<R>(rng);
   const double lx = log10(xran);
-  const double lf1 = draine_logfreq(m, im, xran, lx);
+  const double lf1 = draine_logfreq<R>(m, im, xran, lx);
   double lf = lf1;
-  if (im + 1 <= m.sg_nemit) lf = lf1 + jmf * (draine_logfreq(m, im + 1, xran, lx) - lf1);
+  if (im + 1 <= m.sg_nemit) lf = dmad<R>(jmf, draine_logfreq<R>(m, im + 1, xran, lx) - lf1, lf1);
   return pow(10.0, lf);
 }
 
@@ -2520,12 +2553,12 @@ __device__ void bin_escape(const DevTallies& t, const TallyDims& d, const RunArg
   int ip = (int)((double)a.nph * phi / kR2p) + 1;
   ip = ip > a.nph ? a.nph : (ip < 1 ? 1 : ip);
   const double dmu = 2.0 / (double)a.nmu;
-  const double u = 1.0 - dmu * ((double)it - 0.5);
-  const double sini = sqrt(1.0 - u * u);
+  const double u = dmad<R>(-dmu, (double)it - 0.5, 1.0);
+  const double sini = sqrt(dmad<R>(-u, u, 1.0));
   const double cp = (double)p.cosp, sp = (double)p.sinp;
-  const double x = ypold * cp - xpold * sp;
-  const double y = zpold * sini - ypold * u * sp - xpold * u * cp;
-  const double rho2 = x * x + y * y;
+  const double x = dmad<R>(ypold, cp, -xmul(xpold, sp));
+  const double y = dmad<R>(-(xpold * u), cp, dmad<R>(zpold, sini, -xmul(xmul(ypold, u), sp)));
+  const double rho2 = dmad<R>(x, x, xmul(y, y));
   if (rho2 < __ldg(a.aperture2 + a.nap - 1) * 1.0001) {
     L.add(HC3D_CNT_FLUX);
     if (iflag == 1) {
@@ -3399,7 +3432,7 @@ __device__ __forceinline__ bool tail_window(const DevModel& m, const DustView<R>
       else q.nub = lucydustfreq<R>(m, __ldg(m.tdust + 4 * (int64_t)c + s), s, d);
     }
     q.cost = R(1) - R(2) * (sg ? u[2] : u[1]);
-    q.sint = xsqrt(R(1) - q.cost * q.cost);
+    q.sint = sin_of(q.cost);
     q.phi = (R)kR2p * (sg ? u[3] : u[2]);
     q.cosp = xcos(q.phi);
     q.sinp = xsin(q.phi);
