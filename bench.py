@@ -214,8 +214,8 @@ def model_grid_throughput(tmp: Path, device: int, n: int = 12, slots: int = 4, n
     pars = model_grid_pars(tmp / "grid", n, np_lo, np_hi, seed=4)
     out = {"models": n, "packets_per_model": f"log-uniform {np_lo:.0e}..{np_hi:.0e} per iteration",
            "iterations": "2 Lucy + 1 peeled", "grids": [list(g) for g in GRID_SHAPES]}
-    # the Lucy iterations of the grid: one batched launch per iteration for all
-    # models (hc3d_run_batch) against one launch per model
+    # the Lucy iterations of the grid: all models side by side, one call per
+    # iteration (hc3d_run_batch), against one model after another
     models = [hc3d.Model(p) for p in pars]
     ctxs = [hc3d.Context(hc3d.PREC_MIXED, device=device).load(m) for m in models]
     lucy = {}
@@ -242,7 +242,7 @@ def model_grid_throughput(tmp: Path, device: int, n: int = 12, slots: int = 4, n
         c.close()
     out["lucy_iterations"] = lucy
     # the whole grid with its Lucy iterations batched: the models built on the
-    # host, both Lucy iterations of all models as one launch each, then the
+    # host, both Lucy iterations of all models as one call each, then the
     # peeled iterations of the models on `slots` host threads, one context each
     from concurrent.futures import ThreadPoolExecutor
 
